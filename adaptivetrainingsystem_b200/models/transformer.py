@@ -478,6 +478,11 @@ class TransformerBlock(nn.Module):
         elif self.ffn_kind == "mod":
             x, _ = self.ffn(h, x, decode=True)
         else:
+            fused = None
+            if next_norm is not None and self.ffn.tp_group is None:
+                fused = ops.serving.mlp_norm(h.reshape(-1, h.shape[-1]), self.ffn.gate_up_proj, self.ffn.down_proj, x.reshape(-1, x.shape[-1]), *next_norm)
+            if fused is not None:
+                return fused[0].view(x.shape), fused[1].view(x.shape)
             x, _ = self.ffn(h, x)
         return x, h_next
 

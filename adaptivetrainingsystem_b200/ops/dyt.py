@@ -77,6 +77,8 @@ def _product_f32(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     N = w.shape[0]
     if a.dtype == torch.float32:
         return torch.nn.functional.linear(a, w).view(1, T, N)
+    if G.skinny_ok(a, w):
+        return G.skinny_partials(a, w)
     splits = G._skinny_splits(T, N, K) if G.SPLIT_K_SKINNY else 1
     part = torch.empty(splits, T, N, dtype=torch.float32, device=a.device)
     kp = K // splits
@@ -86,13 +88,13 @@ def _product_f32(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
     return part
 
 
-# bf16 products whose reduction is not split over the SMs do the element-wise step in their epilogue; ATS_BLOCK_EPILOGUE=0 runs it as a
-# launch of its own instead (for comparison)
+# bf16 products that do not leave partial products do the element-wise step in their epilogue; ATS_BLOCK_EPILOGUE=0 runs it as a launch of its
+# own instead (for comparison)
 FUSED_EPILOGUE = os.environ.get("ATS_BLOCK_EPILOGUE", "1") == "1"
 
 
 def _fused(a: torch.Tensor, w: torch.Tensor) -> bool:
-    return FUSED_EPILOGUE and a.dtype == torch.bfloat16 and (not G.SPLIT_K_SKINNY or G._skinny_splits(a.shape[0], w.shape[0], a.shape[1]) == 1)
+    return FUSED_EPILOGUE and a.dtype == torch.bfloat16 and (not G.SPLIT_K_SKINNY or G.skinny_ok(a, w) or G._skinny_splits(a.shape[0], w.shape[0], a.shape[1]) == 1)
 
 
 def _block_gemm(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, bias: Optional[torch.Tensor], x: Optional[torch.Tensor], c: Optional[DytChain]) -> None:
@@ -115,7 +117,10 @@ def linear_residual(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tenso
         return (torch.tanh(c.a2 * x) * c.w2 + c.b2).to(a.dtype)
     h = torch.empty(T, N, dtype=a.dtype, device=a.device)
     if _fused(a, w):
-        _block_gemm(a, w, h, bias, x, c)
+        if G.skinny_ok(a, w):
+            G.skinny(a, w, h, G.SK_DYT, bias=bias, x=x, chain=(c.w1, c.b1, c.a1, c.w2, c.b2, c.a2))
+        else:
+            _block_gemm(a, w, h, bias, x, c)
         return h
     part = _product_f32(a, w)
     _lib.check(_fns().ats_fold_dyt(_lib.ptr(part), part.shape[0], T * N, _lib.ptr(bias), _lib.ptr(x), _lib.ptr(c.w1), _lib.ptr(c.b1), c.a1, _lib.ptr(c.w2),
@@ -130,7 +135,10 @@ def linear_gelu(a: torch.Tensor, w: torch.Tensor, bias: Optional[torch.Tensor]) 
         return gelu_tanh(torch.nn.functional.linear(a.float(), w.float(), bias)).to(a.dtype)
     out = torch.empty(T, N, dtype=a.dtype, device=a.device)
     if _fused(a, w):
-        _block_gemm(a, w, out, bias, None, None)
+        if G.skinny_ok(a, w):
+            G.skinny(a, w, out, G.SK_GELU, bias=bias)
+        else:
+            _block_gemm(a, w, out, bias, None, None)
         return out
     part = _product_f32(a, w)
     _lib.check(_fns().ats_fold_gelu(_lib.ptr(part), part.shape[0], T * N, _lib.ptr(bias), _lib.ptr(out), int(out.dtype == torch.float32), T, N,

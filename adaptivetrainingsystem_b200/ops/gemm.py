@@ -23,6 +23,12 @@ _c_int, _c_ll, _c_f, _vp = ctypes.c_int, ctypes.c_longlong, ctypes.c_float, ctyp
 _configured = False
 
 
+class _Skinny(ctypes.Structure):   # csrc/skinny.cuh
+    _fields_ = [("T", _c_int), ("N", _c_int), ("K", _c_int), ("mode", _c_int), ("up_offset", _c_int), ("act_cols", _c_int), ("head_dim", _c_int), ("early", _c_int), ("alpha", _c_f), ("a1", _c_f), ("a2", _c_f),
+                ("ldx", _c_int), ("out", _vp), ("ldo", _c_ll), ("add", _vp), ("ldadd", _c_ll), ("bias", _vp), ("x", _vp), ("w1", _vp), ("b1", _vp), ("w2", _vp),
+                ("b2", _vp), ("pos", _vp), ("status", _vp)]
+
+
 def _fn():
     global _configured
     lib = _lib.cuda_lib()
@@ -40,6 +46,8 @@ def _fn():
             _vp, _c_int, _vp]  # status, max_ctas, stream
         lib.ats_splitk_reduce.restype = _c_int
         lib.ats_splitk_reduce.argtypes = [_vp, _c_int, _c_ll, _c_ll, _vp, _vp, _vp]
+        lib.ats_gemm_skinny.restype = _c_int
+        lib.ats_gemm_skinny.argtypes = [_vp, _c_ll, _vp, _c_ll, _c_ll, ctypes.POINTER(_Skinny), _c_int, _vp]
         lib.ats_gemm_set_pair.restype = None
         lib.ats_gemm_set_pair.argtypes = [_c_int]
         if os.environ.get("ATS_GEMM_PAIR") is not None:
@@ -81,8 +89,9 @@ def _check2d(t: torch.Tensor) -> torch.Tensor:
 
 
 # Skinny products (a decode step: M = batch rows, few 256-column output tiles) would occupy N / 256 of the 148 SMs and stream
-# the weight at a fraction of HBM bandwidth; the reduction dimension is split over groups of the grouped kernel instead, every
-# group writing an fp32 partial product that a small reduction folds.  ATS_SPLIT_K=0 switches it off.
+# the weight at a fraction of HBM bandwidth; their reduction dimension is split over the SMs instead: bf16 products by a kernel of their own
+# (``csrc/gemm_skinny.cu``), 8-bit ones over groups of the grouped kernel, every group writing an fp32 partial product that a small
+# reduction folds.  ATS_SPLIT_K=0 switches it off.
 SPLIT_K_SKINNY = os.environ.get("ATS_SPLIT_K", "1") == "1"
 
 
@@ -115,6 +124,58 @@ def _gemm_nt_split_k(a, b, out, add, alpha, splits):
     return out
 
 
+SKINNY_MAX_ROWS = 64
+SK_PART, SK_STORE, SK_F32, SK_SWIGLU, SK_SILU, SK_GELU, SK_DYT, SK_ROPE = range(8)
+
+
+def skinny_ok(a: torch.Tensor, w: torch.Tensor, n: Optional[int] = None) -> bool:
+    """Whether ``a`` [T, K] @ ``w`` [N, K]^T runs on the decode kernel (``csrc/gemm_skinny.cu``), where the product is a stream of the weight.
+    Up to 64 rows it is the faster one at every size (2560 x 2048: 7.0 us against 14.4 with one row, 9.8 / 15.2 with 64; 32000 x 2048: 24.0 /
+    33.5 and 27.3 / 29.2); up to 128 rows only for narrow outputs (2048 x 2048: 13.6 / 20.2; 6144 x 4096: 37 / 26), because one CTA fills an SM
+    then and nothing runs under its epilogue."""
+    T, N = a.shape[0], w.shape[0] if n is None else n
+    return SPLIT_K_SKINNY and a.dim() == 2 and 1 <= T <= (128 if N <= 4096 else SKINNY_MAX_ROWS) and a.shape[1] % 8 == 0 and N % 8 == 0
+
+
+def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:
+    """Reduction slices of a decode product: as many as there are CTA slots (two per SM; one beyond 64 rows, whose rings are larger), but no
+    slice below four 64-element blocks, where start-up and the sum of the slices cost more than the further SMs bring, and at most eight (a
+    cluster; four beyond 64 rows, where clusters of eight whole SMs leave the rest of a processing cluster idle)."""
+    tiles, slots, most = (N + width - 1) // width, 296 if T <= 64 else 148, 8 if T <= 64 else 4
+    s = max(1, min(most, slots // tiles, (K + 63) // 64 // 4))
+    return s if s <= 4 else 4 if s < 8 else 8
+
+
+def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Optional[int] = None, splits: Optional[int] = None, add: Optional[torch.Tensor] = None,
+           alpha: float = 1.0, up_offset: int = 0, act_cols: int = 0, bias: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None, chain=None,
+           head_dim: int = 0, pos: Optional[torch.Tensor] = None) -> None:
+    """One launch of the decode kernel; ``chain`` = (w1, b1, a1, w2, b2, a2) of the residual step ``SK_DYT``; for ``SK_ROPE``
+    w1 and w2 are the cosine and sine tables, ``pos`` the positions (int32) and ``act_cols`` the rotated columns."""
+    _fn()
+    a, w = _check2d(a), _check2d(w)
+    (T, K), N = a.shape, w.shape[0] if n is None else n
+    if splits is None:
+        splits = skinny_splits(T, N, K, 64 if mode == SK_SWIGLU else 128)
+    w1, b1, a1, w2, b2, a2 = chain if chain is not None else (None, None, 0.0, None, None, 0.0)
+
+    def at(t):
+        return None if t is None else t.data_ptr()
+    args = _Skinny(T, N, K, mode, up_offset, act_cols, head_dim, 0, alpha, a1, a2, 0 if x is None else x.stride(0), at(out), out.stride(-2), at(add), 0 if add is None else add.stride(0),
+                   at(bias), at(x), at(w1), at(b1), at(w2), at(b2), at(pos),
+                   at(_lib.status_tensor(a.device)))
+    _lib.check(_lib.cuda_lib().ats_gemm_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), w.shape[0], ctypes.byref(args), splits, _lib.stream_ptr(a.device)),
+               "ats_gemm_skinny")
+
+
+def skinny_partials(a: torch.Tensor, w: torch.Tensor) -> torch.Tensor:
+    """-> the slices [splits, T, N] in fp32, for a fold that works on whole rows."""
+    T, K = a.shape
+    splits = skinny_splits(T, w.shape[0], K)
+    part = torch.empty(splits, T, w.shape[0], dtype=torch.float32, device=a.device)
+    skinny(a, w, part, SK_PART, splits=splits)
+    return part
+
+
 def _fold_partials(part: torch.Tensor, splits: int, n_inner: int, n_outer: int, out: torch.Tensor, add: Optional[torch.Tensor] = None) -> None:
     """out[o, :] = sum over the ``splits`` fp32 partial blocks of problem ``o`` (+ add), written as bf16."""
     _fn()
@@ -143,11 +204,14 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     a, b = _check2d(a), _check2d(b)
     M, K = a.shape
     N = b.shape[0]
+    if out is None:
+        out = torch.empty(M, N, dtype=torch.float32 if out_fp32 else a.dtype, device=a.device)
+    if skinny_ok(a, b) and not accumulate and not max_ctas and (add is None or not out_fp32):
+        skinny(a, b, out, SK_F32 if out_fp32 else SK_STORE, add=add, alpha=alpha)
+        return out
     splits = _skinny_splits(M, N, K) if not out_fp32 and SPLIT_K_SKINNY else 1
     if splits > 1:
         return _gemm_nt_split_k(a, b, out, add, alpha, splits)
-    if out is None:
-        out = torch.empty(M, N, dtype=torch.float32 if out_fp32 else a.dtype, device=a.device)
     epi = EPI_F32 if out_fp32 else (EPI_ADDC if add is not None else EPI_STORE)
     _raw(a, M, K, a.stride(0), 0, b, N, K, b.stride(0), 0, out, out.stride(0), add, add.stride(0) if add is not None else 0,
          None, 0, M, N, K, alpha=alpha, beta=int(accumulate), epilogue=epi, max_ctas=max_ctas)
@@ -272,6 +336,9 @@ def gemm_nt_swiglu(a: torch.Tensor, w_gate_up: torch.Tensor, out: Optional[torch
     M, K = a.shape
     if out is None:
         out = torch.empty(M, inter, dtype=a.dtype, device=a.device)
+    if pre_act is None and not max_ctas and skinny_ok(a, w, inter):
+        skinny(a, w, out, SK_SWIGLU, n=inter, up_offset=inter)
+        return out
     _raw(a, M, K, a.stride(0), 0, w, 2 * inter, K, w.stride(0), 0, out, out.stride(0), None, 0,
          pre_act, pre_act.stride(0) if pre_act is not None else 0, M, inter, K, epilogue=EPI_SWIGLU,
          up_offset=inter, max_ctas=max_ctas)

@@ -104,6 +104,9 @@ def linear_silu(a: torch.Tensor, w: torch.Tensor, act_cols: int) -> torch.Tensor
     out = torch.empty(T, N, dtype=a.dtype, device=a.device)
     if _dyt._fused(a, w):
         a = G._check2d(a)
+        if G.skinny_ok(a, w):
+            G.skinny(a, w, out, G.SK_SILU, act_cols=act_cols)
+            return out
         _lib.check(_dyt._fns().ats_gemm_bf16_block(_lib.ptr(a), a.stride(0), _lib.ptr(w), w.stride(0), _lib.ptr(out), out.stride(0), T, N, a.shape[1], None, None, 0,
                                                    None, None, 0.0, None, None, 0.0, act_cols, _lib.ptr(_lib.status_tensor(a.device)), 0,
                                                    _lib.stream_ptr(a.device)), "ats_gemm_bf16_block")

@@ -49,9 +49,10 @@ def _buf(key, numel: int, dtype, device) -> torch.Tensor:
 
 
 # ----------------------------------------------------------------------------------------------------------
-# Fused pieces of a decode step.  With a handful of tokens a projection splits its reduction over the SMs and leaves fp32 partial
-# products; the launch that folds them also does what would otherwise be the next launch: the rotary embedding of the packed
-# q / k / v projection, or the residual add and the RMSNorm that follows the output projection.
+# Fused pieces of a decode step.  With a handful of tokens a projection splits its reduction over the SMs.  Where the decode kernel takes
+# it (csrc/gemm_skinny.cu) the slices are summed inside the launch, which also rotates q and k or adds the residual; beyond its sizes the
+# launch that folds the partial products does what would otherwise be the next launch: the rotary embedding of the packed q / k / v
+# projection, or the residual add and the RMSNorm that follows the output projection.
 # ----------------------------------------------------------------------------------------------------------
 FUSE_DECODE = __import__("os").environ.get("ATS_DECODE_FUSED", "1") == "1"
 # Flash-decoding merge inside the attention kernel (the CTA that arrives last for a sequence and KV head merges the chunk
@@ -61,19 +62,24 @@ FUSE_DECODE = __import__("os").environ.get("ATS_DECODE_FUSED", "1") == "1"
 MERGE_INSIDE = __import__("os").environ.get("ATS_DECODE_MERGE_INSIDE", "0") == "1"
 
 
+DECODE_KERNEL = "decode kernel"
+
+
 def _partial_products(x2: torch.Tensor, w: torch.Tensor):
-    """fp32 partial products [splits, T, N] of x2 [T, K] @ w [N, K]^T over slices of the reduction, or ``None`` when this shape
-    does not split (the caller then uses the ordinary product)."""
+    """fp32 partial products [splits, T, N] of x2 [T, K] @ w [N, K]^T over slices of the reduction, ``None`` when this shape
+    does not split (the caller then uses the ordinary product), or ``DECODE_KERNEL`` for the shapes whose kernel sums its slices itself."""
     from . import gemm as G
     T, K = x2.shape
     N = w.shape[0]
     if not (FUSE_DECODE and _lib.use_cuda_kernels(x2) and x2.dtype == torch.bfloat16 and w.dtype == torch.bfloat16 and w.dim() == 2
             and x2.is_contiguous() and w.is_contiguous() and not getattr(w, "_ats_z3", None) and G.SPLIT_K_SKINNY):
         return None
-    from . import int4
+    from . import fp8, int4, int8
     if int4.enabled() and int4.lookup(w) is not None:
         return None          # a 4-bit weight: the caller's ordinary product streams the packed copy
     splits = G._skinny_splits(T, N, K)
+    if G.skinny_ok(x2, w) and (splits > 1 or not (fp8.enabled() or int8.enabled())):
+        return DECODE_KERNEL   # (with 8-bit copies around, the products that the 8-bit kernels do not split stay with them)
     if splits < 2:
         return None
     kp = K // splits
@@ -94,6 +100,12 @@ def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torc
         return None
     T, N = h2.shape[0], w_qkv.shape[0]
     out = torch.empty(T, N, dtype=h2.dtype, device=h2.device)
+    if part is DECODE_KERNEL:
+        from . import gemm as G
+        if 128 % d == 0:   # whole heads in a tile of the product: it rotates them itself
+            G.skinny(h2, w_qkv, out, G.SK_ROPE, act_cols=(n_q + n_kv) * d, chain=(cos, None, 0.0, sin, None, 0.0), head_dim=d, pos=positions)
+            return out
+        part = G.skinny_partials(h2, w_qkv)
     err = _fns().ats_fold_rope(_lib.ptr(part), part.shape[0], _lib.ptr(out), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions), T, N, n_q, n_kv, d,
                                _lib.stream_ptr(h2.device))
     _lib.check(err, "ats_fold_rope")
@@ -101,12 +113,18 @@ def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torc
 
 
 def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float):
-    """x = a2 @ w_o^T + residual2 and h = RMSNorm(x) * norm_w from one product + one fold launch -> (x, h), or ``None``."""
+    """x = a2 @ w_o^T + residual2 and h = RMSNorm(x) * norm_w from one product + one fold or norm launch -> (x, h), or
+    ``None``."""
     if norm_w.dtype != torch.bfloat16 or residual2 is None or not residual2.is_contiguous():
         return None
     part = _partial_products(a2, w_o)
     if part is None:
         return None
+    if part is DECODE_KERNEL:
+        from . import gemm as G
+        from .functional import rms_norm
+        x = G.gemm_nt(a2, w_o, add=residual2)
+        return x, rms_norm(x, norm_w, eps)
     T, H = a2.shape[0], w_o.shape[0]
     x = torch.empty(T, H, dtype=a2.dtype, device=a2.device)
     h = torch.empty_like(x)
@@ -114,6 +132,16 @@ def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, 
                                    _lib.stream_ptr(a2.device))
     _lib.check(err, "ats_fold_add_norm")
     return x, h
+
+
+def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float):
+    """SwiGLU feed-forward of a decode step whose down projection adds the residual, and the norm in front of the next block -> (x, h), or
+    ``None`` (8-bit or 4-bit copies of the weights, gathered weights, more than a decode step's rows)."""
+    from . import fp8, gemm as G, int4, int8
+    if (fp8.enabled() or int8.enabled() or (int4.enabled() and int4.lookup(w_gate_up) is not None) or getattr(w_gate_up, "_ats_z3", None)
+            or not _lib.use_cuda_kernels(h2) or w_gate_up.dtype != torch.bfloat16 or not G.skinny_ok(h2, w_down) or not FUSE_DECODE or norm_w.dtype != torch.bfloat16 or not residual2.is_contiguous()):
+        return None
+    return out_proj_norm(G.gemm_nt_swiglu(h2, w_gate_up), w_down, residual2, norm_w, eps)
 
 
 def decode_attention_available(qkv: torch.Tensor, n_q: int, n_kv: int, d: int) -> bool:

@@ -1,0 +1,33 @@
+// Arguments of the decode-sized product (gemm_skinny.cu); mirrored by ops/gemm.py.
+#pragma once
+#include <cuda_bf16.h>
+
+namespace ats {
+
+enum SkinnyMode : int {
+  kSkPart = 0,     // out [splits, T, N] fp32: the slices of the reduction
+  kSkStore = 1,    // out bf16 (+ add)
+  kSkF32 = 2,      // out fp32
+  kSkSwiglu = 3,   // out bf16 = silu(gate) * up
+  kSkSilu = 4,     // out bf16, silu on the first act_cols columns
+  kSkGelu = 5,     // out bf16 = gelu_tanh(v + bias)
+  kSkDyt = 6,      // x += tanh(a1 (v + bias)) w1 + b1, out bf16 = tanh(a2 x) w2 + b2
+  kSkRope = 7,     // out bf16, heads of head_dim columns; those below act_cols are rotated (half-split) by the tables w1 (cosine), w2 (sine) at pos[t]
+};
+
+struct SkinnyArgs {
+  int T, N, K, mode, up_offset, act_cols, head_dim, early;
+  float alpha, a1, a2;
+  int ldx;
+  void* out;
+  long long ldo;
+  const __nv_bfloat16* add;
+  long long ldadd;
+  const float* bias;
+  float* x;
+  const float *w1, *b1, *w2, *b2;
+  const int* pos;
+  int* status;
+};
+
+}  // namespace ats
