@@ -22,6 +22,7 @@ import torch
 
 from ..models.cache import SequenceCache
 from ..models.transformer import DeepSeekTransformer
+from ..ops.gemm import chained_launches
 
 GENERATION_MODES: Dict[str, Dict[str, float]] = {
     "standard": dict(temperature=0.8, top_p=0.9, top_k=50, repetition_penalty=1.1),
@@ -311,7 +312,10 @@ class GraphDecoder:
         cache.device_active.fill_(1)
 
     def _run(self) -> torch.Tensor:
-        logits = self.model(self.tokens, cache=self.cache, last_token_only=True, return_aux_loss=False)[:, -1, :]
+        # weights do not change inside a step, so its launches may overlap (several ranks: their barriers keep launches in order)
+        alone = not (torch.distributed.is_available() and torch.distributed.is_initialized() and torch.distributed.get_world_size() > 1)
+        with chained_launches(alone and self.cache.device.type == "cuda"):
+            logits = self.model(self.tokens, cache=self.cache, last_token_only=True, return_aux_loss=False)[:, -1, :]
         self.cache.device_advance()
         return logits
 

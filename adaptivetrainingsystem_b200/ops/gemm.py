@@ -9,6 +9,7 @@ group ``e`` actually used; pad rows up to the next multiple of 128 must be zero)
 """
 from __future__ import annotations
 
+import contextlib
 import ctypes
 import os
 from typing import Optional
@@ -24,7 +25,7 @@ _configured = False
 
 
 class _Skinny(ctypes.Structure):   # csrc/skinny.cuh
-    _fields_ = [("T", _c_int), ("N", _c_int), ("K", _c_int), ("mode", _c_int), ("up_offset", _c_int), ("act_cols", _c_int), ("head_dim", _c_int), ("early", _c_int), ("alpha", _c_f), ("a1", _c_f), ("a2", _c_f),
+    _fields_ = [("T", _c_int), ("N", _c_int), ("K", _c_int), ("mode", _c_int), ("up_offset", _c_int), ("act_cols", _c_int), ("head_dim", _c_int), ("alpha", _c_f), ("a1", _c_f), ("a2", _c_f),
                 ("ldx", _c_int), ("out", _vp), ("ldo", _c_ll), ("add", _vp), ("ldadd", _c_ll), ("bias", _vp), ("x", _vp), ("w1", _vp), ("b1", _vp), ("w2", _vp),
                 ("b2", _vp), ("pos", _vp), ("status", _vp)]
 
@@ -48,6 +49,8 @@ def _fn():
         lib.ats_splitk_reduce.argtypes = [_vp, _c_int, _c_ll, _c_ll, _vp, _vp, _vp]
         lib.ats_gemm_skinny.restype = _c_int
         lib.ats_gemm_skinny.argtypes = [_vp, _c_ll, _vp, _c_ll, _c_ll, ctypes.POINTER(_Skinny), _c_int, _vp]
+        lib.ats_chain_launches.restype = None
+        lib.ats_chain_launches.argtypes = [_c_int]
         lib.ats_gemm_set_pair.restype = None
         lib.ats_gemm_set_pair.argtypes = [_c_int]
         if os.environ.get("ATS_GEMM_PAIR") is not None:
@@ -124,6 +127,22 @@ def _gemm_nt_split_k(a, b, out, add, alpha, splits):
     return out
 
 
+@contextlib.contextmanager
+def chained_launches(on: bool = True):
+    """Kernels launched inside (by this thread) may start while the kernel before them still runs, and the decode products fetch their first
+    weights then.  For a decode step: no kernel launched inside may write a weight that a product inside reads."""
+    if not on or not torch.cuda.is_available():
+        yield
+        return
+    _fn()
+    lib = _lib.cuda_lib()
+    lib.ats_chain_launches(1)   # counted per thread
+    try:
+        yield
+    finally:
+        lib.ats_chain_launches(0)
+
+
 SKINNY_MAX_ROWS = 64
 SK_PART, SK_STORE, SK_F32, SK_SWIGLU, SK_SILU, SK_GELU, SK_DYT, SK_ROPE = range(8)
 
@@ -160,7 +179,7 @@ def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Op
 
     def at(t):
         return None if t is None else t.data_ptr()
-    args = _Skinny(T, N, K, mode, up_offset, act_cols, head_dim, 0, alpha, a1, a2, 0 if x is None else x.stride(0), at(out), out.stride(-2), at(add), 0 if add is None else add.stride(0),
+    args = _Skinny(T, N, K, mode, up_offset, act_cols, head_dim, alpha, a1, a2, 0 if x is None else x.stride(0), at(out), out.stride(-2), at(add), 0 if add is None else add.stride(0),
                    at(bias), at(x), at(w1), at(b1), at(w2), at(b2), at(pos),
                    at(_lib.status_tensor(a.device)))
     _lib.check(_lib.cuda_lib().ats_gemm_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), w.shape[0], ctypes.byref(args), splits, _lib.stream_ptr(a.device)),

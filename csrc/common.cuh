@@ -441,22 +441,17 @@ int make_tmap_heads(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
 // layer).  A kernel that begins with pdl_prologue() may be launched with launch_pdl(): its CTAs are then scheduled as soon as
 // every CTA of the kernel before it has started, and wait inside the prologue until that kernel has completed and its writes are
 // visible, so the launch latency disappears behind the predecessor.  Nothing before the prologue may touch global memory.
-// Launched the ordinary way, the two instructions do nothing.  Off unless ATS_PDL=1: inside a replayed CUDA graph the gap between
-// dependent kernels is already about a microsecond, and the attribute measured 1.7 % on the decode step of the 22-layer MoE model
-// and nothing on the Mixtral shape (the fixed cost of a decode layer is the duration of its small kernels, not their launches).
+// Launched the ordinary way, the two instructions do nothing.  On for the launches that a thread makes between ats_chain_launches(1) and
+// ats_chain_launches(0) (a decode step being captured: 458 -> 360 us for one sequence through eight 2048-wide layers, 752 -> 717 us for 64, because the
+// products then fetch their first weights under the kernel before them) and everywhere with ATS_PDL=1.
 // ----------------------------------------------------------------------------------------------
 __device__ __forceinline__ void pdl_prologue() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
 }
-inline bool pdl_enabled() {
-  static int on = -1;
-  if (on < 0) {
-    const char* e = getenv("ATS_PDL");
-    on = (e && e[0] == '1') ? 1 : 0;
-  }
-  return on == 1;
-}
+// (gemm_tcgen05.cu, the file that every library has)
+bool pdl_enabled();
+bool chained_launches();   // the calling thread vouches that no kernel in flight writes a weight that its next launches read
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

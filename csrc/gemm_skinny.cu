@@ -15,8 +15,7 @@
 // 64 rows 15.2 -> 9.8; 11264 x 2048 21.0 -> 11.9 / 21.4 -> 16.0; 2048 x 5632 17.1 -> 9.0 / 17.2 -> 12.2; 28672 x 4096 55 -> 40 / 47.6 -> 45.7.
 // What is left is start-up (a launch of 1024 x 1024 takes 4.8 us) and, with 64 rows, the exchange of the slices (2 to 3 us).
 //
-// With `early` the first ring of weight tiles is requested before the kernel waits for its predecessor (programmatic dependent launch); the
-// caller vouches that no kernel in flight writes the weight.
+// In a chain of launches (common.cuh) the first ring of weight tiles is requested before the kernel waits for its predecessor.
 #include "skinny.cuh"
 #include "typed.cuh"
 
@@ -121,7 +120,7 @@ __device__ __forceinline__ void by_mode(int mode, F&& f) {
 // NT: token columns of the accumulator (tokens rounded up to 16, 32, 64 or 128).  grid (splits, tiles), cluster (splits, 1, 1) unless kSkPart.
 template <int NT>
 __global__ void __launch_bounds__(SK_THREADS)
-skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkinnyArgs p) {
+skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_a, const SkinnyArgs p, const int early) {
   constexpr int STAGES = sk_stages(NT), STAGE = sk_stage_bytes(NT);
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -177,9 +176,9 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
       };
       auto tokens = [&](int kb, int stage) { tma_load_2d(smem + stage * STAGE + SK_ROWS * 128, &map_a, &full[stage], kb * SK_BK, 0); };
       const int first = min(STAGES, kb1 - kb0);
-      if (!p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < first; ++i) weights(kb0 + i, i);
-      if (p.early) asm volatile("griddepcontrol.wait;" ::: "memory");
+      if (early) asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < first; ++i) tokens(kb0 + i, i);
       int stage = 0, phase = 0;
       for (int kb = kb0 + first; kb < kb1; ++kb) {
@@ -372,7 +371,7 @@ int sk_launch(const CUtensorMap& mw, const CUtensorMap& ma, const SkinnyArgs& p,
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  cudaError_t ce = cudaLaunchKernelEx(&cfg, skinny_kernel<NT>, mw, ma, p);
+  cudaError_t ce = cudaLaunchKernelEx(&cfg, skinny_kernel<NT>, mw, ma, p, int(chained_launches()));
   return int(ce != cudaSuccess ? ce : cudaGetLastError());
 }
 

@@ -1104,6 +1104,18 @@ static int num_sms() {
 
 using namespace ats;
 
+// Programmatic dependent launches (common.cuh) of the calling thread.
+static thread_local int t_chained = 0;
+bool ats::pdl_enabled() {
+  static const bool everywhere = [] {
+    const char* e = getenv("ATS_PDL");
+    return e && e[0] == '1';
+  }();
+  return everywhere || t_chained > 0;
+}
+bool ats::chained_launches() { return t_chained > 0; }
+ATS_API void ats_chain_launches(int on) { t_chained = on ? t_chained + 1 : t_chained > 0 ? t_chained - 1 : 0; }
+
 // Wait budget of every peer wait in this library (nanoseconds of %globaltimer).  A host-side value handed to the kernels as
 // an argument, so a test can make a wait give up after a few milliseconds and production runs can allow slow peers more
 // than the one-second default.  (Here, in the file that every library has, because the gathering products need it.)

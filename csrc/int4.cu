@@ -104,8 +104,9 @@ template <int R, bool SWIGLU, int NT, int DEPTH, int MINB>
 __global__ void __launch_bounds__(GEMV_WARPS * 32, MINB)
 gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta, const __nv_bfloat16* __restrict__ x, long long ldx,
                  const __nv_bfloat16* __restrict__ add, long long ld_add, __nv_bfloat16* __restrict__ out, long long ld_out,
-                 int M, int N, int K, int group_shift) {
-  pdl_prologue();
+                 int M, int N, int K, int group_shift, int early) {
+  if (!early) pdl_prologue();   // early: a chained launch, whose first packed words are requested under the kernel before it (common.cuh)
+  else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float s_red[GEMV_WARPS][R][8 * NT][16];  // [warp][tile][token][feature of the tile]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int n_super = K >> 6, n_tiles = N >> 4;
@@ -135,7 +136,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
   auto w_slot = [&](int d, int r) { return my_ring + d * STAGE + r * 512 + lane * 16; };
   auto m_slot = [&](int d, int r) { return my_ring + d * STAGE + R * 512 + r * 256 + lane * 8; };
   auto x_slot = [&](int d, int i) { return my_ring + d * STAGE + R * 768 + i * 512 + lane * 16; };
-  auto issue = [&](int d, int S) {
+  auto issue_w = [&](int d, int S) {
     const long long grp = S >> (group_shift - 6);
 #pragma unroll
     for (int r = 0; r < R; ++r) {
@@ -144,6 +145,8 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
       cp_async4(m_slot(d, r), mrow);
       cp_async4(m_slot(d, r) + 4, mrow + 8);
     }
+  };
+  auto issue_x = [&](int d, int S) {
 #pragma unroll
     for (int n = 0; n < NT; ++n) {  // lanes without a token get zeros
       cp_async16_or_zero(x_slot(d, 2 * n), xrow[n] + S * 8, tok[n]);
@@ -194,10 +197,20 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
     }
   };
 
-  // group i of this lane's copies holds super-step warp + 8 i; one group is committed per step, empty past the end
+  // group i of this lane's copies holds super-step warp + 8 i; one group is committed per step, empty past the end (an early launch has the
+  // weights of the whole ring in its first group)
+  if (early) {
+#pragma unroll
+    for (int d = 0; d < DEPTH; ++d)
+      if (warp + d * GEMV_WARPS < n_super) issue_w(d, warp + d * GEMV_WARPS);
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
 #pragma unroll
   for (int d = 0; d < DEPTH; ++d) {
-    if (warp + d * GEMV_WARPS < n_super) issue(d, warp + d * GEMV_WARPS);
+    if (warp + d * GEMV_WARPS < n_super) {
+      if (!early) issue_w(d, warp + d * GEMV_WARPS);
+      issue_x(d, warp + d * GEMV_WARPS);
+    }
     cp_async_commit();
   }
   for (int S0 = warp; S0 < n_super; S0 += GEMV_WARPS * DEPTH) {
@@ -208,7 +221,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
         cp_async_wait<DEPTH - 1>();  // all but the DEPTH - 1 youngest groups have landed: this step's is among them
         compute(d);
         const int Sn = S + GEMV_WARPS * DEPTH;
-        if (Sn < n_super) issue(d, Sn);  // the slots just read are refilled (their values are in registers by now)
+        if (Sn < n_super) issue_w(d, Sn), issue_x(d, Sn);  // the slots just read are refilled (their values are in registers by now)
         cp_async_commit();
       }
     }
@@ -297,6 +310,7 @@ static int int4_group_shift(int group) {
 // out[M, N or N / 2] = x[M, K] @ W^T (+ add), M <= 16.  swiglu: W = [gate; up], out = silu(gate) * up (N % 32 == 0).
 ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long long ldx, const void* add, long long ld_add, void* out,
                           long long ld_out, int M, int N, int K, int group, int swiglu, void* stream) {
+  const int early = ats::chained_launches();
   if (!int4_shape_ok(N, K, group) || M < 1 || M > 16 || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15)) return 1003;
   if (swiglu && (N % 32)) return 1003;
   auto s = static_cast<cudaStream_t>(stream);
@@ -320,7 +334,7 @@ ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long 
       attr_set = true;                                                                                                               \
     }                                                                                                                                \
     return ats::launch_pdl(ats::gemv_int4_kernel<R_, SW_, NT_, D_, B_>, dim3(GRID_), block, kRing, s, w4, mt, xp, ldx, ap, ld_add,  \
-                           op, ld_out, M, N, K, gs);                                                                                 \
+                           op, ld_out, M, N, K, gs, early);                                                                               \
   }()
   const bool two = M > 8;
   if (swiglu)

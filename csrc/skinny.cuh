@@ -16,7 +16,7 @@ enum SkinnyMode : int {
 };
 
 struct SkinnyArgs {
-  int T, N, K, mode, up_offset, act_cols, head_dim, early;
+  int T, N, K, mode, up_offset, act_cols, head_dim;
   float alpha, a1, a2;
   int ldx;
   void* out;
