@@ -130,7 +130,8 @@ def _gemm_nt_split_k(a, b, out, add, alpha, splits):
 @contextlib.contextmanager
 def chained_launches(on: bool = True):
     """Kernels launched inside (by this thread) may start while the kernel before them still runs, and the decode products fetch their first
-    weights then.  For a decode step: no kernel launched inside may write a weight that a product inside reads."""
+    weights, the decode attention its first cached keys, then.  For a decode step: no kernel launched inside may write a weight that a product
+    inside reads, a length, or a cached row below its sequence's length (the row at the length is the step's own)."""
     if not on or not torch.cuda.is_available():
         yield
         return

@@ -1,5 +1,5 @@
 """Grouped-query attention over a full key / value cache with normed queries and keys, partial interleaved rotation, capped scores and
-one output gate per head (``csrc/gqa_attention.cu``, ``csrc/gqa_attention_tcgen05.cu``, ``decode_attn_mma_kernel`` of ``csrc/inference.cu``).
+one output gate per head (``csrc/gqa_attention.cu``, ``csrc/gqa_attention_tcgen05.cu``, ``decode_attn_kernel`` of ``csrc/inference.cu``).
 
 ``GqaShape`` carries every size and constant.  :func:`gqa_prepare` norms and rotates queries and keys and appends keys and values to the
 cache (queries only for a layer that reads another layer's cache); :func:`gqa_portion` attends for portions of a prompt, :func:`gqa_decode`
@@ -171,8 +171,7 @@ def gqa_portion(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, gate: Optiona
 
 def decode_tc_ok(q: torch.Tensor, s: GqaShape, k: torch.Tensor, v: torch.Tensor) -> bool:
     """The warp-MMA decode kernel covers these sizes."""
-    from . import serving
-    return (q.shape[0] * s.kv_heads <= serving.MAX_COUNTERS and q.dtype == torch.bfloat16 and TENSOR_CORES and s.dim == s.vdim and s.dim in (64, 128) and s.heads // s.kv_heads in (1, 2, 4, 8)
+    return (q.dtype == torch.bfloat16 and TENSOR_CORES and s.dim == s.vdim and s.dim in (64, 128) and s.heads // s.kv_heads in (1, 2, 4, 8)
             and k.stride(0) == v.stride(0))
 
 

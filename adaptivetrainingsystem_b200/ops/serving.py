@@ -23,12 +23,12 @@ def _fns():
     global _sig
     lib = _lib.cuda_lib()
     if not _sig:
-        lib.ats_decode_attn_chunks.restype = _ci
-        lib.ats_decode_attn_chunks.argtypes = [_ci]
+        lib.ats_decode_attn_parts.restype = _ci
+        lib.ats_decode_attn_parts.argtypes = [_ci] * 4
         lib.ats_decode_attn.restype = _ci
         lib.ats_decode_attn.argtypes = [_vp, _cll, _ci, _ci, _ci, _vp, _vp, _cll, _vp, _ci, _ci, _ci, _ci, _ci, _ci, _ci, _vp, _vp, _vp, _vp, _vp]
         lib.ats_decode_attn_cached.restype = _ci
-        lib.ats_decode_attn_cached.argtypes = [_vp, _cll, _vp, _vp, _cll, _vp, _ci, _ci, _ci, _ci, _ci, _cf, _cf, _vp, _cll, _vp, _vp, _vp, _vp, _cll, _vp]
+        lib.ats_decode_attn_cached.argtypes = [_vp, _cll, _vp, _vp, _cll, _vp, _ci, _ci, _ci, _ci, _ci, _cf, _cf, _vp, _cll, _vp, _vp, _vp, _cll, _vp, _vp]
         lib.ats_fold_rope.restype = _ci
         lib.ats_fold_rope.argtypes = [_vp, _ci, _vp, _vp, _vp, _vp, _ci, _ci, _ci, _ci, _ci, _vp]
         lib.ats_fold_add_norm.restype = _ci
@@ -55,11 +55,6 @@ def _buf(key, numel: int, dtype, device) -> torch.Tensor:
 # projection, or the residual add and the RMSNorm that follows the output projection.
 # ----------------------------------------------------------------------------------------------------------
 FUSE_DECODE = __import__("os").environ.get("ATS_DECODE_FUSED", "1") == "1"
-# Flash-decoding merge inside the attention kernel (the CTA that arrives last for a sequence and KV head merges the chunk
-# partials) instead of a launch of its own.  Off by default: measured on one box it changed the decode step by -0.5 % on the
-# 22-layer model (64-wide heads) and +1.6 % on the Mixtral shape, where the merge lengthens the tail of a kernel that is already
-# the long pole of the layer.
-MERGE_INSIDE = __import__("os").environ.get("ATS_DECODE_MERGE_INSIDE", "0") == "1"
 
 
 DECODE_KERNEL = "decode kernel"
@@ -149,6 +144,14 @@ def decode_attention_available(qkv: torch.Tensor, n_q: int, n_kv: int, d: int) -
             and n_q % n_kv == 0 and n_q // n_kv in (1, 2, 4, 8) and qkv.shape[-1] % 8 == 0)
 
 
+def _partials(B: int, n_q: int, n_kv: int, d: int, tokens: int, device):
+    """Scratch of a cache so long that several clusters share a (sequence, key head): partial outputs and their softmax statistics."""
+    parts = _fns().ats_decode_attn_parts(B, n_kv, d, tokens)
+    if parts < 2:
+        return None, None
+    return (torch.empty(B * n_q * parts * d, dtype=torch.float32, device=device), torch.empty(B * n_q * parts * 2, dtype=torch.float32, device=device))
+
+
 def decode_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, length, n_q: int, n_kv: int, d: int,
                      max_tokens: Optional[int] = None) -> torch.Tensor:
     """qkv: [B, 1, (n_q + 2 n_kv) d] projection of the new token (RoPE already applied).  k_cache / v_cache:
@@ -162,27 +165,14 @@ def decode_attention(qkv: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Te
         raise RuntimeError(f"KV cache overflow: {longest}+1 > {max_len}")
     if not decode_attention_available(qkv, n_q, n_kv, d):
         return decode_attention_reference(qkv, k_cache, v_cache, length, n_q, n_kv, d)
-    lib = _fns()
-    chunks = lib.ats_decode_attn_chunks(max_len)
-    part_o = _buf("dec_o", B * n_q * chunks * d, torch.float32, qkv.device)
-    part_ml = _buf("dec_ml", B * n_q * chunks * 2, torch.float32, qkv.device)
-    # arrival counters of the (sequence, KV head) pairs: the CTA that arrives last merges the chunk partials and puts its counter
-    # back to zero, so the buffer is zeroed once, when it is made
-    key = ("dec_cnt", torch.int32, qkv.device.index)
-    done = _scratch.get(key)
-    if done is None or done.numel() < B * n_kv:
-        done = torch.zeros(max(B * n_kv, 1024), dtype=torch.int32, device=qkv.device)
-        _scratch[key] = done
+    part_o, part_ml = _partials(B, n_q, n_kv, d, longest + 1, qkv.device)
     out = torch.empty(B, 1, n_q * d, dtype=qkv.dtype, device=qkv.device)
-    err = lib.ats_decode_attn(_lib.ptr(qkv), qkv.stride(0), 0, n_q * d, (n_q + n_kv) * d, _lib.ptr(k_cache), _lib.ptr(v_cache),
-                              k_cache.stride(0), _lib.ptr(length) if per_seq else None, 0 if per_seq else int(length), longest, B, n_q,
-                              n_kv, d, max_len, _lib.ptr(part_o), _lib.ptr(part_ml), _lib.ptr(done) if MERGE_INSIDE else None, _lib.ptr(out),
-                              _lib.stream_ptr(qkv.device))
+    err = _fns().ats_decode_attn(_lib.ptr(qkv), qkv.stride(0), 0, n_q * d, (n_q + n_kv) * d, _lib.ptr(k_cache), _lib.ptr(v_cache),
+                                 k_cache.stride(0), _lib.ptr(length) if per_seq else None, 0 if per_seq else int(length), longest, B, n_q,
+                                 n_kv, d, max_len, _lib.ptr(part_o), _lib.ptr(part_ml), _lib.ptr(out), _lib.ptr(_lib.status_tensor(qkv.device)),
+                                 _lib.stream_ptr(qkv.device))
     _lib.check(err, "ats_decode_attn")
     return out
-
-
-MAX_COUNTERS = 1 << 16   # (sequence, key head) pairs of one decode_attention_cached call
 
 
 def decode_attention_cached(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, lengths: torch.Tensor, n_q: int, n_kv: int, d: int, scale: float,
@@ -190,18 +180,11 @@ def decode_attention_cached(q: torch.Tensor, k_cache: torch.Tensor, v_cache: tor
     """The kernel of :func:`decode_attention` for a cache [B, max_len, n_kv * d] that holds the new token's row already: q [B, >= n_q d]
     (prepared), lengths int32 [B] (position of the new token), ``cap`` > 0: scores become ``cap tanh(score / cap)``, gate [B, .] (strided view,
     one column per head) or ``None`` -> out [B, >= n_q d], merged and gated in the same launch."""
-    B, max_len, dev = q.shape[0], k_cache.shape[1], q.device
-    lib = _fns()
-    chunks = lib.ats_decode_attn_chunks(max_len)
-    part_o = torch.empty(B * n_q * chunks * d, dtype=torch.float32, device=dev)
-    part_ml = torch.empty(B * n_q * chunks * 2, dtype=torch.float32, device=dev)
-    done = _scratch.get(("dec_cached_cnt", dev.index))
-    if done is None:
-        # arrival counters, back at zero after every launch; one allocation for good, because captured graphs keep its address
-        done = _scratch[("dec_cached_cnt", dev.index)] = torch.zeros(MAX_COUNTERS, dtype=torch.int32, device=dev)
-    _lib.check(lib.ats_decode_attn_cached(_lib.ptr(q), q.stride(0), _lib.ptr(k_cache), _lib.ptr(v_cache), k_cache.stride(0), _lib.ptr(lengths), B, n_q, n_kv, d, max_len,
-                                          scale, cap, _lib.ptr(gate), 0 if gate is None else gate.stride(0), _lib.ptr(part_o), _lib.ptr(part_ml), _lib.ptr(done),
-                                          _lib.ptr(out), out.stride(0), _lib.stream_ptr(dev)), "ats_decode_attn_cached")
+    B, max_len = q.shape[0], k_cache.shape[1]
+    part_o, part_ml = _partials(B, n_q, n_kv, d, max_len, q.device)
+    _lib.check(_fns().ats_decode_attn_cached(_lib.ptr(q), q.stride(0), _lib.ptr(k_cache), _lib.ptr(v_cache), k_cache.stride(0), _lib.ptr(lengths), B, n_q, n_kv, d, max_len,
+                                             scale, cap, _lib.ptr(gate), 0 if gate is None else gate.stride(0), _lib.ptr(part_o), _lib.ptr(part_ml), _lib.ptr(out),
+                                             out.stride(0), _lib.ptr(_lib.status_tensor(q.device)), _lib.stream_ptr(q.device)), "ats_decode_attn_cached")
 
 
 def decode_attention_reference(qkv, k_cache, v_cache, length, n_q, n_kv, d) -> torch.Tensor:

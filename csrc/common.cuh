@@ -451,7 +451,7 @@ __device__ __forceinline__ void pdl_prologue() {
 }
 // (gemm_tcgen05.cu, the file that every library has)
 bool pdl_enabled();
-bool chained_launches();   // the calling thread vouches that no kernel in flight writes a weight that its next launches read
+bool chained_launches();   // the calling thread vouches that no kernel in flight writes what its next launches read early: weights, cached rows, lengths
 template <typename... KArgs, typename... Args>
 inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, Args&&... args) {
   cudaLaunchConfig_t cfg = {};

@@ -10,7 +10,7 @@
 // * gqa_prepare: norm, rotation, cache append; a warp (few tokens: a CTA) for a token's queries and one for its key and value.
 // * gqa_portion: L queries of a prompt at positions pos0 .. against the cache, any sizes, bf16 and fp32 (gqa_attention_tcgen05.cu is the
 //   tensor-core form).
-// * gqa_decode + gqa_merge: one query token per sequence, any sizes (decode_attn_mma_kernel in inference.cu serves bf16 heads of 64 and 128).
+// * gqa_decode + gqa_merge: one query token per sequence, any sizes (decode_attn_kernel in inference.cu serves bf16 heads of 64 and 128).
 #include "typed.cuh"
 
 namespace ats {

@@ -2,10 +2,9 @@
 // sampling.  Both are memory / latency bound (no tensor-core shape), so they are plain CUDA-core kernels laid out so
 // that every K / V byte of the cache is read exactly once per step.
 //
-// * ats_decode_attn: one new query token per sequence.  Grid (key chunk of 256, kv head, sequence); a CTA scores its
-//   256 keys for every query head of the group (K read once per group, not once per query head), does the softmax of
-//   the chunk in shared memory and reduces P V; a second kernel merges the chunks (flash-decoding).  The new token's
-//   K / V are written into the cache by the CTA whose chunk contains that position, so no separate append is needed.
+// * ats_decode_attn: one new query token per sequence.  Every warp scores units of 32 or 16 keys for all query heads of a group (K read once
+//   per group, not once per query head) and keeps a running softmax; warps are folded through shared memory, the CTAs of a (sequence, KV
+//   head) through distributed shared memory.  The new token's K / V are written into the cache here, so no separate append is needed.
 // * ats_sample: repetition penalty -> temperature -> top-k -> top-p -> multinomial (or arg-max when temperature <= 0) for
 //   one row of logits per CTA, without sorting: the top-k and top-p cut-offs are found by bisection on the order-preserving
 //   integer image of the floats.
@@ -17,12 +16,14 @@
 
 namespace ats {
 
-constexpr int DEC_CHUNK = 256;
-constexpr int DEC_THREADS = 256;
+int make_tmap_cache(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t batch_stride, uint32_t box_rows);
+
+constexpr int DEC_WARPS = 4;
+constexpr int DEC_THREADS = 32 * DEC_WARPS;
 
 struct DecodeArgs {
   const __nv_bfloat16* q;      // [B, *] packed projection of the new token; head h at q + b * ld_qkv + q_col0 + h * D
-  const __nv_bfloat16* k_new;  // same buffer, k_col0 / v_col0
+  const __nv_bfloat16* k_new;  // same buffer, k_col0 / v_col0; nullptr: the cache holds the new token's row already
   const __nv_bfloat16* v_new;
   long long ld_qkv;
   __nv_bfloat16* k_cache;  // [B, max_len, Hkv, D]
@@ -32,286 +33,149 @@ struct DecodeArgs {
   int length;
   int B, Hq, Hkv, D, max_len;
   float scale;
-  float* part_o;   // [B, Hq, n_chunks, D]
-  float* part_ml;  // [B, Hq, n_chunks, 2]
-  int n_chunks;
-  __nv_bfloat16* out;  // [B, Hq * D]
-  int* chunk_done;     // [B, Hkv] arrival counters (zero between launches) or nullptr: the last CTA of a (sequence, KV head) merges
-  // k_new == nullptr: the cache holds the new token's row already.  cap > 0: scores become cap tanh(score / cap).  gate ([B, ld_gate] + head
-  // or null): sigmoid(gate) scales the head's output.  out rows are ld_out elements apart.  (decode_attn_mma_kernel only)
+  int parts;       // clusters of a (sequence, KV head); more than one: the partial results of each go to part_o / part_ml
+  float* part_o;   // [B, Hq, parts, D]
+  float* part_ml;  // [B, Hq, parts, 2]
+  __nv_bfloat16* out;  // [B, ld_out]
+  // cap > 0: scores become cap tanh(score / cap).  gate ([B, ld_gate] + head or null): sigmoid(gate) scales the head's output.
   float cap;
   const __nv_bfloat16* gate;
   long long ld_gate, ld_out;
+  int* status;
 };
 
-template <int D, int REP>
-__global__ void __launch_bounds__(DEC_THREADS) decode_attn_kernel(const DecodeArgs p) {
-  __shared__ float s_q[REP][D];
-  __shared__ float s_p[REP][DEC_CHUNK];
-  __shared__ float s_red[DEC_THREADS / 32][REP][D];
-  const int chunk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int n_old = p.lengths ? p.lengths[b] : p.length;
-  const int n_tot = n_old + 1;  // the new token attends to itself
-  const int k0 = chunk * DEC_CHUNK;
-  const bool active = k0 < n_tot;
-  const int k_end = min(k0 + DEC_CHUNK, n_tot);
-
-  // query heads of the group -> shared memory (fp32, pre-scaled)
-  for (int i = tid; i < REP * D; i += DEC_THREADS) {
-    const int h = i / D, d = i % D;
-    s_q[h][d] = __bfloat162float(p.q[(long long)b * p.ld_qkv + (hk * REP + h) * D + d]) * p.scale;
-  }
-  // the new token's K / V row goes into the cache (by the CTA that owns its position)
-  __nv_bfloat16* kc = p.k_cache + (long long)b * p.cache_b_stride + (long long)hk * D;
-  __nv_bfloat16* vc = p.v_cache + (long long)b * p.cache_b_stride + (long long)hk * D;
-  const long long row_stride = (long long)p.Hkv * D;
-  if (active && n_old >= k0 && n_old < k0 + DEC_CHUNK && n_old < p.max_len) {
-    for (int d = tid; d < D; d += DEC_THREADS) {
-      kc[n_old * row_stride + d] = p.k_new[(long long)b * p.ld_qkv + hk * D + d];
-      vc[n_old * row_stride + d] = p.v_new[(long long)b * p.ld_qkv + hk * D + d];
-    }
-  }
-  __syncthreads();
-
-  // ---- scores: D / 8 lanes share a key row (one 16-byte load each, so a warp's load covers whole rows: with one thread per
-  // row every load instruction touched 32 cache lines and the kernel was bound by L1 wavefronts at a third of HBM speed);
-  // the partial dot products are folded with shuffles.  Four rows per lane group are requested before the first is used.
-  {
-    constexpr int LPR = D / 8, RPW = 32 / LPR, ROWS_PER_PASS = (DEC_THREADS / 32) * RPW, SUNR = 4;
-    const int sub = lane / LPR, l8 = lane % LPR;
-    float q[REP][8];
-#pragma unroll
-    for (int h = 0; h < REP; ++h)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) q[h][e] = s_q[h][8 * l8 + e];
-    for (int r0 = warp * RPW + sub; r0 < DEC_CHUNK; r0 += ROWS_PER_PASS * SUNR) {
-      uint4 kv[SUNR];
-#pragma unroll
-      for (int u = 0; u < SUNR; ++u) {
-        const int key = k0 + r0 + u * ROWS_PER_PASS;
-        if (active && key < k_end) {
-          const __nv_bfloat16* krow = (key == n_old) ? p.k_new + (long long)b * p.ld_qkv + hk * D : kc + key * row_stride;
-          kv[u] = *reinterpret_cast<const uint4*>(krow + 8 * l8);
-        } else {
-          kv[u] = make_uint4(0, 0, 0, 0);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < SUNR; ++u) {
-        const int r = r0 + u * ROWS_PER_PASS;
-        const float2 a = unpack_bf16x2(kv[u].x), bq = unpack_bf16x2(kv[u].y), c = unpack_bf16x2(kv[u].z), e = unpack_bf16x2(kv[u].w);
-        float part[REP];
-#pragma unroll
-        for (int h = 0; h < REP; ++h)
-          part[h] = a.x * q[h][0] + a.y * q[h][1] + bq.x * q[h][2] + bq.y * q[h][3] + c.x * q[h][4] + c.y * q[h][5] + e.x * q[h][6] + e.y * q[h][7];
-#pragma unroll
-        for (int off = LPR / 2; off > 0; off >>= 1)
-#pragma unroll
-          for (int h = 0; h < REP; ++h) part[h] += __shfl_xor_sync(0xffffffffu, part[h], off);
-        if (l8 == 0 && r < DEC_CHUNK) {
-          const bool valid = active && (k0 + r) < k_end;
-#pragma unroll
-          for (int h = 0; h < REP; ++h) s_p[h][r] = valid ? part[h] : -INFINITY;
-        }
-      }
-    }
-  }
-  __syncthreads();
-  // ---- chunk softmax: warp h handles head h (REP <= 8 = number of warps)
-  if (warp < REP) {
-    float m = -INFINITY;
-    for (int i = lane; i < DEC_CHUNK; i += 32) m = fmaxf(m, s_p[warp][i]);
-    m = warp_max(m);
-    float l = 0.f;
-    for (int i = lane; i < DEC_CHUNK; i += 32) {
-      const float e = (m == -INFINITY) ? 0.f : __expf(s_p[warp][i] - m);
-      s_p[warp][i] = e;
-      l += e;
-    }
-    l = warp_sum(l);
-    if (lane == 0) {
-      float* ml = p.part_ml + (((long long)b * p.Hq + hk * REP + warp) * p.n_chunks + chunk) * 2;
-      ml[0] = m;
-      ml[1] = l;
-    }
-  }
-  __syncthreads();
-  // ---- P V: thread (g, d8) sums keys g, g + G, ... for the eight dims 8 d8 .. 8 d8 + 7 of every head.  A row is read by
-  // D / 8 threads with 16-byte loads and four rows are requested before the first is used: the loop is bound by the number of
-  // bytes in flight, not by arithmetic.
-  constexpr int TPR = D / 8, G = DEC_THREADS / TPR;  // threads per row, row groups
-  const int g = tid / TPR, d8 = tid % TPR;
-  float o[REP][8];
-#pragma unroll
-  for (int h = 0; h < REP; ++h)
-#pragma unroll
-    for (int e = 0; e < 8; ++e) o[h][e] = 0.f;
-  if (active) {
-    constexpr int UNR = 4;
-    for (int kk = k0 + g; kk < k_end; kk += G * UNR) {
-      uint4 vv[UNR];
-#pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const int kr = kk + u * G;
-        if (kr < k_end) {
-          const __nv_bfloat16* vrow = (kr == n_old) ? p.v_new + (long long)b * p.ld_qkv + hk * D : vc + kr * row_stride;
-          vv[u] = *reinterpret_cast<const uint4*>(vrow + 8 * d8);
-        } else {
-          vv[u] = make_uint4(0, 0, 0, 0);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < UNR; ++u) {
-        const int kr = kk + u * G;
-        if (kr >= k_end) break;
-        const float2 v0 = unpack_bf16x2(vv[u].x), v1 = unpack_bf16x2(vv[u].y), v2 = unpack_bf16x2(vv[u].z), v3 = unpack_bf16x2(vv[u].w);
-#pragma unroll
-        for (int h = 0; h < REP; ++h) {
-          const float pr = s_p[h][kr - k0];
-          o[h][0] += pr * v0.x; o[h][1] += pr * v0.y; o[h][2] += pr * v1.x; o[h][3] += pr * v1.y;
-          o[h][4] += pr * v2.x; o[h][5] += pr * v2.y; o[h][6] += pr * v3.x; o[h][7] += pr * v3.y;
-        }
-      }
-    }
-  }
-  // fold the row groups that share a warp (lanes d8 and d8 + TPR, ...), then the warps through shared memory
-#pragma unroll
-  for (int off = TPR; off < 32; off <<= 1)
-#pragma unroll
-    for (int h = 0; h < REP; ++h)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) o[h][e] += __shfl_xor_sync(0xffffffffu, o[h][e], off);
-  if (lane < TPR) {
-#pragma unroll
-    for (int h = 0; h < REP; ++h)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) s_red[warp][h][8 * d8 + e] = o[h][e];
-  }
-  __syncthreads();
-  for (int i = tid; i < REP * D; i += DEC_THREADS) {
-    const int h = i / D, d = i % D;
-    float t = 0.f;
-#pragma unroll
-    for (int w = 0; w < DEC_THREADS / 32; ++w) t += s_red[w][h][d];
-    p.part_o[(((long long)b * p.Hq + hk * REP + h) * p.n_chunks + chunk) * D + d] = t;
-  }
-}
-
-// ------------------------------------------------------------------------------------------------
-// Tensor-core form of the same kernel (default).  With fp32 FMAs the kernel above issues ~1300 warp instructions per 32 keys
-// (four query heads per KV head, D = 128) and is bound by instruction issue at a third of HBM speed; both products are
-// therefore done with warp-level MMAs (m16n8k16, bf16 in, fp32 out) whose 16 rows hold the query heads of the group.  A
-// decode step is bandwidth-bound, so the warp-level MMA is enough; no shared-memory staging or transposing loads are needed:
-//
-// * S = Q K^T: the sum over the head dimension does not care about the order of its terms, so the dimension index is permuted
-//   such that the 16-byte piece a lane loads from a key row IS its B fragment for two consecutive k-steps (words 0,1 and 2,3);
-//   the Q fragments are read from global memory with the same permutation.
-// * O = P V: B wants two KEYS of one dimension in a register, memory holds two DIMENSIONS of one key in a word.  A lane loads
-//   16 bytes (four such words) of four keys and two byte permutes per word turn them into the fragments of TWO column tiles, one
-//   holding the even and one the odd dimension of the words; output columns are just another order of the dimensions.
-// Every warp handles 32 keys of the chunk for all dimensions; the warps' partial outputs are folded through shared memory.
-// ------------------------------------------------------------------------------------------------
 __device__ __forceinline__ void mma_16816_bf16(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
+__device__ __forceinline__ float ld_cluster_f32(uint32_t addr) {
+  float v;
+  asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(addr));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_shared_v4(uint32_t addr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
+  return v;
+}
+// scores carry a factor of log2(e), so that a power of two is all the softmax needs
+__device__ __forceinline__ float exp2_fast(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
+}
+__device__ __forceinline__ float exp_from(float m, float base) { return m == -INFINITY ? 0.f : exp2_fast(m - base); }
 
-// OCC: CTAs per SM the register allocation is cut for (2: 116 registers, no spills; 3: 80 registers, about 240 bytes of spills
-// but half again as many loads in flight).
-template <int D, int REP, int OCC = 2>
-__global__ void __launch_bounds__(DEC_THREADS, OCC) decode_attn_mma_kernel(const DecodeArgs p) {
-  pdl_prologue();
-  static_assert(REP <= 8 && D % 32 == 0, "query heads of a group sit in rows 0..7 of the MMA");
-  __shared__ float s_p[REP][DEC_CHUNK];
-  __shared__ __align__(16) float s_red[DEC_THREADS / 32][REP][D];
-  const int chunk = blockIdx.x, hk = blockIdx.y, b = blockIdx.z;
+// ------------------------------------------------------------------------------------------------
+// A decode step reads every K and V row once, so the kernel is a stream of the cache: what counts is the number of bytes in flight.  Plain
+// loads stop at 3.3 TB/s whatever their number (16 warps an SM with 8 KB each in registers measured the same as four dependent rounds of
+// loads), so every warp moves its keys with TMA copies into a ring of its own: two units of 8 KB (K and V of 2048 / D keys), up to 192 KB an SM.
+// No warp waits for another until its units are done; the softmax is the running one.  Both products are warp-level MMAs (m16n8k16,
+// bf16 in, fp32 out) whose 16 rows hold the query heads of the group (with fp32 FMAs the kernel is bound by instruction issue):
+//
+// * S = Q K^T: the sum over the head dimension does not care about the order of its terms, so the dimension index is permuted
+//   such that the 16-byte piece a lane reads of a key row IS its B fragment for two consecutive k-steps (words 0,1 and 2,3);
+//   the Q fragments are read from global memory with the same permutation.
+// * O = P V: B wants two KEYS of one dimension in a register, memory holds two DIMENSIONS of one key in a word.  A lane reads
+//   16 bytes (four such words) of four keys and two byte permutes per word turn them into the fragments of TWO column tiles, one
+//   holding the even and one the odd dimension of the words; output columns are just another order of the dimensions.  The accumulator
+//   fragment of S is the A fragment of P, so the probabilities stay in registers.
+//
+// In a chain of launches (common.cuh) the first units are requested before the kernel waits for its predecessor: only the new token's row
+// and the query come from it.  Units are dealt out over the parts x S x 4 warps of a (sequence, KV head) by its actual length.  The S CTAs
+// of a cluster fold their results through distributed shared memory, so there is no merge launch and no scratch below `parts` = 2.
+// Measured (us, caches larger than L2 in turn; before: 256-key chunks by plain loads and a merge launch): 64 sequences x 4 KV heads of 64,
+// 1,152 keys 29.6 -> 26.1; 64 x 8 of 128, 1,100 keys 94.6 -> 65.5 (4.4 TB/s), 1,500 keys 114 -> 78.6 (5.0 TB/s); one sequence, 640 keys 7.5 -> 4.9,
+// 32,000 keys 68.5 -> 15.2.  64 x 4 CTAs do not fill the SMs evenly: what is left there is a CTA's fixed time.
+// ------------------------------------------------------------------------------------------------
+template <bool V>
+struct BoolC {
+  static constexpr bool value = V;
+};
+constexpr int DEC_STAGES = 2;
+constexpr int DEC_UNIT_BYTES = 8192;
+constexpr int DEC_SMEM = 1024 + DEC_WARPS * DEC_STAGES * DEC_UNIT_BYTES;
+
+template <int D, int REP>
+__global__ void __launch_bounds__(DEC_THREADS, 3) decode_attn_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v,
+                                                                     const DecodeArgs p, const int early) {
+  static_assert(REP <= 8 && (D == 64 || D == 128), "query heads of a group sit in rows 0..7 of the MMA");
+  static_assert(REP * D * 4 <= DEC_STAGES * DEC_UNIT_BYTES, "a warp's result fits its ring");
+  constexpr int UNIT = 2048 / D, NT = UNIT / 8, KB = UNIT / 16, JD = D / 32, RD = D / 64;
+  extern __shared__ uint8_t dec_smem[];
+  __shared__ uint64_t s_full[DEC_WARPS][DEC_STAGES];
+  __shared__ float s_m[DEC_WARPS][REP], s_l[DEC_WARPS][REP];
+  __shared__ float s_ml[2][REP];
+  __shared__ int s_abort;
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (!early) asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int S = int(gridDim.x) / p.parts, part = int(blockIdx.x) / S, rank = int(blockIdx.x) - part * S;
+  const int hk = blockIdx.y, b = blockIdx.z;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
-  int n_old = p.lengths ? p.lengths[b] : p.length;
-  if (!ATS_DBG_CHECK(n_old >= 0 && n_old < p.max_len, kDbgDecodeAttn, n_old)) return;
+  const int n_old = p.lengths ? p.lengths[b] : p.length;
+  if (!ATS_DBG_CHECK(n_old >= 0 && n_old < p.max_len, kDbgDecodeAttn, n_old)) return;   // (every CTA of the cluster)
   const int n_tot = min(n_old + 1, p.max_len);  // the new token attends to itself
-  const int k0 = chunk * DEC_CHUNK;
-  const bool active = k0 < n_tot;
-  const int k_end = min(k0 + DEC_CHUNK, n_tot);
+  uint8_t* base_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dec_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* ring = base_smem + warp * (DEC_STAGES * DEC_UNIT_BYTES);
+  uint64_t* full = s_full[warp];
+  if (lane == 0) {
+    for (int i = 0; i < DEC_STAGES; ++i) mbar_init(&full[i], 1);
+    mbar_fence_init();
+  }
+  if (tid == 0) s_abort = 0;
+  __syncthreads();
+  const bool appended = p.k_new == nullptr;
+  const long long row_stride = (long long)p.Hkv * D;
   __nv_bfloat16* kc = p.k_cache + (long long)b * p.cache_b_stride + (long long)hk * D;
   __nv_bfloat16* vc = p.v_cache + (long long)b * p.cache_b_stride + (long long)hk * D;
-  const long long row_stride = (long long)p.Hkv * D;
-  const bool appended = p.k_new == nullptr;
-  const __nv_bfloat16* k_new = appended ? kc + n_old * row_stride : p.k_new + (long long)b * p.ld_qkv + hk * D;
-  const __nv_bfloat16* v_new = appended ? vc + n_old * row_stride : p.v_new + (long long)b * p.ld_qkv + hk * D;
-  // the new token's K / V row goes into the cache (by the CTA that owns its position); this CTA reads it from the projection
-  if (!appended && active && n_old >= k0 && n_old < k0 + DEC_CHUNK && n_old < p.max_len) {
+  const __nv_bfloat16* k_new = p.k_new + (long long)b * p.ld_qkv + hk * D;   // (not used when appended)
+  const __nv_bfloat16* v_new = p.v_new + (long long)b * p.ld_qkv + hk * D;
+
+  const int stride = p.parts * S * DEC_WARPS * UNIT, first = (int(blockIdx.x) * DEC_WARPS + warp) * UNIT;
+  const int count = first < n_tot ? (n_tot - first + stride - 1) / stride : 0;
+  auto request = [&](int i) {   // lane 0; rows from max_len on read as zero
+    uint8_t* dst = ring + (i % DEC_STAGES) * DEC_UNIT_BYTES;
+    uint64_t* bar = &full[i % DEC_STAGES];
+    const int k0 = first + i * stride;
+    mbar_expect_tx(bar, DEC_UNIT_BYTES);
+#pragma unroll
+    for (int rd = 0; rd < RD; ++rd) {
+      tma_load_3d(dst + rd * UNIT * 128, &map_k, bar, hk * D + 64 * rd, k0, b);
+      tma_load_3d(dst + DEC_UNIT_BYTES / 2 + rd * UNIT * 128, &map_v, bar, hk * D + 64 * rd, k0, b);
+    }
+  };
+  if (lane == 0) {
+    const int n = min(count, DEC_STAGES);
+    int i = 0;
+    // the new token's row is not taken from the cache unless it was appended: then its unit waits for the kernel that wrote it
+    if (early)
+      for (; i < n && (!appended || first + i * stride + UNIT <= n_old); ++i) request(i);
+    if (early) asm volatile("griddepcontrol.wait;" ::: "memory");
+    for (; i < n; ++i) request(i);
+  } else if (early) {
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+  }
+  __syncwarp();
+  // the new token's K / V row goes into the cache; this kernel itself reads it from the projection
+  if (!appended && blockIdx.x == 0 && n_old < p.max_len) {
     for (int d = tid; d < D; d += DEC_THREADS) {
       kc[n_old * row_stride + d] = k_new[d];
       vc[n_old * row_stride + d] = v_new[d];
     }
   }
-  const int kw0 = warp * 32;  // this warp's keys inside the chunk
-
-  // ---- S = Q K^T
+  uint32_t qa[D / 16][2];  // A fragments (rows g < REP): [virtual k-step][a0, a2]
   {
-    uint32_t qa[D / 16][2];  // A fragments (rows g < REP): [virtual k-step][a0, a2]
     const uint32_t* qrow = reinterpret_cast<const uint32_t*>(p.q + (long long)b * p.ld_qkv + (hk * REP + (g < REP ? g : 0)) * D);
 #pragma unroll
-    for (int j = 0; j < D / 32; ++j) {
+    for (int j = 0; j < JD; ++j) {
       uint4 w = make_uint4(0, 0, 0, 0);
       if (g < REP) w = *reinterpret_cast<const uint4*>(qrow + 4 * (4 * j + t));
       qa[2 * j][0] = w.x; qa[2 * j][1] = w.y; qa[2 * j + 1][0] = w.z; qa[2 * j + 1][1] = w.w;
     }
-#pragma unroll
-    for (int nt = 0; nt < 4; ++nt) {
-      const int r = kw0 + nt * 8 + g;  // the key whose row this lane loads (column g of the tile)
-      const int key = k0 + r;
-      const bool ok = active && key < k_end;
-      const __nv_bfloat16* krow = (key == n_old) ? k_new : kc + key * row_stride;
-      uint4 kv[D / 32];
-#pragma unroll
-      for (int j = 0; j < D / 32; ++j) kv[j] = ok ? *reinterpret_cast<const uint4*>(krow + 8 * (4 * j + t)) : make_uint4(0, 0, 0, 0);
-      float c[4] = {0.f, 0.f, 0.f, 0.f};
-#pragma unroll
-      for (int j = 0; j < D / 32; ++j) {
-        mma_16816_bf16(c, qa[2 * j][0], 0u, qa[2 * j][1], 0u, kv[j].x, kv[j].y);
-        mma_16816_bf16(c, qa[2 * j + 1][0], 0u, qa[2 * j + 1][1], 0u, kv[j].z, kv[j].w);
-      }
-      if (g < REP) {  // c[0], c[1]: head g, keys 2t and 2t + 1 of the tile
-        const int c0 = kw0 + nt * 8 + 2 * t;
-        float s0 = c[0] * p.scale, s1 = c[1] * p.scale;
-        if (p.cap > 0.f) {
-          const float inv = __fdividef(1.f, p.cap);
-          s0 = p.cap * tanh_fast(s0 * inv);
-          s1 = p.cap * tanh_fast(s1 * inv);
-        }
-        s_p[g][c0] = (active && k0 + c0 < k_end) ? s0 : -INFINITY;
-        s_p[g][c0 + 1] = (active && k0 + c0 + 1 < k_end) ? s1 : -INFINITY;
-      }
-    }
   }
-  __syncthreads();
-  // ---- chunk softmax: warp h handles head h (REP <= 8 = number of warps)
-  if (warp < REP) {
-    float m = -INFINITY;
-    for (int i = lane; i < DEC_CHUNK; i += 32) m = fmaxf(m, s_p[warp][i]);
-    m = warp_max(m);
-    float l = 0.f;
-    for (int i = lane; i < DEC_CHUNK; i += 32) {
-      const float e = (m == -INFINITY) ? 0.f : __expf(s_p[warp][i] - m);
-      s_p[warp][i] = e;
-      l += e;
-    }
-    l = warp_sum(l);
-    if (lane == 0) {
-      float* ml = p.part_ml + (((long long)b * p.Hq + hk * REP + warp) * p.n_chunks + chunk) * 2;
-      ml[0] = m;
-      ml[1] = l;
-    }
-  }
-  __syncthreads();
-  // ---- O = P V over this warp's 32 keys (two blocks of 16), all dimensions.  Lane (g, t) loads 16 bytes (dims 64 rd + 8 g .. + 7)
-  // of four keys: eight lanes cover 128 contiguous bytes of a row.  Word i of the piece holds dims 8 g + 2 i, + 1: the low halves of
-  // two keys form the B fragment of the column tile "even dims of word i", the high halves that of "odd dims of word i".
-  constexpr int RD = D / 64;
+  const float inv_cap = p.cap > 0.f ? __fdividef(1.f, p.cap) : 0.f;
   float oe[RD][4][4], oo[RD][4][4];
 #pragma unroll
   for (int rd = 0; rd < RD; ++rd)
@@ -319,31 +183,101 @@ __global__ void __launch_bounds__(DEC_THREADS, OCC) decode_attn_mma_kernel(const
     for (int i = 0; i < 4; ++i)
 #pragma unroll
       for (int e = 0; e < 4; ++e) oe[rd][i][e] = oo[rd][i][e] = 0.f;
-  if (active && k0 + kw0 < k_end) {
+  float m = -INFINITY, l = 0.f;   // of head g, over this warp's units (l: this lane's keys)
+  const float scale2 = p.scale * 1.4426950408889634f, cap2 = p.cap * 1.4426950408889634f;
+  const uint32_t k_at = smem_u32(ring) + g * 128, v_at = smem_u32(ring) + DEC_UNIT_BYTES / 2 + 2 * t * 128;
+  // the pieces of key 8 nt + g and of the values' keys 2 t, 2 t + 1 (+ 8), swizzled by their rows modulo eight
+  const uint32_t piece[2] = {uint32_t((t ^ g) << 4), uint32_t(((4 + t) ^ g) << 4)}, vpiece[2] = {uint32_t((g ^ (2 * t)) << 4), uint32_t((g ^ (2 * t + 1)) << 4) + 128};
+  bool ok = true;
+  uint32_t stage = 0, parity = 0;
+  // LAST: the unit holds the new token or rows behind it
+  auto unit = [&](auto last_c, const int k0) {
+    constexpr bool LAST = decltype(last_c)::value;
+    const uint32_t ks = k_at + stage * DEC_UNIT_BYTES, vs = v_at + stage * DEC_UNIT_BYTES;
+    uint4 vv[KB][RD][4];
+    float s[NT][2];
 #pragma unroll
-    for (int kb = 0; kb < 2; ++kb) {
-      const int kk0 = kw0 + kb * 16;
-      if (k0 + kk0 >= k_end) break;
-      uint32_t pa0 = 0u, pa2 = 0u;  // P fragments (bf16 pairs): keys 2t, 2t + 1 and 2t + 8, 2t + 9 of head g
-      if (g < REP) {
-        pa0 = pack_bf16x2(s_p[g][kk0 + 2 * t], s_p[g][kk0 + 2 * t + 1]);
-        pa2 = pack_bf16x2(s_p[g][kk0 + 2 * t + 8], s_p[g][kk0 + 2 * t + 9]);
+    for (int nt = 0; nt < NT; ++nt) {   // column g of the tile: this lane reads pieces of key nt * 8 + g
+      uint4 kv[JD];
+#pragma unroll
+      for (int j = 0; j < JD; ++j) {
+        kv[j] = ld_shared_v4(ks + ((j >> 1) * UNIT + nt * 8) * 128 + piece[j & 1]);
+        if (LAST && !appended && k0 + nt * 8 + g == n_old) kv[j] = *reinterpret_cast<const uint4*>(k_new + 8 * (4 * j + t));
       }
-      uint4 w[RD][4];
+      float c[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const int key = k0 + kk0 + 2 * t + (i & 1) + (i >> 1) * 8;
-        const __nv_bfloat16* vrow = (key == n_old) ? v_new : vc + key * row_stride;
-#pragma unroll
-        for (int rd = 0; rd < RD; ++rd)
-          w[rd][i] = key < k_end ? *reinterpret_cast<const uint4*>(vrow + 64 * rd + 8 * g) : make_uint4(0, 0, 0, 0);
+      for (int j = 0; j < JD; ++j) {
+        mma_16816_bf16(c, qa[2 * j][0], 0u, qa[2 * j][1], 0u, kv[j].x, kv[j].y);
+        mma_16816_bf16(c, qa[2 * j + 1][0], 0u, qa[2 * j + 1][1], 0u, kv[j].z, kv[j].w);
       }
+      s[nt][0] = c[0];   // head g, keys 2t and 2t + 1 of the tile
+      s[nt][1] = c[1];
+    }
+    // lane (g, t) reads 16 bytes (dims 64 rd + 8 g .. + 7) of four keys
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb)
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int rd = 0; rd < RD; ++rd) {
+          vv[kb][rd][i] = ld_shared_v4(vs + (rd * UNIT + kb * 16 + (i >> 1) * 8) * 128 + vpiece[i & 1]);
+          if (LAST) {
+            const int row = kb * 16 + 2 * t + (i & 1) + (i >> 1) * 8;
+            if (!appended && k0 + row == n_old) vv[kb][rd][i] = *reinterpret_cast<const uint4*>(v_new + 64 * rd + 8 * g);
+            if (k0 + row >= n_tot) vv[kb][rd][i] = make_uint4(0, 0, 0, 0);   // whatever earlier generations left there
+          }
+        }
+    if (p.cap > 0.f) {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) s[nt][e] = cap2 * tanh_fast(s[nt][e] * p.scale * inv_cap);
+    } else {
+#pragma unroll
+      for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+        for (int e = 0; e < 2; ++e) s[nt][e] *= scale2;
+    }
+    float top = m;
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        if (LAST && k0 + nt * 8 + 2 * t + e >= n_tot) s[nt][e] = -INFINITY;
+        top = fmaxf(top, s[nt][e]);
+      }
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 1));
+    top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, 2));
+    const float base = top == -INFINITY ? 0.f : top;
+    if (__any_sync(0xffffffffu, top > m)) {
+      const float keep = exp_from(m, base);
+      m = top;
+      l *= keep;
+#pragma unroll
+      for (int rd = 0; rd < RD; ++rd)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) oe[rd][i][e] *= keep, oo[rd][i][e] *= keep;
+    }
+#pragma unroll
+    for (int nt = 0; nt < NT; ++nt)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) {
+        s[nt][e] = exp2_fast(s[nt][e] - base);
+        l += s[nt][e];
+      }
+    // Word i of a V piece holds dims 8 g + 2 i, + 1: the low halves of two keys form the B fragment of the column tile "even dims of
+    // word i", the high halves that of "odd dims of word i".
+#pragma unroll
+    for (int kb = 0; kb < KB; ++kb) {
+      const uint32_t pa0 = pack_bf16x2(s[2 * kb][0], s[2 * kb][1]), pa2 = pack_bf16x2(s[2 * kb + 1][0], s[2 * kb + 1][1]);
 #pragma unroll
       for (int rd = 0; rd < RD; ++rd) {
-        const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&w[rd][0]);
-        const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&w[rd][1]);
-        const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&w[rd][2]);
-        const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&w[rd][3]);
+        const uint32_t* w0 = reinterpret_cast<const uint32_t*>(&vv[kb][rd][0]);
+        const uint32_t* w1 = reinterpret_cast<const uint32_t*>(&vv[kb][rd][1]);
+        const uint32_t* w2 = reinterpret_cast<const uint32_t*>(&vv[kb][rd][2]);
+        const uint32_t* w3 = reinterpret_cast<const uint32_t*>(&vv[kb][rd][3]);
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           mma_16816_bf16(oe[rd][i], pa0, 0u, pa2, 0u, __byte_perm(w0[i], w1[i], 0x5410), __byte_perm(w2[i], w3[i], 0x5410));
@@ -351,12 +285,33 @@ __global__ void __launch_bounds__(DEC_THREADS, OCC) decode_attn_mma_kernel(const
         }
       }
     }
+  };
+#pragma unroll 1
+  for (int u = 0; u < count; ++u) {
+    ok = __all_sync(0xffffffffu, mbar_wait_bounded(&full[stage], parity, &s_abort, p.status, kTimeoutFull));
+    if (!ok) break;
+    const int k0 = first + u * stride;
+    if (k0 + UNIT > n_old) unit(BoolC<true>{}, k0);
+    else unit(BoolC<false>{}, k0);
+    __syncwarp();   // the stage has been read
+    if (lane == 0 && u + DEC_STAGES < count) request(u + DEC_STAGES);
+    if (++stage == DEC_STAGES) stage = 0, parity ^= 1;
   }
+  if (!ok) {   // copies that were issued land before the CTA gives its shared memory back
+    const uint64_t t0 = globaltimer_ns();
+    while (globaltimer_ns() - t0 < 10000000ull) {
+    }
+  }
+  l += __shfl_xor_sync(0xffffffffu, l, 1);
+  l += __shfl_xor_sync(0xffffffffu, l, 2);
+  // results lie in the warps' rings
+  auto red = [&](int w, int h, int d) { return reinterpret_cast<float*>(base_smem + w * (DEC_STAGES * DEC_UNIT_BYTES)) + h * D + d; };
   // lane (g, t), head g: accumulator column 2t is dim 64 rd + 16 t + 2 i (+ 1 for the odd tile), column 2t + 1 eight dims further
   if (g < REP) {
+    if (t == 0) s_m[warp][g] = m, s_l[warp][g] = l;
 #pragma unroll
     for (int rd = 0; rd < RD; ++rd) {
-      float* dst = &s_red[warp][g][64 * rd + 16 * t];
+      float* dst = red(warp, g, 64 * rd + 16 * t);
       *reinterpret_cast<float4*>(dst) = make_float4(oe[rd][0][0], oo[rd][0][0], oe[rd][1][0], oo[rd][1][0]);
       *reinterpret_cast<float4*>(dst + 4) = make_float4(oe[rd][2][0], oo[rd][2][0], oe[rd][3][0], oo[rd][3][0]);
       *reinterpret_cast<float4*>(dst + 8) = make_float4(oe[rd][0][1], oo[rd][0][1], oe[rd][1][1], oo[rd][1][1]);
@@ -364,67 +319,69 @@ __global__ void __launch_bounds__(DEC_THREADS, OCC) decode_attn_mma_kernel(const
     }
   }
   __syncthreads();
+  // the warps of the CTA: into warp 0's block (each element is read and written by one thread)
   for (int i = tid; i < REP * D; i += DEC_THREADS) {
     const int h = i / D, d = i % D;
-    float acc = 0.f;
+    float top = -INFINITY;
 #pragma unroll
-    for (int w = 0; w < DEC_THREADS / 32; ++w) acc += s_red[w][h][d];
-    p.part_o[(((long long)b * p.Hq + hk * REP + h) * p.n_chunks + chunk) * D + d] = acc;
-  }
-  if (p.chunk_done == nullptr) return;
-  // The CTA that arrives last for this (sequence, KV head) merges the chunk partials of its query heads: no separate merge launch.
-  __shared__ int s_last;
-  __threadfence();
-  __syncthreads();
-  if (tid == 0) {
-    int* cnt = p.chunk_done + b * p.Hkv + hk;
-    s_last = atomicAdd(cnt, 1) == int(gridDim.x) - 1;
-    if (s_last) *cnt = 0;  // every CTA of this launch has arrived: ready for the next launch on the stream
-  }
-  __syncthreads();
-  if (!s_last || warp >= REP) return;
-  __threadfence();
-  const long long wq = (long long)b * p.Hq + hk * REP + warp;
-  const float* ml = p.part_ml + wq * p.n_chunks * 2;
-  float m = -INFINITY;
-  for (int c = 0; c < p.n_chunks; ++c) m = fmaxf(m, __ldcg(ml + 2 * c));
-  float l = 0.f;
-  for (int c = 0; c < p.n_chunks; ++c) {
-    const float mc = __ldcg(ml + 2 * c);
-    l += __ldcg(ml + 2 * c + 1) * ((mc == -INFINITY) ? 0.f : __expf(mc - m));
-  }
-  float inv = l > 0.f ? 1.f / l : 0.f;
-  if (p.gate) inv = __fdividef(inv, 1.f + __expf(-__bfloat162float(p.gate[(long long)b * p.ld_gate + hk * REP + warp])));
-  for (int d = lane; d < D; d += 32) {
-    float acc = 0.f;
-    for (int c = 0; c < p.n_chunks; ++c) {
-      const float mc = __ldcg(ml + 2 * c);
-      const float f = (mc == -INFINITY) ? 0.f : __expf(mc - m);
-      acc += __ldcg(p.part_o + (wq * p.n_chunks + c) * D + d) * f;
+    for (int w = 0; w < DEC_WARPS; ++w) top = fmaxf(top, s_m[w][h]);
+    const float base = top == -INFINITY ? 0.f : top;
+    float acc = 0.f, sum = 0.f;
+#pragma unroll
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float f = exp_from(s_m[w][h], base);
+      acc += *red(w, h, d) * f;
+      sum += s_l[w][h] * f;
     }
-    p.out[(long long)b * p.ld_out + (hk * REP + warp) * D + d] = __float2bfloat16(acc * inv);
+    *red(0, h, d) = acc;
+    if (d == 0) s_ml[0][h] = top, s_ml[1][h] = sum;
   }
+  // the CTAs of the cluster: every one finishes its share of the elements
+  if (S > 1) cluster_sync_all();
+  else __syncthreads();
+  const uint32_t at_o = smem_u32(red(0, 0, 0)), at_ml = smem_u32(&s_ml[0][0]);
+  for (int i = rank * DEC_THREADS + tid; i < REP * D; i += S * DEC_THREADS) {
+    const int h = i / D, d = i % D;
+    float top = -INFINITY, acc = 0.f, sum = 0.f;
+    for (int r = 0; r < S; ++r) top = fmaxf(top, ld_cluster_f32(mapa_shared(at_ml + h * 4, r)));
+    const float base = top == -INFINITY ? 0.f : top;
+#pragma unroll 4
+    for (int r = 0; r < S; ++r) {
+      const float f = exp_from(ld_cluster_f32(mapa_shared(at_ml + h * 4, r)), base);
+      sum += ld_cluster_f32(mapa_shared(at_ml + (REP + h) * 4, r)) * f;
+      acc += ld_cluster_f32(mapa_shared(at_o + i * 4, r)) * f;
+    }
+    const long long head = hk * REP + h;
+    if (p.parts > 1) {
+      const long long at = ((long long)b * p.Hq + head) * p.parts + part;
+      p.part_o[at * D + d] = acc;
+      if (d == 0) p.part_ml[2 * at] = top, p.part_ml[2 * at + 1] = sum;
+    } else {
+      float inv = sum > 0.f ? 1.f / sum : 0.f;
+      if (p.gate) inv = __fdividef(inv, 1.f + __expf(-__bfloat162float(p.gate[(long long)b * p.ld_gate + head])));
+      p.out[(long long)b * p.ld_out + head * D + d] = __float2bfloat16(acc * inv);
+    }
+  }
+  if (S > 1) cluster_sync_all();   // nobody leaves while its shared memory is read
 }
 
-// one warp per (sequence, query head): merge the chunk partials
-__global__ void decode_merge_kernel(const float* __restrict__ part_o, const float* __restrict__ part_ml,
-                                    __nv_bfloat16* __restrict__ out, int BH, int n_chunks, int D) {
+// one warp per (sequence, query head): merge the partial results of several clusters
+__global__ void decode_merge_kernel(const DecodeArgs p) {
   pdl_prologue();
   const int w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
-  if (w >= BH) return;
-  const float* ml = part_ml + (long long)w * n_chunks * 2;
+  if (w >= p.B * p.Hq) return;
+  const int b = w / p.Hq, head = w - b * p.Hq;
+  const float* ml = p.part_ml + (long long)w * p.parts * 2;
   float m = -INFINITY;
-  for (int c = 0; c < n_chunks; ++c) m = fmaxf(m, ml[2 * c]);
+  for (int c = 0; c < p.parts; ++c) m = fmaxf(m, ml[2 * c]);
   float l = 0.f;
-  for (int c = 0; c < n_chunks; ++c) l += ml[2 * c + 1] * ((ml[2 * c] == -INFINITY) ? 0.f : __expf(ml[2 * c] - m));
-  const float inv = l > 0.f ? 1.f / l : 0.f;
-  for (int d = lane; d < D; d += 32) {
+  for (int c = 0; c < p.parts; ++c) l += ml[2 * c + 1] * exp_from(ml[2 * c], m);
+  float inv = l > 0.f ? 1.f / l : 0.f;
+  if (p.gate) inv = __fdividef(inv, 1.f + __expf(-__bfloat162float(p.gate[(long long)b * p.ld_gate + head])));
+  for (int d = lane; d < p.D; d += 32) {
     float t = 0.f;
-    for (int c = 0; c < n_chunks; ++c) {
-      const float f = (ml[2 * c] == -INFINITY) ? 0.f : __expf(ml[2 * c] - m);
-      t += part_o[((long long)w * n_chunks + c) * D + d] * f;
-    }
-    out[(long long)w * D + d] = __float2bfloat16(t * inv);
+    for (int c = 0; c < p.parts; ++c) t += p.part_o[((long long)w * p.parts + c) * p.D + d] * exp_from(ml[2 * c], m);
+    p.out[(long long)b * p.ld_out + (long long)head * p.D + d] = __float2bfloat16(t * inv);
   }
 }
 
@@ -860,38 +817,82 @@ __global__ void __launch_bounds__(256) fold_add_norm_kernel(const float* __restr
 
 using namespace ats;
 
-// 1 (default): warp-level tensor-core kernel; 0: the fp32 CUDA-core kernel (kept for comparison, ATS_DECODE_ATTN_MMA=0)
-static int g_decode_mma = -1;
-static int g_decode_occ = 2;  // ATS_DECODE_ATTN_OCC=3 selects the 80-register build of the tensor-core kernel
-template <int D, int REP>
-static int launch_decode(const DecodeArgs& p, cudaStream_t s) {
-  if (g_decode_mma < 0) {
-    const char* e = getenv("ATS_DECODE_ATTN_MMA");
-    g_decode_mma = (e && e[0] == '0') ? 0 : 1;
-    const char* o = getenv("ATS_DECODE_ATTN_OCC");
-    if (o && o[0] == '3') g_decode_occ = 3;
+// How many CTAs share a (sequence, KV head) (`cluster`, a power of two up to the portable cluster size) and how many such clusters (`parts`).
+// A CTA costs 4 to 5 us whatever it reads, so there are no more of them than fill the SMs once (three each) unless a warp would walk
+// through more than ten units: 256 pairs with 1,152 keys take 27.0 us with one CTA each, 26.1 with two, 27.6 with four and 57 with eight;
+// 512 pairs with 1,100 keys of 128 dimensions 65 with two, 68 with four, 102 with eight.
+static void decode_split(int pairs, int D, int tokens, int* cluster, int* parts) {
+  const int units = (tokens + 2048 / D - 1) / (2048 / D);
+  int s = 1, n = 1;
+  while (s < 8 && s * DEC_WARPS < units && (pairs * s < 3 * 148 || s * DEC_WARPS * 10 < units)) s *= 2;
+  while (pairs * s * n < 2 * 148 && s * n * DEC_WARPS * 4 < units) n *= 2;
+  *cluster = s;
+  *parts = n;
+}
+// Partial results per (sequence, query head) of `ats_decode_attn` / `ats_decode_attn_cached` for up to `tokens` keys: above one, part_o
+// holds B * Hq * parts * D floats and part_ml B * Hq * parts * 2; at one they are not used.
+ATS_API int ats_decode_attn_parts(int B, int Hkv, int D, int tokens) {
+  if (B < 1 || Hkv < 1 || D < 1) return 1;
+  int s, n;
+  decode_split(B * Hkv, D, tokens, &s, &n);
+  return n;
+}
+
+static int decode_attn(DecodeArgs& p, int tokens, cudaStream_t s) {
+  int cluster, rep = p.Hq / p.Hkv;
+  decode_split(p.B * p.Hkv, p.D, tokens, &cluster, &p.parts);
+  if (p.parts > 1 && (!p.part_o || !p.part_ml)) return 1003;
+  CUtensorMap mk, mv;
+  const unsigned long long ld = (unsigned long long)p.Hkv * p.D, bs = p.B > 1 ? p.cache_b_stride : ld * p.max_len;
+  int e;
+  if ((e = make_tmap_cache(&mk, p.k_cache, ld, p.max_len, p.B, bs, 2048 / p.D)) || (e = make_tmap_cache(&mv, p.v_cache, ld, p.max_len, p.B, bs, 2048 / p.D))) return e;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster * p.parts, p.Hkv, p.B);
+  cfg.blockDim = dim3(DEC_THREADS);
+  cfg.dynamicSmemBytes = DEC_SMEM;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  int n = 0;
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
   }
-  dim3 grid(p.n_chunks, p.Hkv, p.B);
-  if (g_decode_mma && g_decode_occ == 3) decode_attn_mma_kernel<D, REP, 3><<<grid, DEC_THREADS, 0, s>>>(p);
-  else if (g_decode_mma) {
-    cudaError_t ce = launch_pdl(decode_attn_mma_kernel<D, REP, 2>, grid, dim3(DEC_THREADS), 0, s, p);
-    return int(ce != cudaSuccess ? ce : cudaGetLastError());
+  if (pdl_enabled()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n].val.programmaticStreamSerializationAllowed = 1;
+    ++n;
   }
-  else decode_attn_kernel<D, REP><<<grid, DEC_THREADS, 0, s>>>(p);
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  const int early = int(chained_launches());
+  cudaError_t ce = cudaErrorInvalidValue;
+  bool known = false;
+#define ATS_DEC(DD, RR)                                                                                                             \
+  if (p.D == DD && rep == RR) {                                                                                                     \
+    known = true;                                                                                                                   \
+    ce = cudaFuncSetAttribute(decode_attn_kernel<DD, RR>, cudaFuncAttributeMaxDynamicSharedMemorySize, DEC_SMEM);                    \
+    if (ce == cudaSuccess) ce = cudaLaunchKernelEx(&cfg, decode_attn_kernel<DD, RR>, mk, mv, p, early);                              \
+  }
+  ATS_DEC(64, 1) ATS_DEC(64, 2) ATS_DEC(64, 4) ATS_DEC(64, 8) ATS_DEC(128, 1) ATS_DEC(128, 2) ATS_DEC(128, 4) ATS_DEC(128, 8)
+#undef ATS_DEC
+  if (!known) return 1004;
+  if (ce != cudaSuccess) return int(ce);
+  if (p.parts > 1) {
+    ce = launch_pdl(decode_merge_kernel, dim3((p.B * p.Hq * 32 + 255) / 256), dim3(256), 0, s, p);
+    if (ce != cudaSuccess) return int(ce);
+  }
   return int(cudaGetLastError());
 }
 
-// Scratch sizes for `ats_decode_attn`: floats needed for part_o and part_ml with a cache of `max_len` positions.
-ATS_API int ats_decode_attn_chunks(int max_len) { return (max_len + DEC_CHUNK - 1) / DEC_CHUNK; }
-
 // qkv: packed projection of the new token [B, ld_qkv]; caches [B, max_len, Hkv, D] (batch stride cache_b_stride elements).
-// lengths: per-sequence cached lengths (device int32) or nullptr for the common `length`.  out: [B, Hq * D] bf16.
+// lengths: per-sequence cached lengths (device int32) or nullptr for the common `length`; none exceeds max_tokens.  out: [B, Hq * D] bf16.
 ATS_API int ats_decode_attn(const void* qkv, long long ld_qkv, int q_col0, int k_col0, int v_col0, void* k_cache, void* v_cache,
                             long long cache_b_stride, const int* lengths, int length, int max_tokens, int B, int Hq, int Hkv, int D,
-                            int max_len, float* part_o, float* part_ml, int* chunk_done, void* out, void* stream) {
-  if ((D != 64 && D != 128) || Hq % Hkv || ((q_col0 | k_col0 | v_col0) & 7) || (ld_qkv & 7)) return 1003;
-  const int rep = Hq / Hkv;
-  DecodeArgs p;
+                            int max_len, float* part_o, float* part_ml, void* out, int* status, void* stream) {
+  if ((D != 64 && D != 128) || Hkv < 1 || Hq % Hkv || ((q_col0 | k_col0 | v_col0) & 7) || (ld_qkv & 7)) return 1003;
+  DecodeArgs p = {};
   const __nv_bfloat16* base = static_cast<const __nv_bfloat16*>(qkv);
   p.q = base + q_col0; p.k_new = base + k_col0; p.v_new = base + v_col0;
   p.ld_qkv = ld_qkv;
@@ -901,29 +902,10 @@ ATS_API int ats_decode_attn(const void* qkv, long long ld_qkv, int q_col0, int k
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.max_len = max_len;
   p.scale = 1.f / sqrtf(float(D));
   p.part_o = part_o; p.part_ml = part_ml;
-  p.cap = 0.f; p.gate = nullptr; p.ld_gate = 0; p.ld_out = (long long)Hq * D;
-  // chunks to launch: enough for the longest sequence (+ the new token)
-  p.n_chunks = (min(max_tokens + 1, max_len) + DEC_CHUNK - 1) / DEC_CHUNK;
-  if (p.n_chunks < 1) p.n_chunks = 1;
+  p.ld_out = (long long)Hq * D;
+  p.status = status;
   p.out = static_cast<__nv_bfloat16*>(out);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (g_decode_mma < 0) {
-    const char* ev = getenv("ATS_DECODE_ATTN_MMA");
-    g_decode_mma = (ev && ev[0] == '0') ? 0 : 1;
-    const char* o = getenv("ATS_DECODE_ATTN_OCC");
-    if (o && o[0] == '3') g_decode_occ = 3;
-  }
-  const bool merge_inside = chunk_done != nullptr && g_decode_mma == 1 && g_decode_occ == 2;
-  p.chunk_done = merge_inside ? chunk_done : nullptr;
-  int e = 1004;
-#define ATS_DEC(DD, RR) if (D == DD && rep == RR) e = launch_decode<DD, RR>(p, s);
-  ATS_DEC(64, 1) ATS_DEC(64, 2) ATS_DEC(64, 4) ATS_DEC(64, 8) ATS_DEC(128, 1) ATS_DEC(128, 2) ATS_DEC(128, 4) ATS_DEC(128, 8)
-#undef ATS_DEC
-  if (e) return e;
-  if (merge_inside) return int(cudaGetLastError());
-  const int BH = B * Hq;
-  launch_pdl(decode_merge_kernel, dim3((BH * 32 + 255) / 256), dim3(256), 0, s, (const float*)part_o, (const float*)part_ml, p.out, BH, p.n_chunks, D);
-  return int(cudaGetLastError());
+  return decode_attn(p, min(max_tokens + 1, max_len), static_cast<cudaStream_t>(stream));
 }
 
 // The same for a cache that holds the new token's row already (written by the kernel that prepared the queries, or by the layer whose
@@ -931,25 +913,20 @@ ATS_API int ats_decode_attn(const void* qkv, long long ld_qkv, int q_col0, int k
 // dimensions, 1, 2, 4 or 8 query heads per key head; anything else returns 1003.
 ATS_API int ats_decode_attn_cached(const void* q, long long ldq, void* k_cache, void* v_cache, long long cache_b_stride, const int* lengths, int B, int Hq,
                                    int Hkv, int D, int max_len, float scale, float cap, const void* gate, long long ld_gate, float* part_o, float* part_ml,
-                                   int* chunk_done, void* out, long long ld_out, void* stream) {
-  if ((D != 64 && D != 128) || Hkv < 1 || Hq % Hkv || (ldq & 7) || !lengths || !chunk_done || max_len < 1) return 1003;
+                                   void* out, long long ld_out, int* status, void* stream) {
+  if ((D != 64 && D != 128) || Hkv < 1 || Hq % Hkv || (ldq & 7) || !lengths || max_len < 1) return 1003;
   const int rep = Hq / Hkv;
+  if (rep != 1 && rep != 2 && rep != 4 && rep != 8) return 1003;
   DecodeArgs p = {};
   p.q = static_cast<const __nv_bfloat16*>(q); p.ld_qkv = ldq;
   p.k_cache = static_cast<__nv_bfloat16*>(k_cache); p.v_cache = static_cast<__nv_bfloat16*>(v_cache);
   p.cache_b_stride = cache_b_stride; p.lengths = lengths;
   p.B = B; p.Hq = Hq; p.Hkv = Hkv; p.D = D; p.max_len = max_len; p.scale = scale; p.cap = cap;
   p.gate = static_cast<const __nv_bfloat16*>(gate); p.ld_gate = ld_gate;
-  p.part_o = part_o; p.part_ml = part_ml; p.n_chunks = (max_len + DEC_CHUNK - 1) / DEC_CHUNK; p.chunk_done = chunk_done;
+  p.part_o = part_o; p.part_ml = part_ml;
   p.out = static_cast<__nv_bfloat16*>(out); p.ld_out = ld_out;
-  const dim3 grid(p.n_chunks, Hkv, B);
-  cudaStream_t s = static_cast<cudaStream_t>(stream);
-  cudaError_t ce = cudaErrorInvalidValue;
-#define ATS_DEC(DD, RR) if (D == DD && rep == RR) ce = launch_pdl(decode_attn_mma_kernel<DD, RR, 2>, grid, dim3(DEC_THREADS), 0, s, p);
-  ATS_DEC(64, 1) ATS_DEC(64, 2) ATS_DEC(64, 4) ATS_DEC(64, 8) ATS_DEC(128, 1) ATS_DEC(128, 2) ATS_DEC(128, 4) ATS_DEC(128, 8)
-#undef ATS_DEC
-  if (rep != 1 && rep != 2 && rep != 4 && rep != 8) return 1003;
-  return int(ce != cudaSuccess ? ce : cudaGetLastError());
+  p.status = status;
+  return decode_attn(p, max_len, static_cast<cudaStream_t>(stream));
 }
 
 // logits [B, V] (row pitch ld elements; fp32 when logits_fp32 else bf16) -> out [B] int64.  work: [B, V] fp32 scratch;
