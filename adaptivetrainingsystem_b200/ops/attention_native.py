@@ -47,12 +47,17 @@ def layout_ok(t: torch.Tensor) -> bool:
 
 
 # Forward variant: "v1" = one query tile per CTA; "v2s" / "v2t" = two query tiles per CTA with the probabilities staged
-# through shared memory / tensor memory (sequence length must be a multiple of 256, else v1 runs).
+# through shared memory / tensor memory (any sequence length; odd multiples of 128 run v1, which wastes no half of its last tile).
 FWD_VARIANT = os.environ.get("ATS_ATTN_FWD", "v2t")
 # Diagnostics: an int64 CUDA tensor of 16 elements receives per-phase cycle totals of one CTA of the two-tile forward kernel
 # ([0:5] MMA thread: total, wait for V, wait for P, issue, iterations; [8:13] one soft-max warp: wait for S, TMEM load, row
 # maximum, exponentials + store, signalling).
 FWD_PHASE_PROFILE = None
+
+
+def _pitch(t) -> int:
+    """Elements between consecutive tokens (a dimension of one token has no stride of its own: there it is the one between sequences)."""
+    return t.stride(1) if t.shape[1] > 1 else t.stride(0)
 
 
 def _fwd(q, k, v):
@@ -61,13 +66,13 @@ def _fwd(q, k, v):
     out = torch.empty(B, L, Hq, D, dtype=q.dtype, device=q.device)
     lse = torch.empty(B, Hq, L, dtype=torch.float32, device=q.device)
     st = _lib.status_tensor(q.device)
-    if FWD_VARIANT != "v1" and L % 256 == 0:
-        err = _lib_fns().ats_attn_fwd2(_lib.ptr(q), q.stride(1), Hq * D, 0, _lib.ptr(k), k.stride(1), Hkv * D, 0, _lib.ptr(v), v.stride(1),
+    if L % 128 or (FWD_VARIANT != "v1" and L % 256 == 0):
+        err = _lib_fns().ats_attn_fwd2(_lib.ptr(q), _pitch(q), Hq * D, 0, _lib.ptr(k), _pitch(k), Hkv * D, 0, _lib.ptr(v), _pitch(v),
                                        Hkv * D, 0, _lib.ptr(out), _lib.ptr(lse), B, L, Hq, Hkv, D, int(FWD_VARIANT == "v2t"), _lib.ptr(st),
                                        _lib.ptr(FWD_PHASE_PROFILE), _lib.stream_ptr(q.device))
         _lib.check(err, "ats_attn_fwd2")
         return out, lse
-    err = _lib_fns().ats_attn_fwd(_lib.ptr(q), q.stride(1), Hq * D, 0, _lib.ptr(k), k.stride(1), Hkv * D, 0, _lib.ptr(v), v.stride(1),
+    err = _lib_fns().ats_attn_fwd(_lib.ptr(q), _pitch(q), Hq * D, 0, _lib.ptr(k), _pitch(k), Hkv * D, 0, _lib.ptr(v), _pitch(v),
                                   Hkv * D, 0, _lib.ptr(out), _lib.ptr(lse), B, L, Hq, Hkv, D, _lib.ptr(st), _lib.stream_ptr(q.device))
     _lib.check(err, "ats_attn_fwd")
     return out, lse
@@ -83,9 +88,9 @@ def _bwd(q, k, v, out, dout, lse, dq, dk, dv):
     Hkv = k.shape[2]
     delta = torch.empty(B, Hq, L, dtype=torch.float32, device=q.device)
     st = _lib.status_tensor(q.device)
-    err = _lib_fns().ats_attn_bwd(_lib.ptr(q), q.stride(1), Hq * D, 0, _lib.ptr(k), k.stride(1), Hkv * D, 0, _lib.ptr(v), v.stride(1),
+    err = _lib_fns().ats_attn_bwd(_lib.ptr(q), _pitch(q), Hq * D, 0, _lib.ptr(k), _pitch(k), Hkv * D, 0, _lib.ptr(v), _pitch(v),
                                   Hkv * D, 0, _lib.ptr(out), _lib.ptr(dout), _lib.ptr(lse), _lib.ptr(delta), _lib.ptr(dq), _lib.ptr(dk),
-                                  _lib.ptr(dv), dq.stride(1), dk.stride(1), B, L, Hq, Hkv, D, _lib.ptr(st), _lib.ptr(PHASE_PROFILE),
+                                  _lib.ptr(dv), _pitch(dq), _pitch(dk), B, L, Hq, Hkv, D, _lib.ptr(st), _lib.ptr(PHASE_PROFILE),
                                   _lib.stream_ptr(q.device))
     _lib.check(err, "ats_attn_bwd")
 

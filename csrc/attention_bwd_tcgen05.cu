@@ -12,12 +12,16 @@
 // the same bytes serve both as a K-major operand (dS K) and as an MN-major operand (P^T dO, dS^T Q).
 //
 //   warp 0: TMA producer   warp 1: TMEM owner + MMA issuer   warps 2..9: two threads per query row (64 key columns each)
+// Any sequence length: rows behind the end of a sequence read as zero (its length is a dimension of the tensor maps).  Queries there get a
+// log-sum-exp of infinity, so their P and dS vanish; keys there are behind every real query; neither is stored.
 // Every wait is bounded (status word + clean unwind); no load uses cluster multicast.
 //
 // Replaces the flash-attn / SDPA backward the reference relies on (reference core/model.py:763-768).
 #include "common.cuh"
 
 namespace ats {
+
+int make_tmap_batched(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_stride, uint32_t box_rows);
 
 #ifndef ATS_AB_SPLIT
 #define ATS_AB_SPLIT 2
@@ -108,7 +112,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int nq = p.L / 128;
+  const int nq = (p.L + 127) / 128;
   const int rep = p.Hq / p.Hkv;
   // Grid = (heads, batch, tiles): CTAs are handed out x-fastest, so with the tile index slowest every CTA of the heaviest
   // tile (of all heads and sequences) starts before any lighter one.  With the tile index fastest, a heavy tile of the
@@ -175,18 +179,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       // ------------------------------------------------------------------ producer
       mbar_expect_tx(res_full, 2 * SM::TB);
       if (MODE == 0) {
-        const int row = b * p.L + fixed * 128;
+        const int row = fixed * 128;
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
-          tma_load_2d(sR1 + c * 16384, &map_k, res_full, p.k_col0 + hk * D + 64 * c, row);
-          tma_load_2d(sR2 + c * 16384, &map_v, res_full, p.v_col0 + hk * D + 64 * c, row);
+          tma_load_3d(sR1 + c * 16384, &map_k, res_full, p.k_col0 + hk * D + 64 * c, row, b);
+          tma_load_3d(sR2 + c * 16384, &map_v, res_full, p.v_col0 + hk * D + 64 * c, row, b);
         }
       } else {
-        const int row = b * p.L + fixed * 128;
+        const int row = fixed * 128;
 #pragma unroll
         for (int c = 0; c < D / 64; ++c) {
-          tma_load_2d(sR1 + c * 16384, &map_q, res_full, p.q_col0 + head * D + 64 * c, row);
-          tma_load_2d(sR2 + c * 16384, &map_do, res_full, head * D + 64 * c, row);
+          tma_load_3d(sR1 + c * 16384, &map_q, res_full, p.q_col0 + head * D + 64 * c, row, b);
+          tma_load_3d(sR2 + c * 16384, &map_do, res_full, head * D + 64 * c, row, b);
         }
       }
       for (int t = 0; t < n_iter; ++t) {
@@ -196,18 +200,18 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         if (!mbar_wait_bounded(&t_empty[s], ph ^ 1, abort_flag, p.status, kTimeoutEmpty)) break;
         mbar_expect_tx(&t_full[s], 2 * SM::TB);
         if (MODE == 0) {
-          const int row = b * p.L + qi * 128;
+          const int row = qi * 128;
 #pragma unroll
           for (int c = 0; c < D / 64; ++c) {
-            tma_load_2d(sT1 + s * SM::TB + c * 16384, &map_q, &t_full[s], p.q_col0 + h * D + 64 * c, row);
-            tma_load_2d(sT2 + s * SM::TB + c * 16384, &map_do, &t_full[s], h * D + 64 * c, row);
+            tma_load_3d(sT1 + s * SM::TB + c * 16384, &map_q, &t_full[s], p.q_col0 + h * D + 64 * c, row, b);
+            tma_load_3d(sT2 + s * SM::TB + c * 16384, &map_do, &t_full[s], h * D + 64 * c, row, b);
           }
         } else {
-          const int row = b * p.L + kj * 128;
+          const int row = kj * 128;
 #pragma unroll
           for (int c = 0; c < D / 64; ++c) {
-            tma_load_2d(sT1 + s * SM::TB + c * 16384, &map_k, &t_full[s], p.k_col0 + hk * D + 64 * c, row);
-            tma_load_2d(sT2 + s * SM::TB + c * 16384, &map_v, &t_full[s], p.v_col0 + hk * D + 64 * c, row);
+            tma_load_3d(sT1 + s * SM::TB + c * 16384, &map_k, &t_full[s], p.k_col0 + hk * D + 64 * c, row, b);
+            tma_load_3d(sT2 + s * SM::TB + c * 16384, &map_v, &t_full[s], p.v_col0 + hk * D + 64 * c, row, b);
           }
         }
       }
@@ -326,8 +330,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       int h, qi, kj;
       decode(t, h, qi, kj);
       const long long idx = ((long long)b * p.Hq + h) * p.L + qi * 128 + r;
-      l2 = p.lse[idx] * 1.4426950408889634f;
-      d = p.delta[idx];
+      const bool real = qi * 128 + r < p.L;
+      l2 = real ? p.lse[idx] * 1.4426950408889634f : INFINITY;
+      d = real ? p.delta[idx] : 0.f;
     };
     float lse2 = 0.f, dl = 0.f, lse2_n = 0.f, dl_n = 0.f;
     if (n_iter > 0) row_stats(0, lse2_n, dl_n);
@@ -412,6 +417,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     }
     if (ok && mbar_wait_bounded(acc_done, 0, abort_flag, p.status, kTimeoutTmemFull)) {
       tc_fence_after();
+      const bool real = fixed * 128 + r < p.L;
       const long long tok = (long long)b * p.L + fixed * 128 + r;
       __nv_bfloat16* o1 = MODE == 0 ? p.dv + tok * p.ld_dkv + head * D : p.dq + tok * p.ld_dq + head * D;
       __nv_bfloat16* o2 = MODE == 0 ? p.dk + tok * p.ld_dkv + head * D : nullptr;
@@ -424,7 +430,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         tmem_ld_wait();
 #pragma unroll
         for (int g = 0; g < 2; ++g)
-          *reinterpret_cast<uint4*>(o1 + c * 16 + g * 8) =
+          if (real) *reinterpret_cast<uint4*>(o1 + c * 16 + g * 8) =
               make_uint4(pack_bf16x2(__uint_as_float(v[8 * g]), __uint_as_float(v[8 * g + 1])), pack_bf16x2(__uint_as_float(v[8 * g + 2]), __uint_as_float(v[8 * g + 3])),
                          pack_bf16x2(__uint_as_float(v[8 * g + 4]), __uint_as_float(v[8 * g + 5])), pack_bf16x2(__uint_as_float(v[8 * g + 6]), __uint_as_float(v[8 * g + 7])));
         if (MODE == 0) {
@@ -432,7 +438,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           tmem_ld_wait();
 #pragma unroll
           for (int g = 0; g < 2; ++g)
-            *reinterpret_cast<uint4*>(o2 + c * 16 + g * 8) =
+            if (real) *reinterpret_cast<uint4*>(o2 + c * 16 + g * 8) =
                 make_uint4(pack_bf16x2(__uint_as_float(v[8 * g]), __uint_as_float(v[8 * g + 1])), pack_bf16x2(__uint_as_float(v[8 * g + 2]), __uint_as_float(v[8 * g + 3])),
                            pack_bf16x2(__uint_as_float(v[8 * g + 4]), __uint_as_float(v[8 * g + 5])), pack_bf16x2(__uint_as_float(v[8 * g + 6]), __uint_as_float(v[8 * g + 7])));
         }
@@ -457,7 +463,7 @@ static int launch_attn_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const C
   using SM = AttnBwdSmem<D, MODE>;
   cudaError_t ce = cudaFuncSetAttribute(attn_bwd_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL);
   if (ce != cudaSuccess) return int(ce);
-  dim3 grid(MODE == 0 ? p.Hkv : p.Hq, p.B, p.L / 128);
+  dim3 grid(MODE == 0 ? p.Hkv : p.Hq, p.B, (p.L + 127) / 128);
   attn_bwd_kernel<D, MODE><<<grid, AB_THREADS, SM::TOTAL, s>>>(mq, mk, mv, mdo, p);
   return int(cudaGetLastError());
 }
@@ -469,7 +475,7 @@ ATS_API int ats_attn_bwd(const void* q, long long ld_q, long long q_cols, int q_
                          long long k_cols, int k_col0, const void* v, long long ld_v, long long v_cols, int v_col0,
                          const void* out, const void* dout, const float* lse, float* delta, void* dq, void* dk, void* dv,
                          long long ld_dq, long long ld_dkv, int B, int L, int Hq, int Hkv, int D, int* status, long long* prof, void* stream) {
-  if ((D != 64 && D != 128) || (L % 128) || Hq % Hkv || (q_col0 & 7) || (k_col0 & 7) || (v_col0 & 7) || (ld_dq & 7) || (ld_dkv & 7))
+  if ((D != 64 && D != 128) || L < 1 || Hq % Hkv || (q_col0 & 7) || (k_col0 & 7) || (v_col0 & 7) || (ld_dq & 7) || (ld_dkv & 7))
     return 1003;
   static thread_local bool ctx_bound = false;
   if (!ctx_bound) {
@@ -479,11 +485,11 @@ ATS_API int ats_attn_bwd(const void* q, long long ld_q, long long q_cols, int q_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   CUtensorMap mq, mk, mv, mdo;
   int e;
-  const unsigned long long rows = (unsigned long long)B * L;
-  if ((e = make_tmap_2d(&mq, q, rows, q_cols, ld_q, 2, 64, 128))) return e;
-  if ((e = make_tmap_2d(&mk, k, rows, k_cols, ld_k, 2, 64, 128))) return e;
-  if ((e = make_tmap_2d(&mv, v, rows, v_cols, ld_v, 2, 64, 128))) return e;
-  if ((e = make_tmap_2d(&mdo, dout, rows, (unsigned long long)Hq * D, (unsigned long long)Hq * D, 2, 64, 128))) return e;
+  const unsigned long long n = L, od = (unsigned long long)Hq * D;
+  if ((e = make_tmap_batched(&mq, q, q_cols, n, B, ld_q, n * ld_q, 128))) return e;
+  if ((e = make_tmap_batched(&mk, k, k_cols, n, B, ld_k, n * ld_k, 128))) return e;
+  if ((e = make_tmap_batched(&mv, v, v_cols, n, B, ld_v, n * ld_v, 128))) return e;
+  if ((e = make_tmap_batched(&mdo, dout, od, n, B, od, n * od, 128))) return e;
   const long long delta_threads = (long long)B * L * Hq * (D / 8);
   attn_delta_kernel<<<unsigned((delta_threads + 255) / 256), 256, 0, s>>>(static_cast<const __nv_bfloat16*>(dout),
                                                                       static_cast<const __nv_bfloat16*>(out), delta, B, L, Hq, D);

@@ -16,11 +16,15 @@
 //
 // PT = true keeps P in tensor memory (bf16 pairs written over the first 64 columns of the S tile, read by the MMA as
 // its A operand); PT = false stages P through shared memory in the 128-byte-swizzled K-major layout.
+// Any sequence length: the tensor maps have the sequence as a dimension of its own, so rows behind its end read as zero (never as
+// the next sequence's); the causal mask hides such keys from every real query, and such queries are not stored.
 // Every wait is bounded (status word + clean unwind); no load uses cluster multicast.
 // Replaces flash_attn_func of the reference model (reference core/model.py:763-768) without expanding K / V per query head.
 #include "common.cuh"
 
 namespace ats {
+
+int make_tmap_batched(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_stride, uint32_t box_rows);
 
 // max of three floats in one instruction (sm_100: max.f32 with three sources)
 __device__ __forceinline__ float max3f(float a, float b, float c) {
@@ -109,7 +113,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const int h = blockIdx.x, b = blockIdx.y;
   const int hk = h / (p.Hq / p.Hkv);
   const int nbA = 2 * t + 1, nbB = 2 * t + 2;  // key blocks seen by tile A / tile B
-  const int row0 = b * p.L + t * 256;
+  const int row0 = t * 256;   // of the sequence
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -149,18 +153,18 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 #pragma unroll
       for (int x = 0; x < 2; ++x)
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_2d(sQ + x * TB + c * 16384, &map_q, q_full, p.q_col0 + h * D + 64 * c, row0 + x * 128);
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sQ + x * TB + c * 16384, &map_q, q_full, p.q_col0 + h * D + 64 * c, row0 + x * 128, b);
       for (int j = 0; j < nbB; ++j) {
-        const int krow = b * p.L + j * 128;
+        const int krow = j * 128;
         const int sk = j % KST, sv = j % VST;
         if (!mbar_wait_bounded(&k_empty[sk], ((j / KST) & 1) ^ 1, abort_flag, p.status, kTimeoutEmpty)) break;
         mbar_expect_tx(&k_full[sk], TB);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_2d(sK + sk * TB + c * 16384, &map_k, &k_full[sk], p.k_col0 + hk * D + 64 * c, krow);
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sK + sk * TB + c * 16384, &map_k, &k_full[sk], p.k_col0 + hk * D + 64 * c, krow, b);
         if (!mbar_wait_bounded(&v_empty[sv], ((j / VST) & 1) ^ 1, abort_flag, p.status, kTimeoutEmpty)) break;
         mbar_expect_tx(&v_full[sv], TB);
 #pragma unroll
-        for (int c = 0; c < D / 64; ++c) tma_load_2d(sV + sv * TB + c * 16384, &map_v, &v_full[sv], p.v_col0 + hk * D + 64 * c, krow);
+        for (int c = 0; c < D / 64; ++c) tma_load_3d(sV + sv * TB + c * 16384, &map_v, &v_full[sv], p.v_col0 + hk * D + 64 * c, krow, b);
       }
       if (*abort_flag) {  // give copies already in flight time to land before the CTA exits
         const uint64_t t0 = globaltimer_ns();
@@ -406,13 +410,15 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                      : mbar_wait_bounded(&o_done[x], 0, abort_flag, p.status, kTimeoutTmemFull))) {
       tc_fence_after();
       const float inv = 1.f / l;
-      const long long tok = (long long)row0 + x * 128 + r;
+      const bool real = row0 + x * 128 + r < p.L;
+      const long long tok = (long long)b * p.L + row0 + x * 128 + r;
       __nv_bfloat16* orow = p.out + (tok * p.Hq + h) * D;
 #pragma unroll
       for (int c = 0; c < D / 32; ++c) {
         uint32_t o[32];
         tmem_ld_32x32(tmem_O + c * 32, o);
         tmem_ld_wait();
+        if (!real) continue;
 #pragma unroll
         for (int g = 0; g < 4; ++g)
           *reinterpret_cast<uint4*>(orow + c * 32 + g * 8) =
@@ -421,7 +427,7 @@ attn_fwd2_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
                          pack_bf16x2(__uint_as_float(o[8 * g + 4]) * inv, __uint_as_float(o[8 * g + 5]) * inv),
                          pack_bf16x2(__uint_as_float(o[8 * g + 6]) * inv, __uint_as_float(o[8 * g + 7]) * inv));
       }
-      if (p.lse) p.lse[((long long)b * p.Hq + h) * p.L + (long long)qt * 128 + r] = (m + log2f(l)) * 0.6931471805599453f;
+      if (p.lse && real) p.lse[((long long)b * p.Hq + h) * p.L + (long long)qt * 128 + r] = (m + log2f(l)) * 0.6931471805599453f;
     }
   }
   tc_fence_before();
@@ -444,7 +450,7 @@ static int launch_fwd2_impl(const CUtensorMap& mq, const CUtensorMap& mk, const 
   using SM = Attn2Smem<D, PT>;
   cudaError_t ce = cudaFuncSetAttribute(attn_fwd2_kernel<D, PT, PROF, POLY>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL);
   if (ce != cudaSuccess) return int(ce);
-  dim3 grid(Hq, B, L / 256);
+  dim3 grid(Hq, B, (L + 255) / 256);
   attn_fwd2_kernel<D, PT, PROF, POLY><<<grid, A2_THREADS, SM::TOTAL, s>>>(mq, mk, mv, p);
   return int(cudaGetLastError());
 }
@@ -466,12 +472,12 @@ ATS_API int ats_attn_fwd2_set_poly(int every) {
   return 0;
 }
 
-// Same contract as ats_attn_fwd, for L a multiple of 256.  p_in_tmem selects where the probabilities are staged.
+// Same contract as ats_attn_fwd, for any L.  p_in_tmem selects where the probabilities are staged.
 // prof: null, or 16 int64 that receive per-phase cycle totals of CTA (0,0,0) (diagnostics).
 ATS_API int ats_attn_fwd2(const void* q, long long ld_q, long long q_cols, int q_col0, const void* k, long long ld_k,
                           long long k_cols, int k_col0, const void* v, long long ld_v, long long v_cols, int v_col0,
                           void* out, float* lse, int B, int L, int Hq, int Hkv, int D, int p_in_tmem, int* status, long long* prof, void* stream) {
-  if ((D != 64 && D != 128) || (L % 256) || Hq % Hkv || (q_col0 & 7) || (k_col0 & 7) || (v_col0 & 7)) return 1003;
+  if ((D != 64 && D != 128) || L < 1 || Hq % Hkv || (q_col0 & 7) || (k_col0 & 7) || (v_col0 & 7)) return 1003;
   static thread_local bool ctx_bound = false;
   if (!ctx_bound) {
     cudaFree(0);
@@ -479,10 +485,9 @@ ATS_API int ats_attn_fwd2(const void* q, long long ld_q, long long q_cols, int q
   }
   CUtensorMap mq, mk, mv;
   int e;
-  const unsigned long long rows = (unsigned long long)B * L;
-  if ((e = make_tmap_2d(&mq, q, rows, q_cols, ld_q, 2, 64, 128))) return e;
-  if ((e = make_tmap_2d(&mk, k, rows, k_cols, ld_k, 2, 64, 128))) return e;
-  if ((e = make_tmap_2d(&mv, v, rows, v_cols, ld_v, 2, 64, 128))) return e;
+  if ((e = make_tmap_batched(&mq, q, q_cols, L, B, ld_q, (unsigned long long)L * ld_q, 128))) return e;
+  if ((e = make_tmap_batched(&mk, k, k_cols, L, B, ld_k, (unsigned long long)L * ld_k, 128))) return e;
+  if ((e = make_tmap_batched(&mv, v, v_cols, L, B, ld_v, (unsigned long long)L * ld_v, 128))) return e;
   Attn2Args p;
   p.B = B; p.L = L; p.Hq = Hq; p.Hkv = Hkv;
   p.q_col0 = q_col0; p.k_col0 = k_col0; p.v_col0 = v_col0;

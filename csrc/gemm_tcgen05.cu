@@ -1089,18 +1089,19 @@ int make_tmap_heads(CUtensorMap* out, const void* base, uint64_t rows, uint64_t 
   return r == CUDA_SUCCESS ? 0 : 1100 + int(r);
 }
 
-// bf16 [batch, rows, cols] with a pitch of its own between the batch entries (elements); box = 64 columns x box_rows rows of one entry, 128-byte
-// swizzle; rows outside read as zero.
-int make_tmap_cache(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t batch_stride, uint32_t box_rows) {
+// bf16 [batch, rows, cols], rows ld and batch entries batch_stride elements apart; box = 64 columns x box_rows rows of one entry, 128-byte
+// swizzle; rows beyond `rows` read as zero, not as the next entry's.
+int make_tmap_batched(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_stride, uint32_t box_rows) {
   EncodeTiledFn enc = get_encode_tiled();
   if (!enc) return 1000;
-  if ((reinterpret_cast<uintptr_t>(base) & 15) || (cols & 7) || (batch_stride & 7)) return 1001;
+  if ((reinterpret_cast<uintptr_t>(base) & 15) || (ld & 7) || (batch_stride & 7)) return 1001;
   cuuint64_t dims[3] = {cols, rows, batch};
-  cuuint64_t strides[2] = {cols * 2, batch_stride * 2};
+  cuuint64_t strides[2] = {ld * 2, batch_stride * 2};
   cuuint32_t box[3] = {64, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   CU_TENSOR_MAP_SWIZZLE_128B, box_rows < 128 ? CU_TENSOR_MAP_L2_PROMOTION_L2_128B : CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : 1100 + int(r);
 }
 

@@ -16,7 +16,7 @@
 
 namespace ats {
 
-int make_tmap_cache(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t batch_stride, uint32_t box_rows);
+int make_tmap_batched(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_stride, uint32_t box_rows);
 
 constexpr int DEC_WARPS = 4;
 constexpr int DEC_THREADS = 32 * DEC_WARPS;
@@ -845,7 +845,8 @@ static int decode_attn(DecodeArgs& p, int tokens, cudaStream_t s) {
   CUtensorMap mk, mv;
   const unsigned long long ld = (unsigned long long)p.Hkv * p.D, bs = p.B > 1 ? p.cache_b_stride : ld * p.max_len;
   int e;
-  if ((e = make_tmap_cache(&mk, p.k_cache, ld, p.max_len, p.B, bs, 2048 / p.D)) || (e = make_tmap_cache(&mv, p.v_cache, ld, p.max_len, p.B, bs, 2048 / p.D))) return e;
+  if ((e = make_tmap_batched(&mk, p.k_cache, ld, p.max_len, p.B, ld, bs, 2048 / p.D))) return e;
+  if ((e = make_tmap_batched(&mv, p.v_cache, ld, p.max_len, p.B, ld, bs, 2048 / p.D))) return e;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(cluster * p.parts, p.Hkv, p.B);
   cfg.blockDim = dim3(DEC_THREADS);
