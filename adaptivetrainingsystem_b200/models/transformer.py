@@ -148,7 +148,7 @@ class GroupedQueryAttention(nn.Module):
 
     def forward(self, h: torch.Tensor, residual: torch.Tensor, rope: RotaryEmbedding,
                 attention_mask: Optional[torch.Tensor] = None, cache: Optional[KVCache] = None,
-                positions: Optional[torch.Tensor] = None, post_norm: Optional["RMSNorm"] = None):
+                positions: Optional[torch.Tensor] = None, post_norm: Optional["RMSNorm"] = None, scaled: bool = False):
         """-> x (= attention output projected + residual).  With ``post_norm`` (graph-replayed decode steps only) -> (x, h) where
         h = post_norm(x) came out of the launch that folded the output projection, or ``None`` when that form did not apply."""
         B, L, _ = h.shape
@@ -168,7 +168,7 @@ class GroupedQueryAttention(nn.Module):
                 qkv = ops.rope_packed(qkv, rope.cos, rope.sin, self.n_q, self.n_kv, self.d, positions=cache.device_positions.view(B, 1))
             a = ops.decode_attention(qkv, cache.k[self.layer_idx], cache.v[self.layer_idx], cache.device_lengths, self.n_q, self.n_kv, self.d)
             if post_norm is not None and self.tp_group is None:  # the fold of the output projection adds the residual and normalises
-                fused = ops.serving.out_proj_norm(a.reshape(B, -1), self.o_proj, residual.reshape(B, -1), post_norm.weight, post_norm.eps)
+                fused = ops.serving.out_proj_norm(a.reshape(B, -1), self.o_proj, residual.reshape(B, -1), post_norm.weight, post_norm.eps, scaled)
                 if fused is not None:
                     return fused[0].view(residual.shape), fused[1].view(residual.shape)
             x = self._project_out(a, residual)
@@ -458,15 +458,23 @@ class TransformerBlock(nn.Module):
             aux = x.new_zeros((), dtype=torch.float32)
         return x, aux
 
-    def decode_step(self, x, rope, cache, h_pre=None, next_norm=None):
+    def takes_scaled_rows(self, rope, cache) -> bool:
+        """Whether this block's projection divides by the norm of its input itself (``ops.serving.ScaledRows``)."""
+        a = self.self_attn
+        return a.tp_group is None and ops.serving.takes_rotated(cache.batch, a.qkv_proj, a.n_q, a.n_kv, a.d, rope.cos, cache.device_positions)
+
+    def decode_step(self, x, rope, cache, h_pre=None, next_norm=None, next_scaled=False):
         """One graph-replayed decode step of this block with the norms folded into their producers: ``h_pre`` is this block's
         normalised input when the block before already produced it, ``next_norm`` = (weight, eps) of the norm that follows this
-        block.  -> (x, normalised x for the next block or None)."""
+        block (``next_scaled``: what follows takes ``ops.serving.ScaledRows``).  -> (x, normalised x for the next block or None)."""
         if h_pre is None:
             h, x = self.input_norm.with_skip(x)
         else:
             h = h_pre
-        res = self.self_attn(h, x, rope, None, cache, None, post_norm=self.post_attn_norm)
+        rows = x.numel() // x.shape[-1]
+        scaled = (self.ffn_kind == "dense" and next_norm is not None and self.ffn.tp_group is None and next_norm[0].dtype == torch.bfloat16
+                  and ops.serving.takes_scaled(rows, self.ffn.gate_up_proj, self.ffn.gate_up_proj.shape[0] // 2) and ops.serving.takes_scaled(rows, self.ffn.down_proj))
+        res = self.self_attn(h, x, rope, None, cache, None, post_norm=self.post_attn_norm, scaled=scaled)
         x, h = res if isinstance(res, tuple) else (res, None)
         if h is None:
             h, x = self.post_attn_norm.with_skip(x)
@@ -480,7 +488,7 @@ class TransformerBlock(nn.Module):
         else:
             fused = None
             if next_norm is not None and self.ffn.tp_group is None:
-                fused = ops.serving.mlp_norm(h.reshape(-1, h.shape[-1]), self.ffn.gate_up_proj, self.ffn.down_proj, x.reshape(-1, x.shape[-1]), *next_norm)
+                fused = ops.serving.mlp_norm(h.reshape(-1, h.shape[-1]), self.ffn.gate_up_proj, self.ffn.down_proj, x.reshape(-1, x.shape[-1]), *next_norm, scaled=next_scaled)
             if fused is not None:
                 return fused[0].view(x.shape), fused[1].view(x.shape)
             x, _ = self.ffn(h, x)
@@ -570,9 +578,11 @@ class DeepSeekTransformer(nn.Module):
             # graph-replayed decode step: every norm that can ride on the launch before it does (no auxiliary losses while serving)
             h_pre = None
             n = len(self.layers)
+            self.rope.ensure(cache.max_len, x.device)
             for i, blk in enumerate(self.layers):
                 nxt = self.layers[i + 1].input_norm if i + 1 < n else self.norm
-                x, h_pre = blk.decode_step(x, self.rope, cache, h_pre, (nxt.weight, nxt.eps))
+                scaled = i + 1 < n and self.layers[i + 1].takes_scaled_rows(self.rope, cache)
+                x, h_pre = blk.decode_step(x, self.rope, cache, h_pre, (nxt.weight, nxt.eps), scaled)
             return (h_pre if h_pre is not None else self.norm(x)), aux_losses
         for blk in self.layers:
             x, aux = blk(x, self.rope, attention_mask, cache, positions, decode)

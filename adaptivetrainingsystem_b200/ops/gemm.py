@@ -27,7 +27,8 @@ _configured = False
 class _Skinny(ctypes.Structure):   # csrc/skinny.cuh
     _fields_ = [("T", _c_int), ("N", _c_int), ("K", _c_int), ("mode", _c_int), ("up_offset", _c_int), ("act_cols", _c_int), ("head_dim", _c_int), ("alpha", _c_f), ("a1", _c_f), ("a2", _c_f),
                 ("ldx", _c_int), ("out", _vp), ("ldo", _c_ll), ("add", _vp), ("ldadd", _c_ll), ("bias", _vp), ("x", _vp), ("w1", _vp), ("b1", _vp), ("w2", _vp),
-                ("b2", _vp), ("pos", _vp), ("status", _vp)]
+                ("b2", _vp), ("pos", _vp), ("next_w", _vp), ("next_out", _vp), ("next_parts", _vp), ("scale_parts", _vp), ("scale_n", _c_int), ("scale_inv", _c_f),
+                ("scale_eps", _c_f), ("status", _vp)]
 
 
 def _fn():
@@ -168,9 +169,10 @@ def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:
 
 def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Optional[int] = None, splits: Optional[int] = None, add: Optional[torch.Tensor] = None,
            alpha: float = 1.0, up_offset: int = 0, act_cols: int = 0, bias: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None, chain=None,
-           head_dim: int = 0, pos: Optional[torch.Tensor] = None) -> None:
+           head_dim: int = 0, pos: Optional[torch.Tensor] = None, next_norm=None, scale=None) -> None:
     """One launch of the decode kernel; ``chain`` = (w1, b1, a1, w2, b2, a2) of the residual step ``SK_DYT``; for ``SK_ROPE``
-    w1 and w2 are the cosine and sine tables, ``pos`` the positions (int32) and ``act_cols`` the rotated columns."""
+    w1 and w2 are the cosine and sine tables, ``pos`` the positions (int32) and ``act_cols`` the rotated columns.  ``next_norm`` = (weight, rows
+    [T, N], sums of squares [T, tiles of 128]) of an RMSNorm that follows ``SK_STORE``; ``scale`` = (sums of squares, eps): ``a`` came from such a product."""
     _fn()
     a, w = _check2d(a), _check2d(w)
     (T, K), N = a.shape, w.shape[0] if n is None else n
@@ -181,8 +183,8 @@ def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Op
     def at(t):
         return None if t is None else t.data_ptr()
     args = _Skinny(T, N, K, mode, up_offset, act_cols, head_dim, alpha, a1, a2, 0 if x is None else x.stride(0), at(out), out.stride(-2), at(add), 0 if add is None else add.stride(0),
-                   at(bias), at(x), at(w1), at(b1), at(w2), at(b2), at(pos),
-                   at(_lib.status_tensor(a.device)))
+                   at(bias), at(x), at(w1), at(b1), at(w2), at(b2), at(pos), *(map(at, next_norm) if next_norm is not None else (None,) * 3),
+                   *((at(scale[0]), scale[0].shape[1], 1.0 / K, scale[1]) if scale is not None else (None, 0, 0.0, 0.0)), at(_lib.status_tensor(a.device)))
     _lib.check(_lib.cuda_lib().ats_gemm_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), w.shape[0], ctypes.byref(args), splits, _lib.stream_ptr(a.device)),
                "ats_gemm_skinny")
 

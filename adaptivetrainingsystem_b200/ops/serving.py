@@ -60,6 +60,29 @@ FUSE_DECODE = __import__("os").environ.get("ATS_DECODE_FUSED", "1") == "1"
 DECODE_KERNEL = "decode kernel"
 
 
+class ScaledRows:
+    """RMSNorm(x) * w of a decode step's rows before the division: ``rows`` = x * w [T, N] (bf16) and ``parts`` [T, tiles], the sums of squares of x per
+    128 columns.  The decode product that reads the rows multiplies its sums by 1 / rms, so the norm costs no launch."""
+
+    def __init__(self, rows: torch.Tensor, parts: torch.Tensor, eps: float, shape):
+        self.rows, self.parts, self.eps, self.shape, self.device = rows, parts, eps, shape, rows.device
+
+    def reshape(self, *_):
+        return self
+
+    def view(self, shape):
+        self.shape = shape
+        return self
+
+
+def takes_scaled(rows: int, w: torch.Tensor, n: Optional[int] = None) -> bool:
+    """Whether the product of ``rows`` rows with w [N, K] (``n`` of its outputs where they are pairs) runs on the decode kernel in a form that scales its sums."""
+    from . import fp8, gemm as G, int4, int8
+    return (FUSE_DECODE and w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and not getattr(w, "_ats_z3", None)
+            and not (fp8.enabled() or int8.enabled()) and not (int4.enabled() and int4.lookup(w) is not None) and not (int4.observing() or int8.observing())
+            and _lib.use_cuda_kernels(w) and w.shape[1] % 8 == 0 and G.skinny_ok(w[:1].expand(rows, -1), w, n))
+
+
 def _partial_products(x2: torch.Tensor, w: torch.Tensor):
     """fp32 partial products [splits, T, N] of x2 [T, K] @ w [N, K]^T over slices of the reduction, ``None`` when this shape
     does not split (the caller then uses the ordinary product), or ``DECODE_KERNEL`` for the shapes whose kernel sums its slices itself."""
@@ -88,28 +111,37 @@ def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torc
              d: int) -> Optional[torch.Tensor]:
     """Packed projection of the new tokens with q and k rotated at ``positions`` [T] (int32): one product + one fold launch.
     ``None`` when the fused form does not apply."""
+    rows, scale = (h2.rows, (h2.parts, h2.eps)) if isinstance(h2, ScaledRows) else (h2, None)
+    if scale is not None and not takes_rotated(rows.shape[0], w_qkv, n_q, n_kv, d, cos, positions):
+        raise RuntimeError("scaled rows reached a projection that does not take them")
     if d % 16 or positions is None or positions.dtype != torch.int32 or cos.dtype != torch.float32 or w_qkv.shape[0] != (n_q + 2 * n_kv) * d:
         return None
-    part = _partial_products(h2, w_qkv)
+    part = _partial_products(rows, w_qkv)
     if part is None:
         return None
-    T, N = h2.shape[0], w_qkv.shape[0]
-    out = torch.empty(T, N, dtype=h2.dtype, device=h2.device)
+    T, N = rows.shape[0], w_qkv.shape[0]
+    out = torch.empty(T, N, dtype=rows.dtype, device=rows.device)
     if part is DECODE_KERNEL:
         from . import gemm as G
         if 128 % d == 0:   # whole heads in a tile of the product: it rotates them itself
-            G.skinny(h2, w_qkv, out, G.SK_ROPE, act_cols=(n_q + n_kv) * d, chain=(cos, None, 0.0, sin, None, 0.0), head_dim=d, pos=positions)
+            G.skinny(rows, w_qkv, out, G.SK_ROPE, act_cols=(n_q + n_kv) * d, chain=(cos, None, 0.0, sin, None, 0.0), head_dim=d, pos=positions, scale=scale)
             return out
-        part = G.skinny_partials(h2, w_qkv)
+        part = G.skinny_partials(rows, w_qkv)
     err = _fns().ats_fold_rope(_lib.ptr(part), part.shape[0], _lib.ptr(out), _lib.ptr(cos), _lib.ptr(sin), _lib.ptr(positions), T, N, n_q, n_kv, d,
-                               _lib.stream_ptr(h2.device))
+                               _lib.stream_ptr(rows.device))
     _lib.check(err, "ats_fold_rope")
     return out
 
 
-def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float):
+def takes_rotated(rows: int, w_qkv: torch.Tensor, n_q: int, n_kv: int, d: int, cos: torch.Tensor, positions: Optional[torch.Tensor]) -> bool:
+    """Whether :func:`qkv_rope` takes :class:`ScaledRows` for this projection."""
+    return (d % 16 == 0 and 128 % d == 0 and positions is not None and positions.dtype == torch.int32 and cos.dtype == torch.float32
+            and w_qkv.shape[0] == (n_q + 2 * n_kv) * d and takes_scaled(rows, w_qkv))
+
+
+def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float, scaled: bool = False):
     """x = a2 @ w_o^T + residual2 and h = RMSNorm(x) * norm_w from one product + one fold or norm launch -> (x, h), or
-    ``None``."""
+    ``None``.  ``scaled``: the consumer of h takes :class:`ScaledRows`, and the norm needs no launch."""
     if norm_w.dtype != torch.bfloat16 or residual2 is None or not residual2.is_contiguous():
         return None
     part = _partial_products(a2, w_o)
@@ -118,6 +150,12 @@ def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, 
     if part is DECODE_KERNEL:
         from . import gemm as G
         from .functional import rms_norm
+        if scaled and w_o.shape[0] % 2 == 0:
+            T, N = a2.shape[0], w_o.shape[0]
+            x, rows = (torch.empty(T, N, dtype=a2.dtype, device=a2.device) for _ in range(2))
+            parts = torch.empty(T, (N + 127) // 128, dtype=torch.float32, device=a2.device)
+            G.skinny(a2, w_o, x, G.SK_STORE, add=residual2, next_norm=(norm_w, rows, parts))
+            return x, ScaledRows(rows, parts, float(eps), x.shape)
         x = G.gemm_nt(a2, w_o, add=residual2)
         return x, rms_norm(x, norm_w, eps)
     T, H = a2.shape[0], w_o.shape[0]
@@ -129,14 +167,25 @@ def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, 
     return x, h
 
 
-def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float):
+def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, residual2: torch.Tensor, norm_w: torch.Tensor, eps: float,
+             scaled: bool = False):
     """SwiGLU feed-forward of a decode step whose down projection adds the residual, and the norm in front of the next block -> (x, h), or
     ``None`` (8-bit or 4-bit copies of the weights, gathered weights, more than a decode step's rows)."""
     from . import fp8, gemm as G, int4, int8
+    if isinstance(h2, ScaledRows):   # (the caller has asked takes_scaled)
+        inter = w_gate_up.shape[0] // 2
+        act = torch.empty(h2.rows.shape[0], inter, dtype=h2.rows.dtype, device=h2.rows.device)
+        G.skinny(h2.rows, w_gate_up, act, G.SK_SWIGLU, n=inter, up_offset=inter, scale=(h2.parts, h2.eps))
+        fused = out_proj_norm(act, w_down, residual2, norm_w, eps, scaled)
+        if fused is None:
+            from .functional import rms_norm
+            x = G.gemm_nt(act, w_down, add=residual2)
+            fused = x, rms_norm(x, norm_w, eps)
+        return fused
     if (fp8.enabled() or int8.enabled() or (int4.enabled() and int4.lookup(w_gate_up) is not None) or getattr(w_gate_up, "_ats_z3", None)
             or not _lib.use_cuda_kernels(h2) or w_gate_up.dtype != torch.bfloat16 or not G.skinny_ok(h2, w_down) or not FUSE_DECODE or norm_w.dtype != torch.bfloat16 or not residual2.is_contiguous()):
         return None
-    return out_proj_norm(G.gemm_nt_swiglu(h2, w_gate_up), w_down, residual2, norm_w, eps)
+    return out_proj_norm(G.gemm_nt_swiglu(h2, w_gate_up), w_down, residual2, norm_w, eps, scaled)
 
 
 def decode_attention_available(qkv: torch.Tensor, n_q: int, n_kv: int, d: int) -> bool:

@@ -15,6 +15,10 @@
 // 64 rows 15.2 -> 9.8; 11264 x 2048 21.0 -> 11.9 / 21.4 -> 16.0; 2048 x 5632 17.1 -> 9.0 / 17.2 -> 12.2; 28672 x 4096 55 -> 40 / 47.6 -> 45.7.
 // What is left is start-up (a launch of 1024 x 1024 takes 4.8 us) and, with 64 rows, the exchange of the slices (2 to 3 us).
 //
+// An RMSNorm between two products needs no launch either (skinny.cuh): the first product writes its rows times the norm's weight and their
+// sums of squares per tile, the second one scales its sums.  With it and the residual read under the product, one decode step of eight
+// 2048-wide layers: one sequence 331 -> 312 us, 64 sequences 626 -> 581 us.
+//
 // In a chain of launches (common.cuh) the first ring of weight tiles is requested before the kernel waits for its predecessor.
 #include "skinny.cuh"
 #include "typed.cuh"
@@ -34,6 +38,7 @@ constexpr int SK_ROWS = 128;      // weight rows of a tile
 constexpr int SK_BK = 64;         // reduction elements of a stage
 constexpr int SK_THREADS = 192;   // TMA warp, MMA warp, four epilogue warps
 constexpr int SK_MAX_SPLIT = 8;   // portable cluster size
+constexpr int SK_TOKENS = 144;    // 128 and the padding of the owners' shares
 
 __host__ __device__ constexpr int sk_stage_bytes(int nt) { return SK_ROWS * 128 + nt * 128; }
 // Ring depth: two CTAs per SM up to 64 tokens (2 x (ring + reduction buffer) <= 227 KB), one beyond.
@@ -50,16 +55,19 @@ __device__ __forceinline__ void st_cluster_v4(uint32_t addr, const uint32_t (&v)
 }
 
 // Four tokens of weight row `n` leave as bf16, two neighbouring rows in one word: even lanes write tokens 0 and 2, odd lanes 1 and 3 of the pair.
-__device__ __forceinline__ void sk_store4(const SkinnyArgs& p, int t, int n, const float (&v)[4], bool row_ok) {
-  __nv_bfloat16* out = static_cast<__nv_bfloat16*>(p.out);
+__device__ __forceinline__ void sk_store4(__nv_bfloat16* out, long long ldo, int T, int t, int n, const float (&v)[4], bool row_ok) {
   const int odd = threadIdx.x & 1;
 #pragma unroll
   for (int e = 0; e < 4; e += 2) {
     const float give = odd ? v[e] : v[e + 1];
     const float got = __shfl_xor_sync(0xffffffffu, give, 1);
     const int tt = t + e + odd;
-    if (row_ok && tt < p.T) *reinterpret_cast<uint32_t*>(out + (long long)tt * p.ldo + (n - odd)) = odd ? pack_bf16x2(got, v[e + 1]) : pack_bf16x2(v[e], got);
+    if (row_ok && tt < T) *reinterpret_cast<uint32_t*>(out + (long long)tt * ldo + (n - odd)) = odd ? pack_bf16x2(got, v[e + 1]) : pack_bf16x2(v[e], got);
   }
+}
+
+__device__ __forceinline__ void sk_store4(const SkinnyArgs& p, int t, int n, const float (&v)[4], bool row_ok) {
+  sk_store4(static_cast<__nv_bfloat16*>(p.out), p.ldo, p.T, t, n, v, row_ok);
 }
 
 // The element-wise steps that need no other row: one weight row n, four tokens at a time (the whole warp calls).
@@ -70,23 +78,26 @@ struct RowStep {
   const int n;
   const bool row_ok;
   bool act = false;
-  float bias = 0.f, w1 = 0.f, b1 = 0.f, w2 = 0.f, b2 = 0.f;
+  float bias = 0.f, w1 = 0.f, b1 = 0.f, w2 = 0.f, b2 = 0.f, next_w = 0.f;
   __device__ __forceinline__ RowStep(const SkinnyArgs& args, int row) : p(args), n(row), row_ok(row < args.N) {
     if (MODE == kSkSilu) act = n < p.act_cols;
     if (row_ok && (kDyt_ || MODE == kSkGelu) && p.bias) bias = p.bias[n];
     if (row_ok && kDyt_) w1 = p.w1[n], b1 = p.b1[n], w2 = p.w2[n], b2 = p.b2[n];
+    if (row_ok && MODE == kSkStore && p.next_out) next_w = __bfloat162float(p.next_w[n]);
   }
+  // Clamped, not guarded: guarded loads are waited for one by one (with one slice and 64 tokens that took 12 us).
   __device__ __forceinline__ void residual(int t, float (&r)[4]) const {
+    const int nn = min(n, p.N - 1);
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
+      const long long tt = min(t + e, p.T - 1);
       r[e] = 0.f;
-      if (row_ok && t + e < p.T) {
-        if (MODE == kSkStore && p.add) r[e] = __bfloat162float(p.add[(long long)(t + e) * p.ldadd + n]);
-        if (kDyt_) r[e] = p.x[(long long)(t + e) * p.ldx + n];
-      }
+      if (MODE == kSkStore && p.add) r[e] = __bfloat162float(p.add[tt * p.ldadd + nn]);
+      if (kDyt_) r[e] = p.x[tt * p.ldx + nn];
     }
   }
-  __device__ __forceinline__ void finish(int t, float (&v)[4], float (&r)[4]) const {
+  // sq: where this warp leaves the sums of squares of the four tokens (kSkStore with next_out)
+  __device__ __forceinline__ void finish(int t, float (&v)[4], float (&r)[4], float* sq) const {
 #pragma unroll
     for (int e = 0; e < 4; ++e) {
       const bool ok = row_ok && t + e < p.T;
@@ -105,6 +116,16 @@ struct RowStep {
       }
     }
     if (MODE != kSkF32) sk_store4(p, t, n, v, row_ok);
+    if (MODE == kSkStore && p.next_out) {   // (the whole warp works on the same tokens)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float b = row_ok ? __bfloat162float(__float2bfloat16(v[e])) : 0.f;
+        const float s = warp_sum(b * b);
+        if ((threadIdx.x & 31) == 0) sq[e] = s;
+        v[e] = b * next_w;
+      }
+      sk_store4(p.next_out, p.N, p.T, t, n, v, row_ok);
+    }
   }
 };
 
@@ -131,6 +152,9 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
   float* red = reinterpret_cast<float*>(smem + STAGES * STAGE + 256);
+  // in the ring's memory once the product is done with it (shared memory of their own would keep small kernels of a chain off the SM)
+  float* s_scale = reinterpret_cast<float*>(smem);                                                  // factor of a token's sums
+  float(*s_sq)[SK_TOKENS] = reinterpret_cast<float(*)[SK_TOKENS]>(s_scale + SK_TOKENS);             // per epilogue warp and token: sum of squares of its 32 results
 
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -164,6 +188,12 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   // one slice and no partner row: the step is done on the accumulator's registers
   const bool direct = S == 1 && p.mode != kSkPart && p.mode != kSkSwiglu && p.mode != kSkRope;
   if (reduce) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");   // waited for before a peer's memory is written
+  float ahead[8];
+
+  auto sums_of_squares = [&](int from, int to) {   // of this tile's columns, in a fixed order
+    for (int t = from + int(threadIdx.x) - 64; t < to; t += 128)
+      p.next_parts[(long long)t * gridDim.y + blockIdx.y] = (s_sq[0][t] + s_sq[1][t]) + (s_sq[2][t] + s_sq[3][t]);
+  };
 
   if (warp == 0) {
     if (lane == 0) {
@@ -215,9 +245,24 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
   } else {
     const int quad = warp & 3, row = quad * 32 + lane;   // tensor-memory lane = weight row of the tile
     asm volatile("griddepcontrol.wait;" ::: "memory");   // outputs may still be read, and residuals written, by the kernels before
+    float factor = p.alpha;
+    if (p.scale_parts && int(threadIdx.x) - 64 < p.T) {
+      const float* parts = p.scale_parts + (long long)(int(threadIdx.x) - 64) * p.scale_n;
+      float ss = 0.f;
+#pragma unroll 8
+      for (int i = 0; i < p.scale_n; ++i) ss += parts[i];
+      factor *= rsqrtf(ss * p.scale_inv + p.scale_eps);
+    }
+    if (reduce && p.mode == kSkStore && p.add) {   // the residual of the first eight owned tokens travels under the product
+      const int nn = min(n0 + int(threadIdx.x) - 64, p.N - 1);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) ahead[i] = __bfloat162float(p.add[(long long)min(split * per + i, p.T - 1) * p.ldadd + nn]);
+    }
     const bool ok = mbar_wait_bounded(done, 0, abort_flag, p.status, kTimeoutTmemFull);
     tc_fence_after();
     __syncwarp();
+    if (p.mode != kSkPart) s_scale[int(threadIdx.x) - 64] = factor;
+    if (direct) asm volatile("bar.sync 1, 128;" ::: "memory");   // (the other paths meet at a barrier of the CTA before they read it)
     if (reduce) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     const uint32_t mine = smem_u32(red) + uint32_t(split * per * SK_ROWS + row * 4) * 4;
     auto chunk = [&](int c, uint32_t (&v)[16]) {
@@ -238,11 +283,15 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
           for (int i = 0; i < 4; ++i) {
             float f[4];
 #pragma unroll
-            for (int e = 0; e < 4; ++e) f[e] = __uint_as_float(v[4 * i + e]) * p.alpha;
-            if (c * 16 + 4 * i < p.T) step.finish(c * 16 + 4 * i, f, r[i]);
+            for (int e = 0; e < 4; ++e) f[e] = __uint_as_float(v[4 * i + e]) * s_scale[c * 16 + 4 * i + e];
+            if (c * 16 + 4 * i < p.T) step.finish(c * 16 + 4 * i, f, r[i], &s_sq[warp - 2][c * 16 + 4 * i]);
           }
         }
       });
+      if (p.next_out) {
+        asm volatile("bar.sync 1, 128;" ::: "memory");
+        sums_of_squares(0, p.T);
+      }
     } else {
 #pragma unroll 1
       for (int c = 0; ok && c * 16 < p.T; ++c) {
@@ -287,7 +336,7 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
           v[0] += a.x; v[1] += a.y; v[2] += a.z; v[3] += a.w;
         }
 #pragma unroll
-        for (int e = 0; e < 4; ++e) v[e] *= p.alpha;
+        for (int e = 0; e < 4; ++e) v[e] *= s_scale[t0 + 4 * q + e];
       };
       if (swiglu) {
         const int col = i0 & 63;
@@ -328,15 +377,25 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
         const int n = n0 + i0;
         auto finish = [&](auto mode_c) {   // one loop per step: the memory accesses of two groups of tokens overlap
           const RowStep<decltype(mode_c)::value> step(p, n);
+          const bool have = reduce && p.mode == kSkStore && p.add;
 #pragma unroll 2
           for (int q = 0; q < groups; ++q) {
             float v[4], r[4];
-            step.residual(t0 + 4 * q, r);
+            if (have && q < 2) {
+#pragma unroll
+              for (int e = 0; e < 4; ++e) r[e] = q ? ahead[4 + e] : ahead[e];
+            } else {
+              step.residual(t0 + 4 * q, r);
+            }
             sum4(i0, q, v);
-            step.finish(t0 + 4 * q, v, r);
+            step.finish(t0 + 4 * q, v, r, &s_sq[warp - 2][t0 + 4 * q]);
           }
         };
         by_mode(p.mode, finish);
+        if (p.next_out) {
+          asm volatile("bar.sync 1, 128;" ::: "memory");
+          sums_of_squares(t0, min(p.T, t0 + 4 * groups));
+        }
       }
     }
   }
@@ -392,6 +451,7 @@ ATS_API int ats_gemm_skinny(const void* a, long long lda, const void* w, long lo
   // pairs of neighbouring columns are written together
   if (p.mode != kSkPart && p.mode != kSkF32 && ((p.N & 1) || (reinterpret_cast<uintptr_t>(p.out) & 3) || (p.ldo & 1))) return 1003;
   if (p.mode == kSkRope && (p.head_dim < 4 || 128 % p.head_dim || p.N % p.head_dim || p.act_cols % p.head_dim || !p.pos || !p.w1 || !p.w2)) return 1003;
+  if ((p.scale_parts && (p.mode == kSkPart || p.scale_n < 1)) || (p.next_out && (p.mode != kSkStore || !p.next_w || !p.next_parts || (p.N & 1)))) return 1003;
   CUtensorMap mw, ma;
   if (int e = make_tmap_2d(&mw, w, w_rows, p.K, ldw, 2, SK_BK, SK_ROWS / 2)) return e;
   if (int e = make_tmap_2d(&ma, a, p.T, p.K, lda, 2, SK_BK, nt)) return e;
