@@ -204,10 +204,11 @@ _status = {}
 
 def status_tensor(device: torch.device) -> torch.Tensor:
     """One int32 word per device that kernels set when a bounded wait runs out."""
-    key = torch.device(device).index or 0
-    if key not in _status:
-        _status[key] = torch.zeros(4, dtype=torch.int32, device=device)
-    return _status[key]
+    key = (device if isinstance(device, torch.device) else torch.device(device)).index or 0
+    t = _status.get(key)
+    if t is None:
+        t = _status[key] = torch.zeros(4, dtype=torch.int32, device=device)
+    return t
 
 
 def check_status(device=None) -> None:
@@ -244,4 +245,6 @@ def ptr(t: Optional[torch.Tensor]) -> ctypes.c_void_p:
 
 
 def stream_ptr(device=None) -> ctypes.c_void_p:
+    if isinstance(device, torch.device) and device.index is not None:
+        return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device.index))   # without the Stream object: 0.3 us instead of 4
     return ctypes.c_void_p(torch.cuda.current_stream(device).cuda_stream)

@@ -74,13 +74,14 @@ def _raw(a, a_rows, a_cols, lda, a_mn, b, b_rows, b_cols, ldb, b_mn, d, ldd, c, 
          M, N, K, alpha=1.0, beta=0, epilogue=EPI_STORE, up_offset=0, groups=1, ragged=0, counts=None,
          a_gs_mn=0, a_gs_k=0, b_gs_mn=0, b_gs_k=0, d_gs=0, c_gs=0, aux_gs=0, max_ctas=0,
          b_div=1, k_segs=1, seg_stride=0, d_table=None, k_split=1, scatter_rows=0):
-    st = _lib.status_tensor(a.device)
-    err = _fn()(_lib.ptr(a), a_rows, a_cols, lda, a_mn, _lib.ptr(b), b_rows, b_cols, ldb, b_mn,
-                _lib.ptr(d), ldd, _lib.ptr(c), ldc, _lib.ptr(aux), ldaux,
-                M, N, K, alpha, beta, epilogue, up_offset, groups, ragged, _lib.ptr(counts),
+    dev = a.device
+    # (addresses as integers: the function's argument types are declared, and a c_void_p per tensor is a third of the call's host time)
+    err = _fn()(a.data_ptr(), a_rows, a_cols, lda, a_mn, b.data_ptr(), b_rows, b_cols, ldb, b_mn,
+                None if d is None else d.data_ptr(), ldd, None if c is None else c.data_ptr(), ldc, None if aux is None else aux.data_ptr(), ldaux,
+                M, N, K, alpha, beta, epilogue, up_offset, groups, ragged, None if counts is None else counts.data_ptr(),
                 a_gs_mn, a_gs_k, b_gs_mn, b_gs_k, d_gs, c_gs, aux_gs,
-                b_div, k_segs, seg_stride, _lib.ptr(d_table), k_split, scatter_rows,
-                _lib.ptr(st), max_ctas, _lib.stream_ptr(a.device))
+                b_div, k_segs, seg_stride, None if d_table is None else d_table.data_ptr(), k_split, scatter_rows,
+                _lib.status_tensor(dev).data_ptr(), max_ctas, _lib.stream_ptr(dev))
     _lib.check(err, "ats_gemm_bf16")
 
 

@@ -195,7 +195,10 @@ def _ptr_table(t: torch.Tensor) -> torch.Tensor:
     """int64 device table with the base address of every expert region of t[E, C, H]."""
     E = t.shape[0]
     step = t.stride(0) * t.element_size()
-    return torch.arange(E, dtype=torch.int64, device=t.device) * step + t.data_ptr()
+    first = t.data_ptr()
+    if step <= 0:
+        return torch.full((E,), first, dtype=torch.int64, device=t.device)
+    return torch.arange(first, first + E * step, step, dtype=torch.int64, device=t.device)   # one launch; addresses stay below 2^53
 
 
 def dispatch(x: torch.Tensor, topk_idx: torch.Tensor, slot_pos: torch.Tensor, counts: torch.Tensor,
