@@ -377,6 +377,8 @@ static int launch_channel(const ChannelArgs& p, cudaStream_t s) {
   if (even) launch_pdl(channel_pairs_kernel<T, 2, true>, grid, block, 0, s, p);
   else launch_pdl(channel_pairs_kernel<T, 2, false>, grid, block, 0, s, p);
   if (p.DK == 64) return launch_channel_scan<T, 4, 8>(p, s);
+  // (as in delta_rule.cu; us with eight / four columns: 16 CTAs 161 / 116, 96 516 / 471, 160 655 / 501, 192 499 / 405, 224 499 / 505, 256 1010 / 1034)
+  if (p.DK == 128 && (long long)((p.vdim + 63) / 64) * p.H * p.B <= SCAN_FEW) return launch_channel_scan<T, 8, 4>(p, s);
   if (p.DK == 128) return launch_channel_scan<T, 8, 8>(p, s);
   return launch_channel_scan<T, 16, 4>(p, s);
 }

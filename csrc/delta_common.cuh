@@ -5,6 +5,8 @@
 namespace ats {
 
 constexpr int DC = 8;  // tokens per group
+// Up to this many CTAs (of 64 columns) the scan kernels of 128 state rows take 32 columns a CTA instead.
+constexpr int SCAN_FEW = 192;
 
 // exp(rate softplus(a)), rate < 0.  The bf16 form uses the fast functions and, where exp(a) is small, the series of log(1 + x), so that a
 // slow decay keeps its digits.

@@ -865,7 +865,14 @@ static int launch_scan(const ScanArgs& p, cudaStream_t s) {
   }
   auto grid = [&](int cpl) { return dim3((p.vdim + 8 * cpl - 1) / (8 * cpl), p.H, p.B); };
   if (p.dim <= 64) launch_pdl(delta_scan_kernel<T, 4, 8, 2>, grid(8), dim3(128), 0, s, p);
-  else if (p.dim <= 128) launch_pdl(delta_scan_kernel<T, 8, 8, 2>, grid(8), dim3(128), 0, s, p);
+  else if (p.dim <= 128) {
+    // Eight columns per lane read each k and q row for twice the products of four, but a CTA's groups follow one another, so while SMs are idle
+    // it is the time of one group that counts.  us with eight / four columns, by CTAs at eight: 16 187 / 117, 96 565 / 459, 128 388 / 312,
+    // 160 640 / 496, 192 532 / 416, 224 534 / 615, 256 1092 / 1270.
+    const dim3 g8 = grid(8);
+    if ((long long)g8.x * g8.y * g8.z <= SCAN_FEW) launch_pdl(delta_scan_kernel<T, 8, 4, 2>, grid(4), dim3(128), 0, s, p);
+    else launch_pdl(delta_scan_kernel<T, 8, 8, 2>, g8, dim3(128), 0, s, p);
+  }
   else if (p.dim <= 256) launch_pdl(delta_scan_kernel<T, 16, 4, 2>, grid(4), dim3(128), 0, s, p);
   else return 1006;
   return int(cudaGetLastError());
