@@ -28,7 +28,7 @@ class _Skinny(ctypes.Structure):   # csrc/skinny.cuh
     _fields_ = [("T", _c_int), ("N", _c_int), ("K", _c_int), ("mode", _c_int), ("up_offset", _c_int), ("act_cols", _c_int), ("head_dim", _c_int), ("alpha", _c_f), ("a1", _c_f), ("a2", _c_f),
                 ("ldx", _c_int), ("out", _vp), ("ldo", _c_ll), ("add", _vp), ("ldadd", _c_ll), ("bias", _vp), ("x", _vp), ("w1", _vp), ("b1", _vp), ("w2", _vp),
                 ("b2", _vp), ("pos", _vp), ("next_w", _vp), ("next_out", _vp), ("next_parts", _vp), ("scale_parts", _vp), ("scale_n", _c_int), ("scale_inv", _c_f),
-                ("scale_eps", _c_f), ("status", _vp)]
+                ("scale_eps", _c_f), ("status", _vp), ("w_ready", _c_int)]
 
 
 def _fn():
@@ -132,8 +132,9 @@ def _gemm_nt_split_k(a, b, out, add, alpha, splits):
 @contextlib.contextmanager
 def chained_launches(on: bool = True):
     """Kernels launched inside (by this thread) may start while the kernel before them still runs, and the decode products fetch their first
-    weights, the decode attention its first cached keys, then.  For a decode step: no kernel launched inside may write a weight that a product
-    inside reads, a length, or a cached row below its sequence's length (the row at the length is the step's own)."""
+    weights, the decode attention its first cached keys, then.  For a decode step: no kernel launched inside may write a parameter, a packed
+    4-bit copy of one, a length, or a cached row below its sequence's length (the row at the length is the step's own).  A product whose weight
+    is the result of a kernel (:func:`_weight_ready`) waits for it."""
     if not on or not torch.cuda.is_available():
         yield
         return
@@ -144,6 +145,12 @@ def chained_launches(on: bool = True):
         yield
     finally:
         lib.ats_chain_launches(0)
+
+
+def _weight_ready(w: torch.Tensor) -> bool:
+    """Whether ``w`` certainly holds its values before a chained step begins: a parameter itself, not a view or a copy of one, nor a matrix that
+    a kernel writes (a dequantised weight, a gathered shard)."""
+    return isinstance(w, torch.nn.Parameter) and getattr(w, "_ats_z3", None) is None
 
 
 SKINNY_MAX_ROWS = 64
@@ -185,7 +192,7 @@ def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Op
         return None if t is None else t.data_ptr()
     args = _Skinny(T, N, K, mode, up_offset, act_cols, head_dim, alpha, a1, a2, 0 if x is None else x.stride(0), at(out), out.stride(-2), at(add), 0 if add is None else add.stride(0),
                    at(bias), at(x), at(w1), at(b1), at(w2), at(b2), at(pos), *(map(at, next_norm) if next_norm is not None else (None,) * 3),
-                   *((at(scale[0]), scale[0].shape[1], 1.0 / K, scale[1]) if scale is not None else (None, 0, 0.0, 0.0)), at(_lib.status_tensor(a.device)))
+                   *((at(scale[0]), scale[0].shape[1], 1.0 / K, scale[1]) if scale is not None else (None, 0, 0.0, 0.0)), at(_lib.status_tensor(a.device)), int(_weight_ready(w)))
     _lib.check(_lib.cuda_lib().ats_gemm_skinny(a.data_ptr(), a.stride(0), w.data_ptr(), w.stride(0), w.shape[0], ctypes.byref(args), splits, _lib.stream_ptr(a.device)),
                "ats_gemm_skinny")
 

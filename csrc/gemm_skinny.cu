@@ -19,7 +19,8 @@
 // sums of squares per tile, the second one scales its sums.  With it and the residual read under the product, one decode step of eight
 // 2048-wide layers: one sequence 331 -> 312 us, 64 sequences 626 -> 581 us.
 //
-// In a chain of launches (common.cuh) the first ring of weight tiles is requested before the kernel waits for its predecessor.
+// In a chain of launches (common.cuh) the first ring of weight tiles is requested before the kernel waits for its predecessor, if the caller says
+// that the weight is not a result of the same step (w_ready).
 #include "skinny.cuh"
 #include "typed.cuh"
 
@@ -430,7 +431,7 @@ int sk_launch(const CUtensorMap& mw, const CUtensorMap& ma, const SkinnyArgs& p,
   }
   cfg.attrs = attr;
   cfg.numAttrs = n;
-  cudaError_t ce = cudaLaunchKernelEx(&cfg, skinny_kernel<NT>, mw, ma, p, int(chained_launches()));
+  cudaError_t ce = cudaLaunchKernelEx(&cfg, skinny_kernel<NT>, mw, ma, p, int(p.w_ready && chained_launches()));
   return int(ce != cudaSuccess ? ce : cudaGetLastError());
 }
 

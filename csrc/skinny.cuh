@@ -37,6 +37,7 @@ struct SkinnyArgs {
   int scale_n;
   float scale_inv, scale_eps;
   int* status;
+  int w_ready;   // no kernel that may still run writes w (it is no result of the same step): in a chain of launches its first tiles are requested early
 };
 
 }  // namespace ats
