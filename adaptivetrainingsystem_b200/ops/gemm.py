@@ -213,6 +213,11 @@ def _fold_partials(part: torch.Tensor, splits: int, n_inner: int, n_outer: int, 
                                                  _lib.stream_ptr(part.device)), "splitk_reduce")
 
 
+def _addressable(t: Optional[torch.Tensor], M: int, N: int, dtype) -> bool:
+    """Whether the epilogues can read or write ``t`` in place: [M, N] of their type, adjacent columns, 16-byte aligned rows."""
+    return (t is None or (t.dtype == dtype and t.shape == (M, N) and t.stride(1) == 1 and t.stride(0) % 8 == 0 and t.data_ptr() % 16 == 0))
+
+
 def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None,
             add: Optional[torch.Tensor] = None, alpha: float = 1.0, out_fp32: bool = False,
             accumulate: bool = False, max_ctas: int = 0) -> torch.Tensor:
@@ -234,8 +239,20 @@ def gemm_nt(a: torch.Tensor, b: torch.Tensor, out: Optional[torch.Tensor] = None
     a, b = _check2d(a), _check2d(b)
     M, K = a.shape
     N = b.shape[0]
+    dtype = torch.float32 if out_fp32 else a.dtype
+    if N % 8 == 0 and not (_addressable(out, M, N, dtype) and _addressable(add, M, N, a.dtype)):
+        # transposed, expanded over the columns, oddly pitched, of another type or of more dimensions: the fp32 product, then torch
+        with torch.no_grad():
+            res = gemm_nt(a, b, alpha=alpha, out_fp32=True, max_ctas=max_ctas)
+            if add is not None:
+                res += add.reshape(M, N) if add.numel() == M * N else add
+            if out is None:
+                return res.to(dtype)
+            dst = out.view(M, N)
+            dst.copy_(dst + res if accumulate and out_fp32 else res)
+        return out
     if out is None:
-        out = torch.empty(M, N, dtype=torch.float32 if out_fp32 else a.dtype, device=a.device)
+        out = torch.empty(M, N, dtype=dtype, device=a.device)
     if skinny_ok(a, b) and not accumulate and not max_ctas and (add is None or not out_fp32):
         skinny(a, b, out, SK_F32 if out_fp32 else SK_STORE, add=add, alpha=alpha)
         return out
