@@ -1050,6 +1050,13 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 // host
 // ------------------------------------------------------------------------------------------------
 EncodeTiledFn get_encode_tiled() {
+  // The encoder is a driver call and fails on a thread without a current context; a thread whose first work is a product or an attention
+  // step has none yet.  (Selecting the device that is selected anyway binds its context, also while a stream is being captured.)
+  static thread_local bool bound = false;
+  if (!bound) {
+    int dev = 0;
+    bound = cudaGetDevice(&dev) == cudaSuccess && cudaSetDevice(dev) == cudaSuccess;
+  }
   static EncodeTiledFn fn = nullptr;
   if (!fn) {
     void* p = nullptr;
