@@ -93,8 +93,8 @@ def _partial_products(x2: torch.Tensor, w: torch.Tensor):
             and x2.is_contiguous() and w.is_contiguous() and not getattr(w, "_ats_z3", None) and G.SPLIT_K_SKINNY):
         return None
     from . import fp8, int4, int8
-    if int4.enabled() and int4.lookup(w) is not None:
-        return None          # a 4-bit weight: the caller's ordinary product streams the packed copy
+    if int4.enabled() and int4.lookup(w) is not None or int4.observing() or int8.observing():
+        return None          # the caller's ordinary product streams the packed copy of a 4-bit weight, and shows its rows to a calibration
     splits = G._skinny_splits(T, N, K)
     if G.skinny_ok(x2, w) and (splits > 1 or not (fp8.enabled() or int8.enabled())):
         return DECODE_KERNEL   # (with 8-bit copies around, the products that the 8-bit kernels do not split stay with them)
@@ -182,7 +182,8 @@ def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, re
             x = G.gemm_nt(act, w_down, add=residual2)
             fused = x, rms_norm(x, norm_w, eps)
         return fused
-    if (fp8.enabled() or int8.enabled() or (int4.enabled() and int4.lookup(w_gate_up) is not None) or getattr(w_gate_up, "_ats_z3", None)
+    if (fp8.enabled() or int8.enabled() or (int4.enabled() and (int4.lookup(w_gate_up) is not None or int4.lookup(w_down) is not None))
+            or int4.observing() or int8.observing() or getattr(w_gate_up, "_ats_z3", None)
             or not _lib.use_cuda_kernels(h2) or w_gate_up.dtype != torch.bfloat16 or not G.skinny_ok(h2, w_down) or not FUSE_DECODE or norm_w.dtype != torch.bfloat16 or not residual2.is_contiguous()):
         return None
     return out_proj_norm(G.gemm_nt_swiglu(h2, w_gate_up), w_down, residual2, norm_w, eps, scaled)
