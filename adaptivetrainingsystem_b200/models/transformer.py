@@ -429,6 +429,14 @@ class MoDFFN(nn.Module):
         return out, aux * self.cfg.mod_aux_weight
 
 
+def _plain(module: nn.Module, kind: type) -> bool:
+    """Whether a decode step may do the work of ``module`` in the launches around it instead of calling it: it is a ``kind`` as defined here and
+    nothing hangs on its call."""
+    m = nn.modules.module
+    return (type(module) is kind and "forward" not in module.__dict__
+            and not (module._forward_hooks or module._forward_pre_hooks or m._global_forward_hooks or m._global_forward_pre_hooks))
+
+
 class TransformerBlock(nn.Module):
     def __init__(self, cfg: ModelConfig, layer_idx: int, ep_size: int = 1, ep_rank: int = 0):
         super().__init__()
@@ -461,20 +469,21 @@ class TransformerBlock(nn.Module):
     def takes_scaled_rows(self, rope, cache) -> bool:
         """Whether this block's projection divides by the norm of its input itself (``ops.serving.ScaledRows``)."""
         a = self.self_attn
-        return a.tp_group is None and ops.serving.takes_rotated(cache.batch, a.qkv_proj, a.n_q, a.n_kv, a.d, rope.cos, cache.device_positions)
+        return _plain(a, GroupedQueryAttention) and a.tp_group is None and ops.serving.takes_rotated(cache.batch, a.qkv_proj, a.n_q, a.n_kv, a.d, rope.cos, cache.device_positions)
 
     def decode_step(self, x, rope, cache, h_pre=None, next_norm=None, next_scaled=False):
         """One graph-replayed decode step of this block with the norms folded into their producers: ``h_pre`` is this block's
         normalised input when the block before already produced it, ``next_norm`` = (weight, eps) of the norm that follows this
-        block (``next_scaled``: what follows takes ``ops.serving.ScaledRows``).  -> (x, normalised x for the next block or None)."""
+        block or ``None`` (``next_scaled``: what follows takes ``ops.serving.ScaledRows``).  -> (x, normalised x for the next block or None)."""
         if h_pre is None:
             h, x = self.input_norm.with_skip(x)
         else:
             h = h_pre
         rows = x.numel() // x.shape[-1]
-        scaled = (self.ffn_kind == "dense" and next_norm is not None and self.ffn.tp_group is None and next_norm[0].dtype == torch.bfloat16
+        folds = self.ffn_kind == "dense" and next_norm is not None and _plain(self.ffn, DenseSwiGLU) and self.ffn.tp_group is None
+        scaled = (folds and _plain(self.self_attn, GroupedQueryAttention) and _plain(self.post_attn_norm, RMSNorm) and next_norm[0].dtype == torch.bfloat16
                   and ops.serving.takes_scaled(rows, self.ffn.gate_up_proj, self.ffn.gate_up_proj.shape[0] // 2) and ops.serving.takes_scaled(rows, self.ffn.down_proj))
-        res = self.self_attn(h, x, rope, None, cache, None, post_norm=self.post_attn_norm, scaled=scaled)
+        res = self.self_attn(h, x, rope, None, cache, None, post_norm=self.post_attn_norm, **({"scaled": True} if scaled else {}))
         x, h = res if isinstance(res, tuple) else (res, None)
         if h is None:
             h, x = self.post_attn_norm.with_skip(x)
@@ -487,7 +496,7 @@ class TransformerBlock(nn.Module):
             x, _ = self.ffn(h, x, decode=True)
         else:
             fused = None
-            if next_norm is not None and self.ffn.tp_group is None:
+            if folds:
                 fused = ops.serving.mlp_norm(h.reshape(-1, h.shape[-1]), self.ffn.gate_up_proj, self.ffn.down_proj, x.reshape(-1, x.shape[-1]), *next_norm, scaled=next_scaled)
             if fused is not None:
                 return fused[0].view(x.shape), fused[1].view(x.shape)
@@ -582,7 +591,8 @@ class DeepSeekTransformer(nn.Module):
             for i, blk in enumerate(self.layers):
                 nxt = self.layers[i + 1].input_norm if i + 1 < n else self.norm
                 scaled = i + 1 < n and self.layers[i + 1].takes_scaled_rows(self.rope, cache)
-                x, h_pre = blk.decode_step(x, self.rope, cache, h_pre, (nxt.weight, nxt.eps), scaled)
+                fold = blk.ffn_kind != "dense" or _plain(nxt, RMSNorm)
+                x, h_pre = blk.decode_step(x, self.rope, cache, h_pre, (nxt.weight, nxt.eps) if fold else None, scaled)
             return (h_pre if h_pre is not None else self.norm(x)), aux_losses
         for blk in self.layers:
             x, aux = blk(x, self.rope, attention_mask, cache, positions, decode)
