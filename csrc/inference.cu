@@ -115,7 +115,10 @@ __global__ void __launch_bounds__(DEC_THREADS, 3) decode_attn_kernel(const __gri
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int n_old = p.lengths ? p.lengths[b] : p.length;
-  if (!ATS_DBG_CHECK(n_old >= 0 && n_old < p.max_len, kDbgDecodeAttn, n_old)) return;   // (every CTA of the cluster)
+  if (!ATS_DBG_CHECK(n_old >= 0 && n_old < p.max_len, kDbgDecodeAttn, n_old)) {   // (every CTA of the cluster)
+    if (early) asm volatile("griddepcontrol.wait;" ::: "memory");   // what follows in a chain counts on this kernel to end after the one before it
+    return;
+  }
   const int n_tot = min(n_old + 1, p.max_len);  // the new token attends to itself
   uint8_t* base_smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dec_smem) + 1023) & ~uintptr_t(1023));
   uint8_t* ring = base_smem + warp * (DEC_STAGES * DEC_UNIT_BYTES);
