@@ -85,9 +85,9 @@ __device__ __forceinline__ float exp_from(float m, float base) { return m == -IN
 // In a chain of launches (common.cuh) the first units are requested before the kernel waits for its predecessor: only the new token's row
 // and the query come from it.  Units are dealt out over the parts x S x 4 warps of a (sequence, KV head) by its actual length.  The S CTAs
 // of a cluster fold their results through distributed shared memory, so there is no merge launch and no scratch below `parts` = 2.
-// Measured (us, caches larger than L2 in turn; before: 256-key chunks by plain loads and a merge launch): 64 sequences x 4 KV heads of 64,
-// 1,152 keys 29.6 -> 26.1; 64 x 8 of 128, 1,100 keys 94.6 -> 65.5 (4.4 TB/s), 1,500 keys 114 -> 78.6 (5.0 TB/s); one sequence, 640 keys 7.5 -> 4.9,
-// 32,000 keys 68.5 -> 15.2.  64 x 4 CTAs do not fill the SMs evenly: what is left there is a CTA's fixed time.
+// Measured (us, caches larger than L2 in turn; before: 256-key chunks by plain loads and a merge launch): 64 sequences x 4 KV heads of 64, 500 keys
+// 18.3 -> 10.8, 2,000 keys 48.9 -> 25.6 (5.1 TB/s); 64 x 8 of 128, 2,000 keys 149 -> 97 (5.4 TB/s); 32 x 4 of 64, 500 keys 10.6 -> 8.7; one
+// sequence, 500 keys 7.2 -> 5.1, 32,000 keys 67.6 -> 15.3.
 // ------------------------------------------------------------------------------------------------
 template <bool V>
 struct BoolC {
@@ -821,14 +821,21 @@ __global__ void __launch_bounds__(256) fold_add_norm_kernel(const float* __restr
 using namespace ats;
 
 // How many CTAs share a (sequence, KV head) (`cluster`, a power of two up to the portable cluster size) and how many such clusters (`parts`).
-// A CTA costs 4 to 5 us whatever it reads, so there are no more of them than fill the SMs once (three each) unless a warp would walk
-// through more than ten units: 256 pairs with 1,152 keys take 27.0 us with one CTA each, 26.1 with two, 27.6 with four and 57 with eight;
-// 512 pairs with 1,100 keys of 128 dimensions 65 with two, 68 with four, 102 with eight.
+// Clusters of eight stop fitting beyond some 400 CTAs (three an SM would be 444), and a second wave costs more than the shorter walk
+// brings.  So the number doubles freely while there is at most one CTA for every SM, up to 384 as long as a warp keeps more than five units
+// (a CTA costs 3 to 4 us whatever it reads), and beyond one wave only where a warp would walk through more than eighteen.  us with 1 / 2 / 4 / 8 CTAs:
+//   pairs x dimensions, keys      pairs x dimensions, keys      pairs x dimensions, keys
+//   64 x 64, 250    4.4  4.7  5.2  8.9     128 x 64, 500    7.2  7.9 11.6 16.2     256 x 64, 1150   16.9 25.0 26.8 40.0
+//   64 x 64, 2000  14.3 11.1 10.0 15.4     128 x 64, 4000  27.8 24.4 30.4 31.2     384 x 128, 1150  41.1 45.1 53.6 77.8
+//   64 x 128, 1150 19.3 14.0 12.5 19.3     128 x 128, 1150 20.6 17.9 24.5 29.6     512 x 128, 4000   194  169  164  184
 static void decode_split(int pairs, int D, int tokens, int* cluster, int* parts) {
   const int units = (tokens + 2048 / D - 1) / (2048 / D);
+  const long long sms = 148, wave = 384;
   int s = 1, n = 1;
-  while (s < 8 && s * DEC_WARPS < units && (pairs * s < 3 * 148 || s * DEC_WARPS * 10 < units)) s *= 2;
-  while (pairs * s * n < 2 * 148 && s * n * DEC_WARPS * 4 < units) n *= 2;
+  while (s < 8 && s * DEC_WARPS < units &&
+         (2ll * s * pairs <= sms || (2ll * s * pairs <= wave && s * DEC_WARPS * 5 < units) || (s == 1 && pairs > 3 * sms && DEC_WARPS * 18 < units)))
+    s *= 2;
+  while (s == 8 && 2ll * pairs * s * n <= wave && s * n * DEC_WARPS * 4 < units) n *= 2;
   *cluster = s;
   *parts = n;
 }
