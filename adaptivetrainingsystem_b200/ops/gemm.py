@@ -169,9 +169,13 @@ def skinny_ok(a: torch.Tensor, w: torch.Tensor, n: Optional[int] = None) -> bool
 def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:
     """Reduction slices of a decode product: as many as there are CTA slots (two per SM; one beyond 64 rows, whose rings are larger), but no
     slice below four 64-element blocks, where start-up and the sum of the slices cost more than the further SMs bring, and at most eight (a
-    cluster; four beyond 64 rows, where clusters of eight whole SMs leave the rest of a processing cluster idle)."""
+    cluster; four beyond 64 rows, where clusters of eight whole SMs leave the rest of a processing cluster idle).  Clusters of three and more
+    do not find all slots: 88 x 3 and 64 x 4 CTAs run at once, 96 x 3 and 74 x 4 in two waves (64 rows, us with two / three / four slices:
+    11264 x 1536 15.5 / 14.2 / 20.1, 12288 x 1536 15.8 / 21.4 / 20.5, 8192 x 1536 14.2 / 13.2 / 12.2, 9472 x 1536 14.4 / 13.5 / 19.3)."""
     tiles, slots, most = (N + width - 1) // width, 296 if T <= 64 else 148, 8 if T <= 64 else 4
     s = max(1, min(most, slots // tiles, (K + 63) // 64 // 4))
+    if s > 2:
+        s = max(2, min(s, slots * 264 // 296 // tiles))
     return s if s <= 4 else 4 if s < 8 else 8
 
 
