@@ -153,17 +153,41 @@ def _weight_ready(w: torch.Tensor) -> bool:
     return isinstance(w, torch.nn.Parameter) and getattr(w, "_ats_z3", None) is None
 
 
-SKINNY_MAX_ROWS = 64
 SK_PART, SK_STORE, SK_F32, SK_SWIGLU, SK_SILU, SK_GELU, SK_DYT, SK_ROPE = range(8)
 
 
 def skinny_ok(a: torch.Tensor, w: torch.Tensor, n: Optional[int] = None) -> bool:
-    """Whether ``a`` [T, K] @ ``w`` [N, K]^T runs on the decode kernel (``csrc/gemm_skinny.cu``), where the product is a stream of the weight.
-    Up to 64 rows it is the faster one at every size (2560 x 2048: 7.0 us against 14.4 with one row, 9.8 / 15.2 with 64; 32000 x 2048: 24.0 /
-    33.5 and 27.3 / 29.2); up to 128 rows only for narrow outputs (2048 x 2048: 13.6 / 20.2; 6144 x 4096: 37 / 26), because one CTA fills an SM
-    then and nothing runs under its epilogue."""
-    T, N = a.shape[0], w.shape[0] if n is None else n
-    return SPLIT_K_SKINNY and a.dim() == 2 and 1 <= T <= (128 if N <= 4096 else SKINNY_MAX_ROWS) and a.shape[1] % 8 == 0 and N % 8 == 0
+    """Whether ``a`` [T, K] @ ``w`` [N, K]^T runs on the decode kernel (``csrc/gemm_skinny.cu``), where the product is a stream of the weight; ``n``:
+    the outputs of a gate / up pair.  The lines are where the general kernel with its fold becomes the faster one (us, decode kernel / general):
+
+    * up to 32 rows hardly ever (2048 x 2048, one row 6.6 / 14.3; 32000 x 2048, 16 rows 24 / 32; 128256 x 384, 32 rows 30.4 / 27.4);
+    * up to 64 rows with very many outputs, where a CTA walks its whole tile alone: 32000 x 2048 27.6 / 29.0, 128256 x 1024 61 / 54; pairs: 64 rows
+      8192 x 2048 19.4 / 22.0, 11008 x 2048 25.3 / 24.1; 48 rows 14336 x 2048 26.7 / 27.0, 28672 x 2048 51 / 47; and with pairs over short
+      reductions, whose epilogue is the longer part: 64 rows 256 x 256 9.0 / 8.5, 256 x 512 8.1 / 9.7; 48 rows 14336 x 136 12.7 / 10.9;
+    * up to 128 rows, where one CTA fills an SM and four slices are the most, with many outputs (8192 x 2048, 128 rows 19.9 / 19.7), one or two
+      tiles or a reduction long for their number (1024 x 8192 20.6 / 19.1, 2048 x 4096 16.4 / 17.4), and short reductions (2048 x 512
+      13.6 / 10.3, 2048 x 1024 11.4 / 12.8; pairs 2816 x 512 12.1 / 10.5, 2816 x 1024 13.4 / 14.4)."""
+    T, K, N = a.shape[0], a.shape[-1], w.shape[0] if n is None else n
+    if not (SPLIT_K_SKINNY and a.dim() == 2 and 1 <= T <= 128 and K % 8 == 0 and N % 8 == 0):
+        return False
+    if T <= 32:
+        return T <= 16 or N <= 65536 or K >= 768
+    if T <= 64:
+        if n is None:
+            return N <= 32768
+        return N <= (14336 if T <= 48 else 8192) and (K >= 512 or (T <= 48 and 128 <= N <= 8192))
+    if N > 4096:
+        return False
+    if n is None:
+        return N >= 128 and K <= max(4096, 4 * N) and (K >= 1024 or T <= 80)
+    return K >= 1024 or (K >= 512 and T <= 80)
+
+
+def skinny_fits(T: int, N: int, K: int) -> bool:
+    """The same for a product whose decode kernel also saves a launch (a rotation, a norm) and fetches its first weights early: a captured step of
+    four 4096-wide layers with 28672 inner columns and 64 rows takes 792 us, with the lines of :func:`skinny_ok` for the pairs 844.  Beyond 64 rows
+    the reduction must not be long for the outputs (1024-wide layers with 28672 inner columns, 96 rows: 416 us, 476 without that)."""
+    return SPLIT_K_SKINNY and K % 8 == 0 and N % 8 == 0 and (1 <= T <= 64 or (T <= 128 and N <= 4096 and K <= max(4096, 4 * N)))
 
 
 def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:

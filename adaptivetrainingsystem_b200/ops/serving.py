@@ -80,7 +80,7 @@ def takes_scaled(rows: int, w: torch.Tensor, n: Optional[int] = None) -> bool:
     from . import fp8, gemm as G, int4, int8
     return (FUSE_DECODE and w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and not getattr(w, "_ats_z3", None)
             and not (fp8.enabled() or int8.enabled()) and not (int4.enabled() and int4.lookup(w) is not None) and not (int4.observing() or int8.observing())
-            and _lib.use_cuda_kernels(w) and w.shape[1] % 8 == 0 and G.skinny_ok(w[:1].expand(rows, -1), w, n))
+            and _lib.use_cuda_kernels(w) and G.skinny_fits(rows, w.shape[0] if n is None else n, w.shape[1]))
 
 
 def _partial_products(x2: torch.Tensor, w: torch.Tensor):
@@ -96,7 +96,7 @@ def _partial_products(x2: torch.Tensor, w: torch.Tensor):
     if int4.enabled() and int4.lookup(w) is not None or int4.observing() or int8.observing():
         return None          # the caller's ordinary product streams the packed copy of a 4-bit weight, and shows its rows to a calibration
     splits = G._skinny_splits(T, N, K)
-    if G.skinny_ok(x2, w) and (splits > 1 or not (fp8.enabled() or int8.enabled())):
+    if G.skinny_fits(T, N, K) and (splits > 1 or not (fp8.enabled() or int8.enabled())):
         return DECODE_KERNEL   # (with 8-bit copies around, the products that the 8-bit kernels do not split stay with them)
     if splits < 2:
         return None
@@ -184,7 +184,7 @@ def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, re
         return fused
     if (fp8.enabled() or int8.enabled() or (int4.enabled() and (int4.lookup(w_gate_up) is not None or int4.lookup(w_down) is not None))
             or int4.observing() or int8.observing() or getattr(w_gate_up, "_ats_z3", None)
-            or not _lib.use_cuda_kernels(h2) or w_gate_up.dtype != torch.bfloat16 or not G.skinny_ok(h2, w_down) or not FUSE_DECODE or norm_w.dtype != torch.bfloat16 or not residual2.is_contiguous()):
+            or not _lib.use_cuda_kernels(h2) or w_gate_up.dtype != torch.bfloat16 or not G.skinny_fits(h2.shape[0], *w_down.shape) or not FUSE_DECODE or norm_w.dtype != torch.bfloat16 or not residual2.is_contiguous()):
         return None
     return out_proj_norm(G.gemm_nt_swiglu(h2, w_gate_up), w_down, residual2, norm_w, eps, scaled)
 

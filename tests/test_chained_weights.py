@@ -32,9 +32,9 @@ def test_results_of_the_step_are_not(launches):
 @pytest.mark.parametrize("rows", [17, 33, 64])
 def test_dequantised_weights_are_not(launches, monkeypatch, rows):
     """More rows than the 4-bit streaming kernel takes: the weight is written out inside the step."""
-    wd = torch.randn(256, 128).bfloat16()
+    wd = torch.randn(256, 512).bfloat16()
     monkeypatch.setattr(int4, "dequantize", lambda *entry: wd)
-    a = torch.randn(rows, 128).bfloat16()
+    a = torch.randn(rows, 512).bfloat16()
     int4._matmul(a, (None, None, 64), None)
     int4._matmul(a, (None, None, 64), None, swiglu=True)
     assert [x.w_ready for x in launches] == [0, 0]
