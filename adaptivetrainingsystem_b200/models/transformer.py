@@ -177,12 +177,12 @@ class GroupedQueryAttention(nn.Module):
         qkv = ops.linear(h, self.qkv_proj, reduce_group=self.tp_group)
         nq, nk = self.n_q * self.d, self.n_kv * self.d
         if (cache is None and attention_mask is None and positions is None and self.d % 16 == 0
-                and ops.attention_packed_available(qkv, self.d, L)):
+                and ops.attention_packed_available(qkv, self.d, L, self.n_q, self.n_kv)):
             # training / scoring path: rotation and attention are one autograd node on the projection buffer
             a = ops.rope_attention_packed(qkv, rope.cos, rope.sin, self.n_q, self.n_kv, self.d, pos_offset=0)
             return self._project_out(a.reshape(B, L, nq), residual)
         qkv = ops.rope_packed(qkv, rope.cos, rope.sin, self.n_q, self.n_kv, self.d, pos_offset=offset, positions=positions)
-        if cache is None and attention_mask is None and ops.attention_packed_available(qkv, self.d, L):
+        if cache is None and attention_mask is None and ops.attention_packed_available(qkv, self.d, L, self.n_q, self.n_kv):
             a = ops.attention_packed(qkv, self.n_q, self.n_kv, self.d)
             return self._project_out(a.reshape(B, L, nq), residual)
         if (cache is not None and L == 1 and attention_mask is None and positions is None

@@ -814,10 +814,35 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, causal: bool = 
 NATIVE_MIN_SEQ = 32
 
 
-def attention_packed_available(qkv: torch.Tensor, d: int, seq_len: int) -> bool:
+def _ragged_native(B: int, L: int, n_q: int, n_kv: int, d: int, grad: bool) -> bool:
+    """Whether sequences that are no multiple of 128 run on the packed kernels or, as before those took them, on the library's and the copies
+    they need.  us a block (norms, projections, feed-forward), library / packed, forward and backward where a gradient is needed:
+
+    * up to 1,024 tokens the packed kernels (2048 wide, 32 / 4 heads of 64: 8 x 300 970 / 920; 16 heads of 128: 8 x 500 1545 / 1372), without a gradient
+      except for many sequences of one tile, which is mostly padding (64 x 40, attention alone: 33 / 90);
+    * up to 2,048 for gradients where the pass over the keys, one CTA for a key head's tile and its whole group, has work for the chip: 16 / 4 heads
+      8 x 2000 2000 / 1936, 32 / 4 heads 1 x 2000 920 / 955, 2 x 2000 1434 / 1536 and 8 x 2000 5182 / 5146; without a gradient 562 / 578 (16 / 4);
+    * beyond that the library (32 / 4 heads: 1 x 4000 1542 / 1870, 1 x 8000 3565 / 4078; 16 heads of 128: 4 x 4000 6261 / 6536), unless the whole
+      block is so small that its launches take longer than its kernels, of which the packed form needs fewer (1024 wide, 16 / 4 heads: 1 x 2000
+      921 / 750, 1 x 8000 1509 / 1722; 512 wide: 1 x 4000 914 / 750, 1 x 8000 994 / 1034)."""
+    if not (1 <= B <= 65535 and L >= NATIVE_MIN_SEQ):
+        return False
+    if L <= 4096 and B * L * (n_q * d) ** 2 < 4e9:
+        return True
+    if grad:
+        return L <= 1024 or (L <= 2048 and B * n_kv * n_kv >= 4 * n_q)
+    return L <= 1024 and (L > 128 or B * n_q <= 256)
+
+
+def attention_packed_available(qkv: torch.Tensor, d: int, seq_len: int, n_q: int = 0, n_kv: int = 0) -> bool:
+    """Whether :func:`attention_packed` takes ``qkv`` and pays (``n_q`` = 0: the head counts are not known)."""
     from . import attn as A
-    return (_lib.use_cuda_kernels(qkv) and A._native_available() and d in (64, 128) and seq_len >= NATIVE_MIN_SEQ and qkv.is_contiguous()
-            and qkv.shape[-1] % 8 == 0)
+    if not (_lib.use_cuda_kernels(qkv) and A._native_available() and d in (64, 128) and qkv.is_contiguous() and qkv.shape[-1] % 8 == 0):
+        return False
+    if seq_len % 128 == 0:
+        return seq_len >= NATIVE_MIN_SEQ
+    heads = qkv.shape[-1] // d
+    return _ragged_native(qkv.shape[0], seq_len, n_q or heads, n_kv if n_q else 1, d, torch.is_grad_enabled() and qkv.requires_grad)
 
 
 def rope_attention_packed(qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, n_q: int, n_kv: int, d: int,
