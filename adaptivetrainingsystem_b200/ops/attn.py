@@ -1,8 +1,9 @@
 """Causal grouped-query attention on CUDA.
 
-``flash_attention`` runs the tcgen05 kernel of ``csrc/attention_tcgen05.cu`` when the shape is one it
-covers (head_dim 64 or 128, sequence a multiple of 128, bf16).  Other shapes use PyTorch's fused SDPA, which
-is a library call and is reported as such by ``backend_for``.
+``flash_attention`` runs the tcgen05 kernels of ``csrc/attention_tcgen05.cu`` and ``csrc/attention_fwd2_tcgen05.cu`` for head sizes of 64
+and 128, bf16, sequences of a multiple of 128 and evenly pitched token rows.  Other operands (the views of a longer cache that a prompt
+attends to among them) use PyTorch's fused SDPA, which is a library call and is reported as such by ``backend_for``.  The kernels take any
+length: the packed entry points (``functional.attention_packed_available``) use that.
 
 Replaces ``flash_attn_func(causal=True)`` plus the ``repeat_interleave`` K/V expansion of the reference
 (``core/model.py:705-768``); K/V heads are shared by the query heads of a group without being copied.

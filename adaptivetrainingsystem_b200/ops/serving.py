@@ -109,8 +109,8 @@ def _partial_products(x2: torch.Tensor, w: torch.Tensor):
 
 def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, positions: torch.Tensor, n_q: int, n_kv: int,
              d: int) -> Optional[torch.Tensor]:
-    """Packed projection of the new tokens with q and k rotated at ``positions`` [T] (int32): one product + one fold launch.
-    ``None`` when the fused form does not apply."""
+    """Packed projection of the new tokens with q and k rotated at ``positions`` [T] (int32): one launch where the decode kernel rotates (whole
+    heads in its tiles), else the product and a fold.  ``None`` when the fused form does not apply."""
     rows, scale = (h2.rows, (h2.parts, h2.eps)) if isinstance(h2, ScaledRows) else (h2, None)
     if scale is not None and not takes_rotated(rows.shape[0], w_qkv, n_q, n_kv, d, cos, positions):
         raise RuntimeError("scaled rows reached a projection that does not take them")

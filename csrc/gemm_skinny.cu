@@ -2,11 +2,12 @@
 // fp32 accumulation.
 //
 // Such a product is a stream of the weight: its floor is N K 2 bytes at the copy bandwidth (2 to 10 us for the projections of a
-// 2048-wide decoder), so what counts is that every SM streams, and that it starts early.  The general GEMM puts the activations on the 128
+// 2048-wide decoder), so what counts is that as many SMs as possible stream, and that they start early.  The general GEMM puts the activations on the 128
 // accumulator rows and tiles N by 256: qkv of a 2048-wide model is 10 tiles (40 CTAs with its four reduction slices), the gate / up product
 // 44, so a third of the SMs streamed.  Here the operands are swapped: 128 weight rows are the rows of the tensor-core tile and the tokens its
 // columns (16 to 128 of them, so one token costs 1/8 of the accumulator instead of a full one), and the reduction of a tile is cut over a
-// cluster of up to eight CTAs, so that a product has up to two CTAs for every SM, each with all of its ring (54 to 96 KB) in flight.
+// cluster of up to eight CTAs, so that a product of up to 64 tokens has up to two CTAs for every SM (2,048 outputs: 16 tiles, 128 CTAs), beyond
+// that one, each with all of its ring (72 to 90 KB; 128 KB beyond 64 tokens) in flight.
 // The slices are summed through distributed shared memory in a fixed order (every CTA of the cluster owns a block of the tokens), and the
 // element-wise step that follows the product (a rotation of the heads among them) is done there: no partial products in memory and no second
 // launch.  Steps on whole rows (a norm) keep their fold kernels: kSkPart writes the slices.

@@ -1,6 +1,6 @@
 // Serving kernels for sm_100a: single-query (decode) attention against a grouped-query KV cache, and batched token
-// sampling.  Both are memory / latency bound (no tensor-core shape), so they are plain CUDA-core kernels laid out so
-// that every K / V byte of the cache is read exactly once per step.
+// sampling.  Attention reads every K / V byte of the cache exactly once per step, through rings of TMA copies into
+// warp-level MMAs; the sampler is bound by latency and runs on the CUDA cores.
 //
 // * ats_decode_attn: one new query token per sequence.  Every warp scores units of 32 or 16 keys for all query heads of a group (K read once
 //   per group, not once per query head) and keeps a running softmax; warps are folded through shared memory, the CTAs of a (sequence, KV
