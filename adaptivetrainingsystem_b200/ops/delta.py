@@ -17,7 +17,7 @@ from . import _lib
 from .latent import _call, _p, pad8
 
 _vp, _ci, _cll, _cf = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float
-GROUP = 8  # tokens the portion kernel advances at a time
+GROUP, GROUP_MMA = 8, 16  # tokens the portion kernels advance at a time (csrc/delta_rule.cu, csrc/delta_rule_mma.cu)
 
 
 @dataclass(frozen=True)
@@ -185,6 +185,11 @@ def delta_prep(proj: torch.Tensor, s: DeltaShape, conv: torch.Tensor, neg_rate: 
     return mixed, rlen, gb
 
 
+def scan_on_tensor_cores(mixed: torch.Tensor, s: DeltaShape) -> bool:
+    """Whether portions run on ``csrc/delta_rule_mma.cu``: bf16 rows of 16-byte pieces, up to 128 state rows."""
+    return mixed.dtype == torch.bfloat16 and s.dim <= 128 and s.dim % 8 == 0 and s.vdim % 8 == 0 and mixed.stride(0) % 8 == 0 and mixed.data_ptr() % 16 == 0
+
+
 def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, s: DeltaShape, L: int, fresh: bool) -> torch.Tensor:
     """Advances ``state`` [B, H, dim, vdim] over portions of L tokens -> read-outs [B * L, H * vdim]; ``fresh``: the state starts at zero."""
     B = state.shape[0]
@@ -199,12 +204,13 @@ def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state:
                 out[t] = o.reshape(-1).to(out.dtype)
             state[b] = S
         return out
-    dev = mixed.device
-    groups = (L + GROUP - 1) // GROUP
-    coef = torch.empty(B, groups, H, 2 * GROUP * GROUP + 3 * GROUP + 8, dtype=torch.float32, device=dev)   # layout: csrc/delta_rule.cu
-    o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=dev)
-    _call("ats_delta_scan", _Scan(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0), B, L, H, KH, s.dim, s.vdim,
-                                  groups, int(fresh)), mixed)
+    mma = scan_on_tensor_cores(mixed, s)
+    groups = -(-L // (GROUP_MMA if mma else GROUP))
+    size = 832 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # layouts: csrc/delta_rule_mma.cu, csrc/delta_rule.cu
+    coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
+    o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
+    args = _Scan(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0), B, L, H, KH, s.dim, s.vdim, groups, int(fresh))
+    _call("ats_delta_scan_mma" if mma else "ats_delta_scan", args, mixed)
     return o
 
 
@@ -261,9 +267,17 @@ def channel_delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor
                 out[t] = o.reshape(-1).to(out.dtype)
             state[b] = S
         return out
-    groups, DK = (L + GROUP - 1) // GROUP, s.scan_rows
-    coef = torch.empty(B, groups, H, 2 * GROUP * GROUP + (3 * GROUP + 1) * DK, dtype=torch.float32, device=mixed.device)   # layout: csrc/channel_delta.cu
+    mma, DK = scan_on_tensor_cores(mixed, s), s.scan_rows
+    groups = -(-L // (GROUP_MMA if mma else GROUP))
+    size = 73 * DK + 768 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # layouts: csrc/channel_delta_mma.cu, csrc/channel_delta.cu
+    coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
     o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
-    _call("ats_channel_delta", _Channel(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(a), a.stride(0), _p(neg_rate), _p(dt_bias), _p(coef), _p(state), state.stride(0),
-                                        _p(o), o.stride(0), B, L, H, s.kv_heads, s.dim, s.vdim, groups, int(fresh), DK), mixed)
+    args = _Channel(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(a), a.stride(0), _p(neg_rate), _p(dt_bias), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0),
+                    B, L, H, s.kv_heads, s.dim, s.vdim, groups, int(fresh), DK)
+    if mma:
+        f = _lib.cuda_lib().ats_channel_delta_mma
+        f.restype, f.argtypes = _ci, [_vp, _vp, _vp]
+        _lib.check(f(ctypes.byref(args), _p(_lib.status_tensor(mixed.device)), _lib.stream_ptr(mixed.device)), "ats_channel_delta_mma")
+    else:
+        _call("ats_channel_delta", args, mixed)
     return o

@@ -13,31 +13,11 @@
 // channel_pairs computes, for all groups in parallel, the 8 x 8 inverse (times beta), kq, and the decayed rows P_i k_i, P_i q_i,
 // k_j g_{j+1} .. g_C, P_C in fp32; all decay products are running products of factors in (0, 1], so nothing overflows however fast a
 // channel decays.  channel_scan does three products with the state per token: sixteen lanes share eight columns, fp32 with packed
-// fma.f32x2, the next group's rows arriving in shared memory by asynchronous copies.
+// fma.f32x2, the next group's rows arriving in shared memory by asynchronous copies.  channel_delta_mma.cu is the faster form for bf16 rows of whole
+// 16-byte pieces and up to 128 state rows.
 #include "delta_common.cuh"
 
 namespace ats {
-
-struct ChannelArgs {
-  const void* mixed;       // [B * L, ldm] convolved q, k, v
-  long long ldm;
-  const float* rlen;       // [B * L, 2 * KH] dim^-1/2 / |q|, 1 / |k|
-  const float* gb;         // [B * L, 2 * H]: step size at H + h
-  const void* a;           // [B * L, lda]: decay input of head h at h * dim
-  long long lda;
-  const float* neg_rate;   // [H] -exp(A)
-  const float* dt_bias;    // [H * dim]
-  float* coef;             // [B, groups, H, size()]
-  float* state;            // [B, H, dim, vdim]
-  long long state_bs;
-  void* o;                 // [B * L, H * vdim]
-  long long ldo;
-  int B, L, H, KH, dim, vdim, groups, fresh;
-  // Per group and head: [DC][2 * DC] inverse (times beta) and kq, then rows of DK floats: DC times P_i k_i, DC times P_i q_i, DC times
-  // k_j g_{j+1} .. g_C, P_C; DK = 64, 128 or 256 (the state rows the scan kernel is built for), zero beyond dim.
-  int DK;
-  __host__ __device__ int size() const { return 2 * DC * DC + (3 * DC + 1) * DK; }
-};
 
 // One warp per (group, head, sequence).  VC channels per lane side by side, so that all of a warp's loads of a pass are in flight together
 // and are whole lines; DK = 32 * VC * passes.

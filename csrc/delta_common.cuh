@@ -49,4 +49,40 @@ __device__ __forceinline__ void inverse_column(const float (&beta)[DC], const KK
   }
 }
 
+// A portion of a prompt: ats_delta_scan (groups of DC tokens) and ats_delta_scan_mma (groups of 16).
+struct ScanArgs {
+  const void* mixed;
+  long long ldm;
+  const float* rlen;
+  const float* gb;
+  float* coef;             // [B, groups, H, .]: constants of a group and head, as the scan kernel wants them
+  float* state;            // [B, H, dim, vdim]
+  long long state_bs;
+  void* o;                 // [B * L, H * vdim]
+  long long ldo;
+  int B, L, H, KH, dim, vdim, groups, fresh;
+};
+
+// The same with one decay per state row: ats_channel_delta (groups of DC tokens), ats_channel_delta_mma (groups of 16, another layout of coef).
+struct ChannelArgs {
+  const void* mixed;       // [B * L, ldm] convolved q, k, v
+  long long ldm;
+  const float* rlen;       // [B * L, 2 * KH] dim^-1/2 / |q|, 1 / |k|
+  const float* gb;         // [B * L, 2 * H]: step size at H + h
+  const void* a;           // [B * L, lda]: decay input of head h at h * dim
+  long long lda;
+  const float* neg_rate;   // [H] -exp(A)
+  const float* dt_bias;    // [H * dim]
+  float* coef;             // [B, groups, H, size()]
+  float* state;            // [B, H, dim, vdim]
+  long long state_bs;
+  void* o;                 // [B * L, H * vdim]
+  long long ldo;
+  int B, L, H, KH, dim, vdim, groups, fresh;
+  // Per group and head: [DC][2 * DC] inverse (times beta) and kq, then rows of DK floats: DC times P_i k_i, DC times P_i q_i, DC times
+  // k_j g_{j+1} .. g_C, P_C; DK = 64, 128 or 256 (the state rows the scan kernel is built for), zero beyond dim.
+  int DK;
+  __host__ __device__ int size() const { return 2 * DC * DC + (3 * DC + 1) * DK; }
+};
+
 }  // namespace ats

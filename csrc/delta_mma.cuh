@@ -1,0 +1,102 @@
+// Warp-level tensor-core pieces of the delta-rule scans (delta_rule_mma.cu): fp32 operands as sums of bf16 values, fragments, asynchronous copies.
+//
+// An fp32 value has 24 significant bits, three bf16 values have 8 each: cut off after every eight bits, the pieces add up to the value exactly,
+// and a product of a piece with a bf16 number is exact in fp32.  So a product of an fp32 matrix with a bf16 one is three
+// tensor-core products, one of two fp32 matrices six (the three pairs of pieces left out are below 2^-24 of the product).
+#pragma once
+#include "delta_common.cuh"
+
+namespace ats {
+
+struct Pieces {   // of an A fragment (16 x 16): hi + mid + lo
+  uint32_t hi[4], mid[4], lo[4];
+};
+
+// Two neighbouring values of a row as three words of two bf16 each.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
+  hi = __byte_perm(ux, uy, 0x7632);
+  const float rx = x - __uint_as_float(ux & 0xffff0000u), ry = y - __uint_as_float(uy & 0xffff0000u);
+  const uint32_t vx = __float_as_uint(rx), vy = __float_as_uint(ry);
+  mid = __byte_perm(vx, vy, 0x7632);
+  lo = __byte_perm(__float_as_uint(rx - __uint_as_float(vx & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(vy & 0xffff0000u)), 0x7632);
+}
+
+// Accumulator tiles of columns 0..7 (a) and 8..15 (b) of a 16 x 16 block as the A operand of the next product.
+__device__ __forceinline__ void split_tiles(const float (&a)[4], const float (&b)[4], Pieces& p) {
+  split_pair(a[0], a[1], p.hi[0], p.mid[0], p.lo[0]);
+  split_pair(a[2], a[3], p.hi[1], p.mid[1], p.lo[1]);
+  split_pair(b[0], b[1], p.hi[2], p.mid[2], p.lo[2]);
+  split_pair(b[2], b[3], p.hi[3], p.mid[3], p.lo[3]);
+}
+
+__device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+// Tensor-core sums are cut off at the last place of the result: all in one direction, half a unit on average.  With c = a x b so computed, adds what was cut
+// off to `small`: the same product on top of -c.  (State of the scan after 300 tokens, relative error against 64 bits 1.28e-7 -> 0.92e-7.)
+__device__ __forceinline__ void add_rest(const float (&c)[4], float (&small)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  float rest[4] = {-c[0], -c[1], -c[2], -c[3]};
+  mma_bf16(rest, a, b0, b1);
+#pragma unroll
+  for (int e = 0; e < 4; ++e) small[e] += rest[e];
+}
+__device__ __forceinline__ void ldsm4(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void ldsm4_t(uint32_t (&r)[4], uint32_t addr) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+__device__ __forceinline__ void stsm4_t(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+// 16 bytes, of which the first `bytes` are read and the rest is zero
+__device__ __forceinline__ void cp_async_fill(uint32_t dst, const void* src, int bytes) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(bytes) : "memory");
+}
+
+// A 16 x 16 fp32 matrix M in shared memory (row pitch 17) as three B operands, element [k][n] = M[n][k]; per piece a lane's 16 bytes: rows
+// n = 0..7 with k = 0..7 and 8..15, then rows 8..15.
+__device__ __forceinline__ void store_split_b(const float (*m)[17], int lane, uint4* dst) {
+  const int g = lane >> 2, t = lane & 3;
+  uint32_t hi[4], mid[4], lo[4];
+#pragma unroll
+  for (int x = 0; x < 4; ++x) {
+    const int i = g + 8 * (x >> 1), j = 2 * t + 8 * (x & 1);
+    split_pair(m[i][j], m[i][j + 1], hi[x], mid[x], lo[x]);
+  }
+  dst[lane] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+  dst[32 + lane] = make_uint4(mid[0], mid[1], mid[2], mid[3]);
+  dst[64 + lane] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+}
+
+// c[2] (16 rows x 16 columns) = a x b for split operands, b as store_split_b leaves it: the large products and the small ones are summed apart.
+__device__ __forceinline__ void split_product(const Pieces& a, const uint4* b, int lane, float (&c)[2][4]) {
+  const uint4 bh = b[lane], bm = b[32 + lane], bl = b[64 + lane];
+  float small[2][4];
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[n][e] = small[n][e] = 0.f;
+  mma_bf16(small[0], a.lo, bh.x, bh.y);
+  mma_bf16(small[1], a.lo, bh.z, bh.w);
+  mma_bf16(c[0], a.hi, bh.x, bh.y);
+  mma_bf16(c[1], a.hi, bh.z, bh.w);
+  mma_bf16(small[0], a.hi, bl.x, bl.y);
+  mma_bf16(small[1], a.hi, bl.z, bl.w);
+  mma_bf16(small[0], a.mid, bm.x, bm.y);
+  mma_bf16(small[1], a.mid, bm.z, bm.w);
+  mma_bf16(small[0], a.mid, bh.x, bh.y);
+  mma_bf16(small[1], a.mid, bh.z, bh.w);
+  mma_bf16(small[0], a.hi, bm.x, bm.y);
+  mma_bf16(small[1], a.hi, bm.z, bm.w);
+  add_rest(c[0], small[0], a.hi, bh.x, bh.y);
+  add_rest(c[1], small[1], a.hi, bh.z, bh.w);
+#pragma unroll
+  for (int n = 0; n < 2; ++n)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) c[n][e] += small[n][e];
+}
+
+}  // namespace ats

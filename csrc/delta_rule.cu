@@ -15,7 +15,8 @@
 // * delta_output: output norm over vdim, weight, silu gate.
 // * delta_step: one decoded token per sequence: state read once and written once, output norm and gate in the same launch.
 //
-// channel_delta.cu holds the portion kernels of the form with one decay per state row; it shares delta_prep (without the decays),
+// delta_rule_mma.cu holds the portion kernels for bf16 rows of whole 16-byte pieces and up to 128 state rows (two to three times as fast); those below serve fp32,
+// larger states and odd widths.  channel_delta.cu holds the portion kernels of the form with one decay per state row; it shares delta_prep (without the decays),
 // delta_output and delta_step.
 //
 // A sequence at position 0 starts from a zero state and zero convolution inputs whatever its buffers hold.
@@ -209,19 +210,6 @@ __global__ void __launch_bounds__(256) delta_tail_kernel(const DeltaArgs p) {
 // G_i / |k_i|, G_i dim^-1/2 / |q_i|, D_Ci / |k_i| (G_i = g_1 .. g_i, D_Ci = g_{i+1} .. g_C), then G_C: with the lengths folded in
 // here, the sequential kernel works on the raw q and k.
 constexpr int CO = 2 * DC * DC + 3 * DC + 8;
-
-struct ScanArgs {
-  const void* mixed;
-  long long ldm;
-  const float* rlen;
-  const float* gb;
-  float* coef;             // [B, groups, H, CO]: see CO
-  float* state;            // [B, H, dim, vdim]
-  long long state_bs;
-  void* o;                 // [B * L, H * vdim]
-  long long ldo;
-  int B, L, H, KH, dim, vdim, groups, fresh;
-};
 
 // 16 x 8 products of one group: rows 0..7 k_i . k_j, rows 8..15 q_i . k_j, sums over dim.  bf16 values: exact products accumulated in
 // fp32 by a warp-level MMA, whose B fragment is the same registers as the upper half of A (the order of the reduction is

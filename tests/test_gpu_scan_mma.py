@@ -1,0 +1,75 @@
+"""Delta scans on the tensor cores (``csrc/delta_rule_mma.cu``, ``csrc/channel_delta_mma.cu``) against the recurrence in 64 bits and the scans in fp32 FMAs."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def _inputs(channel, B, L, H, KH, dim, vdim, slow):
+    from adaptivetrainingsystem_b200.ops import delta as D
+    g = torch.Generator(device="cuda").manual_seed(B + L + H + dim + vdim)
+
+    def r(*shape):
+        return torch.randn(*shape, generator=g, device="cuda")
+    if channel:
+        s = D.ChannelDeltaShape(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5, decay_rank=8, gate_rank=8)
+    else:
+        s = D.DeltaShape(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5)
+    proj, conv, tail = r(B, L, s.proj_width).bfloat16(), r(s.taps, s.channels) * 0.5, r(B, 3, s.channels).bfloat16()
+    rate, shift = -torch.exp(r(H) * 0.5), -6.0 if slow else -2.0
+    start = r(2 * B, H, dim, vdim)[::2]      # sequences that do not lie side by side
+    if channel:
+        mixed, rlen, gb = D.delta_prep(proj, s, conv, None, None, tail)
+        a, bias = r(B * L, H * dim).bfloat16(), r(H * dim) * 0.5 + shift
+        decay = torch.exp(rate.double()[:, None] * torch.nn.functional.softplus(a.double() + bias.double()).view(-1, H, dim)).view(B, L, H, dim)
+
+        def scan(state, fresh):
+            return D.channel_delta_scan(mixed, rlen, gb, a, rate, bias, state, s, L, fresh)
+    else:
+        mixed, rlen, gb = D.delta_prep(proj, s, conv, rate, r(H) * 0.5 + shift, tail)
+        decay = gb.double()[:, :H].view(B, L, H, 1)
+
+        def scan(state, fresh):
+            return D.delta_scan(mixed, rlen, gb, state, s, L, fresh)
+    return s, mixed, rlen, gb, decay, start, scan
+
+
+def _exact(s, mixed, rlen, gb, decay, start, L, fresh):
+    B, H, KH, dim = start.shape[0], s.heads, s.kv_heads, s.dim
+    m, rl = mixed.double(), rlen.double()
+    q = (m[:, :KH * dim].view(B, L, KH, dim) * rl[:, :KH].view(B, L, KH, 1)).repeat_interleave(H // KH, 2)
+    k = (m[:, KH * dim:2 * KH * dim].view(B, L, KH, dim) * rl[:, KH:].view(B, L, KH, 1)).repeat_interleave(H // KH, 2)
+    v, beta = m[:, 2 * KH * dim:s.channels].view(B, L, H, s.vdim), gb.double()[:, H:].view(B, L, H, 1)
+    S, out = (torch.zeros_like(start) if fresh else start).double(), []
+    for t in range(L):
+        S = S * decay[:, t, :, :, None]
+        u = beta[:, t] * (v[:, t] - torch.einsum("bhdv,bhd->bhv", S, k[:, t]))
+        S = S + k[:, t, :, :, None] * u[:, :, None, :]
+        out.append(torch.einsum("bhdv,bhd->bhv", S, q[:, t]))
+    return torch.stack(out, 1).view(B * L, -1), S
+
+
+# lengths around the groups of 16 tokens and their halves; state rows and columns around the tiles of 64, 128 and 16; one to three heads a key head
+@pytest.mark.parametrize("B,L,H,KH,dim,vdim,slow", [(1, 1, 2, 2, 128, 128, False), (2, 8, 3, 1, 8, 8, False), (2, 15, 4, 2, 64, 96, True), (1, 16, 2, 1, 72, 40, False),
+                                                    (3, 17, 3, 3, 128, 64, False), (1, 25, 6, 2, 120, 16, True), (2, 331, 4, 2, 128, 128, True)])
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("fresh", [False, True])
+def test_against_recurrence_and_fma_scan(monkeypatch, channel, B, L, H, KH, dim, vdim, slow, fresh):
+    from adaptivetrainingsystem_b200.ops import delta as D
+    s, mixed, rlen, gb, decay, start, scan = _inputs(channel, B, L, H, KH, dim, vdim, slow)
+    assert D.scan_on_tensor_cores(mixed, s)
+    state = start.clone()
+    out = scan(state, fresh)
+    want, S = _exact(s, mixed, rlen, gb, decay, start, L, fresh)
+    monkeypatch.setattr(D, "scan_on_tensor_cores", lambda *_: False)
+    fma_state = start.clone()
+    fma_out = scan(fma_state, fresh)
+
+    def rel(a, b):
+        return float((a.double() - b).norm() / b.norm())
+    # Read-outs carry the rounding to bf16 (2^-9 an element at most).  States: 32-bit sums; with a decay per row the error of the fast exponential of
+    # each token's decay (a few 1e-7) adds up over the tokens that a state remembers.  Neither is further off than the FMA scan by more than
+    # rounding errors differ from one order of sums to another.
+    assert rel(out, want) < 2.0 ** -8
+    assert rel(state, S) < (4e-6 if channel else 6e-7)
+    assert rel(state, S) < 1.5 * rel(fma_state, S) + 6e-8 and rel(out, want) < rel(fma_out, want) + 1e-5
