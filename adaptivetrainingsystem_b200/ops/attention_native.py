@@ -78,8 +78,8 @@ def _fwd(q, k, v):
     return out, lse
 
 
-# Diagnostics: set to an int64 CUDA tensor of 32 elements to receive per-phase cycle totals of one CTA of each backward
-# pass ([0:16] dK/dV pass, [16:32] dQ pass: total, waits of the MMA thread, issue time; [8:13] phases of one softmax warp).
+# Diagnostics: set to an int64 CUDA tensor of 32 elements to receive cycle totals of one CTA of each backward pass ([0:16] dK/dV pass,
+# [16:32] dQ pass; [0] all, [1] waits of the thread that issues the products, [5] iterations).
 PHASE_PROFILE = None
 
 

@@ -88,10 +88,8 @@ def main():
         AN.PHASE_PROFILE = AN.FWD_PHASE_PROFILE = None
         out["phases_fwd"] = dict(zip(["total", "wait_v", "wait_p", "issue", "iterations"], fp[:5]))
         out["phases_fwd"].update(dict(zip(["sm_wait_s", "sm_tmem_load", "sm_max", "sm_exp_store", "sm_signal"], fp[8:13])))
-        names = ["total", "wait_tile", "wait_scores_read", "wait_p_ds", "issue", "iterations", "", "", "sm_wait_scores", "sm_tmem_load", "sm_math",
-                 "sm_wait_products", "sm_store"]
-        out["phases_dkv"] = {n: v for n, v in zip(names, pp[:13]) if n}
-        out["phases_dq"] = {n: v for n, v in zip(names, pp[16:29]) if n}
+        for name, at in (("phases_dkv", 0), ("phases_dq", 16)):   # of the thread that issues the products
+            out[name] = {"total": pp[at], "waits": pp[at + 1], "iterations": pp[at + 5]}
     ops.check_status()
     print(json.dumps(out))
 

@@ -8,10 +8,20 @@
 //   MODE 1 (dQ):     one CTA per (128-query tile i, query head, batch).  Q_i and dO_i stay resident, K_j / V_j stream for
 //           j <= i, and dQ += dS K accumulates in TMEM; dS goes back to tensor memory as bf16 and is the MMA's A operand.
 // S and dP are recomputed in both passes (7 tile products per tile pair instead of 5) in exchange for an atomics-free,
-// deterministic dQ.  P and dS live in shared memory as [query x key] bf16 tiles in the 128-byte-swizzled layout, which
-// the same bytes serve both as a K-major operand (dS K) and as an MN-major operand (P^T dO, dS^T Q).
+// deterministic dQ.
 //
-//   warp 0: TMA producer   warp 1: TMEM owner + MMA issuer   warps 2..9: two threads per query row (64 key columns each)
+// The dK/dV pass needs P^T and dS^T as A operands.
+//   64 dimensions:  P and dS go to shared memory as [query x key] bf16 tiles in the 128-byte-swizzled layout, which the same bytes serve as an
+//           MN-major operand.
+//   128 dimensions (OVER): those tiles would take the room of a second stage, and copies, products and exponentials would follow one another
+//           (568 us for one sequence of 4,096 tokens, 32 / 8 heads).  So the scores are computed transposed, S^T = K Q^T and dP^T = V dO^T, with keys
+//           as the lanes of tensor memory: P^T and dS^T are written over the scores they come from and are read from there.  The scores of pair t + 1
+//           run under dS of pair t, dP of t + 1 under the exponentials of t + 1: 309 us.  At 64 dimensions that form is the slower one (579 us
+//           against 543 for 8 x 2,048 tokens, 32 / 4 heads): products with an A operand in tensor memory and 64 columns take longer than from shared
+//           memory, and the statistics of a query are read per column.
+// In the other forms the scores of pair t + 1 run as soon as S of pair t is in registers, dP of t + 1 as soon as dP of t is (dQ pass 446 -> 435 us).
+//
+//   warp 0: TMA producer   warp 1: TMEM owner + MMA issuer   warps 2..9: two threads per row of the scores (64 columns each)
 // Any sequence length: rows behind the end of a sequence read as zero (its length is a dimension of the tensor maps).  Queries there get a
 // log-sum-exp of infinity, so their P and dS vanish; keys there are behind every real query; neither is stored.
 // Every wait is bounded (status word + clean unwind); no load uses cluster multicast.
@@ -23,11 +33,8 @@ namespace ats {
 
 int make_tmap_batched(CUtensorMap* out, const void* base, uint64_t cols, uint64_t rows, uint64_t batch, uint64_t ld, uint64_t batch_stride, uint32_t box_rows);
 
-#ifndef ATS_AB_SPLIT
-#define ATS_AB_SPLIT 2
-#endif
-constexpr int AB_SPLIT = ATS_AB_SPLIT;             // threads per query row in the softmax-gradient stage (2 or 4)
-constexpr int AB_COLS = 128 / AB_SPLIT;           // key columns per thread
+constexpr int AB_SPLIT = 2;                       // threads per row of the scores in the softmax-gradient stage
+constexpr int AB_COLS = 128 / AB_SPLIT;           // columns per thread
 constexpr int AB_THREADS = 64 + 128 * AB_SPLIT;   // TMA warp, MMA warp, 4 * AB_SPLIT softmax-gradient warps
 
 struct AttnBwdArgs {
@@ -41,21 +48,23 @@ struct AttnBwdArgs {
   long long ld_dq, ld_dkv;
   float scale, scale_log2;
   int* status;
-  long long* prof;  // optional [16]: cycle totals per phase, written by one CTA (diagnostics; null in normal use)
+  long long* prof;  // optional [16]: cycle totals, written by one CTA (diagnostics; null in normal use)
 };
 
 template <int D, int MODE>
 struct AttnBwdSmem {
   // streamed stages: a stage is held until the gradient products that read it have finished, and a refill takes a
   // TMA round trip, so the ring must be deep enough to have the next tiles in flight meanwhile
-  static constexpr int ST = (D == 64) ? 4 : (MODE == 1 ? 2 : 1);
+  static constexpr int ST = (D == 64) ? 4 : 2;
   static constexpr int TB = 128 * D * 2;
   static constexpr int R1 = 0, R2 = TB;
   static constexpr int T1 = 2 * TB;            // ST stages
   static constexpr int T2 = T1 + ST * TB;      // ST stages
-  static constexpr int P_OFF = T2 + ST * TB;   // MODE 0 only
-  static constexpr int DS_OFF = P_OFF + (MODE == 0 ? 32768 : 0);
-  static constexpr int BAR_OFF = DS_OFF + (MODE == 0 ? 32768 : 0);  // the dQ pass keeps dS in tensor memory
+  static constexpr bool OVER = MODE == 0 && D == 128;
+  static constexpr int P_OFF = T2 + ST * TB;     // MODE 0 at 64 dimensions: P, dS
+  static constexpr int DS_OFF = P_OFF + (MODE == 0 && !OVER ? 32768 : 0);
+  static constexpr int ROW_OFF = DS_OFF + (MODE == 0 && !OVER ? 32768 : 0);   // OVER: [2][-lse, -delta][128 queries] of two iterations
+  static constexpr int BAR_OFF = ROW_OFF + (OVER ? 2048 : 0);
   static constexpr int TOTAL = BAR_OFF + 256 + 1024;
 };
 
@@ -99,16 +108,20 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   uint8_t* sT2 = smem + SM::T2;
   uint8_t* sP = smem + SM::P_OFF;
   uint8_t* sDS = smem + SM::DS_OFF;
+  float* sRow = reinterpret_cast<float*>(smem + SM::ROW_OFF);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + SM::BAR_OFF);
   uint64_t* res_full = bars;       // 1
   uint64_t* t_full = bars + 1;     // [4]
   uint64_t* t_empty = bars + 5;    // [4]
-  uint64_t* s_full = bars + 9;     // S and dP ready
-  uint64_t* sd_free = bars + 10;   // one arrival per softmax warp: S / dP read out of TMEM
-  uint64_t* pds_full = bars + 11;  // one arrival per softmax warp: P / dS written to shared memory
-  uint64_t* pds_free = bars + 12;  // accumulate MMAs have consumed P / dS
-  uint64_t* acc_done = bars + 13;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 14);
+  uint64_t* s_full = bars + 9;     // S ready
+  uint64_t* dp_full = bars + 10;   // dP ready
+  uint64_t* s_free = bars + 11;    // one arrival per softmax warp: S read out of TMEM
+  uint64_t* dp_free = bars + 12;   // the same for dP
+  uint64_t* p_full = bars + 13;    // OVER: one arrival per softmax warp, P written to TMEM
+  uint64_t* ds_full = bars + 14;   // the same for dS (VIA_SMEM: P and dS written to shared memory)
+  uint64_t* ds_free = bars + 15;   // without OVER: the products that read P and dS are done
+  uint64_t* acc_done = bars + 16;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -138,9 +151,12 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       mbar_init(&t_empty[s], 1);
     }
     mbar_init(s_full, 1);
-    mbar_init(sd_free, 4 * AB_SPLIT);
-    mbar_init(pds_full, 4 * AB_SPLIT);
-    mbar_init(pds_free, 1);
+    mbar_init(dp_full, 1);
+    mbar_init(s_free, 4 * AB_SPLIT);
+    mbar_init(dp_free, 4 * AB_SPLIT);
+    mbar_init(p_full, 4 * AB_SPLIT);
+    mbar_init(ds_full, 4 * AB_SPLIT);
+    mbar_init(ds_free, 1);
     mbar_init(acc_done, 1);
     *abort_flag = 0;
     mbar_fence_init();
@@ -158,7 +174,11 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   const uint32_t tmem_S = tmem_base, tmem_dP = tmem_base + 128, tmem_A1 = tmem_base + 256, tmem_A2 = tmem_base + 256 + D;
-  const uint32_t tmem_dS = tmem_base + 384;  // MODE 1: dS as bf16 pairs, 64 columns, the A operand of dQ += dS K
+  // OVER: P and dS as bf16 pairs over the scores that their thread has read, so the second half of the columns starts 64 further on.  MODE 1: dS
+  // in 64 columns of its own.
+  constexpr bool OVER = SM::OVER, VIA_SMEM = MODE == 0 && !OVER;
+  const uint32_t tmem_P = tmem_S, tmem_dS = OVER ? tmem_dP : tmem_base + 384;
+  constexpr uint32_t HALF = OVER ? 64 : 32;   // columns from the first 64 reduction elements to the others
 
   // iteration t -> (query head, query tile, key tile)
   auto decode = [&](int t, int& h, int& qi, int& kj) {
@@ -225,195 +245,242 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     if (lane == 0) {
       // ------------------------------------------------------------------ MMA issuer
       const uint32_t idesc_s = make_idesc(128, 128, 1, 1, 0, 0);
-      const uint32_t idesc_acc0 = make_idesc(128, D, 1, 1, 1, 1);  // A^T B with both operands MN-major
-      const uint32_t idesc_acc1 = make_idesc(128, D, 1, 1, 0, 1);  // dS (K-major) x K (MN-major)
+      const uint32_t idesc_acc = make_idesc(128, D, 1, 1, VIA_SMEM, 1);  // A from tensor memory or MN-major, B MN-major
       // Descriptors are built once: per operand one base descriptor for the K-major view and one for the MN-major view;
       // inside the loops a descriptor is the base plus a constant (the issue rate of this one thread bounds the kernel).
       const uint64_t r1_k = make_smem_desc_sw128(smem_u32(sR1), 16, 1024), r2_k = make_smem_desc_sw128(smem_u32(sR2), 16, 1024);
-      const uint64_t r1_mn = make_smem_desc_sw128(smem_u32(sR1), 16384, 1024), r2_mn = make_smem_desc_sw128(smem_u32(sR2), 16384, 1024);
       const uint64_t t1_k = make_smem_desc_sw128(smem_u32(sT1), 16, 1024), t2_k = make_smem_desc_sw128(smem_u32(sT2), 16, 1024);
       const uint64_t t1_mn = make_smem_desc_sw128(smem_u32(sT1), 16384, 1024), t2_mn = make_smem_desc_sw128(smem_u32(sT2), 16384, 1024);
       const uint64_t p_mn = make_smem_desc_sw128(smem_u32(sP), 16384, 1024), ds_mn = make_smem_desc_sw128(smem_u32(sDS), 16384, 1024);
-      auto issue_scores = [&](int t) {  // S = Q K^T and dP = dO V^T of iteration t
-        const uint32_t so = uint32_t(t % ST) * SM::TB;
-        const uint64_t q_d = MODE == 0 ? desc_advance(t1_k, so) : r1_k, do_d = MODE == 0 ? desc_advance(t2_k, so) : r2_k;
-        const uint64_t k_d = MODE == 0 ? r1_k : desc_advance(t1_k, so), v_d = MODE == 0 ? r2_k : desc_advance(t2_k, so);
+      // S (which = 0: R1 and T1) or dP (1: R2 and T2) of iteration t; lanes are the rows of the resident tile, VIA_SMEM: of the streamed one
+      auto issue_score = [&](int t, int which) {
+        const uint64_t fixed_d = which ? r2_k : r1_k, moving = desc_advance(which ? t2_k : t1_k, uint32_t(t % ST) * SM::TB);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-          tc_mma_f16(tmem_S, desc_advance(q_d, off), desc_advance(k_d, off), idesc_s, k != 0);
+          const uint64_t f = desc_advance(fixed_d, off), m = desc_advance(moving, off);
+          tc_mma_f16(which ? tmem_dP : tmem_S, VIA_SMEM ? m : f, VIA_SMEM ? f : m, idesc_s, k != 0);
         }
-#pragma unroll
-        for (int k = 0; k < D / 16; ++k) {
-          const uint32_t off = (k >> 2) * 16384 + (k & 3) * 32;
-          tc_mma_f16(tmem_dP, desc_advance(do_d, off), desc_advance(v_d, off), idesc_s, k != 0);
-        }
-        tc_commit(s_full);
+        tc_commit(which ? dp_full : s_full);
       };
-      auto issue_acc = [&](int t) {  // the gradient products that consume P / dS of iteration t
-        const int s = t % ST;
-        const uint32_t so = uint32_t(s) * SM::TB;
-        if (MODE == 0) {
-          const uint64_t do_d = desc_advance(t2_mn, so), q_d = desc_advance(t1_mn, so);
+      auto issue_acc = [&](int t, uint32_t acc, uint32_t a, uint64_t rows_mn) {   // reduction over the 128 rows of the streamed tile, 16 per step
+        const uint64_t bb = desc_advance(rows_mn, uint32_t(t % ST) * SM::TB);
 #pragma unroll
-          for (int k = 0; k < 8; ++k)  // reduction over the 128 queries, 16 per step
-            tc_mma_f16(tmem_A1, desc_advance(p_mn, k * 2048), desc_advance(do_d, k * 2048), idesc_acc0, (t | k) != 0);
+        for (int k = 0; k < 8; ++k) tc_mma_f16_ts(acc, a + (k >> 2) * HALF + (k & 3) * 8, desc_advance(bb, k * 2048), idesc_acc, (t | k) != 0);
+      };
+      auto issue_acc_smem = [&](int t, uint32_t acc, uint64_t a_mn, uint64_t rows_mn) {
+        const uint64_t bb = desc_advance(rows_mn, uint32_t(t % ST) * SM::TB);
 #pragma unroll
-          for (int k = 0; k < 8; ++k) tc_mma_f16(tmem_A2, desc_advance(ds_mn, k * 2048), desc_advance(q_d, k * 2048), idesc_acc0, (t | k) != 0);
+        for (int k = 0; k < 8; ++k) tc_mma_f16(acc, desc_advance(a_mn, k * 2048), desc_advance(bb, k * 2048), idesc_acc, (t | k) != 0);
+      };
+      long long waited = 0, c0 = 0;
+      const bool rec = p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
+      auto wait = [&](uint64_t* bar, int parity, int code) {
+        if (rec) c0 = clock64();
+        const bool got = mbar_wait_bounded(bar, parity, abort_flag, p.status, code);
+        if (rec) waited += clock64() - c0;
+        tc_fence_after();
+        return got;
+      };
+      const long long t_begin = clock64();
+      bool ok = wait(res_full, 0, kTimeoutFull) && (n_iter == 0 || wait(&t_full[0], 0, kTimeoutFull));
+      if (ok && n_iter > 0) {
+        issue_score(0, 0);
+        issue_score(0, 1);
+      }
+      for (int t = 0; ok && t < n_iter; ++t) {
+        const bool more = t + 1 < n_iter;
+        auto next_scores = [&] {
+          ok = ok && wait(&t_full[(t + 1) % ST], ((t + 1) / ST) & 1, kTimeoutFull) && (OVER || wait(s_free, t & 1, kTimeoutTmemEmpty));
+          if (ok) issue_score(t + 1, 0);
+        };
+        auto next_dp = [&] {
+          ok = ok && (OVER || wait(dp_free, t & 1, kTimeoutTmemEmpty));
+          if (ok) issue_score(t + 1, 1);
+        };
+        if (OVER) {
+          ok = ok && wait(p_full, t & 1, kTimeoutTmemFull);
+          if (!ok) break;
+          issue_acc(t, tmem_A1, tmem_P, t2_mn);   // dV += P^T dO
+          if (more) next_scores();   // (products are executed in the order of their issue: P has been read when S is written)
+        } else if (more) {
+          next_scores();
+          next_dp();
+        }
+        ok = ok && wait(ds_full, t & 1, kTimeoutTmemFull);
+        if (!ok) break;
+        if (VIA_SMEM) {
+          issue_acc_smem(t, tmem_A1, p_mn, t2_mn);
+          issue_acc_smem(t, tmem_A2, ds_mn, t1_mn);
         } else {
-          const uint64_t k_d = desc_advance(t1_mn, so);
-#pragma unroll
-          for (int k = 0; k < 8; ++k)  // reduction over the 128 keys; dS is read from tensor memory (8 columns per 16 keys)
-            tc_mma_f16_ts(tmem_A1, tmem_dS + k * 8, desc_advance(k_d, k * 2048), idesc_acc1, (t | k) != 0);
+          issue_acc(t, MODE == 0 ? tmem_A2 : tmem_A1, tmem_dS, t1_mn);   // dK += dS^T Q, dQ += dS K
         }
-        tc_commit(pds_free);
-        tc_commit(&t_empty[s]);
-      };
-      bool ok = mbar_wait_bounded(res_full, 0, abort_flag, p.status, kTimeoutFull);
-      if (ST >= 2) {
-        // The scores of iteration t + 1 are issued as soon as the soft-max threads have S / dP of iteration t in registers,
-        // so the tensor cores work on them while those threads do the exponentials of iteration t.
-        ok = ok && mbar_wait_bounded(&t_full[0], 0, abort_flag, p.status, kTimeoutFull);
-        if (ok) {
-          tc_fence_after();
-          issue_scores(0);
-        }
-        const bool rec = p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0;
-        long long w_tfull = 0, w_sdfree = 0, w_pdsfull = 0, t_issue = 0, c0 = 0, c1 = 0;
-        const long long t_begin = clock64();
-        for (int t = 0; ok && t < n_iter; ++t) {
-          if (t + 1 < n_iter) {
-            if (rec) c0 = clock64();
-            if (!mbar_wait_bounded(&t_full[(t + 1) % ST], ((t + 1) / ST) & 1, abort_flag, p.status, kTimeoutFull)) break;
-            if (rec) { c1 = clock64(); w_tfull += c1 - c0; }
-            if (!mbar_wait_bounded(sd_free, t & 1, abort_flag, p.status, kTimeoutTmemEmpty)) break;
-            if (rec) { c0 = clock64(); w_sdfree += c0 - c1; }
-            tc_fence_after();
-            issue_scores(t + 1);
-            if (rec) { c1 = clock64(); t_issue += c1 - c0; }
-          }
-          if (rec) c0 = clock64();
-          if (!mbar_wait_bounded(pds_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) break;
-          if (rec) { c1 = clock64(); w_pdsfull += c1 - c0; }
-          tc_fence_after();
-          issue_acc(t);
-          if (rec) { c0 = clock64(); t_issue += c0 - c1; }
-        }
-        if (rec) {
-          p.prof[0] = clock64() - t_begin;
-          p.prof[1] = w_tfull; p.prof[2] = w_sdfree; p.prof[3] = w_pdsfull; p.prof[4] = t_issue; p.prof[5] = n_iter;
-        }
-      } else {
-        // one streamed stage: the next tile can only be fetched after this iteration's products, so the order is serial
-        for (int t = 0; ok && t < n_iter; ++t) {
-          if (!mbar_wait_bounded(&t_full[0], t & 1, abort_flag, p.status, kTimeoutFull)) break;
-          if (!mbar_wait_bounded(sd_free, (t & 1) ^ 1, abort_flag, p.status, kTimeoutTmemEmpty)) break;
-          tc_fence_after();
-          issue_scores(t);
-          if (!mbar_wait_bounded(pds_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) break;
-          tc_fence_after();
-          issue_acc(t);
-        }
+        if (!OVER) tc_commit(ds_free);
+        tc_commit(&t_empty[t % ST]);
+        if (OVER && more) next_dp();
+      }
+      if (rec) {
+        p.prof[0] = clock64() - t_begin;
+        p.prof[1] = waited;
+        p.prof[5] = n_iter;
       }
       tc_commit(acc_done);
     }
   } else {
     // ---------------------------------------- softmax-gradient threads: a TMEM lane quadrant is open to warps with the
-    // same (warp % 4), so the AB_SPLIT warps w, w + 4, ... share 32 query rows and take AB_COLS key columns each
+    // same (warp % 4), so the AB_SPLIT warps w, w + 4, ... share 32 rows and take AB_COLS columns each
     const int quad = warp & 3;
     const int part = (warp - 2) >> 2;  // which AB_COLS key columns of the 128
     const int r = quad * 32 + lane;
     const uint32_t lane_base = uint32_t(quad * 32) << 16;
     bool ok = true;
-    // log-sum-exp and delta of this thread's query row, fetched one iteration ahead so the loads never sit on the critical path
-    auto row_stats = [&](int t, float& l2, float& d) {
-      int h, qi, kj;
-      decode(t, h, qi, kj);
-      const long long idx = ((long long)b * p.Hq + h) * p.L + qi * 128 + r;
-      const bool real = qi * 128 + r < p.L;
-      l2 = real ? p.lse[idx] * 1.4426950408889634f : INFINITY;
-      d = real ? p.delta[idx] : 0.f;
+    // Query tile and head of the next statistics to fetch (MODE 1: of all of them), and of the iteration at hand whether it is on the diagonal.
+    int tile = fixed, stat_head = MODE == 0 ? head * rep : head, to_diagonal = 0;
+    // log-sum-exp (times -log2 e) and delta (times -scale) of query `row` of that tile
+    auto row_stat = [&](int row, bool lse) {
+      const long long idx = ((long long)b * p.Hq + stat_head) * p.L + tile * 128 + row;
+      const bool real = tile * 128 + row < p.L;
+      return lse ? (real ? p.lse[idx] * -1.4426950408889634f : -INFINITY) : (real ? -p.delta[idx] * p.scale : 0.f);
     };
-    float lse2 = 0.f, dl = 0.f, lse2_n = 0.f, dl_n = 0.f;
-    if (n_iter > 0) row_stats(0, lse2_n, dl_n);
+    auto next_tile = [&] {
+      if (++tile == nq) tile = fixed, ++stat_head;
+    };
+    // OVER: queries are the columns; each thread fetches one value an iteration ahead and leaves it in shared memory, where everyone reads it.
+    // Otherwise they are the rows, and a thread fetches those of its row (VIA_SMEM: of the next iteration's row, ahead).
+    const int id = int(threadIdx.x) - 64;
+    float row_l = 0.f, row_d = 0.f, ahead = 0.f, ahead_d = 0.f;
+    if (OVER) {
+      if (n_iter > 0) sRow[id] = row_stat(id & 127, id < 128);
+      next_tile();
+      if (n_iter > 1) ahead = row_stat(id & 127, id < 128);
+    } else if (n_iter > 0) {
+      row_l = ahead = row_stat(r, true), row_d = ahead_d = row_stat(r, false);
+    }
     const float2 sc2 = make_float2(p.scale_log2, p.scale_log2), scale2 = make_float2(p.scale, p.scale);
-    const bool rec = p.prof != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && warp == 2 && lane == 0;
-    long long w_sfull = 0, t_load = 0, t_math = 0, w_pdsfree = 0, t_store = 0, c0 = 0, c1 = 0;
+    const uint32_t col = lane_base + part * AB_COLS, bf_col = lane_base + part * HALF;
     for (int t = 0; t < n_iter; ++t) {
-      int h, qi, kj;
-      decode(t, h, qi, kj);
-      lse2 = lse2_n;
-      dl = dl_n;
-      if (t + 1 < n_iter && (MODE == 0)) row_stats(t + 1, lse2_n, dl_n);  // MODE 1 keeps the same query rows throughout
-      if (rec) c0 = clock64();
+      const bool diag = MODE == 0 ? to_diagonal == 0 : t == n_iter - 1;
+      if (MODE == 0 && ++to_diagonal == nq - fixed) to_diagonal = 0;
+      const float* nl = sRow + (t & 1) * 256 + part * AB_COLS;   // of this thread's columns; 128 floats on those of delta
+      if (OVER) {
+        asm volatile("bar.sync 1, %0;" ::"n"(128 * AB_SPLIT) : "memory");   // the values of this iteration are there, those of the one before are read
+        if (t + 1 < n_iter) sRow[((t + 1) & 1) * 256 + id] = ahead;
+        next_tile();
+        if (t + 2 < n_iter) ahead = row_stat(id & 127, id < 128);
+      } else if (VIA_SMEM) {
+        row_l = ahead, row_d = ahead_d;
+        next_tile();
+        if (t + 1 < n_iter) ahead = row_stat(r, true), ahead_d = row_stat(r, false);
+      }
       if (!mbar_wait_bounded(s_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) {
         ok = false;
         break;
       }
-      if (rec) { c1 = clock64(); w_sfull += c1 - c0; }
       tc_fence_after();
-      // this thread's columns of S, then of dP; the exponentials start while the dP load is still in flight
-      uint32_t sv[AB_COLS], dv[AB_COLS];
+      uint32_t sv[AB_COLS];
 #pragma unroll
-      for (int c = 0; c < AB_COLS / 32; ++c) tmem_ld_32x32(tmem_S + lane_base + part * AB_COLS + c * 32, reinterpret_cast<uint32_t(&)[32]>(sv[c * 32]));
+      for (int c = 0; c < AB_COLS / 32; ++c) tmem_ld_32x32(tmem_S + col + c * 32, reinterpret_cast<uint32_t(&)[32]>(sv[c * 32]));
       tmem_ld_wait();
-      if (rec) { c0 = clock64(); t_load += c0 - c1; }
-#pragma unroll
-      for (int c = 0; c < AB_COLS / 32; ++c) tmem_ld_32x32(tmem_dP + lane_base + part * AB_COLS + c * 32, reinterpret_cast<uint32_t(&)[32]>(dv[c * 32]));
-      const float2 nl2 = make_float2(-lse2, -lse2), ndl2 = make_float2(-dl, -dl);
-      const bool diag = (qi == kj);
-      float2 pr[AB_COLS / 2];
-      uint32_t pk[AB_COLS / 2], dk[AB_COLS / 2];
-#pragma unroll
-      for (int i = 0; i < AB_COLS / 2; ++i) {
-        const float2 xs = __ffma2_rn(make_float2(__uint_as_float(sv[2 * i]), __uint_as_float(sv[2 * i + 1])), sc2, nl2);
-        pr[i] = make_float2(exp2f(xs.x), exp2f(xs.y));
-        if (diag) {
-          if (part * AB_COLS + 2 * i > r) pr[i].x = 0.f;
-          if (part * AB_COLS + 2 * i + 1 > r) pr[i].y = 0.f;
-        }
-        pk[i] = pack_bf16x2(pr[i].x, pr[i].y);
+      if (!OVER) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(s_free);
       }
-      tmem_ld_wait();
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(sd_free);  // S and dP are in registers: the tensor cores may start the next scores
+      // dP^T or dP: without OVER it is on its way while the exponentials are taken
+      uint32_t dv[AB_COLS];
+      auto load_dp = [&] {
+        if (!mbar_wait_bounded(dp_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) return false;
+        tc_fence_after();
 #pragma unroll
-      for (int i = 0; i < AB_COLS / 2; ++i) {
-        const float2 dd = __fmul2_rn(__fmul2_rn(pr[i], scale2), __fadd2_rn(make_float2(__uint_as_float(dv[2 * i]), __uint_as_float(dv[2 * i + 1])), ndl2));
-        dk[i] = pack_bf16x2(dd.x, dd.y);
-      }
-      // the gradient products of the previous iteration must be done with P / dS before they are overwritten
-      if (rec) { c1 = clock64(); t_math += c1 - c0; }
-      if (!mbar_wait_bounded(pds_free, (t & 1) ^ 1, abort_flag, p.status, kTimeoutTmemEmpty)) {
+        for (int c = 0; c < AB_COLS / 32; ++c) tmem_ld_32x32(tmem_dP + col + c * 32, reinterpret_cast<uint32_t(&)[32]>(dv[c * 32]));
+        return true;
+      };
+      if (!OVER && !load_dp()) {
         ok = false;
         break;
       }
-      if (rec) { c0 = clock64(); w_pdsfree += c0 - c1; }
-      if (MODE == 1) {
-        // dQ pass: dS never touches shared memory
-        if (AB_COLS == 64) tmem_st_32x32(tmem_dS + lane_base + part * 32, reinterpret_cast<uint32_t(&)[32]>(dk[0]));
-        else tmem_st_32x16(tmem_dS + lane_base + part * 16, reinterpret_cast<uint32_t(&)[16]>(dk[0]));
+      float2 pr[AB_COLS / 2];
+#pragma unroll
+      for (int i = 0; i < AB_COLS / 2; i += 2) {
+        float4 n4 = make_float4(row_l, row_l, row_l, row_l);
+        if (OVER) n4 = *reinterpret_cast<const float4*>(nl + 2 * i);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float2 xs = __ffma2_rn(make_float2(__uint_as_float(sv[2 * (i + x)]), __uint_as_float(sv[2 * (i + x) + 1])), sc2,
+                                       x ? make_float2(n4.z, n4.w) : make_float2(n4.x, n4.y));
+          pr[i + x] = make_float2(exp2f(xs.x), exp2f(xs.y));
+        }
+      }
+      if (diag) {   // keys behind the query: rows above the column (OVER) or columns behind the row
+#pragma unroll
+        for (int i = 0; i < AB_COLS / 2; ++i) {
+          const int c = part * AB_COLS + 2 * i;
+          if (OVER ? c < r : c > r) pr[i].x = 0.f;
+          if (OVER ? c + 1 < r : c + 1 > r) pr[i].y = 0.f;
+        }
+      }
+      if (!OVER) {
+        tmem_ld_wait();
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(dp_free);
+      }
+      // P and dS in shared memory: chunk g of eight columns of this thread's row
+      const int roff = part * 16384 + (r >> 3) * 1024 + (r & 7) * 128;
+      auto put = [&](uint8_t* tile, int g, uint4 v) { *reinterpret_cast<uint4*>(tile + roff + ((g ^ (r & 7)) << 4)) = v; };
+      uint32_t pk[VIA_SMEM ? 32 : 1];
+      if (VIA_SMEM)
+#pragma unroll
+        for (int i = 0; i < 32; ++i) pk[i] = pack_bf16x2(pr[i].x, pr[i].y);
+      if (OVER) {   // (S of this iteration was written behind the product that read the P before it)
+#pragma unroll
+        for (int c = 0; c < 32; c += 16) {   // (half a row at a time: registers)
+          uint32_t half[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) half[i] = pack_bf16x2(pr[c + i].x, pr[c + i].y);
+          tmem_st_32x16(tmem_P + bf_col + c, half);
+        }
         tmem_st_wait();
         tc_fence_before();
-      } else {
-        constexpr int CH = AB_COLS / 8;  // 16-byte chunks per thread
-        const int col0 = part * AB_COLS;
-        const int roff = (col0 >> 6) * 16384 + (r >> 3) * 1024 + (r & 7) * 128;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(p_full);
+        if (!load_dp()) {
+          ok = false;
+          break;
+        }
+        tmem_ld_wait();
+      }
+      uint32_t dk[32];
 #pragma unroll
-        for (int g = 0; g < CH; ++g) {
-          const int chunk = ((((col0 & 63) >> 3) + g) ^ (r & 7)) << 4;
-          *reinterpret_cast<uint4*>(sP + roff + chunk) = make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]);
-          *reinterpret_cast<uint4*>(sDS + roff + chunk) = make_uint4(dk[4 * g], dk[4 * g + 1], dk[4 * g + 2], dk[4 * g + 3]);
+      for (int i = 0; i < 32; i += 2) {
+        float4 n4 = make_float4(row_d, row_d, row_d, row_d);
+        if (OVER) n4 = *reinterpret_cast<const float4*>(nl + 128 + 2 * i);
+#pragma unroll
+        for (int x = 0; x < 2; ++x) {
+          const float2 dd = __fmul2_rn(pr[i + x], __ffma2_rn(make_float2(__uint_as_float(dv[2 * (i + x)]), __uint_as_float(dv[2 * (i + x) + 1])), scale2,
+                                                             x ? make_float2(n4.z, n4.w) : make_float2(n4.x, n4.y)));
+          dk[i + x] = pack_bf16x2(dd.x, dd.y);
+        }
+      }
+      // the products of the previous iteration must be done with P and dS before they are overwritten
+      if (!OVER && !mbar_wait_bounded(ds_free, (t & 1) ^ 1, abort_flag, p.status, kTimeoutTmemEmpty)) {
+        ok = false;
+        break;
+      }
+      if (VIA_SMEM) {
+#pragma unroll
+        for (int g = 0; g < 8; ++g) {
+          put(sP, g, make_uint4(pk[4 * g], pk[4 * g + 1], pk[4 * g + 2], pk[4 * g + 3]));
+          put(sDS, g, make_uint4(dk[4 * g], dk[4 * g + 1], dk[4 * g + 2], dk[4 * g + 3]));
         }
         fence_proxy_async_smem();
+      } else {
+        tmem_st_32x32(tmem_dS + bf_col, dk);
+        tmem_st_wait();
+        tc_fence_before();
       }
       __syncwarp();
-      if (lane == 0) mbar_arrive(pds_full);
-      if (rec) { c1 = clock64(); t_store += c1 - c0; }
-    }
-    if (rec) {
-      p.prof[8] = w_sfull; p.prof[9] = t_load; p.prof[10] = t_math; p.prof[11] = w_pdsfree; p.prof[12] = t_store;
+      if (lane == 0) mbar_arrive(ds_full);
     }
     if (ok && mbar_wait_bounded(acc_done, 0, abort_flag, p.status, kTimeoutTmemFull)) {
       tc_fence_after();
@@ -470,7 +537,7 @@ static int launch_attn_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const C
 
 // q/k/v as for ats_attn_fwd; out, dout: [B, L, Hq, D] contiguous; lse [B, Hq, L]; delta: fp32 scratch [B, Hq, L];
 // dq: rows = tokens with pitch ld_dq, dk / dv with pitch ld_dkv (so all three can be slices of one packed gradient).
-// prof: null, or 32 int64 that receive per-phase cycle totals of CTA (0,0,0) of each pass (diagnostics).
+// prof: null, or 32 int64 that receive cycle totals of CTA (0,0,0) of each pass (diagnostics).
 ATS_API int ats_attn_bwd(const void* q, long long ld_q, long long q_cols, int q_col0, const void* k, long long ld_k,
                          long long k_cols, int k_col0, const void* v, long long ld_v, long long v_cols, int v_col0,
                          const void* out, const void* dout, const float* lse, float* delta, void* dq, void* dk, void* dv,
