@@ -13,7 +13,7 @@
 // * Epilogues: store bf16 | add bf16 C | fp32 store/accumulate | SwiGLU (gate and up halves of the accumulator
 //   are combined, optionally also writing the pre-activations for backward).
 //
-// CTA layout (192 threads): warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..5 = epilogue
+// CTA layout: warp 0 = TMA producer, warp 1 = TMEM owner + MMA issuer, warps 2..5 (2..9 where two share the columns) = epilogue
 // (one TMEM lane quadrant each).  Two 256-column accumulators ping-pong so the epilogue of tile i overlaps
 // the main loop of tile i+1.  No load in this file uses cluster multicast.
 //
@@ -37,6 +37,9 @@ constexpr int MAX_GROUPS = 256;
 constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + (MAX_GROUPS + 1) * 4;
 
 enum Epilogue : int { kStore = 0, kAddC = 1, kF32 = 2, kSwiGLU = 3, kSwiGLUBwd = 4, kGelu = 5, kDyt = 6, kSilu = 7 };
+// Each class has a tile function and a pair kernel of its own (kGluClass also takes the plain epilogues of a launch that gathers B).
+enum EpilogueClass : int { kPlainClass, kGluClass, kBlockClass };
+__host__ __device__ constexpr EpilogueClass class_of(int epilogue) { return epilogue <= kF32 ? kPlainClass : epilogue <= kSwiGLUBwd ? kGluClass : kBlockClass; }
 
 struct GemmArgs {
   int M, N, K;
@@ -227,7 +230,7 @@ __device__ __forceinline__ bool wait_chunk(const GemmArgs& p, ChunkRange& r, int
 
 // Epilogue of one tile for one warp: `taddr` = TMEM address of the accumulator at this warp's lane quadrant, `row_in_tile` =
 // the accumulator row (TMEM lane) that this thread owns.
-__device__ __forceinline__ void epilogue_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile) {
+__device__ __forceinline__ void epilogue_glu_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile) {
   const int row = t.m0 + row_in_tile;
   const bool row_ok = row < t.valid;
   const bool have_acc = t.k_iters > 0;
@@ -314,72 +317,7 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& p, const TileCoord
         }
       }
     }
-  } else if (p.epilogue == kGelu || p.epilogue == kDyt || p.epilogue == kSilu) {
-    const bool dyt = p.epilogue == kDyt;
-    __nv_bfloat16* drow = p.D + (long long)row * p.ldd;
-    float* xrow = dyt ? p.x + (long long)row * p.ldx : nullptr;
-#pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      const int colbase = t.n0 + c * 32;
-      if (colbase >= p.N) break;
-      uint4 xq[8];  // 32 residual values, requested before the accumulator is read (N is a multiple of 8, x rows are 32-byte aligned)
-      if (dyt && row_ok) {
-#pragma unroll
-        for (int v = 0; v < 4; ++v)
-          if (colbase + v * 8 < p.N) ld_global_32B(xrow + colbase + v * 8, xq[2 * v], xq[2 * v + 1]);
-      }
-      uint32_t r[32];
-      tmem_ld_32x32(taddr + c * 32, r);
-      tmem_ld_wait();
-      if (!row_ok) continue;
-      auto piece = [&](int v, int col) -> uint4 {  // eight columns
-        float f[8];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) f[e] = have_acc ? __uint_as_float(r[v * 8 + e]) * rs : 0.f;
-        if (p.bias) {
-          const float4 b0 = *reinterpret_cast<const float4*>(p.bias + col), b1 = *reinterpret_cast<const float4*>(p.bias + col + 4);
-          f[0] += b0.x; f[1] += b0.y; f[2] += b0.z; f[3] += b0.w;
-          f[4] += b1.x; f[5] += b1.y; f[6] += b1.z; f[7] += b1.w;
-        }
-        if (dyt) {
-          float* xf = reinterpret_cast<float*>(&xq[2 * v]);
-#pragma unroll
-          for (int q = 0; q < 2; ++q) {
-            const float4 w1 = *reinterpret_cast<const float4*>(p.w1 + col + 4 * q), b1 = *reinterpret_cast<const float4*>(p.b1 + col + 4 * q);
-            const float4 w2 = *reinterpret_cast<const float4*>(p.w2 + col + 4 * q), b2 = *reinterpret_cast<const float4*>(p.b2 + col + 4 * q);
-            xf[4 * q] += tanh_fast(p.a1 * f[4 * q]) * w1.x + b1.x;
-            xf[4 * q + 1] += tanh_fast(p.a1 * f[4 * q + 1]) * w1.y + b1.y;
-            xf[4 * q + 2] += tanh_fast(p.a1 * f[4 * q + 2]) * w1.z + b1.z;
-            xf[4 * q + 3] += tanh_fast(p.a1 * f[4 * q + 3]) * w1.w + b1.w;
-            f[4 * q] = tanh_fast(p.a2 * xf[4 * q]) * w2.x + b2.x;
-            f[4 * q + 1] = tanh_fast(p.a2 * xf[4 * q + 1]) * w2.y + b2.y;
-            f[4 * q + 2] = tanh_fast(p.a2 * xf[4 * q + 2]) * w2.z + b2.z;
-            f[4 * q + 3] = tanh_fast(p.a2 * xf[4 * q + 3]) * w2.w + b2.w;
-          }
-          st_global_32B(xrow + col, xq[2 * v], xq[2 * v + 1]);
-        } else if (p.epilogue == kSilu) {
-          if (col < p.act_cols)
-#pragma unroll
-            for (int e = 0; e < 8; ++e) f[e] = __fdividef(f[e], 1.f + __expf(-f[e]));
-        } else {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = 0.5f * f[e] * (1.f + tanh_fast(0.7978845608028654f * (f[e] + 0.044715f * f[e] * f[e] * f[e])));
-        }
-        return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
-      };
-#pragma unroll
-      for (int v = 0; v < 4; v += 2) {
-        const int col = colbase + v * 8;
-        if (p.wide && col + 16 <= p.N) {
-          const uint4 lo = piece(v, col), hi = piece(v + 1, col + 8);
-          st_global_32B(drow + col, lo, hi);
-        } else {
-          if (col < p.N) *reinterpret_cast<uint4*>(drow + col) = piece(v, col);
-          if (col + 8 < p.N) *reinterpret_cast<uint4*>(drow + col + 8) = piece(v + 1, col + 8);
-        }
-      }
-    }
-  } else if (p.epilogue == kSwiGLUBwd) {
+  } else {  // kSwiGLUBwd
     __nv_bfloat16* dbase = p.D + p.d_gs * t.g + (long long)row * p.ldd;
     const __nv_bfloat16* arow = p.aux + p.aux_gs * t.g + (long long)row * p.ldaux;
     __nv_bfloat16* hrow = p.out2 ? p.out2 + p.out2_gs * t.g + (long long)row * p.ldout2 : nullptr;
@@ -459,98 +397,226 @@ __device__ __forceinline__ void epilogue_tile(const GemmArgs& p, const TileCoord
         }
       }
     }
-  } else {
+  }
+}
+
+// kStore, kAddC and kF32.  With PARTS = 2 two warps share the rows: `part` says which half of the columns.
+template <int PARTS>
+__device__ __forceinline__ void epilogue_plain_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
+  const int c_begin = part * (BN / 32 / PARTS), c_end = c_begin + BN / 32 / PARTS;  // chunks of 32 columns
+  const int row = t.m0 + row_in_tile;
+  const bool row_ok = row < t.valid;
+  const bool have_acc = t.k_iters > 0;
+  const float rs = (p.row_scale && row_ok) ? p.row_scale[p.rs_gs * t.g + row] * p.alpha : p.alpha;
+  const float* cs = p.col_scale ? p.col_scale + p.cs_gs * (t.g / p.k_split / p.b_div) : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      uint32_t r[32];
-      if (have_acc) {
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-        if (p.fp8 == 2) {  // int8 operands: the accumulator columns hold s32
+  for (int c = c_begin; c < c_end; ++c) {
+    const int colbase = t.n0 + c * 32;
+    uint4 old[8];  // the 32 values that are added to (bf16 in the first four), requested before the accumulator is read
+    if (p.wide && row_ok) {
+      if (p.epilogue == kAddC) {
+        const __nv_bfloat16* crow = p.C + p.c_gs * t.g + (long long)row * p.ldc;
 #pragma unroll
-          for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__int2float_rn(int(r[i])));
+        for (int v = 0; v < 4; v += 2)
+          if (colbase + v * 8 + 16 <= p.N) ld_global_32B(crow + colbase + v * 8, old[v], old[v + 1]);
+      } else if (p.epilogue == kF32 && p.beta) {
+        const float* drow = p.Df32 + p.d_gs * t.g + (long long)row * p.ldd;
+#pragma unroll
+        for (int v = 0; v < 4; ++v)
+          if (colbase + v * 8 < p.N) ld_global_32B(drow + colbase + v * 8, old[2 * v], old[2 * v + 1]);
+      }
+    }
+    uint32_t r[32];
+    if (have_acc) {
+      tmem_ld_32x32(taddr + c * 32, r);
+      tmem_ld_wait();
+      if (p.fp8 == 2) {  // int8 operands: the accumulator columns hold s32
+#pragma unroll
+        for (int i = 0; i < 32; ++i) r[i] = __float_as_uint(__int2float_rn(int(r[i])));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = 0;
+    }
+    if (!row_ok) continue;
+    if (p.epilogue == kF32 && p.scatter_rows > 0) {
+      const int owner = row / p.scatter_rows;
+      float* drow = static_cast<float*>(p.d_table[owner]) + (long long)(row - owner * p.scatter_rows) * p.ldd;
+#pragma unroll
+      for (int v = 0; v < 8; ++v) {
+        const int col = colbase + v * 4;
+        if (col < p.N)
+          asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(drow + col), "f"(__uint_as_float(r[v * 4]) * p.alpha),
+                       "f"(__uint_as_float(r[v * 4 + 1]) * p.alpha), "f"(__uint_as_float(r[v * 4 + 2]) * p.alpha),
+                       "f"(__uint_as_float(r[v * 4 + 3]) * p.alpha)
+                       : "memory");
+      }
+    } else if (p.epilogue == kF32) {
+      float* drow = p.Df32 + p.d_gs * t.g + (long long)row * p.ldd;
+      auto four = [&](int v, int col, const float4& prev) -> float4 {
+        // rs = alpha (x the row scale of an 8-bit product); cs = its column scales: both distribute over the sum of the slices
+        float4 o = make_float4(__uint_as_float(r[v * 4]) * rs, __uint_as_float(r[v * 4 + 1]) * rs, __uint_as_float(r[v * 4 + 2]) * rs,
+                               __uint_as_float(r[v * 4 + 3]) * rs);
+        if (cs) {
+          const float4 c4 = *reinterpret_cast<const float4*>(cs + col);
+          o.x *= c4.x; o.y *= c4.y; o.z *= c4.z; o.w *= c4.w;
+        }
+        if (p.beta) {
+          o.x += prev.x; o.y += prev.y; o.z += prev.z; o.w += prev.w;
+        }
+        return o;
+      };
+      if (p.wide) {  // N is a multiple of 8: whole sectors of eight values (accumulating, 32,000 x 1,024 x 3,000: 225 -> 176 us)
+#pragma unroll
+        for (int v = 0; v < 8; v += 2) {
+          const int col = colbase + v * 4;
+          if (col < p.N) {
+            float4 lo = four(v, col, *reinterpret_cast<const float4*>(&old[v])), hi = four(v + 1, col + 4, *reinterpret_cast<const float4*>(&old[v + 1]));
+            st_global_32B(drow + col, *reinterpret_cast<uint4*>(&lo), *reinterpret_cast<uint4*>(&hi));
+          }
         }
       } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) r[i] = 0;
-      }
-      if (!row_ok) continue;
-      const int colbase = t.n0 + c * 32;
-      if (p.epilogue == kF32 && p.scatter_rows > 0) {
-        const int owner = row / p.scatter_rows;
-        float* drow = static_cast<float*>(p.d_table[owner]) + (long long)(row - owner * p.scatter_rows) * p.ldd;
 #pragma unroll
         for (int v = 0; v < 8; ++v) {
           const int col = colbase + v * 4;
           if (col < p.N)
-            asm volatile("red.relaxed.sys.global.add.v4.f32 [%0], {%1, %2, %3, %4};" ::"l"(drow + col), "f"(__uint_as_float(r[v * 4]) * p.alpha),
-                         "f"(__uint_as_float(r[v * 4 + 1]) * p.alpha), "f"(__uint_as_float(r[v * 4 + 2]) * p.alpha),
-                         "f"(__uint_as_float(r[v * 4 + 3]) * p.alpha)
-                         : "memory");
+            *reinterpret_cast<float4*>(drow + col) = four(v, col, p.beta ? *reinterpret_cast<const float4*>(drow + col) : make_float4(0.f, 0.f, 0.f, 0.f));
         }
-      } else if (p.epilogue == kF32) {
-        float* drow = p.Df32 + p.d_gs * t.g + (long long)row * p.ldd;
+      }
+    } else {
+      __nv_bfloat16* dbase = p.d_table ? static_cast<__nv_bfloat16*>(p.d_table[t.g]) : p.D + p.d_gs * t.g;
+      __nv_bfloat16* drow = dbase + (long long)row * p.ldd;
+      const __nv_bfloat16* crow =
+          p.epilogue == kAddC ? p.C + p.c_gs * t.g + (long long)row * p.ldc : nullptr;
+      auto piece = [&](int v, int col, const uint4& cv) -> uint4 {
+        float f[8];
 #pragma unroll
-        for (int v = 0; v < 8; ++v) {
-          const int col = colbase + v * 4;
-          if (col < p.N) {
-            // rs = alpha (x the row scale of an 8-bit product); cs = its column scales: both distribute over the sum of the slices
-            float4 o = make_float4(__uint_as_float(r[v * 4]) * rs, __uint_as_float(r[v * 4 + 1]) * rs,
-                                   __uint_as_float(r[v * 4 + 2]) * rs, __uint_as_float(r[v * 4 + 3]) * rs);
-            if (cs) {
-              const float4 c4 = *reinterpret_cast<const float4*>(cs + col);
-              o.x *= c4.x; o.y *= c4.y; o.z *= c4.z; o.w *= c4.w;
-            }
-            if (p.beta) {
-              float4 old = *reinterpret_cast<float4*>(drow + col);
-              o.x += old.x; o.y += old.y; o.z += old.z; o.w += old.w;
-            }
-            *reinterpret_cast<float4*>(drow + col) = o;
+        for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v * 8 + e]) * rs;
+        if (cs) {
+          const float4 c0 = *reinterpret_cast<const float4*>(cs + col), c1 = *reinterpret_cast<const float4*>(cs + col + 4);
+          f[0] *= c0.x; f[1] *= c0.y; f[2] *= c0.z; f[3] *= c0.w;
+          f[4] *= c1.x; f[5] *= c1.y; f[6] *= c1.z; f[7] *= c1.w;
+        }
+        if (crow) {
+          float2 c0 = unpack_bf16x2(cv.x), c1 = unpack_bf16x2(cv.y), c2 = unpack_bf16x2(cv.z), c3 = unpack_bf16x2(cv.w);
+          f[0] += c0.x; f[1] += c0.y; f[2] += c1.x; f[3] += c1.y;
+          f[4] += c2.x; f[5] += c2.y; f[6] += c3.x; f[7] += c3.y;
+        }
+        return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+      };
+      const uint4 zero4 = make_uint4(0, 0, 0, 0);
+      if (p.wide) {
+#pragma unroll
+        for (int v = 0; v < 4; v += 2) {
+          const int col = colbase + v * 8;
+          if (col + 16 <= p.N) {
+            st_global_32B(drow + col, piece(v, col, old[v]), piece(v + 1, col + 8, old[v + 1]));
+          } else if (col < p.N) {
+            *reinterpret_cast<uint4*>(drow + col) = piece(v, col, crow ? *reinterpret_cast<const uint4*>(crow + col) : zero4);
           }
         }
       } else {
-        __nv_bfloat16* dbase = p.d_table ? static_cast<__nv_bfloat16*>(p.d_table[t.g]) : p.D + p.d_gs * t.g;
-        __nv_bfloat16* drow = dbase + (long long)row * p.ldd;
-        const __nv_bfloat16* crow =
-            p.epilogue == kAddC ? p.C + p.c_gs * t.g + (long long)row * p.ldc : nullptr;
-        auto piece = [&](int v, int col, const uint4& cv) -> uint4 {
-          float f[8];
 #pragma unroll
-          for (int e = 0; e < 8; ++e) f[e] = __uint_as_float(r[v * 8 + e]) * rs;
-          if (cs) {
-            const float4 c0 = *reinterpret_cast<const float4*>(cs + col), c1 = *reinterpret_cast<const float4*>(cs + col + 4);
-            f[0] *= c0.x; f[1] *= c0.y; f[2] *= c0.z; f[3] *= c0.w;
-            f[4] *= c1.x; f[5] *= c1.y; f[6] *= c1.z; f[7] *= c1.w;
-          }
-          if (crow) {
-            float2 c0 = unpack_bf16x2(cv.x), c1 = unpack_bf16x2(cv.y), c2 = unpack_bf16x2(cv.z), c3 = unpack_bf16x2(cv.w);
-            f[0] += c0.x; f[1] += c0.y; f[2] += c1.x; f[3] += c1.y;
-            f[4] += c2.x; f[5] += c2.y; f[6] += c3.x; f[7] += c3.y;
-          }
-          return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
-        };
-        const uint4 zero4 = make_uint4(0, 0, 0, 0);
-        if (p.wide) {
-#pragma unroll
-          for (int v = 0; v < 4; v += 2) {
-            const int col = colbase + v * 8;
-            if (col + 16 <= p.N) {
-              uint4 c0 = zero4, c1 = zero4;
-              if (crow) ld_global_32B(crow + col, c0, c1);
-              st_global_32B(drow + col, piece(v, col, c0), piece(v + 1, col + 8, c1));
-            } else if (col < p.N) {
-              *reinterpret_cast<uint4*>(drow + col) = piece(v, col, crow ? *reinterpret_cast<const uint4*>(crow + col) : zero4);
-            }
-          }
-        } else {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int col = colbase + v * 8;
-            if (col < p.N) *reinterpret_cast<uint4*>(drow + col) = piece(v, col, crow ? *reinterpret_cast<const uint4*>(crow + col) : zero4);
-          }
+        for (int v = 0; v < 4; ++v) {
+          const int col = colbase + v * 8;
+          if (col < p.N) *reinterpret_cast<uint4*>(drow + col) = piece(v, col, crow ? *reinterpret_cast<const uint4*>(crow + col) : zero4);
         }
       }
     }
+  }
+}
+
+// The block steps (kGelu, kDyt, kSilu), shared between warps in the same way.
+template <int PARTS>
+__device__ __forceinline__ void epilogue_block_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
+  const int c_begin = part * (BN / 32 / PARTS), c_end = c_begin + BN / 32 / PARTS;  // chunks of 32 columns
+  const int row = t.m0 + row_in_tile;
+  const bool row_ok = row < t.valid;
+  const bool have_acc = t.k_iters > 0;
+  const float rs = p.alpha;
+  const bool dyt = p.epilogue == kDyt;
+  __nv_bfloat16* drow = p.D + (long long)row * p.ldd;
+  float* xrow = dyt ? p.x + (long long)row * p.ldx : nullptr;
+#pragma unroll 1
+  for (int c = c_begin; c < c_end; ++c) {
+    const int colbase = t.n0 + c * 32;
+    if (colbase >= p.N) break;
+    uint4 xq[8];  // 32 residual values, requested before the accumulator is read (N is a multiple of 8, x rows are 32-byte aligned)
+    if (dyt && row_ok) {
+#pragma unroll
+      for (int v = 0; v < 4; ++v)
+        if (colbase + v * 8 < p.N) ld_global_32B(xrow + colbase + v * 8, xq[2 * v], xq[2 * v + 1]);
+    }
+    uint32_t r[32];
+    tmem_ld_32x32(taddr + c * 32, r);
+    tmem_ld_wait();
+    if (!row_ok) continue;
+    auto piece = [&](int v, int col) -> uint4 {  // eight columns
+      float f[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) f[e] = have_acc ? __uint_as_float(r[v * 8 + e]) * rs : 0.f;
+      if (p.bias) {
+        const float4 b0 = *reinterpret_cast<const float4*>(p.bias + col), b1 = *reinterpret_cast<const float4*>(p.bias + col + 4);
+        f[0] += b0.x; f[1] += b0.y; f[2] += b0.z; f[3] += b0.w;
+        f[4] += b1.x; f[5] += b1.y; f[6] += b1.z; f[7] += b1.w;
+      }
+      if (dyt) {
+        float* xf = reinterpret_cast<float*>(&xq[2 * v]);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          const float4 w1 = *reinterpret_cast<const float4*>(p.w1 + col + 4 * q), b1 = *reinterpret_cast<const float4*>(p.b1 + col + 4 * q);
+          const float4 w2 = *reinterpret_cast<const float4*>(p.w2 + col + 4 * q), b2 = *reinterpret_cast<const float4*>(p.b2 + col + 4 * q);
+          xf[4 * q] += tanh_fast(p.a1 * f[4 * q]) * w1.x + b1.x;
+          xf[4 * q + 1] += tanh_fast(p.a1 * f[4 * q + 1]) * w1.y + b1.y;
+          xf[4 * q + 2] += tanh_fast(p.a1 * f[4 * q + 2]) * w1.z + b1.z;
+          xf[4 * q + 3] += tanh_fast(p.a1 * f[4 * q + 3]) * w1.w + b1.w;
+          f[4 * q] = tanh_fast(p.a2 * xf[4 * q]) * w2.x + b2.x;
+          f[4 * q + 1] = tanh_fast(p.a2 * xf[4 * q + 1]) * w2.y + b2.y;
+          f[4 * q + 2] = tanh_fast(p.a2 * xf[4 * q + 2]) * w2.z + b2.z;
+          f[4 * q + 3] = tanh_fast(p.a2 * xf[4 * q + 3]) * w2.w + b2.w;
+        }
+        st_global_32B(xrow + col, xq[2 * v], xq[2 * v + 1]);
+      } else if (p.epilogue == kSilu) {
+        if (col < p.act_cols)
+#pragma unroll
+          for (int e = 0; e < 8; ++e) f[e] = __fdividef(f[e], 1.f + __expf(-f[e]));
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) f[e] = 0.5f * f[e] * (1.f + tanh_fast(0.7978845608028654f * (f[e] + 0.044715f * f[e] * f[e] * f[e])));
+      }
+      return make_uint4(pack_bf16x2(f[0], f[1]), pack_bf16x2(f[2], f[3]), pack_bf16x2(f[4], f[5]), pack_bf16x2(f[6], f[7]));
+    };
+#pragma unroll
+    for (int v = 0; v < 4; v += 2) {
+      const int col = colbase + v * 8;
+      if (p.wide && col + 16 <= p.N) {
+        const uint4 lo = piece(v, col), hi = piece(v + 1, col + 8);
+        st_global_32B(drow + col, lo, hi);
+      } else {
+        if (col < p.N) *reinterpret_cast<uint4*>(drow + col) = piece(v, col);
+        if (col + 8 < p.N) *reinterpret_cast<uint4*>(drow + col + 8) = piece(v + 1, col + 8);
+      }
+    }
+  }
+}
+
+// What the epilogue of a tile reads beside the accumulator (the matrix or the sums that are added to, the residual stream) is asked into L2 while
+// the tile's main loop runs: each thread asks for its row's share, whole stretches of it, where the epilogue itself reads 64 bytes a time.
+// `tile` may lie behind the last one.  (The saved pre-activations of the SwiGLU backward are not: reading twice as many bytes as such a product
+// stores, that epilogue is bound by the requests to L2, and more of them made it slower, 375 -> 412 us for 16,384 x 5,632 x 2,048.)
+template <int PARTS>
+__device__ __forceinline__ void prefetch_epilogue(const GemmArgs& p, const int* prefix, int tile, int total_tiles, int g_hint, int row_in_tile, int part, int bm) {
+  if (tile >= total_tiles || !(p.wide || p.epilogue == kDyt)) return;
+  const TileCoord t = decode_tile(p, prefix, tile, g_hint, bm);
+  const int row = t.m0 + row_in_tile, col = t.n0 + part * (BN / PARTS);
+  const int cols = min(BN / PARTS, p.N - col);  // N is a multiple of 8
+  if (row >= t.valid || cols <= 0) return;
+  if (p.epilogue == kAddC) {
+    l2_prefetch(p.C + p.c_gs * t.g + (long long)row * p.ldc + col, cols * 2);
+  } else if (p.epilogue == kDyt) {
+    l2_prefetch(p.x + (long long)row * p.ldx + col, cols * 4);
+  } else if (p.epilogue == kF32) {
+    l2_prefetch(p.Df32 + p.d_gs * t.g + (long long)row * p.ldd + col, cols * 4);
   }
 }
 
@@ -775,7 +841,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (!mbar_wait_bounded(&tfull[acc], acc_phase, abort_flag, p.status, kTimeoutTmemFull)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
-      epilogue_tile(p, t, taddr, row_in_tile);
+      const EpilogueClass cls = class_of(p.epilogue);
+      if (cls == kPlainClass) epilogue_plain_tile<1>(p, t, taddr, row_in_tile, 0);
+      else if (cls == kGluClass) epilogue_glu_tile(p, t, taddr, row_in_tile);
+      else epilogue_block_tile<1>(p, t, taddr, row_in_tile, 0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -814,10 +883,18 @@ constexpr int PAIR_BM = 2 * BM;
 constexpr int PAIR_STAGES = ATS_PAIR_STAGES;
 constexpr int PAIR_B_STAGE_BYTES = (BN / 2) * BK * 2;
 constexpr int PAIR_STAGE_BYTES = A_STAGE_BYTES + PAIR_B_STAGE_BYTES;
-constexpr int PAIR_THREADS = 192;
 constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 + (MAX_GROUPS + 1) * 4;
+// Epilogue warps per CTA.  With four, a warp walks the 256 columns of its 32 rows alone and hides neither its TMEM round trips nor its loads behind
+// anything: the Dynamic-Tanh step took 33 us a tile, GELU 17, where the main loop of a 2,048-long reduction takes 14, and in a product of one wave
+// the epilogue is the last thing that runs.  With eight, two share the columns: 16,384 x 2,048 x 2,048 with the Dynamic-Tanh step 230 -> 174 us,
+// 16,384 x 8,192 x 2,048 with GELU 479 -> 410, 3,000 x 1,024 x 1,024 stored 19.5 -> 18.5, added to a matrix 25.6 -> 21.5.  The gated products stay at
+// four: theirs (two values read and three stored for each of the backward) are bound by their requests to L2, and eight warps made them slower
+// (16,384 x 5,632 x 2,048 375 -> 382 us), as does their share of registers.
+constexpr int pair_epi_warps(int cls) { return cls == kGluClass ? 4 : 8; }
+constexpr int pair_threads(int cls) { return 64 + 32 * pair_epi_warps(cls); }  // and two copy warps in launches that gather B
 
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS + 64, 1)
+template <int CLASS, int EW = pair_epi_warps(CLASS)>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(CLASS) + (CLASS == kGluClass ? 64 : 0), 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_b_own, const GemmArgs p) {
   extern __shared__ uint8_t smem_raw[];
@@ -844,7 +921,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
     }
     for (int b = 0; b < 2; ++b) {
       mbar_init(&tfull[b], 1);
-      mbar_init(&tempty[b], 8);  // four epilogue warps in each of the two CTAs
+      mbar_init(&tempty[b], 2 * EW);  // the epilogue warps of both CTAs
     }
     *abort_flag = 0;
     mbar_fence_init();
@@ -874,9 +951,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
   const int first_tile = int(cluster_id_x());
   const int tile_step = int(cluster_count_x());
 
-  if (warp >= 6) {
+  if (warp >= 2 + EW) {
     // ------------------------------------------------------------------ copy warps (launches that gather B from its owners)
-    if (p.n_copy) copy_remote_shards(p, warp - 6, lane);
+    if (p.n_copy) copy_remote_shards(p, warp - 2 - EW, lane);
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
@@ -1015,17 +1092,26 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       }
     }
   } else {
-    // ------------------------------------------------------------------ epilogue (warps 2..5 of both CTAs)
+    // ------------------------------------------------------------------ epilogue (warps 2 .. 1 + EW of both CTAs)
     const int quad = warp & 3;
     const int row_in_tile = quad * 32 + lane;
     int acc = 0, acc_phase = 0, g_hint = 0;
+    // epilogues that read: the next tile's operands are asked for when a tile's accumulator is ready
+    const bool reads = CLASS == kBlockClass ? p.epilogue == kDyt
+                                            : CLASS == kPlainClass && (p.epilogue == kAddC || (p.epilogue == kF32 && p.beta && !p.scatter_rows));
+    const int part = (warp - 2) >> 2;
+    if (reads) prefetch_epilogue<EW / 4>(p, prefix, first_tile, total_tiles, 0, int(rank) * BM + row_in_tile, part, PAIR_BM);
     for (int tile = first_tile; tile < total_tiles; tile += tile_step) {
       TileCoord t = decode_tile(p, prefix, tile, g_hint, PAIR_BM);
       t.m0 += int(rank) * BM;
       if (!mbar_wait_bounded(&tfull[acc], acc_phase, abort_flag, p.status, kTimeoutTmemFull)) break;
       tc_fence_after();
+      if (reads) prefetch_epilogue<EW / 4>(p, prefix, tile + tile_step, total_tiles, g_hint, int(rank) * BM + row_in_tile, part, PAIR_BM);
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
-      epilogue_tile(p, t, taddr, row_in_tile);
+      if constexpr (CLASS == kBlockClass) epilogue_block_tile<EW / 4>(p, t, taddr, row_in_tile, part);
+      else if constexpr (CLASS == kPlainClass) epilogue_plain_tile<EW / 4>(p, t, taddr, row_in_tile, part);
+      else if (class_of(p.epilogue) == kPlainClass) epilogue_plain_tile<1>(p, t, taddr, row_in_tile, 0);
+      else epilogue_glu_tile(p, t, taddr, row_in_tile);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty[acc]), 0));
@@ -1412,7 +1498,7 @@ ATS_API int ats_gemm_bf16_gathered(const void* A, long long lda, const void* B_l
 // Whole-sector stores need every row of D (and of aux for SwiGLU) to start 32-byte aligned at every 16th column.
 static int sector_aligned_outputs(const GemmArgs& p) {
   if (!g_gemm_wide || p.d_table) return 0;
-  if (p.epilogue == kF32) return 0;
+  if (p.epilogue == kF32) return (reinterpret_cast<uintptr_t>(p.Df32) & 31) == 0 && (p.ldd & 7) == 0 && (p.d_gs & 7) == 0 && (p.N & 7) == 0;
   auto ok = [](const void* ptr, long long ld, long long gs) { return (reinterpret_cast<uintptr_t>(ptr) & 31) == 0 && (ld & 15) == 0 && (gs & 15) == 0; };
   if (!ok(p.D, p.ldd, p.d_gs)) return 0;
   if (p.epilogue == kAddC && !ok(p.C, p.ldc, p.c_gs)) return 0;
@@ -1420,6 +1506,34 @@ static int sector_aligned_outputs(const GemmArgs& p) {
     return ok(p.aux, p.ldaux, p.aux_gs) && (p.up_offset & 15) == 0 && (!p.out2 || ok(p.out2, p.ldout2, p.out2_gs));
   if (p.epilogue == kSwiGLU && p.aux && (!ok(p.aux, p.ldaux, p.aux_gs) || (p.up_offset & 15))) return 0;
   return 1;
+}
+
+template <int CLASS>
+static int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb_own, const GemmArgs& p, long long tiles, int max_ctas,
+                        void* stream) {
+  const bool gather = CLASS == kGluClass && p.n_copy > 0;
+  const int threads = pair_threads(CLASS) + (gather ? 64 : 0);  // the two copy warps exist only in launches that gather B from peers
+  static int pair_clusters = -1;
+  if (pair_clusters < 0) {
+    cudaError_t ce = cudaFuncSetAttribute(gemm_bf16_pair_kernel<CLASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
+    if (ce != cudaSuccess) return int(ce);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(unsigned(num_sms() & ~1));
+    cfg.blockDim = dim3(pair_threads(CLASS));
+    cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
+    int n = 0;
+    ce = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<CLASS>, &cfg);
+    if (ce != cudaSuccess) return int(ce);
+    pair_clusters = n < 1 ? 1 : (n > num_sms() / 2 ? num_sms() / 2 : n);
+  }
+  int clusters = pair_clusters;
+  if (!gather) {  // (producers of a gathering launch wait on the copy warps of other CTAs: its whole grid stays resident)
+    if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2 < 1 ? 1 : max_ctas / 2;
+    if (tiles < clusters) clusters = int(tiles);
+  }
+  if (clusters < 1) return 0;
+  gemm_bf16_pair_kernel<CLASS><<<2 * clusters, threads, PAIR_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(ma, mb, mb_own, p);
+  return int(cudaGetLastError());
 }
 
 static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmArgs& p_in, int epilogue, int groups, int M, int N,
@@ -1436,32 +1550,11 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmA
   const int tn = epilogue == kSwiGLU ? (N + 127) / 128 : (N + BN - 1) / BN;
   if (g_gemm_pair && M >= PAIR_BM) {
     // two SMs per 256 x 256 tile
-    static int pair_clusters = -1;
-    if (pair_clusters < 0) {
-      cudaError_t ce = cudaFuncSetAttribute(gemm_bf16_pair_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
-      if (ce != cudaSuccess) return int(ce);
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3(unsigned(num_sms() & ~1));
-      cfg.blockDim = dim3(PAIR_THREADS);
-      cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
-      int n = 0;
-      ce = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel, &cfg);
-      if (ce != cudaSuccess) return int(ce);
-      pair_clusters = n < 1 ? 1 : (n > num_sms() / 2 ? num_sms() / 2 : n);
-    }
-    const long long pair_tiles = (long long)groups * ((M + PAIR_BM - 1) / PAIR_BM) * tn;
-    int clusters = pair_clusters;
-    if (p.n_copy > 0) {
-      // producers wait on the copy warps of other CTAs of this launch: keep the whole grid resident
-    } else {
-      if (max_ctas > 0 && max_ctas / 2 < clusters) clusters = max_ctas / 2 < 1 ? 1 : max_ctas / 2;
-      if (pair_tiles < clusters) clusters = int(pair_tiles);
-    }
-    if (clusters < 1) return 0;
-    // the two copy warps exist only in launches that gather B from peers
-    gemm_bf16_pair_kernel<<<2 * clusters, p.n_copy ? PAIR_THREADS + 64 : PAIR_THREADS, PAIR_SMEM_BYTES, static_cast<cudaStream_t>(stream)>>>(
-        ma, mb, mb_own ? *mb_own : mb, p);
-    return int(cudaGetLastError());
+    const long long tiles = (long long)groups * ((M + PAIR_BM - 1) / PAIR_BM) * tn;
+    const EpilogueClass cls = class_of(epilogue);
+    if (cls == kBlockClass) return launch_pairs<kBlockClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+    return cls == kGluClass || p.n_copy > 0 ? launch_pairs<kGluClass>(ma, mb, mb_own ? *mb_own : mb, p, tiles, max_ctas, stream)
+                                            : launch_pairs<kPlainClass>(ma, mb, mb, p, tiles, max_ctas, stream);
   }
   long long upper = (long long)groups * ((M + BM - 1) / BM) * tn;
   int grid = num_sms();

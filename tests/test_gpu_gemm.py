@@ -294,3 +294,32 @@ def test_weight_gradient_product_with_reduction_slices():
     err = (acc.float() - ref2).norm(dim=-1) / (ref2.norm(dim=-1) + 1e-6)
     assert err.max().item() < 1e-2
     ops.check_status()
+
+
+@pytest.mark.parametrize("M,N", [(256, 8), (300, 128), (513, 136), (256, 264), (1000, 1160)])
+def test_pair_epilogues_match_single_ctas(M, N):
+    """Two warps share a tile's columns in the pair kernels, one takes them all in the single-CTA kernel; sums run in the same order, so results are
+    the same bits.  Sizes: a second half without columns, one that begins or ends in the middle, rows behind the end, several tiles."""
+    from adaptivetrainingsystem_b200.ops import dyt, postnorm
+    torch.manual_seed(N)
+    K = 136
+    a, w = _rand(M, K), _rand(N, K, scale=K ** -0.5)
+    c = _rand(M, N)
+    x, v = torch.randn(M, N, device=DEV), [torch.randn(N, device=DEV) for _ in range(5)]
+
+    def results():
+        acc, xr = x.clone(), x.clone()
+        odd = torch.zeros(M * N + 4, device=DEV)[4:].view(M, N)   # begins in the middle of a sector
+        G.gemm_nt(a, w, out=acc, out_fp32=True, accumulate=True)
+        G.gemm_nt(a, w, out=odd, out_fp32=True, accumulate=True)
+        h = dyt.linear_residual(a, w, v[4], xr, dyt.DytChain(v[0], v[1], 0.7, v[2], v[3], 0.4))
+        return [G.gemm_nt(a, w), G.gemm_nt(a, w, add=c), acc, odd, dyt.linear_gelu(a, w, v[4]), postnorm.linear_silu(a, w, N // 2 // 8 * 8), h, xr]
+    pairs = results()
+    G.set_pair_kernels(False)
+    try:
+        single = results()
+    finally:
+        G.set_pair_kernels(True)
+    for name, p, s in zip(("store", "add", "accumulate", "fp32", "gelu", "silu", "dyt", "residual"), pairs, single):
+        assert torch.equal(p, s), name
+    _close(pairs[2], x + a.float() @ w.float().t(), tol=1e-2)
