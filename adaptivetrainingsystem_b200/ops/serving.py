@@ -78,9 +78,10 @@ class ScaledRows:
 def takes_scaled(rows: int, w: torch.Tensor, n: Optional[int] = None) -> bool:
     """Whether the product of ``rows`` rows with w [N, K] (``n`` of its outputs where they are pairs) runs on the decode kernel in a form that scales its sums."""
     from . import fp8, gemm as G, int4, int8
+    if int4.enabled() and int4.lookup(w) is not None:
+        return FUSE_DECODE and not int8.observing() and int4.streams(rows, w)
     return (FUSE_DECODE and w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.is_contiguous() and not getattr(w, "_ats_z3", None)
-            and not (fp8.enabled() or int8.enabled()) and not (int4.enabled() and int4.lookup(w) is not None) and not (int4.observing() or int8.observing())
-            and _lib.use_cuda_kernels(w) and G.skinny_fits(rows, w.shape[0] if n is None else n, w.shape[1]))
+            and not (fp8.enabled() or int8.enabled()) and not (int4.observing() or int8.observing()) and _lib.use_cuda_kernels(w) and G.skinny_fits(rows, w.shape[0] if n is None else n, w.shape[1]))
 
 
 def _partial_products(x2: torch.Tensor, w: torch.Tensor):
@@ -116,6 +117,9 @@ def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torc
         raise RuntimeError("scaled rows reached a projection that does not take them")
     if d % 16 or positions is None or positions.dtype != torch.int32 or cos.dtype != torch.float32 or w_qkv.shape[0] != (n_q + 2 * n_kv) * d:
         return None
+    from . import int4
+    if rows.dtype == torch.bfloat16 and takes_rotated(rows.shape[0], w_qkv, n_q, n_kv, d, cos, positions) and int4.enabled() and (entry := int4.lookup(w_qkv)) is not None:
+        return int4.gemv(rows, *entry, scale=scale, rope=(cos, sin, positions, (n_q + n_kv) * d, d))
     part = _partial_products(rows, w_qkv)
     if part is None:
         return None
@@ -135,7 +139,9 @@ def qkv_rope(h2: torch.Tensor, w_qkv: torch.Tensor, cos: torch.Tensor, sin: torc
 
 def takes_rotated(rows: int, w_qkv: torch.Tensor, n_q: int, n_kv: int, d: int, cos: torch.Tensor, positions: Optional[torch.Tensor]) -> bool:
     """Whether :func:`qkv_rope` takes :class:`ScaledRows` for this projection."""
-    return (d % 16 == 0 and 128 % d == 0 and positions is not None and positions.dtype == torch.int32 and cos.dtype == torch.float32
+    from . import int4
+    whole = d % 32 == 0 if int4.enabled() and int4.lookup(w_qkv) is not None else d % 16 == 0 and 128 % d == 0
+    return (whole and positions is not None and positions.dtype == torch.int32 and cos.dtype == torch.float32
             and w_qkv.shape[0] == (n_q + 2 * n_kv) * d and takes_scaled(rows, w_qkv))
 
 
@@ -144,6 +150,15 @@ def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, 
     ``None``.  ``scaled``: the consumer of h takes :class:`ScaledRows`, and the norm needs no launch."""
     if norm_w.dtype != torch.bfloat16 or residual2 is None or not residual2.is_contiguous():
         return None
+    from . import int4
+    if scaled and a2.dtype == torch.bfloat16 and int4.enabled() and (entry := int4.lookup(w_o)) is not None:
+        if not takes_scaled(a2.shape[0], w_o):
+            return None
+        T, N = a2.shape[0], w_o.shape[0]
+        rows = torch.empty(T, N, dtype=a2.dtype, device=a2.device)
+        parts = torch.empty(T, N // 16, dtype=torch.float32, device=a2.device)
+        x = int4.gemv(a2, *entry, add=residual2, next_norm=(norm_w, rows, parts))
+        return x, ScaledRows(rows, parts, float(eps), x.shape)
     part = _partial_products(a2, w_o)
     if part is None:
         return None
@@ -174,12 +189,15 @@ def mlp_norm(h2: torch.Tensor, w_gate_up: torch.Tensor, w_down: torch.Tensor, re
     from . import fp8, gemm as G, int4, int8
     if isinstance(h2, ScaledRows):   # (the caller has asked takes_scaled)
         inter = w_gate_up.shape[0] // 2
-        act = torch.empty(h2.rows.shape[0], inter, dtype=h2.rows.dtype, device=h2.rows.device)
-        G.skinny(h2.rows, w_gate_up, act, G.SK_SWIGLU, n=inter, up_offset=inter, scale=(h2.parts, h2.eps))
+        if int4.enabled() and (entry := int4.lookup(w_gate_up)) is not None:
+            act = int4.gemv(h2.rows, *entry, swiglu=True, scale=(h2.parts, h2.eps))
+        else:
+            act = torch.empty(h2.rows.shape[0], inter, dtype=h2.rows.dtype, device=h2.rows.device)
+            G.skinny(h2.rows, w_gate_up, act, G.SK_SWIGLU, n=inter, up_offset=inter, scale=(h2.parts, h2.eps))
         fused = out_proj_norm(act, w_down, residual2, norm_w, eps, scaled)
         if fused is None:
             from .functional import rms_norm
-            x = G.gemm_nt(act, w_down, add=residual2)
+            x = int4.linear_int4(act, w_down, residual2) if int4.usable(act, w_down) else G.gemm_nt(act, w_down, add=residual2)
             fused = x, rms_norm(x, norm_w, eps)
         return fused
     if (fp8.enabled() or int8.enabled() or (int4.enabled() and (int4.lookup(w_gate_up) is not None or int4.lookup(w_down) is not None))

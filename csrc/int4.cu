@@ -69,8 +69,6 @@ __device__ __forceinline__ void dq_word(uint32_t w, const Int4Consts& k, uint32_
   a[3] = dq_scale(and_or(shr_mulhi(w, k.m12), k.mask, k.magic), zB, sB);
 }
 
-constexpr int GEMV_WARPS = 8;
-
 // Asynchronous copies global -> shared (each lane copies into slots only it reads back, so no barrier is involved: a lane waits
 // for its own copy groups).  Loads into registers did not pipeline here: with five loads per step and stage the kernel waited
 // a full round trip to memory in every step whatever the prefetch depth (1.9 TB/s, warps 68 % of the time on the long
@@ -93,21 +91,42 @@ __device__ __forceinline__ void cp_async_wait() {
 
 // bytes one warp holds per stage: packed words and scale words of R tiles, 16 activations per lane and token tile
 __host__ __device__ constexpr int int4_stage_bytes(int R, int NT) { return 32 * (R * 16 + R * 8 + NT * 32); }
-__host__ __device__ constexpr int int4_ring_bytes(int R, int NT, int DEPTH) { return GEMV_WARPS * DEPTH * int4_stage_bytes(R, NT); }
+__host__ __device__ constexpr int int4_ring_bytes(int WARPS, int R, int NT, int DEPTH) { return WARPS * DEPTH * int4_stage_bytes(R, NT); }
 
-// R tiles per CTA: one, or with SWIGLU the gate tile and the up tile of the same features.  The warps split the super-steps;
+// What a decode step does around its products, instead of launches of their own (all optional):
+//   scale: x holds the rows of an RMSNorm before the division, x * w, and scale_parts [M, scale_n] sums of squares of x: the sums are divided by the rms;
+//   next:  the RMSNorm behind the product: next_out [M, N] = (the stored values) * next_w, next_parts [M, N / 16] = their sums of squares per tile;
+//   rope:  the first act_cols features are rotated in pairs half a head apart, at positions pos [M].
+// With them a step of four rows has five launches a layer instead of eight (eight 2,048-wide layers with 5,632 inner columns: 298 -> 277 us).
+struct Int4Step {
+  const float* scale_parts;
+  int scale_n;
+  float scale_inv, scale_eps;
+  const __nv_bfloat16* next_w;
+  __nv_bfloat16* next_out;
+  float* next_parts;
+  const int* pos;
+  const float* cos_t;
+  const float* sin_t;   // [positions, head_dim / 2]
+  int act_cols, head_dim;
+};
+enum Int4Mode : int { kI4Store = 0, kI4SwiGLU = 1, kI4Rope = 2 };
+
+// R tiles per CTA: one, or with kI4SwiGLU the gate tile and the up tile of the same features, with kI4Rope two tiles half a head apart.  The warps split the super-steps;
 // every warp keeps the copies of DEPTH of its super-steps in flight (a ring in shared memory), so that a CTA's few microseconds
 // are spent streaming and not waiting for one round trip to memory per step.  One tile per CTA and MINB resident CTAs per SM keep
 // the grid fine-grained: with two tiles and 72 registers the 28,672-feature projection ran as 2.02 waves of CTAs, i.e. three.
 // NT: token tiles of eight rows (the code fragments of a step feed NT MMAs).
-template <int R, bool SWIGLU, int NT, int DEPTH, int MINB>
-__global__ void __launch_bounds__(GEMV_WARPS * 32, MINB)
+template <int MODE, int WARPS, int NT, int DEPTH, int MINB>
+__global__ void __launch_bounds__(WARPS * 32, MINB)
 gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta, const __nv_bfloat16* __restrict__ x, long long ldx,
                  const __nv_bfloat16* __restrict__ add, long long ld_add, __nv_bfloat16* __restrict__ out, long long ld_out,
-                 int M, int N, int K, int group_shift, int early) {
+                 int M, int N, int K, int group_shift, int early, const Int4Step st) {
+  constexpr int R = MODE == kI4Store ? 1 : 2;
   if (!early) pdl_prologue();   // early: a chained launch, whose first packed words are requested under the kernel before it (common.cuh)
   else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  __shared__ float s_red[GEMV_WARPS][R][8 * NT][16];  // [warp][tile][token][feature of the tile]
+  __shared__ float s_red[WARPS][R][8 * NT][16];  // [warp][tile][token][feature of the tile]
+  __shared__ float s_scale[8 * NT];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int n_super = K >> 6, n_tiles = N >> 4;
   // constants the extraction wants in registers; built from a kernel argument so that they are not folded back into immediates
@@ -115,7 +134,10 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
   const Int4Consts kc = {0x000f000fu * one, 0x43004300u * one, one << 28, one << 24, one << 20, 0x3f803f80u * one};
   int tile[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) tile[r] = SWIGLU ? int(blockIdx.x) + r * (N >> 5) : int(blockIdx.x) * R + r;
+  for (int r = 0; r < R; ++r) {
+    const int per_half = st.head_dim >> 5;  // kI4Rope: tiles of half a head
+    tile[r] = MODE == kI4Rope ? int(blockIdx.x) / per_half * 2 * per_half + int(blockIdx.x) % per_half + r * per_half : int(blockIdx.x) + r * (N >> 5);
+  }
   float c[R][NT][4];
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -202,25 +224,35 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
   if (early) {
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d)
-      if (warp + d * GEMV_WARPS < n_super) issue_w(d, warp + d * GEMV_WARPS);
+      if (warp + d * WARPS < n_super) issue_w(d, warp + d * WARPS);
     asm volatile("griddepcontrol.wait;" ::: "memory");
   }
 #pragma unroll
   for (int d = 0; d < DEPTH; ++d) {
-    if (warp + d * GEMV_WARPS < n_super) {
-      if (!early) issue_w(d, warp + d * GEMV_WARPS);
-      issue_x(d, warp + d * GEMV_WARPS);
+    if (warp + d * WARPS < n_super) {
+      if (!early) issue_w(d, warp + d * WARPS);
+      issue_x(d, warp + d * WARPS);
     }
     cp_async_commit();
   }
-  for (int S0 = warp; S0 < n_super; S0 += GEMV_WARPS * DEPTH) {
+  // (while the first copies travel)
+  for (int m = warp; m < 8 * NT; m += WARPS) {
+    float f = 1.f;
+    if (st.scale_parts && m < M) {
+      float ss = 0.f;
+      for (int i = lane; i < st.scale_n; i += 32) ss += __ldcg(st.scale_parts + (long long)m * st.scale_n + i);
+      f = rsqrtf(warp_sum(ss) * st.scale_inv + st.scale_eps);
+    }
+    if (lane == 0) s_scale[m] = f;
+  }
+  for (int S0 = warp; S0 < n_super; S0 += WARPS * DEPTH) {
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) {
-      const int S = S0 + d * GEMV_WARPS;
+      const int S = S0 + d * WARPS;
       if (S < n_super) {  // the same for every lane of the warp
         cp_async_wait<DEPTH - 1>();  // all but the DEPTH - 1 youngest groups have landed: this step's is among them
         compute(d);
-        const int Sn = S + GEMV_WARPS * DEPTH;
+        const int Sn = S + WARPS * DEPTH;
         if (Sn < n_super) issue_w(d, Sn), issue_x(d, Sn);  // the slots just read are refilled (their values are in registers by now)
         cp_async_commit();
       }
@@ -238,24 +270,48 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
       s_red[warp][r][8 * n + 2 * t + 1][g + 8] = c[r][n][3];
     }
   __syncthreads();
-  constexpr int OUT_TILES = SWIGLU ? 1 : R;
-  for (int e = tid; e < OUT_TILES * NT * 128; e += GEMV_WARPS * 32) {
-    const int r = e / (NT * 128), m = (e >> 4) & (8 * NT - 1), f = e & 15;
-    if (m >= M) continue;
-    float v = 0.f;
+  for (int e = tid; e < NT * 128; e += WARPS * 32) {  // (whole warps: 16 lanes have the tile's features of one token)
+    const int m = e >> 4, f = e & 15, col = tile[0] * 16 + f;
+    const bool live = m < M;
+    float v = 0.f, u = 0.f;
 #pragma unroll
-    for (int w = 0; w < GEMV_WARPS; ++w) v += s_red[w][r][m][f];
-    const int col = (SWIGLU ? int(blockIdx.x) : int(blockIdx.x) * R + r) * 16 + f;
-    if (SWIGLU) {
-      float u = 0.f;
-#pragma unroll
-      for (int w = 0; w < GEMV_WARPS; ++w) u += s_red[w][R - 1][m][f];
+    for (int w = 0; w < WARPS; ++w) {
+      v += s_red[w][0][m][f];
+      if (R == 2) u += s_red[w][R - 1][m][f];
+    }
+    v *= s_scale[m];
+    u *= s_scale[m];
+    if (MODE == kI4Rope) {
+      const int half = st.head_dim >> 1, col_u = tile[R - 1] * 16 + f;
+      if (!live) continue;
+      if (col < st.act_cols) {
+        // rounded to bf16 first: the values that a separate rotation would read
+        const float a = __bfloat162float(__float2bfloat16(v)), b = __bfloat162float(__float2bfloat16(u));
+        const long long at = (long long)st.pos[m] * half + col % st.head_dim;
+        const float cs = st.cos_t[at], sn = st.sin_t[at];
+        v = a * cs - b * sn;
+        u = a * sn + b * cs;
+      }
+      out[(long long)m * ld_out + col] = __float2bfloat16(v);
+      out[(long long)m * ld_out + col_u] = __float2bfloat16(u);
+      continue;
+    }
+    if (MODE == kI4SwiGLU) {
       // the gate and up products are rounded to bf16 first, as the unfused form stores them
       const float gf = __bfloat162float(__float2bfloat16(v)), uf = __bfloat162float(__float2bfloat16(u));
       v = gf / (1.f + __expf(-gf)) * uf;
     }
-    if (add) v += __bfloat162float(add[(long long)m * ld_add + col]);
-    out[(long long)m * ld_out + col] = __float2bfloat16(v);
+    if (add && live) v += __bfloat162float(add[(long long)m * ld_add + col]);
+    const __nv_bfloat16 o = __float2bfloat16(v);
+    if (live) out[(long long)m * ld_out + col] = o;
+    if (MODE == kI4Store && st.next_out) {
+      const float b = __bfloat162float(o);
+      float sq = b * b;
+#pragma unroll
+      for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
+      if (live) st.next_out[(long long)m * N + col] = __float2bfloat16(b * __bfloat162float(st.next_w[col]));
+      if (live && f == 0) st.next_parts[(long long)m * n_tiles + tile[0]] = sq;
+    }
   }
 }
 
@@ -307,12 +363,20 @@ static int int4_group_shift(int group) {
   return s;
 }
 
-// out[M, N or N / 2] = x[M, K] @ W^T (+ add), M <= 16.  swiglu: W = [gate; up], out = silu(gate) * up (N % 32 == 0).
+// out[M, N or N / 2] = x[M, K] @ W^T (+ add), M <= 16.  mode kI4SwiGLU: W = [gate; up], out = silu(gate) * up (N % 32 == 0).  `step` may be null.
 ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long long ldx, const void* add, long long ld_add, void* out,
-                          long long ld_out, int M, int N, int K, int group, int swiglu, void* stream) {
+                          long long ld_out, int M, int N, int K, int group, int mode, const ats::Int4Step* step, void* stream) {
   const int early = ats::chained_launches();
   if (!int4_shape_ok(N, K, group) || M < 1 || M > 16 || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15)) return 1003;
-  if (swiglu && (N % 32)) return 1003;
+  if (mode < ats::kI4Store || mode > ats::kI4Rope || (mode != ats::kI4Store && (N % 32))) return 1003;
+  ats::Int4Step st = {};
+  if (step) st = *step;
+  if ((st.scale_parts && st.scale_n < 1) || (st.next_out && (mode != ats::kI4Store || !st.next_w || !st.next_parts))) return 1003;
+  if (mode == ats::kI4Rope) {
+    if (add || !st.pos || !st.cos_t || !st.sin_t || st.head_dim < 32 || (st.head_dim & 31) || N % st.head_dim || st.act_cols < 0 || st.act_cols % st.head_dim) return 1003;
+  } else {
+    st.head_dim = 32;
+  }
   auto s = static_cast<cudaStream_t>(stream);
   const auto* w4 = static_cast<const uint4*>(wq);
   const auto* mt = static_cast<const uint32_t*>(meta);
@@ -322,25 +386,40 @@ ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long 
   const int tiles = N / 16;
   const int gs = int4_group_shift(group);
   cudaError_t err;
-  const dim3 block(ats::GEMV_WARPS * 32);
-#define ATS_GEMV4(R_, SW_, NT_, D_, B_, GRID_)                                                                                        \
+  constexpr int kSms = 148;
+#define ATS_GEMV4(MODE_, W_, NT_, D_, B_, GRID_)                                                                                      \
   [&]() -> cudaError_t {                                                                                                             \
-    constexpr int kRing = ats::int4_ring_bytes(R_, NT_, D_);                                                                         \
+    constexpr int kRing = ats::int4_ring_bytes(W_, MODE_ == ats::kI4Store ? 1 : 2, NT_, D_);                                         \
     static bool attr_set = false;                                                                                                    \
     if (!attr_set) {                                                                                                                 \
-      cudaError_t ce = cudaFuncSetAttribute(ats::gemv_int4_kernel<R_, SW_, NT_, D_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
+      cudaError_t ce = cudaFuncSetAttribute(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                             kRing);                                                                                  \
       if (ce != cudaSuccess) return ce;                                                                                              \
       attr_set = true;                                                                                                               \
     }                                                                                                                                \
-    return ats::launch_pdl(ats::gemv_int4_kernel<R_, SW_, NT_, D_, B_>, dim3(GRID_), block, kRing, s, w4, mt, xp, ldx, ap, ld_add,  \
-                           op, ld_out, M, N, K, gs, early);                                                                               \
+    return ats::launch_pdl(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_>, dim3(GRID_), dim3(W_ * 32), kRing, s, w4, mt, xp, ldx, ap, ld_add,     \
+                           op, ld_out, M, N, K, gs, early, st);                                                                      \
   }()
+  // Warps, ring and CTAs per SM, from a chain of launches (us a launch; one or four rows / sixteen rows):
+  // * one tile per CTA: with a CTA for each SM at most, sixteen warps have the whole of a short reduction in flight: 5,632 -> 2,048 8.2 -> 4.7 /
+  //   9.9 -> 5.9, 2,048 -> 2,048 3.0 -> 2.5 / 5.0 -> 3.1; with two, rings of three steps let both run at once: 14,336 -> 4,096 21.5 -> 14.9 / 23.2
+  //   (rings of four: 17.3); more tiles are more waves, and their CTAs stay small;
+  // * gate and up tiles: more than two CTAs per SM run at once with rings of two steps: 2,048 -> 11,264 7.6 -> 6.5 / 11.0 -> 10.1,
+  //   4,096 -> 28,672 26.7 -> 24.5 / 39.7 -> 36.0; two find the deep rings faster: 1,024 -> 5,632 3.0 (rings of two: 3.6), not with sixteen rows;
+  // * heads of two tiles: deep rings (4,096 -> 6,144 8.5, rings of two 10.3), with sixteen rows while one CTA per SM is enough (2,048 -> 2,560 4.5,
+  //   rings of two 5.8; 4,096 -> 6,144 13.7 and 11.8).
   const bool two = M > 8;
-  if (swiglu)
-    err = two ? ATS_GEMV4(2, true, 2, 3, 2, tiles / 2) : ATS_GEMV4(2, true, 1, 4, 2, tiles / 2);
+  const int pairs = tiles / 2;
+  if (mode == ats::kI4SwiGLU)
+    err = two ? ATS_GEMV4(ats::kI4SwiGLU, 8, 2, 2, 2, pairs) : pairs > 2 * kSms ? ATS_GEMV4(ats::kI4SwiGLU, 8, 1, 2, 3, pairs) : ATS_GEMV4(ats::kI4SwiGLU, 8, 1, 4, 2, pairs);
+  else if (mode == ats::kI4Rope)
+    err = !two ? ATS_GEMV4(ats::kI4Rope, 8, 1, 4, 2, pairs) : pairs > kSms ? ATS_GEMV4(ats::kI4Rope, 8, 2, 2, 2, pairs) : ATS_GEMV4(ats::kI4Rope, 8, 2, 4, 1, pairs);
+  else if (tiles > 2 * kSms)
+    err = two ? ATS_GEMV4(ats::kI4Store, 8, 2, 4, 2, tiles) : ATS_GEMV4(ats::kI4Store, 8, 1, 4, 3, tiles);
+  else if (two)
+    err = ATS_GEMV4(ats::kI4Store, 16, 2, 2, 1, tiles);
   else
-    err = two ? ATS_GEMV4(1, false, 2, 4, 2, tiles) : ATS_GEMV4(1, false, 1, 4, 3, tiles);
+    err = tiles > kSms ? ATS_GEMV4(ats::kI4Store, 16, 1, 3, 2, tiles) : ATS_GEMV4(ats::kI4Store, 16, 1, 4, 1, tiles);
 #undef ATS_GEMV4
   return int(err);
 }

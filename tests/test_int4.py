@@ -325,6 +325,56 @@ def test_gemv_kernel_swiglu_epilogue(M, inter, K):
     assert (out.float() - ref).abs().max().item() < 2.0 ** -6 * ref.abs().max().item() + 1e-3
 
 
+# rows around the token tiles, one tile of a norm and many, heads of one tile pair and of several, rotated columns that end before the matrix
+@pytest.mark.gpu
+@pytest.mark.parametrize("M,N,K,d,group", [(1, 64, 128, 32, 128), (4, 2560, 2048, 64, 128), (8, 1536, 1024, 128, 64), (9, 96, 64, 32, 64), (16, 1024, 2816, 64, 128)])
+def test_gemv_kernel_with_the_steps_around_it(M, N, K, d, group):
+    from adaptivetrainingsystem_b200 import ops
+    dev = torch.device("cuda")
+    g = torch.Generator(device="cuda").manual_seed(M + N)
+    first, second, gated = _packed(N, K, group, dev, 6), _packed(N, N // 64 * 64, 64, dev, 7), _packed(N // 32 * 32, N // 64 * 64, 64, dev, 8)
+    x, res = torch.randn(M, K, generator=g, device=dev).bfloat16(), torch.randn(M, N, generator=g, device=dev).bfloat16()
+    norm, eps = (1 + 0.1 * torch.randn(N, generator=g, device=dev)).bfloat16(), 1e-6
+    rows, parts = torch.full((M, N), float("nan"), dtype=torch.bfloat16, device=dev), torch.full((M, N // 16), float("nan"), device=dev)
+    y = int4.gemv(x, *first, group, add=res, next_norm=(norm, rows, parts))
+    assert torch.equal(y, int4.gemv(x, *first, group, add=res)) and torch.equal(rows, y * norm)   # the result itself does not change
+    ss = (y.double() ** 2).view(M, -1, 16).sum(-1)
+    assert bool(((parts.double() - ss).abs() <= 16 * 2.0 ** -23 * ss).all())
+    def exact(packed, meta, group):   # (the kernel takes (code - zero) * scale without the rounding of a bf16 weight)
+        scale, zero = (t.to(dev).double() for t in int4.unpack_meta(meta.cpu()))
+        q = int4.unpack(packed.cpu()).to(dev).double()
+        w = ((q.view(q.shape[0], -1, group) - zero[:, :, None]) * scale[:, :, None]).view_as(q)
+        return w, (2 * 143 * scale.amax(1, keepdim=True)).expand_as(w)   # and the terms that it sums: 128 + code and 128 + zero times the scale
+    # rotation: the fp32 sums (K ulp of the terms) are rounded to bf16, rotated and rounded again
+    cos, sin = (torch.rand(40, d // 2, generator=g, device=dev) * 2 - 1 for _ in range(2))
+    pos, cols = torch.randint(0, 40, (M,), generator=g, device=dev, dtype=torch.int32), (N // d + 1) // 2 * d
+    got = int4.gemv(x, *first, group, rope=(cos, sin, pos, cols, d)).double()
+    w, most = exact(*first, group)
+    ref, slack = x.double() @ w.t(), (K + 8) * 2.0 ** -23 * (x.double().abs() @ most.t())
+    a, b = ref[:, :cols].view(M, -1, 2, d // 2).unbind(2)
+    ta, tb = (2.0 ** -8 * ref.abs() + slack)[:, :cols].view(M, -1, 2, d // 2).unbind(2)
+    c, s = cos[pos.long()].double()[:, None], sin[pos.long()].double()[:, None]
+    want, tol = torch.stack([a * c - b * s, a * s + b * c], 2), torch.stack([ta * c.abs() + tb * s.abs(), ta * s.abs() + tb * c.abs()], 2)
+    assert bool(((got[:, :cols].view_as(want) - want).abs() <= 2.0 ** -8 * want.abs() + 1.01 * tol).all())
+    assert bool(((got[:, cols:] - ref[:, cols:]).abs() <= 2.0 ** -8 * ref[:, cols:].abs() + slack[:, cols:]).all())
+    # a product that divides by the rms: fp32 sums (k ulp of the terms), bf16 result
+    k = N // 64 * 64
+    r = torch.rsqrt((y.double() ** 2).mean(-1, keepdim=True) * (N / k) + eps)
+    def bound(packed, meta):
+        w, most = exact(packed, meta, 64)
+        ref = r * (rows[:, :k].double() @ w.t())
+        return ref, 2.0 ** -8 * ref.abs() + (k + 8) * 2.0 ** -23 * r * (rows[:, :k].double().abs() @ most.t())
+    if k:
+        out = int4.gemv(rows[:, :k], *second, 64, scale=(parts, eps))
+        ref, tol = bound(*second)
+        assert bool(((out.double() - ref).abs() <= tol).all())
+        out = int4.gemv(rows[:, :k], *gated, 64, swiglu=True, scale=(parts, eps))
+        ref, tol = bound(*gated)
+        (gate, up), (tg, tu) = ref.chunk(2, -1), tol.chunk(2, -1)
+        want = torch.nn.functional.silu(gate) * up   # (the slope of silu is at most 1.1)
+        assert bool(((out.double() - want).abs() <= 2.0 ** -8 * want.abs() + 1.1 * tg * (up.abs() + tu) + tu * gate.abs() + 1e-6).all())
+
+
 @pytest.mark.gpu
 def test_int4_model_matches_its_dequantised_weights():
     """Weights replaced by their dequantised 4-bit values give the oracle.  The 4-bit kernels (a prompt through dequantise +
