@@ -24,7 +24,7 @@ from .mixers import CappedAttention, ChannelDelta, LightningAttention, SwigluMLP
 
 
 class Nemipel(LayeredDecoder):
-    KERNEL_SOURCES = ("gemm_tcgen05.cu", "gemm_skinny.cu", "postnorm.cu", "lightning.cu", "lightning_tcgen05.cu", "gqa_attention.cu", "gqa_attention_tcgen05.cu", "inference.cu",
+    KERNEL_SOURCES = ("gemm_tcgen05.cu", "gemm_skinny.cu", "gemv_bf16.cu", "postnorm.cu", "lightning.cu", "lightning_tcgen05.cu", "gqa_attention.cu", "gqa_attention_tcgen05.cu", "inference.cu",
                       "delta_rule.cu", "channel_delta.cu", "channel_delta_mma.cu", "dyt.cu")
 
     def __init__(self, config: NemipelConfig):

@@ -24,7 +24,7 @@ from .mixers import GatedDelta, GeluMLP, LatentAttention, padded, vector
 
 
 class Vimodra(LayeredDecoder):
-    KERNEL_SOURCES = ("gemm_tcgen05.cu", "gemm_skinny.cu", "dyt.cu", "latent_attention.cu",
+    KERNEL_SOURCES = ("gemm_tcgen05.cu", "gemm_skinny.cu", "gemv_bf16.cu", "dyt.cu", "latent_attention.cu",
                       "latent_decode.cu", "attention_window_tcgen05.cu", "delta_rule.cu", "delta_rule_mma.cu")
 
     def __init__(self, config: VimodraConfig):

@@ -31,6 +31,27 @@ class _Skinny(ctypes.Structure):   # csrc/skinny.cuh
                 ("scale_eps", _c_f), ("status", _vp), ("w_ready", _c_int)]
 
 
+class StreamStep(ctypes.Structure):   # csrc/stream_step.cuh
+    _fields_ = [("scale_parts", _vp), ("scale_n", _c_int), ("scale_inv", _c_f), ("scale_eps", _c_f), ("next_w", _vp), ("next_out", _vp), ("next_parts", _vp),
+                ("pos", _vp), ("cos_t", _vp), ("sin_t", _vp), ("act_cols", _c_int), ("head_dim", _c_int)]
+
+
+def stream_step(K: int, scale=None, next_norm=None, rope=None) -> Optional[StreamStep]:
+    """``scale`` = (sums of squares [M, n], eps), ``next_norm`` = (weight, rows [M, N], sums of squares [M, N / 16]), ``rope`` = (cos, sin, positions [M]
+    int32, rotated columns, head width) of a streaming product with ``K`` terms; the tensors outlive the launch's call."""
+    if scale is None and next_norm is None and rope is None:
+        return None
+    step = StreamStep()
+    if scale is not None:
+        step.scale_parts, step.scale_n, step.scale_inv, step.scale_eps = scale[0].data_ptr(), scale[0].shape[1], 1.0 / K, scale[1]
+    if next_norm is not None:
+        step.next_w, step.next_out, step.next_parts = (t.data_ptr() for t in next_norm)
+    if rope is not None:
+        step.cos_t, step.sin_t, step.pos = (t.data_ptr() for t in rope[:3])
+        step.act_cols, step.head_dim = rope[3:]
+    return step
+
+
 def _fn():
     global _configured
     lib = _lib.cuda_lib()
@@ -50,6 +71,8 @@ def _fn():
         lib.ats_splitk_reduce.argtypes = [_vp, _c_int, _c_ll, _c_ll, _vp, _vp, _vp]
         lib.ats_gemm_skinny.restype = _c_int
         lib.ats_gemm_skinny.argtypes = [_vp, _c_ll, _vp, _c_ll, _c_ll, ctypes.POINTER(_Skinny), _c_int, _vp]
+        lib.ats_gemv_bf16.restype = _c_int
+        lib.ats_gemv_bf16.argtypes = [_vp, _c_ll, _vp, _c_ll, _vp, _c_ll, _vp, _c_ll, _c_int, _c_int, _c_int, _c_int, ctypes.POINTER(StreamStep), _c_int, _vp]
         lib.ats_chain_launches.restype = None
         lib.ats_chain_launches.argtypes = [_c_int]
         lib.ats_gemm_set_pair.restype = None
@@ -203,15 +226,49 @@ def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:
     return s if s <= 4 else 4 if s < 8 else 8
 
 
+_STREAM_MODES = {SK_STORE: 0, SK_SWIGLU: 1, SK_ROPE: 2}
+
+
+def stream_fits(T: int, N: int, K: int, mode: int = SK_STORE, head_dim: int = 0) -> bool:
+    """Whether a decode product runs on the streaming kernel (``csrc/gemv_bf16.cu``); ``N``: the outputs.  The lines are where a CTA per tile no longer
+    has an SM to itself, or its warps walk a long reduction alone where the decode kernel cuts it over clusters (us in a chain of launches, decode
+    kernel / streaming kernel; one to eight rows, then sixteen):
+
+    * up to 148 tiles of 16 outputs: 2048 x 2048 4.5 / 2.9, 5.0 / 3.8; 2048 x 5632 8.0 / 5.9, 8.3 / 7.3; 2368 x 14336 15.5 / 13.3, 15.9 / 15.2, but
+      with sixteen rows 1024 x 14336 12.1 / 12.8; more tiles: 3072 x 5632 9.0 / 10.0, 9.4 / 12.8;
+    * up to 148 pairs of tiles of rotated heads: 2560 x 2048 5.2 / 3.7, 5.6 / 4.6; 4608 x 4096 11.0 / 8.7, 12.0 / 9.4; more: 6144 x 2048 7.6 / 8.1;
+    * up to 296 pairs of gate and up tiles, whose CTAs have half the warps: 2816 x 1024 4.8 / 3.3, 5.1 / 4.1; 4736 x 2048 9.3 / 7.5, 9.7 / 9.0; longer
+      reductions: 2048 x 4096 8.7 / 9.3, 9.0 / 11.0; more: 5632 x 2048 9.4 / 10.0."""
+    if not (SPLIT_K_SKINNY and 1 <= T <= 16 and N % 16 == 0 and K % 64 == 0 and mode in _STREAM_MODES):
+        return False
+    if mode == SK_ROPE:
+        return head_dim >= 32 and head_dim % 32 == 0 and N % head_dim == 0 and N <= 148 * 32 and K <= 4096
+    if mode == SK_SWIGLU:
+        return N <= 296 * 16 and K <= 2048
+    return N <= 148 * 16 and K <= (14336 if T <= 8 else 8192)
+
+
+def norm_parts(T: int, N: int, K: int) -> int:
+    """Sums of squares that :func:`skinny` leaves for each row of a ``SK_STORE`` product with an RMSNorm behind it."""
+    return N // 16 if stream_fits(T, N, K) else (N + 127) // 128
+
+
 def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Optional[int] = None, splits: Optional[int] = None, add: Optional[torch.Tensor] = None,
            alpha: float = 1.0, up_offset: int = 0, act_cols: int = 0, bias: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None, chain=None,
            head_dim: int = 0, pos: Optional[torch.Tensor] = None, next_norm=None, scale=None) -> None:
     """One launch of the decode kernel; ``chain`` = (w1, b1, a1, w2, b2, a2) of the residual step ``SK_DYT``; for ``SK_ROPE``
     w1 and w2 are the cosine and sine tables, ``pos`` the positions (int32) and ``act_cols`` the rotated columns.  ``next_norm`` = (weight, rows
-    [T, N], sums of squares [T, tiles of 128]) of an RMSNorm that follows ``SK_STORE``; ``scale`` = (sums of squares, eps): ``a`` came from such a product."""
+    [T, N], sums of squares [T, norm_parts]) of an RMSNorm that follows ``SK_STORE``; ``scale`` = (sums of squares, eps): ``a`` came from such a product."""
     _fn()
     a, w = _check2d(a), _check2d(w)
     (T, K), N = a.shape, w.shape[0] if n is None else n
+    if (splits is None and alpha == 1.0 and stream_fits(T, N, K, mode, head_dim) and (mode != SK_SWIGLU or (add is None and up_offset == N and w.shape[0] == 2 * N))
+            and (next_norm is None or next_norm[2].shape[1] == N // 16) and (mode != SK_ROPE or add is None and act_cols % head_dim == 0)):
+        step = stream_step(K, scale, next_norm, (chain[0], chain[3], pos, act_cols, head_dim) if mode == SK_ROPE else None)
+        _lib.check(_lib.cuda_lib().ats_gemv_bf16(w.data_ptr(), w.stride(0), a.data_ptr(), a.stride(0), None if add is None else add.data_ptr(), 0 if add is None else add.stride(0),
+                                                 out.data_ptr(), out.stride(-2), T, w.shape[0] if mode == SK_SWIGLU else N, K, _STREAM_MODES[mode], step, int(_weight_ready(w)),
+                                                 _lib.stream_ptr(a.device)), "ats_gemv_bf16")
+        return
     if splits is None:
         splits = skinny_splits(T, N, K, 64 if mode == SK_SWIGLU else 128)
     w1, b1, a1, w2, b2, a2 = chain if chain is not None else (None, None, 0.0, None, None, 0.0)

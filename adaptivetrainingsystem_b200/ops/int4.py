@@ -38,11 +38,6 @@ _weights: Dict[int, Tuple[int, Tuple[int, int], torch.Tensor, torch.Tensor, int]
 _hessians: Dict[int, Tuple[torch.Tensor, int]] = {}                                       # storage -> (sum of x^T x, rows seen)
 
 
-class _Step(ctypes.Structure):   # csrc/int4.cu, Int4Step
-    _fields_ = [("scale_parts", _vp), ("scale_n", _ci), ("scale_inv", ctypes.c_float), ("scale_eps", ctypes.c_float), ("next_w", _vp), ("next_out", _vp), ("next_parts", _vp),
-                ("pos", _vp), ("cos_t", _vp), ("sin_t", _vp), ("act_cols", _ci), ("head_dim", _ci)]
-
-
 def set_enabled(flag: bool) -> None:
     global _enabled
     _enabled = bool(flag)
@@ -57,7 +52,7 @@ def _fns():
     lib = _lib.cuda_lib()
     if not _sig:
         lib.ats_gemv_int4.restype = _ci
-        lib.ats_gemv_int4.argtypes = [_vp, _vp, _vp, _cll, _vp, _cll, _vp, _cll, _ci, _ci, _ci, _ci, _ci, ctypes.POINTER(_Step), _vp]
+        lib.ats_gemv_int4.argtypes = [_vp, _vp, _vp, _cll, _vp, _cll, _vp, _cll, _ci, _ci, _ci, _ci, _ci, ctypes.POINTER(G.StreamStep), _vp]
         lib.ats_dequant_int4.restype = _ci
         lib.ats_dequant_int4.argtypes = [_vp, _vp, _vp, _cll, _ci, _ci, _ci, _vp]
         _sig = True
@@ -228,16 +223,7 @@ def gemv(x2: torch.Tensor, packed: torch.Tensor, meta: torch.Tensor, group: int 
     if add is not None and (add.stride(1) != 1 or tuple(add.shape) != (M, n_out)):
         add = add.expand(M, n_out).contiguous()
     out = torch.empty(M, n_out, dtype=torch.bfloat16, device=x2.device)
-    step = None
-    if scale is not None or next_norm is not None or rope is not None:
-        step = _Step()
-        if scale is not None:
-            step.scale_parts, step.scale_n, step.scale_inv, step.scale_eps = scale[0].data_ptr(), scale[0].shape[1], 1.0 / K, scale[1]
-        if next_norm is not None:
-            step.next_w, step.next_out, step.next_parts = (t.data_ptr() for t in next_norm)
-        if rope is not None:
-            step.cos_t, step.sin_t, step.pos = (t.data_ptr() for t in rope[:3])
-            step.act_cols, step.head_dim = rope[3:]
+    step = G.stream_step(K, scale, next_norm, rope)
     err = _fns().ats_gemv_int4(_lib.ptr(packed), _lib.ptr(meta), _lib.ptr(x2), x2.stride(0), _lib.ptr(add), add.stride(0) if add is not None else 0,
                                _lib.ptr(out), out.stride(0), M, N, K, group, 2 if rope is not None else int(swiglu), step, _lib.stream_ptr(x2.device))
     _lib.check(err, "ats_gemv_int4")

@@ -62,7 +62,7 @@ DECODE_KERNEL = "decode kernel"
 
 class ScaledRows:
     """RMSNorm(x) * w of a decode step's rows before the division: ``rows`` = x * w [T, N] (bf16) and ``parts`` [T, tiles], the sums of squares of x per
-    128 columns.  The decode product that reads the rows multiplies its sums by 1 / rms, so the norm costs no launch."""
+    16 or 128 columns.  The decode product that reads the rows multiplies its sums by 1 / rms, so the norm costs no launch."""
 
     def __init__(self, rows: torch.Tensor, parts: torch.Tensor, eps: float, shape):
         self.rows, self.parts, self.eps, self.shape, self.device = rows, parts, eps, shape, rows.device
@@ -168,7 +168,7 @@ def out_proj_norm(a2: torch.Tensor, w_o: torch.Tensor, residual2: torch.Tensor, 
         if scaled and w_o.shape[0] % 2 == 0:
             T, N = a2.shape[0], w_o.shape[0]
             x, rows = (torch.empty(T, N, dtype=a2.dtype, device=a2.device) for _ in range(2))
-            parts = torch.empty(T, (N + 127) // 128, dtype=torch.float32, device=a2.device)
+            parts = torch.empty(T, G.norm_parts(T, N, a2.shape[1]), dtype=torch.float32, device=a2.device)
             G.skinny(a2, w_o, x, G.SK_STORE, add=residual2, next_norm=(norm_w, rows, parts))
             return x, ScaledRows(rows, parts, float(eps), x.shape)
         x = G.gemm_nt(a2, w_o, add=residual2)

@@ -251,8 +251,16 @@ skinny_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__
     if (p.scale_parts && int(threadIdx.x) - 64 < p.T) {
       const float* parts = p.scale_parts + (long long)(int(threadIdx.x) - 64) * p.scale_n;
       float ss = 0.f;
+      if ((p.scale_n & 3) == 0 && (reinterpret_cast<uintptr_t>(p.scale_parts) & 15) == 0) {  // (a streaming product leaves a part for every 16 columns)
 #pragma unroll 8
-      for (int i = 0; i < p.scale_n; ++i) ss += parts[i];
+        for (int i = 0; i < p.scale_n; i += 4) {
+          const float4 v = *reinterpret_cast<const float4*>(parts + i);
+          ss += v.x; ss += v.y; ss += v.z; ss += v.w;
+        }
+      } else {
+#pragma unroll 8
+        for (int i = 0; i < p.scale_n; ++i) ss += parts[i];
+      }
       factor *= rsqrtf(ss * p.scale_inv + p.scale_eps);
     }
     if (reduce && p.mode == kSkStore && p.add) {   // the residual of the first eight owned tokens travels under the product

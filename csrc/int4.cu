@@ -28,15 +28,9 @@
 //
 // Counterparts in the reference: the GPTQ hook of training/trainer.py:681-710 (AutoGPTQ, 4 bits, group 128) and the Triton GPTQ
 // matmul of its vendored inference engine (colossalai/kernel/triton/gptq_triton.py).
-#include "common.cuh"
+#include "stream_step.cuh"
 
 namespace ats {
-
-__device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
-  asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
-               : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3])
-               : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
-}
 
 // (128 + q) pairs -> (q - zero) * scale, in bf16 pairs.  The integer ALU issues a warp instruction every other cycle and is the
 // pipe this kernel fills first (measured: 60 % busy with the plain C++ form, 15 of its instructions per packed word), so the
@@ -73,46 +67,11 @@ __device__ __forceinline__ void dq_word(uint32_t w, const Int4Consts& k, uint32_
 // for its own copy groups).  Loads into registers did not pipeline here: with five loads per step and stage the kernel waited
 // a full round trip to memory in every step whatever the prefetch depth (1.9 TB/s, warps 68 % of the time on the long
 // scoreboard); copy groups are counted, not score-boarded.
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async16_or_zero(void* smem, const void* gmem, bool valid) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem), "r"(valid ? 16 : 0)
-               : "memory");
-}
-__device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
-
 // bytes one warp holds per stage: packed words and scale words of R tiles, 16 activations per lane and token tile
 __host__ __device__ constexpr int int4_stage_bytes(int R, int NT) { return 32 * (R * 16 + R * 8 + NT * 32); }
 __host__ __device__ constexpr int int4_ring_bytes(int WARPS, int R, int NT, int DEPTH) { return WARPS * DEPTH * int4_stage_bytes(R, NT); }
 
-// What a decode step does around its products, instead of launches of their own (all optional):
-//   scale: x holds the rows of an RMSNorm before the division, x * w, and scale_parts [M, scale_n] sums of squares of x: the sums are divided by the rms;
-//   next:  the RMSNorm behind the product: next_out [M, N] = (the stored values) * next_w, next_parts [M, N / 16] = their sums of squares per tile;
-//   rope:  the first act_cols features are rotated in pairs half a head apart, at positions pos [M].
-// With them a step of four rows has five launches a layer instead of eight (eight 2,048-wide layers with 5,632 inner columns: 298 -> 277 us).
-struct Int4Step {
-  const float* scale_parts;
-  int scale_n;
-  float scale_inv, scale_eps;
-  const __nv_bfloat16* next_w;
-  __nv_bfloat16* next_out;
-  float* next_parts;
-  const int* pos;
-  const float* cos_t;
-  const float* sin_t;   // [positions, head_dim / 2]
-  int act_cols, head_dim;
-};
-enum Int4Mode : int { kI4Store = 0, kI4SwiGLU = 1, kI4Rope = 2 };
-
-// R tiles per CTA: one, or with kI4SwiGLU the gate tile and the up tile of the same features, with kI4Rope two tiles half a head apart.  The warps split the super-steps;
+// R tiles per CTA: one, or with kStreamSwiGLU the gate tile and the up tile of the same features, with kStreamRope two tiles half a head apart.  The warps split the super-steps;
 // every warp keeps the copies of DEPTH of its super-steps in flight (a ring in shared memory), so that a CTA's few microseconds
 // are spent streaming and not waiting for one round trip to memory per step.  One tile per CTA and MINB resident CTAs per SM keep
 // the grid fine-grained: with two tiles and 72 registers the 28,672-feature projection ran as 2.02 waves of CTAs, i.e. three.
@@ -121,8 +80,8 @@ template <int MODE, int WARPS, int NT, int DEPTH, int MINB>
 __global__ void __launch_bounds__(WARPS * 32, MINB)
 gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta, const __nv_bfloat16* __restrict__ x, long long ldx,
                  const __nv_bfloat16* __restrict__ add, long long ld_add, __nv_bfloat16* __restrict__ out, long long ld_out,
-                 int M, int N, int K, int group_shift, int early, const Int4Step st) {
-  constexpr int R = MODE == kI4Store ? 1 : 2;
+                 int M, int N, int K, int group_shift, int early, const StreamStep st) {
+  constexpr int R = MODE == kStreamStore ? 1 : 2;
   if (!early) pdl_prologue();   // early: a chained launch, whose first packed words are requested under the kernel before it (common.cuh)
   else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float s_red[WARPS][R][8 * NT][16];  // [warp][tile][token][feature of the tile]
@@ -134,10 +93,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
   const Int4Consts kc = {0x000f000fu * one, 0x43004300u * one, one << 28, one << 24, one << 20, 0x3f803f80u * one};
   int tile[R];
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
-    const int per_half = st.head_dim >> 5;  // kI4Rope: tiles of half a head
-    tile[r] = MODE == kI4Rope ? int(blockIdx.x) / per_half * 2 * per_half + int(blockIdx.x) % per_half + r * per_half : int(blockIdx.x) + r * (N >> 5);
-  }
+  for (int r = 0; r < R; ++r) tile[r] = stream_tile<MODE>(st, N, r);
   float c[R][NT][4];
 #pragma unroll
   for (int r = 0; r < R; ++r)
@@ -235,16 +191,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
     }
     cp_async_commit();
   }
-  // (while the first copies travel)
-  for (int m = warp; m < 8 * NT; m += WARPS) {
-    float f = 1.f;
-    if (st.scale_parts && m < M) {
-      float ss = 0.f;
-      for (int i = lane; i < st.scale_n; i += 32) ss += __ldcg(st.scale_parts + (long long)m * st.scale_n + i);
-      f = rsqrtf(warp_sum(ss) * st.scale_inv + st.scale_eps);
-    }
-    if (lane == 0) s_scale[m] = f;
-  }
+  stream_scales<WARPS, NT>(st, M, s_scale);  // (while the first copies travel)
   for (int S0 = warp; S0 < n_super; S0 += WARPS * DEPTH) {
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) {
@@ -270,49 +217,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
       s_red[warp][r][8 * n + 2 * t + 1][g + 8] = c[r][n][3];
     }
   __syncthreads();
-  for (int e = tid; e < NT * 128; e += WARPS * 32) {  // (whole warps: 16 lanes have the tile's features of one token)
-    const int m = e >> 4, f = e & 15, col = tile[0] * 16 + f;
-    const bool live = m < M;
-    float v = 0.f, u = 0.f;
-#pragma unroll
-    for (int w = 0; w < WARPS; ++w) {
-      v += s_red[w][0][m][f];
-      if (R == 2) u += s_red[w][R - 1][m][f];
-    }
-    v *= s_scale[m];
-    u *= s_scale[m];
-    if (MODE == kI4Rope) {
-      const int half = st.head_dim >> 1, col_u = tile[R - 1] * 16 + f;
-      if (!live) continue;
-      if (col < st.act_cols) {
-        // rounded to bf16 first: the values that a separate rotation would read
-        const float a = __bfloat162float(__float2bfloat16(v)), b = __bfloat162float(__float2bfloat16(u));
-        const long long at = (long long)st.pos[m] * half + col % st.head_dim;
-        const float cs = st.cos_t[at], sn = st.sin_t[at];
-        v = a * cs - b * sn;
-        u = a * sn + b * cs;
-      }
-      out[(long long)m * ld_out + col] = __float2bfloat16(v);
-      out[(long long)m * ld_out + col_u] = __float2bfloat16(u);
-      continue;
-    }
-    if (MODE == kI4SwiGLU) {
-      // the gate and up products are rounded to bf16 first, as the unfused form stores them
-      const float gf = __bfloat162float(__float2bfloat16(v)), uf = __bfloat162float(__float2bfloat16(u));
-      v = gf / (1.f + __expf(-gf)) * uf;
-    }
-    if (add && live) v += __bfloat162float(add[(long long)m * ld_add + col]);
-    const __nv_bfloat16 o = __float2bfloat16(v);
-    if (live) out[(long long)m * ld_out + col] = o;
-    if (MODE == kI4Store && st.next_out) {
-      const float b = __bfloat162float(o);
-      float sq = b * b;
-#pragma unroll
-      for (int off = 8; off > 0; off >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, off);
-      if (live) st.next_out[(long long)m * N + col] = __float2bfloat16(b * __bfloat162float(st.next_w[col]));
-      if (live && f == 0) st.next_parts[(long long)m * n_tiles + tile[0]] = sq;
-    }
-  }
+  stream_finish<MODE, WARPS, NT>(st, s_red, s_scale, tile, add, ld_add, out, ld_out, M, N);
 }
 
 // one thread per (tile, super-step, lane): 16 + 16 consecutive values of features g and g + 8
@@ -363,20 +268,16 @@ static int int4_group_shift(int group) {
   return s;
 }
 
-// out[M, N or N / 2] = x[M, K] @ W^T (+ add), M <= 16.  mode kI4SwiGLU: W = [gate; up], out = silu(gate) * up (N % 32 == 0).  `step` may be null.
+// out[M, N or N / 2] = x[M, K] @ W^T (+ add), M <= 16.  mode kStreamSwiGLU: W = [gate; up], out = silu(gate) * up (N % 32 == 0).  `step` may be null.
 ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long long ldx, const void* add, long long ld_add, void* out,
-                          long long ld_out, int M, int N, int K, int group, int mode, const ats::Int4Step* step, void* stream) {
+                          long long ld_out, int M, int N, int K, int group, int mode, const ats::StreamStep* step, void* stream) {
   const int early = ats::chained_launches();
   if (!int4_shape_ok(N, K, group) || M < 1 || M > 16 || (ldx & 7) || (reinterpret_cast<uintptr_t>(x) & 15)) return 1003;
-  if (mode < ats::kI4Store || mode > ats::kI4Rope || (mode != ats::kI4Store && (N % 32))) return 1003;
-  ats::Int4Step st = {};
+  if (mode < ats::kStreamStore || mode > ats::kStreamRope || (mode != ats::kStreamStore && (N % 32))) return 1003;
+  ats::StreamStep st = {};
   if (step) st = *step;
-  if ((st.scale_parts && st.scale_n < 1) || (st.next_out && (mode != ats::kI4Store || !st.next_w || !st.next_parts))) return 1003;
-  if (mode == ats::kI4Rope) {
-    if (add || !st.pos || !st.cos_t || !st.sin_t || st.head_dim < 32 || (st.head_dim & 31) || N % st.head_dim || st.act_cols < 0 || st.act_cols % st.head_dim) return 1003;
-  } else {
-    st.head_dim = 32;
-  }
+  if (!ats::stream_step_ok(st, mode, N, add != nullptr)) return 1003;
+  if (mode != ats::kStreamRope) st.head_dim = 32;
   auto s = static_cast<cudaStream_t>(stream);
   const auto* w4 = static_cast<const uint4*>(wq);
   const auto* mt = static_cast<const uint32_t*>(meta);
@@ -389,7 +290,7 @@ ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long 
   constexpr int kSms = 148;
 #define ATS_GEMV4(MODE_, W_, NT_, D_, B_, GRID_)                                                                                      \
   [&]() -> cudaError_t {                                                                                                             \
-    constexpr int kRing = ats::int4_ring_bytes(W_, MODE_ == ats::kI4Store ? 1 : 2, NT_, D_);                                         \
+    constexpr int kRing = ats::int4_ring_bytes(W_, MODE_ == ats::kStreamStore ? 1 : 2, NT_, D_);                                         \
     static bool attr_set = false;                                                                                                    \
     if (!attr_set) {                                                                                                                 \
       cudaError_t ce = cudaFuncSetAttribute(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
@@ -410,16 +311,16 @@ ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long 
   //   rings of two 5.8; 4,096 -> 6,144 13.7 and 11.8).
   const bool two = M > 8;
   const int pairs = tiles / 2;
-  if (mode == ats::kI4SwiGLU)
-    err = two ? ATS_GEMV4(ats::kI4SwiGLU, 8, 2, 2, 2, pairs) : pairs > 2 * kSms ? ATS_GEMV4(ats::kI4SwiGLU, 8, 1, 2, 3, pairs) : ATS_GEMV4(ats::kI4SwiGLU, 8, 1, 4, 2, pairs);
-  else if (mode == ats::kI4Rope)
-    err = !two ? ATS_GEMV4(ats::kI4Rope, 8, 1, 4, 2, pairs) : pairs > kSms ? ATS_GEMV4(ats::kI4Rope, 8, 2, 2, 2, pairs) : ATS_GEMV4(ats::kI4Rope, 8, 2, 4, 1, pairs);
+  if (mode == ats::kStreamSwiGLU)
+    err = two ? ATS_GEMV4(ats::kStreamSwiGLU, 8, 2, 2, 2, pairs) : pairs > 2 * kSms ? ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 2, 3, pairs) : ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 4, 2, pairs);
+  else if (mode == ats::kStreamRope)
+    err = !two ? ATS_GEMV4(ats::kStreamRope, 8, 1, 4, 2, pairs) : pairs > kSms ? ATS_GEMV4(ats::kStreamRope, 8, 2, 2, 2, pairs) : ATS_GEMV4(ats::kStreamRope, 8, 2, 4, 1, pairs);
   else if (tiles > 2 * kSms)
-    err = two ? ATS_GEMV4(ats::kI4Store, 8, 2, 4, 2, tiles) : ATS_GEMV4(ats::kI4Store, 8, 1, 4, 3, tiles);
+    err = two ? ATS_GEMV4(ats::kStreamStore, 8, 2, 4, 2, tiles) : ATS_GEMV4(ats::kStreamStore, 8, 1, 4, 3, tiles);
   else if (two)
-    err = ATS_GEMV4(ats::kI4Store, 16, 2, 2, 1, tiles);
+    err = ATS_GEMV4(ats::kStreamStore, 16, 2, 2, 1, tiles);
   else
-    err = tiles > kSms ? ATS_GEMV4(ats::kI4Store, 16, 1, 3, 2, tiles) : ATS_GEMV4(ats::kI4Store, 16, 1, 4, 1, tiles);
+    err = tiles > kSms ? ATS_GEMV4(ats::kStreamStore, 16, 1, 3, 2, tiles) : ATS_GEMV4(ats::kStreamStore, 16, 1, 4, 1, tiles);
 #undef ATS_GEMV4
   return int(err);
 }
