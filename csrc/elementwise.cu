@@ -430,6 +430,17 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
   }
 }
 
+// out = bf16(in * bf16(*scale)): a gradient times the upstream one, which is on the device.  (The framework's product with a one-element tensor
+// does not vectorise: 84 us for 16,384 x 2,048, this 23.)  n is a multiple of 8.
+__global__ void __launch_bounds__(256) scale_bf16_kernel(const uint4* __restrict__ in, const float* __restrict__ scale, uint4* __restrict__ out, long long nvec) {
+  const float s = __bfloat162float(__float2bfloat16(*scale));
+  for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {
+    const uint4 a = in[i];
+    const float2 x0 = unpack_bf16x2(a.x), x1 = unpack_bf16x2(a.y), x2 = unpack_bf16x2(a.z), x3 = unpack_bf16x2(a.w);
+    out[i] = make_uint4(pack_bf16x2(x0.x * s, x0.y * s), pack_bf16x2(x1.x * s, x1.y * s), pack_bf16x2(x2.x * s, x2.y * s), pack_bf16x2(x3.x * s, x3.y * s));
+  }
+}
+
 static inline int grid_for(long long work_items, int threads, int cap = 148 * 16) {
   long long b = (work_items + threads - 1) / threads;
   if (b < 1) b = 1;
@@ -588,6 +599,13 @@ ATS_API int ats_cast_f32_bf16(const float* in, void* out, long long n, int accum
   if (n == 0) return 0;
   cast_f32_bf16_kernel<<<grid_for((n + 3) / 4, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(
       in, static_cast<__nv_bfloat16*>(out), n, accumulate, scale);
+  return int(cudaGetLastError());
+}
+
+ATS_API int ats_scale_bf16(const void* in, const float* scale, void* out, long long n, void* stream) {
+  if ((n & 7) || (reinterpret_cast<uintptr_t>(in) & 15) || (reinterpret_cast<uintptr_t>(out) & 15)) return 1003;
+  if (n == 0) return 0;
+  scale_bf16_kernel<<<grid_for(n >> 3, 256), 256, 0, static_cast<cudaStream_t>(stream)>>>(static_cast<const uint4*>(in), scale, static_cast<uint4*>(out), n >> 3);
   return int(cudaGetLastError());
 }
 

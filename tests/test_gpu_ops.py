@@ -1005,3 +1005,30 @@ def test_fp8_experts_in_the_serving_path():
         fp8.set_enabled(False)
         fp8.clear_weight_cache()
     ops.check_status()
+
+
+@pytest.mark.parametrize("T,V", [(1, 8), (300, 2048), (512, 1000)])
+def test_linear_cross_entropy_in_one_chunk(T, V):
+    """One chunk (the weight gradient is a product of the backward pass) against several (summed in fp32 beside the loss): the same loss, input gradients
+    of the same bits, weight gradients of the same sums in another order; an upstream gradient that is not one; a gradient that is accumulated."""
+    torch.manual_seed(T)
+    H = 256
+    h0, w0 = _rand(T, H), _rand(V, H, scale=0.05)
+    labels = torch.randint(0, V, (T,), device=DEV)
+    labels[:T // 10] = -100
+    got = []
+    for rows in (T, max(1, T // 3)):
+        h, w = h0.clone().requires_grad_(), w0.clone().requires_grad_()
+        loss = ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows)[0]
+        (loss * 0.37).backward()
+        first, sink = w.grad.clone(), torch.full((V, H), 0.25, device=DEV, dtype=torch.bfloat16)
+        w._ats_grad, w._ats_grad_fresh, w.grad = sink, False, None   # as an engine that sums micro-batches has it
+        ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows)[0].backward()
+        assert w.grad is None
+        got.append((loss.detach(), h.grad, first, sink))
+    one, many = got
+    assert torch.equal(one[0], many[0]) and torch.equal(one[1], many[1])
+    scale = many[2].float().abs().max()
+    # the sums differ by T fp32 roundings, which can take the result to the neighbouring bf16 number (they are up to 2^-7 of the value apart)
+    for a, b in ((one[2], many[2]), (one[3], many[3])):
+        assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + T * 2.0 ** -23 * scale).all())
