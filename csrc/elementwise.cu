@@ -3,7 +3,7 @@
 //
 // Counterparts in the reference: core/transformer_ops.cu:61-315 (fp32 CUDA-core RMSNorm / RoPE / SwiGLU) and
 // the eager PyTorch paths in core/model.py:228-304, 470-524, 1082-1088, 1924-1931.
-#include "common.cuh"
+#include "async_copy.cuh"
 #include <cstdlib>
 
 namespace ats {
@@ -150,87 +150,127 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// Warp-per-row form of the RMSNorm backward for rows of up to 32 * 8 * NV elements: a warp keeps its whole row (x, dy and
-// the residual-branch gradient) in registers as packed bf16, reduces with shuffles only and never meets a CTA barrier
-// inside the row loop, so every warp keeps 3 * NV 16-byte loads in flight.  The weight-gradient partials of the four warps
-// of a CTA are folded in shared memory (fixed order) into one partial row per CTA.
-template <int NV>
-__global__ void __launch_bounds__(128, 2)
-rmsnorm_bwd_warp_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w,
-                        const __nv_bfloat16* __restrict__ dy, const float* __restrict__ rstd,
-                        const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
+// RMSNorm backward over many rows: one CTA of eight warps per SM, groups of WPR warps take a row each (up to 2,048 WPR columns with NV = 8 vectors of
+// eight per lane).  The kernel moves four matrices and does little with them, so what counts is what is in flight: every lane copies its vectors of
+// the group's next rows (x, dy and the gradient of the residual branch) asynchronously into slots that only it reads, two rows ahead, so that a row's
+// reduction never waits for its loads (98 KB in flight per SM at 2,048 columns; loading a row, reducing it and only then asking for the residual
+// branch kept a third of that).  16,384 x 2,048 with a residual branch 91.8 -> 47.6 us (41.6 at the copy rate),
+// 4,096 x 4,096 64.0 -> 29.5 (20.8) and 13.5 -> 3.5 for the fold of its partial sums, 16,384 x 5,120 446 -> 160, 3,000 x 1,024 9.3 -> 8.7.
+// The weight-gradient sums of a lane's columns stay in registers and are folded over the groups at the end.
+template <int NV, int WPR>
+__global__ void __launch_bounds__(256, 1)
+rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy,
+                        const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows, int cols) {
-  extern __shared__ float fold[];  // [4][cols] fp32, then the weight row as bf16 (zero-padded to 256 * NV elements)
-  const int lane = threadIdx.x & 31, wib = threadIdx.x >> 5;
+  constexpr int G = 8 / WPR, S = 2, SLOTS = 32 * WPR * NV;  // row groups, rows in flight, vectors of a row
+  extern __shared__ __align__(16) unsigned char rows_smem[];
+  __shared__ float s_dot[2][8];
+  uint4* ring = reinterpret_cast<uint4*>(rows_smem);        // [G][S][3][SLOTS]
+  uint4* wsm = ring + G * S * 3 * SLOTS;                    // the weight, zero-padded
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / WPR, at = (warp % WPR) * 32 + lane;
   const int nvec = cols >> 3;
   const float inv_cols = 1.f / float(cols);
-  uint4* wsm = reinterpret_cast<uint4*>(fold + 4 * cols);
-  for (int v = threadIdx.x; v < 32 * NV; v += 128) wsm[v] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : make_uint4(0, 0, 0, 0);
+  for (int v = threadIdx.x; v < SLOTS; v += 256) wsm[v] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : make_uint4(0, 0, 0, 0);
   __syncthreads();
+  uint4* mine = ring + group * S * 3 * SLOTS + at;
+  const long long first = (long long)blockIdx.x * G + group, stride = (long long)gridDim.x * G;
+  float rq[S];
+  auto issue = [&](int d, long long row) {
+    if (row < rows) {
+      rq[d] = rstd[row];
+      uint4* slot = mine + d * 3 * SLOTS;
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = at + 32 * WPR * i;
+        if (v < nvec) {
+          cp_async16(slot + 32 * WPR * i, reinterpret_cast<const uint4*>(x + row * cols) + v);
+          cp_async16(slot + SLOTS + 32 * WPR * i, reinterpret_cast<const uint4*>(dy + row * cols) + v);
+          if (dres_in) cp_async16(slot + 2 * SLOTS + 32 * WPR * i, reinterpret_cast<const uint4*>(dres_in + row * cols) + v);
+        }
+      }
+    }
+    cp_async_commit();
+  };
   float dwacc[NV][8];
 #pragma unroll
-  for (int i = 0; i < NV; ++i) {
+  for (int i = 0; i < NV; ++i)
 #pragma unroll
     for (int e = 0; e < 8; ++e) dwacc[i][e] = 0.f;
-  }
-  for (long long row = blockIdx.x * 4 + wib; row < rows; row += 4LL * gridDim.x) {
-    const float r = rstd[row];
-    const uint4* xr = reinterpret_cast<const uint4*>(x + row * cols);
-    const uint4* dr = reinterpret_cast<const uint4*>(dy + row * cols);
-    const uint4* cr = dres_in ? reinterpret_cast<const uint4*>(dres_in + row * cols) : nullptr;
-    uint4 a[NV], b[NV];
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = lane + 32 * i;
-      const bool in = v < nvec;
-      a[i] = in ? xr[v] : make_uint4(0, 0, 0, 0);
-      b[i] = in ? dr[v] : make_uint4(0, 0, 0, 0);
-    }
-    float dot = 0.f;
+  for (int d = 0; d < S; ++d) issue(d, first + d * stride);
+  int parity = 0;
+  for (long long row0 = first; row0 < rows; row0 += S * stride) {
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const uint4 wq = wsm[lane + 32 * i];
-      const uint32_t au[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, bu[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
-      const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w};
+    for (int d = 0; d < S; ++d) {
+      const long long row = row0 + d * stride;
+      if (row >= rows) break;  // the same for the whole group
+      cp_async_wait<S - 1>();
+      const uint4* slot = mine + d * 3 * SLOTS;
+      const float r = rq[d];
+      auto vec = [&](int m, int i) { return at + 32 * WPR * i < nvec ? slot[m * SLOTS + 32 * WPR * i] : make_uint4(0, 0, 0, 0); };
+      float dot = 0.f;
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 xv = unpack_bf16x2(au[e]), dv = unpack_bf16x2(bu[e]), ww = unpack_bf16x2(wu[e]);
-        const float xh0 = xv.x * r, xh1 = xv.y * r;
-        dot += dv.x * ww.x * xh0 + dv.y * ww.y * xh1;
-        dwacc[i][2 * e] += dv.x * xh0;
-        dwacc[i][2 * e + 1] += dv.y * xh1;
+      for (int i = 0; i < NV; ++i) {
+        const uint4 wq = wsm[at + 32 * WPR * i], a = vec(0, i), b = vec(1, i);
+        const uint32_t au[4] = {a.x, a.y, a.z, a.w}, bu[4] = {b.x, b.y, b.z, b.w};
+        const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 xv = unpack_bf16x2(au[e]), dv = unpack_bf16x2(bu[e]), ww = unpack_bf16x2(wu[e]);
+          const float xh0 = xv.x * r, xh1 = xv.y * r;
+          dot += dv.x * ww.x * xh0 + dv.y * ww.y * xh1;
+          dwacc[i][2 * e] += dv.x * xh0;
+          dwacc[i][2 * e + 1] += dv.y * xh1;
+        }
       }
-    }
-    dot = warp_sum(dot) * inv_cols;
-    uint4* outr = reinterpret_cast<uint4*>(dx + row * cols);
+      dot = warp_sum(dot);
+      if (WPR > 1) {  // (two sets: a warp that is a row ahead writes the other one)
+        if (lane == 0) s_dot[parity][warp] = dot;
+        asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(32 * WPR) : "memory");
+        dot = 0.f;
 #pragma unroll
-    for (int i = 0; i < NV; ++i) {
-      const int v = lane + 32 * i;
-      const uint4 wq = wsm[v];
-      const uint4 cq = (cr && v < nvec) ? cr[v] : make_uint4(0, 0, 0, 0);
-      const uint32_t au[4] = {a[i].x, a[i].y, a[i].z, a[i].w}, bu[4] = {b[i].x, b[i].y, b[i].z, b[i].w};
-      const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w}, cu[4] = {cq.x, cq.y, cq.z, cq.w};
-      uint32_t o[4];
-#pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 xv = unpack_bf16x2(au[e]), dv = unpack_bf16x2(bu[e]), ww = unpack_bf16x2(wu[e]), cc = unpack_bf16x2(cu[e]);
-        o[e] = pack_bf16x2(r * (dv.x * ww.x - xv.x * r * dot) + cc.x, r * (dv.y * ww.y - xv.y * r * dot) + cc.y);
+        for (int j = 0; j < WPR; ++j) dot += s_dot[parity][group * WPR + j];
+        parity ^= 1;
       }
-      if (v < nvec) outr[v] = make_uint4(o[0], o[1], o[2], o[3]);
+      dot *= inv_cols;
+      uint4* outr = reinterpret_cast<uint4*>(dx + row * cols);
+#pragma unroll
+      for (int i = 0; i < NV; ++i) {
+        const int v = at + 32 * WPR * i;
+        const uint4 wq = wsm[v], a = vec(0, i), b = vec(1, i), cq = dres_in ? vec(2, i) : make_uint4(0, 0, 0, 0);
+        const uint32_t au[4] = {a.x, a.y, a.z, a.w}, bu[4] = {b.x, b.y, b.z, b.w};
+        const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w}, cu[4] = {cq.x, cq.y, cq.z, cq.w};
+        uint32_t o[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float2 xv = unpack_bf16x2(au[e]), dv = unpack_bf16x2(bu[e]), ww = unpack_bf16x2(wu[e]), cc = unpack_bf16x2(cu[e]);
+          o[e] = pack_bf16x2(r * (dv.x * ww.x - xv.x * r * dot) + cc.x, r * (dv.y * ww.y - xv.y * r * dot) + cc.y);
+        }
+        if (v < nvec) outr[v] = make_uint4(o[0], o[1], o[2], o[3]);
+      }
+      issue(d, row + S * stride);  // (a lane refills the slots that it has just read itself)
     }
   }
+  cp_async_wait<0>();
+  __syncthreads();
+  float* fold = reinterpret_cast<float*>(rows_smem);  // [G][cols], over the ring
 #pragma unroll
   for (int i = 0; i < NV; ++i) {
-    const int v = lane + 32 * i;
+    const int v = at + 32 * WPR * i;
     if (v < nvec) {
-      float* f = fold + wib * cols + 8 * v;
-      reinterpret_cast<float4*>(f)[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
-      reinterpret_cast<float4*>(f)[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
+      float4* f = reinterpret_cast<float4*>(fold + group * cols + 8 * v);
+      f[0] = make_float4(dwacc[i][0], dwacc[i][1], dwacc[i][2], dwacc[i][3]);
+      f[1] = make_float4(dwacc[i][4], dwacc[i][5], dwacc[i][6], dwacc[i][7]);
     }
   }
   __syncthreads();
   float* out = dw_partial + (long long)blockIdx.x * cols;
-  for (int col = threadIdx.x; col < cols; col += 128) out[col] = (fold[col] + fold[cols + col]) + (fold[2 * cols + col] + fold[3 * cols + col]);
+  for (int col = threadIdx.x; col < cols; col += 256) {
+    float t = 0.f;
+#pragma unroll
+    for (int j = 0; j < G; ++j) t += fold[j * cols + col];
+    out[col] = t;
+  }
 }
 
 // dw[c] (+)= sum_b partial[b][c]; output bf16 or fp32.  One CTA per 32 columns: 8 row lanes x 32 columns read the partials
@@ -476,7 +516,7 @@ ATS_API int ats_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
 // dw_partial: fp32 scratch of nblocks*cols; dw written as bf16 (dw_bf16) and/or fp32 (dw_f32).
 static int rmsnorm_bwd_launch(const void* x, const void* w, const void* dy, const float* rstd, const void* dres_in, void* dx,
                               float* dw_partial, int nblocks, void* dw_bf16, float* dw_f32, int accumulate, long long rows,
-                              int cols, void* stream, bool warp_rows) {
+                              int cols, void* stream, bool many_rows) {
   if (cols & 7) return 1003;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   auto X = static_cast<const __nv_bfloat16*>(x);
@@ -484,16 +524,21 @@ static int rmsnorm_bwd_launch(const void* x, const void* w, const void* dy, cons
   auto DY = static_cast<const __nv_bfloat16*>(dy);
   auto DR = static_cast<const __nv_bfloat16*>(dres_in);
   auto DX = static_cast<__nv_bfloat16*>(dx);
-  static const bool warp_rows_on = [] {
-    const char* e = getenv("ATS_NORM_WARP_ROWS");  // "0" keeps the CTA-per-row kernels everywhere (for comparisons)
-    return !(e && e[0] == '0');
-  }();
-  if (warp_rows && warp_rows_on && cols <= 2048 && rows >= 1024 && nblocks >= 1) {
-    // many rows of moderate width: one warp per row, two CTAs of four warps per SM
-    const int nb = nblocks < 296 ? nblocks : 296;
-    const size_t sm = size_t(4) * cols * sizeof(float) + (cols <= 1024 ? 4 : 8) * 512;
-    if (cols <= 1024) rmsnorm_bwd_warp_kernel<4><<<nb, 128, sm, s>>>(X, W, DY, rstd, DR, DX, dw_partial, (int)rows, cols);
-    else rmsnorm_bwd_warp_kernel<8><<<nb, 128, sm, s>>>(X, W, DY, rstd, DR, DX, dw_partial, (int)rows, cols);
+  if (many_rows && rows >= 1024 && cols <= 16384 && nblocks >= 1) {
+    const int nb = nblocks < 148 ? nblocks : 148;
+    auto go = [&](auto kernel, int nv, int wpr) -> int {
+      const int smem = (8 / wpr * 2 * 3 + 1) * 32 * wpr * nv * 16;
+      if (cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return int(ce);
+      kernel<<<nb, 256, smem, s>>>(X, W, DY, rstd, DR, DX, dw_partial, (int)rows, cols);
+      return int(cudaGetLastError());
+    };
+    int e;
+    if (cols <= 1024) e = go(rmsnorm_bwd_rows_kernel<4, 1>, 4, 1);
+    else if (cols <= 2048) e = go(rmsnorm_bwd_rows_kernel<8, 1>, 8, 1);
+    else if (cols <= 4096) e = go(rmsnorm_bwd_rows_kernel<8, 2>, 8, 2);
+    else if (cols <= 8192) e = go(rmsnorm_bwd_rows_kernel<8, 4>, 8, 4);
+    else e = go(rmsnorm_bwd_rows_kernel<8, 8>, 8, 8);
+    if (e) return e;
     colsum_partial_kernel<<<(cols + 31) / 32, 256, 0, s>>>(dw_partial, nb, cols, static_cast<__nv_bfloat16*>(dw_bf16), dw_f32, accumulate);
     return int(cudaGetLastError());
   }

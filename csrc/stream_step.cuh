@@ -1,7 +1,7 @@
 // What the weight-streaming products of a decode step share (csrc/int4.cu, csrc/gemv_bf16.cu): a CTA owns one tile of 16 output features, or two
 // that belong together, its warps split the reduction, and what a decode step does around a product is done with the sums.
 #pragma once
-#include "common.cuh"
+#include "async_copy.cuh"
 
 namespace ats {
 
@@ -12,20 +12,12 @@ __device__ __forceinline__ void mma_16816(float (&c)[4], uint32_t a0, uint32_t a
                : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem) : "memory");
-}
 __device__ __forceinline__ void cp_async16_or_zero(void* smem, const void* gmem, bool valid) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 16, %2;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem), "r"(valid ? 16 : 0)
                : "memory");
 }
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(uint32_t(__cvta_generic_to_shared(smem))), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() {
-  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
 }
 
 // What a decode step does around its products, instead of launches of their own (all optional):
