@@ -37,9 +37,12 @@ constexpr int MAX_GROUPS = 256;
 constexpr int GEMM_SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + (MAX_GROUPS + 1) * 4;
 
 enum Epilogue : int { kStore = 0, kAddC = 1, kF32 = 2, kSwiGLU = 3, kSwiGLUBwd = 4, kGelu = 5, kDyt = 6, kSilu = 7 };
-// Each class has a tile function and a pair kernel of its own (kGluClass also takes the plain epilogues of a launch that gathers B).
-enum EpilogueClass : int { kPlainClass, kGluClass, kBlockClass };
-__host__ __device__ constexpr EpilogueClass class_of(int epilogue) { return epilogue <= kF32 ? kPlainClass : epilogue <= kSwiGLUBwd ? kGluClass : kBlockClass; }
+// Each class has a tile function and a pair kernel of its own, which then gets the registers that it needs and no others; launches that gather B have
+// one kernel for all but the block steps.
+enum EpilogueClass : int { kPlainClass, kSwiGLUClass, kSwiGLUBwdClass, kBlockClass, kGatherClass };
+__host__ __device__ constexpr EpilogueClass class_of(int epilogue) {
+  return epilogue <= kF32 ? kPlainClass : epilogue == kSwiGLU ? kSwiGLUClass : epilogue == kSwiGLUBwd ? kSwiGLUBwdClass : kBlockClass;
+}
 
 struct GemmArgs {
   int M, N, K;
@@ -229,158 +232,75 @@ __device__ __forceinline__ bool wait_chunk(const GemmArgs& p, ChunkRange& r, int
 }
 
 // Epilogue of one tile for one warp: `taddr` = TMEM address of the accumulator at this warp's lane quadrant, `row_in_tile` =
-// the accumulator row (TMEM lane) that this thread owns.
-__device__ __forceinline__ void epilogue_glu_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile) {
+// the accumulator row (TMEM lane) that this thread owns.  With PARTS = 2 two warps share the rows: `part` says
+// which half of the columns.
+template <int PARTS>
+__device__ __forceinline__ void epilogue_swiglu_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
   const int row = t.m0 + row_in_tile;
   const bool row_ok = row < t.valid;
-  const bool have_acc = t.k_iters > 0;
   const float rs = (p.row_scale && row_ok) ? p.row_scale[p.rs_gs * t.g + row] * p.alpha : p.alpha;
   const float* cs = p.col_scale ? p.col_scale + p.cs_gs * (t.g / p.k_split / p.b_div) : nullptr;
-  if (p.epilogue == kSwiGLU) {
-    __nv_bfloat16* dbase = p.d_table ? static_cast<__nv_bfloat16*>(p.d_table[t.g]) : p.D + p.d_gs * t.g;
-    __nv_bfloat16* drow = dbase + (long long)row * p.ldd;
-    __nv_bfloat16* arow = p.aux ? p.aux + p.aux_gs * t.g + (long long)row * p.ldaux : nullptr;
+  __nv_bfloat16* dbase = p.d_table ? static_cast<__nv_bfloat16*>(p.d_table[t.g]) : p.D + p.d_gs * t.g;
+  __nv_bfloat16* drow = dbase + (long long)row * p.ldd;
+  __nv_bfloat16* arow = p.aux ? p.aux + p.aux_gs * t.g + (long long)row * p.ldaux : nullptr;
 #pragma unroll 1
-    for (int c = 0; c < 4; ++c) {
-      uint32_t gr[32], ur[32];
-      tmem_ld_32x32(taddr + c * 32, gr);
-      tmem_ld_32x32(taddr + 128 + c * 32, ur);
-      tmem_ld_wait();
-      if (p.fp8 == 2) {  // int8 operands: the accumulator columns hold s32
+  for (int c = part * (4 / PARTS); c < (part + 1) * (4 / PARTS); ++c) {
+    uint32_t gr[32], ur[32];
+    tmem_ld_32x32(taddr + c * 32, gr);
+    tmem_ld_32x32(taddr + 128 + c * 32, ur);
+    tmem_ld_wait();
+    if (p.fp8 == 2) {  // int8 operands: the accumulator columns hold s32
 #pragma unroll
-        for (int i = 0; i < 32; ++i) {
-          gr[i] = __float_as_uint(__int2float_rn(int(gr[i])));
-          ur[i] = __float_as_uint(__int2float_rn(int(ur[i])));
-        }
-      }
-      if (row_ok) {
-        // eight columns: h, gate and up as four packed bf16 pairs each
-        auto piece = [&](int v, int col, uint4& hq, uint4& gq4, uint4& uq4) {
-          uint32_t h[4], gg[4], uu[4];
-#pragma unroll
-          for (int e = 0; e < 4; ++e) {
-            float g0 = __uint_as_float(gr[v * 8 + 2 * e]) * rs, g1 = __uint_as_float(gr[v * 8 + 2 * e + 1]) * rs;
-            float u0 = __uint_as_float(ur[v * 8 + 2 * e]) * rs, u1 = __uint_as_float(ur[v * 8 + 2 * e + 1]) * rs;
-            if (cs) {
-              g0 *= cs[col + 2 * e];
-              g1 *= cs[col + 2 * e + 1];
-              u0 *= cs[p.up_offset + col + 2 * e];
-              u1 *= cs[p.up_offset + col + 2 * e + 1];
-            }
-            gg[e] = pack_bf16x2(g0, g1);
-            uu[e] = pack_bf16x2(u0, u1);
-            // activation on the bf16-rounded values so a separate SwiGLU pass gives identical bits
-            float2 gq = unpack_bf16x2(gg[e]), uq = unpack_bf16x2(uu[e]);
-            h[e] = pack_bf16x2(silu_f(gq.x) * uq.x, silu_f(gq.y) * uq.y);
-          }
-          hq = make_uint4(h[0], h[1], h[2], h[3]);
-          gq4 = make_uint4(gg[0], gg[1], gg[2], gg[3]);
-          uq4 = make_uint4(uu[0], uu[1], uu[2], uu[3]);
-        };
-        if (p.wide) {
-#pragma unroll
-          for (int v = 0; v < 4; v += 2) {
-            const int col = t.n0 + c * 32 + v * 8;
-            if (col + 16 <= p.N) {
-              uint4 h0, g0, u0, h1, g1, u1;
-              piece(v, col, h0, g0, u0);
-              piece(v + 1, col + 8, h1, g1, u1);
-              st_global_32B(drow + col, h0, h1);
-              if (arow) {
-                st_global_32B(arow + col, g0, g1);
-                st_global_32B(arow + p.up_offset + col, u0, u1);
-              }
-            } else if (col < p.N) {
-              uint4 h0, g0, u0;
-              piece(v, col, h0, g0, u0);
-              *reinterpret_cast<uint4*>(drow + col) = h0;
-              if (arow) {
-                *reinterpret_cast<uint4*>(arow + col) = g0;
-                *reinterpret_cast<uint4*>(arow + p.up_offset + col) = u0;
-              }
-            }
-          }
-        } else {
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            const int col = t.n0 + c * 32 + v * 8;
-            if (col < p.N) {
-              uint4 h0, g0, u0;
-              piece(v, col, h0, g0, u0);
-              *reinterpret_cast<uint4*>(drow + col) = h0;
-              if (arow) {
-                *reinterpret_cast<uint4*>(arow + col) = g0;
-                *reinterpret_cast<uint4*>(arow + p.up_offset + col) = u0;
-              }
-            }
-          }
-        }
+      for (int i = 0; i < 32; ++i) {
+        gr[i] = __float_as_uint(__int2float_rn(int(gr[i])));
+        ur[i] = __float_as_uint(__int2float_rn(int(ur[i])));
       }
     }
-  } else {  // kSwiGLUBwd
-    __nv_bfloat16* dbase = p.D + p.d_gs * t.g + (long long)row * p.ldd;
-    const __nv_bfloat16* arow = p.aux + p.aux_gs * t.g + (long long)row * p.ldaux;
-    __nv_bfloat16* hrow = p.out2 ? p.out2 + p.out2_gs * t.g + (long long)row * p.ldout2 : nullptr;
-#pragma unroll 1
-    for (int c = 0; c < BN / 32; ++c) {
-      uint4 g[4], u[4];  // the chunk's 32 gate and 32 up values, requested before the accumulator is read
-      if (p.wide && row_ok) {
-#pragma unroll
-        for (int v = 0; v < 4; v += 2) {
-          const int col = t.n0 + c * 32 + v * 8;
-          if (col + 16 <= p.N) {
-            ld_global_32B(arow + col, g[v], g[v + 1]);
-            ld_global_32B(arow + p.up_offset + col, u[v], u[v + 1]);
-          } else if (col < p.N) {
-            g[v] = *reinterpret_cast<const uint4*>(arow + col);
-            u[v] = *reinterpret_cast<const uint4*>(arow + p.up_offset + col);
-          }
-        }
-      }
-      uint32_t r[32];
-      if (have_acc) {
-        tmem_ld_32x32(taddr + c * 32, r);
-        tmem_ld_wait();
-      } else {
-#pragma unroll
-        for (int i = 0; i < 32; ++i) r[i] = 0;
-      }
-      if (!row_ok) continue;
-      // eight columns from the saved gate / up values and the accumulator
-      auto piece = [&](int v, const uint4& gq, const uint4& uq, uint4& og4, uint4& ou4, uint4& oh4) {
-        const uint32_t gg[4] = {gq.x, gq.y, gq.z, gq.w}, uu[4] = {uq.x, uq.y, uq.z, uq.w};
-        uint32_t og[4], ou[4], oh[4];
+    if (row_ok) {
+      // eight columns: h, gate and up as four packed bf16 pairs each
+      auto piece = [&](int v, int col, uint4& hq, uint4& gq4, uint4& uq4) {
+        uint32_t h[4], gg[4], uu[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          // dh rounded to bf16 first: bit-identical to writing dh and running the separate backward kernel
-          const float2 d = unpack_bf16x2(pack_bf16x2(__uint_as_float(r[v * 8 + 2 * e]) * rs, __uint_as_float(r[v * 8 + 2 * e + 1]) * rs));
-          const float2 a = unpack_bf16x2(gg[e]), b = unpack_bf16x2(uu[e]);
-          const float s0 = 1.f / (1.f + __expf(-a.x)), s1 = 1.f / (1.f + __expf(-a.y));
-          const float si0 = a.x * s0, si1 = a.y * s1;
-          og[e] = pack_bf16x2(d.x * b.x * (s0 + si0 * (1.f - s0)), d.y * b.y * (s1 + si1 * (1.f - s1)));
-          ou[e] = pack_bf16x2(d.x * si0, d.y * si1);
-          oh[e] = pack_bf16x2(si0 * b.x, si1 * b.y);
+          float g0 = __uint_as_float(gr[v * 8 + 2 * e]) * rs, g1 = __uint_as_float(gr[v * 8 + 2 * e + 1]) * rs;
+          float u0 = __uint_as_float(ur[v * 8 + 2 * e]) * rs, u1 = __uint_as_float(ur[v * 8 + 2 * e + 1]) * rs;
+          if (cs) {
+            g0 *= cs[col + 2 * e];
+            g1 *= cs[col + 2 * e + 1];
+            u0 *= cs[p.up_offset + col + 2 * e];
+            u1 *= cs[p.up_offset + col + 2 * e + 1];
+          }
+          gg[e] = pack_bf16x2(g0, g1);
+          uu[e] = pack_bf16x2(u0, u1);
+          // activation on the bf16-rounded values so a separate SwiGLU pass gives identical bits
+          float2 gq = unpack_bf16x2(gg[e]), uq = unpack_bf16x2(uu[e]);
+          h[e] = pack_bf16x2(silu_f(gq.x) * uq.x, silu_f(gq.y) * uq.y);
         }
-        og4 = make_uint4(og[0], og[1], og[2], og[3]);
-        ou4 = make_uint4(ou[0], ou[1], ou[2], ou[3]);
-        oh4 = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+        hq = make_uint4(h[0], h[1], h[2], h[3]);
+        gq4 = make_uint4(gg[0], gg[1], gg[2], gg[3]);
+        uq4 = make_uint4(uu[0], uu[1], uu[2], uu[3]);
       };
       if (p.wide) {
 #pragma unroll
         for (int v = 0; v < 4; v += 2) {
           const int col = t.n0 + c * 32 + v * 8;
-          uint4 a0, b0, c0, a1, b1, c1;
           if (col + 16 <= p.N) {
-            piece(v, g[v], u[v], a0, b0, c0);
-            piece(v + 1, g[v + 1], u[v + 1], a1, b1, c1);
-            st_global_32B(dbase + col, a0, a1);
-            st_global_32B(dbase + p.up_offset + col, b0, b1);
-            if (hrow) st_global_32B(hrow + col, c0, c1);
+            uint4 h0, g0, u0, h1, g1, u1;
+            piece(v, col, h0, g0, u0);
+            piece(v + 1, col + 8, h1, g1, u1);
+            st_global_32B(drow + col, h0, h1);
+            if (arow) {
+              st_global_32B(arow + col, g0, g1);
+              st_global_32B(arow + p.up_offset + col, u0, u1);
+            }
           } else if (col < p.N) {
-            piece(v, g[v], u[v], a0, b0, c0);
-            *reinterpret_cast<uint4*>(dbase + col) = a0;
-            *reinterpret_cast<uint4*>(dbase + p.up_offset + col) = b0;
-            if (hrow) *reinterpret_cast<uint4*>(hrow + col) = c0;
+            uint4 h0, g0, u0;
+            piece(v, col, h0, g0, u0);
+            *reinterpret_cast<uint4*>(drow + col) = h0;
+            if (arow) {
+              *reinterpret_cast<uint4*>(arow + col) = g0;
+              *reinterpret_cast<uint4*>(arow + p.up_offset + col) = u0;
+            }
           }
         }
       } else {
@@ -388,11 +308,13 @@ __device__ __forceinline__ void epilogue_glu_tile(const GemmArgs& p, const TileC
         for (int v = 0; v < 4; ++v) {
           const int col = t.n0 + c * 32 + v * 8;
           if (col < p.N) {
-            uint4 a0, b0, c0;
-            piece(v, *reinterpret_cast<const uint4*>(arow + col), *reinterpret_cast<const uint4*>(arow + p.up_offset + col), a0, b0, c0);
-            *reinterpret_cast<uint4*>(dbase + col) = a0;
-            *reinterpret_cast<uint4*>(dbase + p.up_offset + col) = b0;
-            if (hrow) *reinterpret_cast<uint4*>(hrow + col) = c0;
+            uint4 h0, g0, u0;
+            piece(v, col, h0, g0, u0);
+            *reinterpret_cast<uint4*>(drow + col) = h0;
+            if (arow) {
+              *reinterpret_cast<uint4*>(arow + col) = g0;
+              *reinterpret_cast<uint4*>(arow + p.up_offset + col) = u0;
+            }
           }
         }
       }
@@ -400,7 +322,95 @@ __device__ __forceinline__ void epilogue_glu_tile(const GemmArgs& p, const TileC
   }
 }
 
-// kStore, kAddC and kF32.  With PARTS = 2 two warps share the rows: `part` says which half of the columns.
+// kSwiGLUBwd
+template <int PARTS>
+__device__ __forceinline__ void epilogue_swiglu_bwd_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
+  const int row = t.m0 + row_in_tile;
+  const bool row_ok = row < t.valid;
+  const bool have_acc = t.k_iters > 0;
+  const float rs = (p.row_scale && row_ok) ? p.row_scale[p.rs_gs * t.g + row] * p.alpha : p.alpha;
+  __nv_bfloat16* dbase = p.D + p.d_gs * t.g + (long long)row * p.ldd;
+  const __nv_bfloat16* arow = p.aux + p.aux_gs * t.g + (long long)row * p.ldaux;
+  __nv_bfloat16* hrow = p.out2 ? p.out2 + p.out2_gs * t.g + (long long)row * p.ldout2 : nullptr;
+#pragma unroll 1
+  for (int c = part * (BN / 32 / PARTS); c < (part + 1) * (BN / 32 / PARTS); ++c) {
+    uint4 g[4], u[4];  // the chunk's 32 gate and 32 up values, requested before the accumulator is read
+    if (p.wide && row_ok) {
+#pragma unroll
+      for (int v = 0; v < 4; v += 2) {
+        const int col = t.n0 + c * 32 + v * 8;
+        if (col + 16 <= p.N) {
+          ld_global_32B(arow + col, g[v], g[v + 1]);
+          ld_global_32B(arow + p.up_offset + col, u[v], u[v + 1]);
+        } else if (col < p.N) {
+          g[v] = *reinterpret_cast<const uint4*>(arow + col);
+          u[v] = *reinterpret_cast<const uint4*>(arow + p.up_offset + col);
+        }
+      }
+    }
+    uint32_t r[32];
+    if (have_acc) {
+      tmem_ld_32x32(taddr + c * 32, r);
+      tmem_ld_wait();
+    } else {
+#pragma unroll
+      for (int i = 0; i < 32; ++i) r[i] = 0;
+    }
+    if (!row_ok) continue;
+    // eight columns from the saved gate / up values and the accumulator
+    auto piece = [&](int v, const uint4& gq, const uint4& uq, uint4& og4, uint4& ou4, uint4& oh4) {
+      const uint32_t gg[4] = {gq.x, gq.y, gq.z, gq.w}, uu[4] = {uq.x, uq.y, uq.z, uq.w};
+      uint32_t og[4], ou[4], oh[4];
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        // dh rounded to bf16 first: bit-identical to writing dh and running the separate backward kernel
+        const float2 d = unpack_bf16x2(pack_bf16x2(__uint_as_float(r[v * 8 + 2 * e]) * rs, __uint_as_float(r[v * 8 + 2 * e + 1]) * rs));
+        const float2 a = unpack_bf16x2(gg[e]), b = unpack_bf16x2(uu[e]);
+        const float s0 = 1.f / (1.f + __expf(-a.x)), s1 = 1.f / (1.f + __expf(-a.y));
+        const float si0 = a.x * s0, si1 = a.y * s1;
+        og[e] = pack_bf16x2(d.x * b.x * (s0 + si0 * (1.f - s0)), d.y * b.y * (s1 + si1 * (1.f - s1)));
+        ou[e] = pack_bf16x2(d.x * si0, d.y * si1);
+        oh[e] = pack_bf16x2(si0 * b.x, si1 * b.y);
+      }
+      og4 = make_uint4(og[0], og[1], og[2], og[3]);
+      ou4 = make_uint4(ou[0], ou[1], ou[2], ou[3]);
+      oh4 = make_uint4(oh[0], oh[1], oh[2], oh[3]);
+    };
+    if (p.wide) {
+#pragma unroll
+      for (int v = 0; v < 4; v += 2) {
+        const int col = t.n0 + c * 32 + v * 8;
+        uint4 a0, b0, c0, a1, b1, c1;
+        if (col + 16 <= p.N) {
+          piece(v, g[v], u[v], a0, b0, c0);
+          piece(v + 1, g[v + 1], u[v + 1], a1, b1, c1);
+          st_global_32B(dbase + col, a0, a1);
+          st_global_32B(dbase + p.up_offset + col, b0, b1);
+          if (hrow) st_global_32B(hrow + col, c0, c1);
+        } else if (col < p.N) {
+          piece(v, g[v], u[v], a0, b0, c0);
+          *reinterpret_cast<uint4*>(dbase + col) = a0;
+          *reinterpret_cast<uint4*>(dbase + p.up_offset + col) = b0;
+          if (hrow) *reinterpret_cast<uint4*>(hrow + col) = c0;
+        }
+      }
+    } else {
+#pragma unroll
+      for (int v = 0; v < 4; ++v) {
+        const int col = t.n0 + c * 32 + v * 8;
+        if (col < p.N) {
+          uint4 a0, b0, c0;
+          piece(v, *reinterpret_cast<const uint4*>(arow + col), *reinterpret_cast<const uint4*>(arow + p.up_offset + col), a0, b0, c0);
+          *reinterpret_cast<uint4*>(dbase + col) = a0;
+          *reinterpret_cast<uint4*>(dbase + p.up_offset + col) = b0;
+          if (hrow) *reinterpret_cast<uint4*>(hrow + col) = c0;
+        }
+      }
+    }
+  }
+}
+
+// kStore, kAddC and kF32
 template <int PARTS>
 __device__ __forceinline__ void epilogue_plain_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
   const int c_begin = part * (BN / 32 / PARTS), c_end = c_begin + BN / 32 / PARTS;  // chunks of 32 columns
@@ -526,7 +536,7 @@ __device__ __forceinline__ void epilogue_plain_tile(const GemmArgs& p, const Til
   }
 }
 
-// The block steps (kGelu, kDyt, kSilu), shared between warps in the same way.
+// The block steps: kGelu, kDyt, kSilu
 template <int PARTS>
 __device__ __forceinline__ void epilogue_block_tile(const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
   const int c_begin = part * (BN / 32 / PARTS), c_end = c_begin + BN / 32 / PARTS;  // chunks of 32 columns
@@ -600,10 +610,18 @@ __device__ __forceinline__ void epilogue_block_tile(const GemmArgs& p, const Til
   }
 }
 
+template <int PARTS>
+__device__ __forceinline__ void epilogue_tile(EpilogueClass cls, const GemmArgs& p, const TileCoord& t, uint32_t taddr, int row_in_tile, int part) {
+  if (cls == kPlainClass) epilogue_plain_tile<PARTS>(p, t, taddr, row_in_tile, part);
+  else if (cls == kSwiGLUClass) epilogue_swiglu_tile<PARTS>(p, t, taddr, row_in_tile, part);
+  else if (cls == kSwiGLUBwdClass) epilogue_swiglu_bwd_tile<PARTS>(p, t, taddr, row_in_tile, part);
+  else epilogue_block_tile<PARTS>(p, t, taddr, row_in_tile, part);
+}
+
 // What the epilogue of a tile reads beside the accumulator (the matrix or the sums that are added to, the residual stream) is asked into L2 while
 // the tile's main loop runs: each thread asks for its row's share, whole stretches of it, where the epilogue itself reads 64 bytes a time.
-// `tile` may lie behind the last one.  (The saved pre-activations of the SwiGLU backward are not: reading twice as many bytes as such a product
-// stores, that epilogue is bound by the requests to L2, and more of them made it slower, 375 -> 412 us for 16,384 x 5,632 x 2,048.)
+// `tile` may lie behind the last one.  (The saved pre-activations of the SwiGLU backward are not: that epilogue moves five values an element, the
+// requests to L2 bound it, and more of them made it slower, 375 -> 412 us for 16,384 x 5,632 x 2,048.)
 template <int PARTS>
 __device__ __forceinline__ void prefetch_epilogue(const GemmArgs& p, const int* prefix, int tile, int total_tiles, int g_hint, int row_in_tile, int part, int bm) {
   if (tile >= total_tiles || !(p.wide || p.epilogue == kDyt)) return;
@@ -841,10 +859,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
       if (!mbar_wait_bounded(&tfull[acc], acc_phase, abort_flag, p.status, kTimeoutTmemFull)) break;
       tc_fence_after();
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
-      const EpilogueClass cls = class_of(p.epilogue);
-      if (cls == kPlainClass) epilogue_plain_tile<1>(p, t, taddr, row_in_tile, 0);
-      else if (cls == kGluClass) epilogue_glu_tile(p, t, taddr, row_in_tile);
-      else epilogue_block_tile<1>(p, t, taddr, row_in_tile, 0);
+      epilogue_tile<1>(class_of(p.epilogue), p, t, taddr, row_in_tile, 0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive(&tempty[acc]);
@@ -887,14 +902,14 @@ constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 + 256 + (M
 // Epilogue warps per CTA.  With four, a warp walks the 256 columns of its 32 rows alone and hides neither its TMEM round trips nor its loads behind
 // anything: the Dynamic-Tanh step took 33 us a tile, GELU 17, where the main loop of a 2,048-long reduction takes 14, and in a product of one wave
 // the epilogue is the last thing that runs.  With eight, two share the columns: 16,384 x 2,048 x 2,048 with the Dynamic-Tanh step 230 -> 174 us,
-// 16,384 x 8,192 x 2,048 with GELU 479 -> 410, 3,000 x 1,024 x 1,024 stored 19.5 -> 18.5, added to a matrix 25.6 -> 21.5.  The gated products stay at
-// four: theirs (two values read and three stored for each of the backward) are bound by their requests to L2, and eight warps made them slower
-// (16,384 x 5,632 x 2,048 375 -> 382 us), as does their share of registers.
-constexpr int pair_epi_warps(int cls) { return cls == kGluClass ? 4 : 8; }
-constexpr int pair_threads(int cls) { return 64 + 32 * pair_epi_warps(cls); }  // and two copy warps in launches that gather B
+// 16,384 x 8,192 x 2,048 with GELU 479 -> 410, 3,000 x 1,024 x 1,024 stored 19.5 -> 18.5, added to a matrix 25.6 -> 21.5, 16,384 x 4,096 x 512 87 -> 77
+// and 169 -> 116; the SwiGLU backward of 16,384 x 5,632 x 2,048 362 -> 347, of 3,000 x 2,816 x 1,024 46 -> 42 (of 4,096 x 11,008 x 4,096, whose main
+// loop hides it, 285 -> 287), SwiGLU 538 -> 533, 41.0 -> 39.9, 474 -> 470.  Launches that gather B have four beside their two copy warps.
+constexpr int pair_epi_warps(int cls) { return cls == kGatherClass ? 4 : 8; }
+constexpr int pair_threads(int cls) { return 64 + 32 * pair_epi_warps(cls) + (cls == kGatherClass ? 64 : 0); }
 
 template <int CLASS, int EW = pair_epi_warps(CLASS)>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(CLASS) + (CLASS == kGluClass ? 64 : 0), 1)
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(pair_threads(CLASS), 1)
 gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                       const __grid_constant__ CUtensorMap map_b_own, const GemmArgs p) {
   extern __shared__ uint8_t smem_raw[];
@@ -953,7 +968,7 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
 
   if (warp >= 2 + EW) {
     // ------------------------------------------------------------------ copy warps (launches that gather B from its owners)
-    if (p.n_copy) copy_remote_shards(p, warp - 2 - EW, lane);
+    if (CLASS == kGatherClass) copy_remote_shards(p, warp - 2 - EW, lane);
   } else if (warp == 0) {
     // ------------------------------------------------------------------ TMA producer (both CTAs)
     if (lane == 0) {
@@ -1108,10 +1123,9 @@ gemm_bf16_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_co
       tc_fence_after();
       if (reads) prefetch_epilogue<EW / 4>(p, prefix, tile + tile_step, total_tiles, g_hint, int(rank) * BM + row_in_tile, part, PAIR_BM);
       const uint32_t taddr = tmem_base + acc * BN + (uint32_t(quad * 32) << 16);
-      if constexpr (CLASS == kBlockClass) epilogue_block_tile<EW / 4>(p, t, taddr, row_in_tile, part);
-      else if constexpr (CLASS == kPlainClass) epilogue_plain_tile<EW / 4>(p, t, taddr, row_in_tile, part);
-      else if (class_of(p.epilogue) == kPlainClass) epilogue_plain_tile<1>(p, t, taddr, row_in_tile, 0);
-      else epilogue_glu_tile(p, t, taddr, row_in_tile);
+      if constexpr (CLASS != kGatherClass) epilogue_tile<EW / 4>(EpilogueClass(CLASS), p, t, taddr, row_in_tile, part);
+      else if (p.epilogue == kSwiGLU) epilogue_swiglu_tile<1>(p, t, taddr, row_in_tile, 0);
+      else epilogue_plain_tile<1>(p, t, taddr, row_in_tile, 0);
       tc_fence_before();
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(mapa_shared(smem_u32(&tempty[acc]), 0));
@@ -1511,15 +1525,15 @@ static int sector_aligned_outputs(const GemmArgs& p) {
 template <int CLASS>
 static int launch_pairs(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb_own, const GemmArgs& p, long long tiles, int max_ctas,
                         void* stream) {
-  const bool gather = CLASS == kGluClass && p.n_copy > 0;
-  const int threads = pair_threads(CLASS) + (gather ? 64 : 0);  // the two copy warps exist only in launches that gather B from peers
+  constexpr bool gather = CLASS == kGatherClass;
+  constexpr int threads = pair_threads(CLASS);
   static int pair_clusters = -1;
   if (pair_clusters < 0) {
     cudaError_t ce = cudaFuncSetAttribute(gemm_bf16_pair_kernel<CLASS>, cudaFuncAttributeMaxDynamicSharedMemorySize, PAIR_SMEM_BYTES);
     if (ce != cudaSuccess) return int(ce);
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(num_sms() & ~1));
-    cfg.blockDim = dim3(pair_threads(CLASS));
+    cfg.blockDim = dim3(threads);
     cfg.dynamicSmemBytes = PAIR_SMEM_BYTES;
     int n = 0;
     ce = cudaOccupancyMaxActiveClusters(&n, gemm_bf16_pair_kernel<CLASS>, &cfg);
@@ -1551,10 +1565,13 @@ static int launch_gemm(const CUtensorMap& ma, const CUtensorMap& mb, const GemmA
   if (g_gemm_pair && M >= PAIR_BM) {
     // two SMs per 256 x 256 tile
     const long long tiles = (long long)groups * ((M + PAIR_BM - 1) / PAIR_BM) * tn;
-    const EpilogueClass cls = class_of(epilogue);
-    if (cls == kBlockClass) return launch_pairs<kBlockClass>(ma, mb, mb, p, tiles, max_ctas, stream);
-    return cls == kGluClass || p.n_copy > 0 ? launch_pairs<kGluClass>(ma, mb, mb_own ? *mb_own : mb, p, tiles, max_ctas, stream)
-                                            : launch_pairs<kPlainClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+    if (p.n_copy > 0) return launch_pairs<kGatherClass>(ma, mb, mb_own ? *mb_own : mb, p, tiles, max_ctas, stream);
+    switch (class_of(epilogue)) {
+      case kPlainClass: return launch_pairs<kPlainClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+      case kSwiGLUClass: return launch_pairs<kSwiGLUClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+      case kSwiGLUBwdClass: return launch_pairs<kSwiGLUBwdClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+      default: return launch_pairs<kBlockClass>(ma, mb, mb, p, tiles, max_ctas, stream);
+    }
   }
   long long upper = (long long)groups * ((M + BM - 1) / BM) * tn;
   int grid = num_sms();
