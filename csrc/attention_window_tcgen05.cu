@@ -67,7 +67,8 @@ window_attn_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_co
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int h = blockIdx.x, b = blockIdx.y, q0 = blockIdx.z * 256;
+  // the tiles with the longest windows first: CTAs are handed out with z slowest, and the short ones of a prompt's first window then fill the end
+  const int h = blockIdx.x, b = blockIdx.y, q0 = int(gridDim.z - 1 - blockIdx.z) * 256;
   const int last_row = p.rows - 1;
   // key blocks of 128 rows start at kb0; tile A uses blocks [0, nA), tile B blocks [jB, nB)
   const int kb0 = max(0, p.n_old + q0 - p.window + 1);

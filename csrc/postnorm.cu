@@ -45,8 +45,10 @@ struct PostNormArgs {
   int N, width;
 };
 
-// QPT quads per thread stay in registers between the passes (N <= 4 * 256 * QPT); QPT = 0: rows of any length go through x.
-template <typename T, int QPT>
+// QPT quads per thread stay in registers between the passes (N <= 4 * 256 * QPT); QPT = 0: rows of any length go through x.  SPLITS > 0: that many
+// blocks, all requested at once with the residual and the weight: a decode step has a CTA for each of its few rows, and one round trip to L2 instead of
+// two per quad and one for the weight is most of its time (us in a chain of launches: 64 rows of 2,048, eight blocks 3.9 -> 2.6, one block 2.8 -> 2.0; 4,503 rows, one block 16.0 -> 14.2).
+template <typename T, int QPT, int SPLITS>
 __global__ void __launch_bounds__(256) fold_postnorm_kernel(const PostNormArgs p) {
   pdl_prologue();
   __shared__ float red[40];
@@ -58,6 +60,7 @@ __global__ void __launch_bounds__(256) fold_postnorm_kernel(const PostNormArgs p
   auto sum = [&](int q) {
     float4 z = *reinterpret_cast<const float4*>(x + 4 * q);
     z.x *= p.alpha; z.y *= p.alpha; z.z *= p.alpha; z.w *= p.alpha;
+#pragma unroll 4
     for (int s = 0; s < p.splits; ++s) {
       const float4 t = *reinterpret_cast<const float4*>(y + s * p.split_stride + 4 * q);
       z.x += t.x; z.y += t.y; z.z += t.z; z.w += t.w;
@@ -65,18 +68,40 @@ __global__ void __launch_bounds__(256) fold_postnorm_kernel(const PostNormArgs p
     return z;
   };
   auto sq = [](const float4& z) { return z.x * z.x + z.y * z.y + z.z * z.z + z.w * z.w; };
-  auto scaled = [](const float4& z, const float* w, float r) {
-    const float4 g = *reinterpret_cast<const float4*>(w);
-    return make_float4(z.x * r * g.x, z.y * r * g.y, z.z * r * g.z, z.w * r * g.w);
-  };
+  auto quad = [](const float* v) { return *reinterpret_cast<const float4*>(v); };
+  auto scaled = [](const float4& z, const float4& g, float r) { return make_float4(z.x * r * g.x, z.y * r * g.y, z.z * r * g.z, z.w * r * g.w); };
   constexpr int R = QPT > 0 ? QPT : 1;
-  float4 z[R];
+  float4 z[R], wv[R];
   float ss = 0.f;
-  if constexpr (QPT > 0) {
+  if constexpr (QPT > 0 && SPLITS > 0) {
+    float4 part[R][SPLITS];
+#pragma unroll
+    for (int i = 0; i < QPT; ++i) {
+      const int q = tid + i * 256;
+      if (q < quads) {
+        z[i] = quad(x + 4 * q);
+#pragma unroll
+        for (int s = 0; s < SPLITS; ++s) part[i][s] = quad(y + s * p.split_stride + 4 * q);
+        wv[i] = quad(p.w + 4 * q);
+      }
+    }
+#pragma unroll
+    for (int i = 0; i < QPT; ++i) {
+      if (tid + i * 256 < quads) {
+        z[i].x *= p.alpha; z[i].y *= p.alpha; z[i].z *= p.alpha; z[i].w *= p.alpha;
+#pragma unroll
+        for (int s = 0; s < SPLITS; ++s) {
+          z[i].x += part[i][s].x; z[i].y += part[i][s].y; z[i].z += part[i][s].z; z[i].w += part[i][s].w;
+        }
+        ss += sq(z[i]);
+      }
+    }
+  } else if constexpr (QPT > 0) {
 #pragma unroll
     for (int i = 0; i < QPT; ++i) {
       const int q = tid + i * 256;
       z[i] = q < quads ? sum(q) : make_float4(0.f, 0.f, 0.f, 0.f);
+      if (q < quads) wv[i] = quad(p.w + 4 * q);
       ss += sq(z[i]);
     }
   } else {
@@ -88,8 +113,8 @@ __global__ void __launch_bounds__(256) fold_postnorm_kernel(const PostNormArgs p
   }
   const float r = 1.f / sqrtf(block_sum(ss, red) / float(p.width) + p.eps);
   float s2 = 0.f;
-  auto finish = [&](int q, float4 t) {
-    t = scaled(t, p.w + 4 * q, r);
+  auto finish = [&](int q, float4 t, const float4& w) {
+    t = scaled(t, w, r);
     *reinterpret_cast<float4*>(x + 4 * q) = t;
     if (p.w2) s2 += sq(t);
     else if (h) Typed<T>::store4(h + 4 * q, t);
@@ -98,18 +123,18 @@ __global__ void __launch_bounds__(256) fold_postnorm_kernel(const PostNormArgs p
   if constexpr (QPT > 0) {
 #pragma unroll
     for (int i = 0; i < QPT; ++i)
-      if (tid + i * 256 < quads) z[i] = finish(tid + i * 256, z[i]);
+      if (tid + i * 256 < quads) z[i] = finish(tid + i * 256, z[i], wv[i]);
   } else {
-    for (int q = tid; q < quads; q += 256) finish(q, *reinterpret_cast<const float4*>(x + 4 * q));
+    for (int q = tid; q < quads; q += 256) finish(q, quad(x + 4 * q), quad(p.w + 4 * q));
   }
   if (!p.w2) return;  // the whole grid agrees
   const float r2 = 1.f / sqrtf(block_sum(s2, red) / float(p.width) + p.eps);
   if constexpr (QPT > 0) {
 #pragma unroll
     for (int i = 0; i < QPT; ++i)
-      if (tid + i * 256 < quads) Typed<T>::store4(h + 4 * (tid + i * 256), scaled(z[i], p.w2 + 4 * (tid + i * 256), r2));
+      if (tid + i * 256 < quads) Typed<T>::store4(h + 4 * (tid + i * 256), scaled(z[i], quad(p.w2 + 4 * (tid + i * 256)), r2));
   } else {
-    for (int q = tid; q < quads; q += 256) Typed<T>::store4(h + 4 * q, scaled(*reinterpret_cast<const float4*>(x + 4 * q), p.w2 + 4 * q, r2));
+    for (int q = tid; q < quads; q += 256) Typed<T>::store4(h + 4 * q, scaled(quad(x + 4 * q), quad(p.w2 + 4 * q), r2));
   }
 }
 
@@ -212,11 +237,24 @@ template <typename T>
 static int launch_postnorm(const PostNormArgs& p, cudaStream_t s) {
   const int q = (p.N / 4 + 255) / 256;
   const dim3 grid{unsigned(p.rows)}, block(256);
-  if (q <= 1) launch_pdl(fold_postnorm_kernel<T, 1>, grid, block, 0, s, p);
-  else if (q <= 2) launch_pdl(fold_postnorm_kernel<T, 2>, grid, block, 0, s, p);
-  else if (q <= 4) launch_pdl(fold_postnorm_kernel<T, 4>, grid, block, 0, s, p);
-  else if (q <= 8) launch_pdl(fold_postnorm_kernel<T, 8>, grid, block, 0, s, p);
-  else launch_pdl(fold_postnorm_kernel<T, 0>, grid, block, 0, s, p);
+  auto go = [&](auto kernel) { launch_pdl(kernel, grid, block, 0, s, p); };
+  auto by_splits = [&](auto one, auto two, auto four, auto eight, auto any) {
+    switch (p.splits) {
+      case 1: return go(one);
+      case 2: return go(two);
+      case 4: return go(four);
+      case 8: return go(eight);
+      default: return go(any);
+    }
+  };
+  if (q <= 1)
+    by_splits(fold_postnorm_kernel<T, 1, 1>, fold_postnorm_kernel<T, 1, 2>, fold_postnorm_kernel<T, 1, 4>, fold_postnorm_kernel<T, 1, 8>, fold_postnorm_kernel<T, 1, 0>);
+  else if (q <= 2)
+    by_splits(fold_postnorm_kernel<T, 2, 1>, fold_postnorm_kernel<T, 2, 2>, fold_postnorm_kernel<T, 2, 4>, fold_postnorm_kernel<T, 2, 8>, fold_postnorm_kernel<T, 2, 0>);
+  else if (q <= 4)  // (eight blocks of four quads would be 128 registers)
+    by_splits(fold_postnorm_kernel<T, 4, 1>, fold_postnorm_kernel<T, 4, 2>, fold_postnorm_kernel<T, 4, 4>, fold_postnorm_kernel<T, 4, 0>, fold_postnorm_kernel<T, 4, 0>);
+  else if (q <= 8) go(fold_postnorm_kernel<T, 8, 0>);
+  else go(fold_postnorm_kernel<T, 0, 0>);
   return int(cudaGetLastError());
 }
 
