@@ -25,14 +25,18 @@ class SequenceCache:
         self.device_active: Optional[torch.Tensor] = None
 
     def enable_device_lengths(self) -> None:
-        self.device_lengths = torch.full((self.batch,), self.length, dtype=torch.int32, device=self.device)
-        self.device_positions = torch.full((self.batch,), self.length, dtype=torch.int32, device=self.device)
+        self._device_counters = torch.full((2, self.batch), self.length, dtype=torch.int32, device=self.device)   # (one launch moves both on)
+        self.device_lengths, self.device_positions = self._device_counters
         self.device_active = torch.ones(self.batch, dtype=torch.int32, device=self.device)
 
     def device_advance(self) -> None:
         """One decoded token of every active row: called inside the captured step."""
-        self.device_lengths += self.device_active
-        self.device_positions += self.device_active
+        rows = (self.device_lengths, self.device_positions)
+        if [t.data_ptr() for t in rows] == [t.data_ptr() for t in self._device_counters]:
+            self._device_counters += self.device_active
+        else:   # (tensors of the caller's in their place)
+            for t in rows:
+                t += self.device_active
 
     def set_row(self, row: int, length: int, active: bool) -> None:
         self.device_lengths[row] = length

@@ -616,12 +616,10 @@ class DeepSeekTransformer(nn.Module):
             logits = logits / math.sqrt(self.config.hidden_size)
         has_aux = self.config.use_moe or self.config.use_mod
         want_aux = has_aux if return_aux_loss is None else return_aux_loss
+        if not want_aux:   # (a decode step: no launch for a sum that nobody reads)
+            return (logits, x) if return_hidden_states else logits
         total_aux = torch.stack(aux_losses).sum() if aux_losses else logits.new_zeros(())
-        if return_hidden_states:
-            return (logits, x, total_aux, aux_losses) if want_aux else (logits, x)
-        if want_aux:
-            return logits, total_aux, aux_losses
-        return logits
+        return (logits, x, total_aux, aux_losses) if return_hidden_states else (logits, total_aux, aux_losses)
 
     def forward_loss(self, input_ids: torch.Tensor, labels: torch.Tensor, loss_weights: Optional[torch.Tensor] = None,
                      attention_mask: Optional[torch.Tensor] = None, ignore_index: int = -100) -> Dict[str, torch.Tensor]:

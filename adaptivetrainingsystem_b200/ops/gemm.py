@@ -71,8 +71,6 @@ def _fn():
         lib.ats_splitk_reduce.argtypes = [_vp, _c_int, _c_ll, _c_ll, _vp, _vp, _vp]
         lib.ats_gemm_skinny.restype = _c_int
         lib.ats_gemm_skinny.argtypes = [_vp, _c_ll, _vp, _c_ll, _c_ll, ctypes.POINTER(_Skinny), _c_int, _vp]
-        lib.ats_gemv_bf16.restype = _c_int
-        lib.ats_gemv_bf16.argtypes = [_vp, _c_ll, _vp, _c_ll, _vp, _c_ll, _vp, _c_ll, _c_int, _c_int, _c_int, _c_int, ctypes.POINTER(StreamStep), _c_int, _vp]
         lib.ats_chain_launches.restype = None
         lib.ats_chain_launches.argtypes = [_c_int]
         lib.ats_gemm_set_pair.restype = None
@@ -226,7 +224,7 @@ def skinny_splits(T: int, N: int, K: int, width: int = 128) -> int:
     return s if s <= 4 else 4 if s < 8 else 8
 
 
-_STREAM_MODES = {SK_STORE: 0, SK_SWIGLU: 1, SK_ROPE: 2}
+_STREAM_MODES = (SK_STORE, SK_SWIGLU, SK_ROPE)
 
 
 def stream_fits(T: int, N: int, K: int, mode: int = SK_STORE, head_dim: int = 0) -> bool:
@@ -256,21 +254,16 @@ def norm_parts(T: int, N: int, K: int) -> int:
 def skinny(a: torch.Tensor, w: torch.Tensor, out: torch.Tensor, mode: int, n: Optional[int] = None, splits: Optional[int] = None, add: Optional[torch.Tensor] = None,
            alpha: float = 1.0, up_offset: int = 0, act_cols: int = 0, bias: Optional[torch.Tensor] = None, x: Optional[torch.Tensor] = None, chain=None,
            head_dim: int = 0, pos: Optional[torch.Tensor] = None, next_norm=None, scale=None) -> None:
-    """One launch of the decode kernel; ``chain`` = (w1, b1, a1, w2, b2, a2) of the residual step ``SK_DYT``; for ``SK_ROPE``
+    """One launch of the decode kernel or, by the lines of :func:`stream_fits`, of the streaming one; ``chain`` = (w1, b1, a1, w2, b2, a2) of the residual step ``SK_DYT``; for ``SK_ROPE``
     w1 and w2 are the cosine and sine tables, ``pos`` the positions (int32) and ``act_cols`` the rotated columns.  ``next_norm`` = (weight, rows
     [T, N], sums of squares [T, norm_parts]) of an RMSNorm that follows ``SK_STORE``; ``scale`` = (sums of squares, eps): ``a`` came from such a product."""
     _fn()
     a, w = _check2d(a), _check2d(w)
     (T, K), N = a.shape, w.shape[0] if n is None else n
-    if (splits is None and alpha == 1.0 and stream_fits(T, N, K, mode, head_dim) and (mode != SK_SWIGLU or (add is None and up_offset == N and w.shape[0] == 2 * N))
-            and (next_norm is None or next_norm[2].shape[1] == N // 16) and (mode != SK_ROPE or add is None and act_cols % head_dim == 0)):
-        step = stream_step(K, scale, next_norm, (chain[0], chain[3], pos, act_cols, head_dim) if mode == SK_ROPE else None)
-        _lib.check(_lib.cuda_lib().ats_gemv_bf16(w.data_ptr(), w.stride(0), a.data_ptr(), a.stride(0), None if add is None else add.data_ptr(), 0 if add is None else add.stride(0),
-                                                 out.data_ptr(), out.stride(-2), T, w.shape[0] if mode == SK_SWIGLU else N, K, _STREAM_MODES[mode], step, int(_weight_ready(w)),
-                                                 _lib.stream_ptr(a.device)), "ats_gemv_bf16")
-        return
     if splits is None:
-        splits = skinny_splits(T, N, K, 64 if mode == SK_SWIGLU else 128)
+        stream = (alpha == 1.0 and stream_fits(T, N, K, mode, head_dim) and (mode != SK_SWIGLU or (add is None and up_offset == N and w.shape[0] == 2 * N))
+                  and (next_norm is None or next_norm[2].shape[1] == N // 16) and (mode != SK_ROPE or (add is None and act_cols % head_dim == 0)))
+        splits = 0 if stream else skinny_splits(T, N, K, 64 if mode == SK_SWIGLU else 128)
     w1, b1, a1, w2, b2, a2 = chain if chain is not None else (None, None, 0.0, None, None, 0.0)
 
     def at(t):

@@ -450,9 +450,10 @@ int sk_launch(const CUtensorMap& mw, const CUtensorMap& ma, const SkinnyArgs& p,
 using namespace ats;
 
 // a [T, K] (row pitch lda), w [N, K] (or [2 N, K] with up_offset rows between gate and up for kSkSwiglu, row pitch ldw); `splits` reduction
-// slices (kSkPart: out is [splits, T, N] fp32).  Both operands 16-byte aligned with row pitches of a multiple of 8.
+// slices (kSkPart: out is [splits, T, N] fp32), or 0 for the streaming kernel.  Both operands 16-byte aligned with row pitches of a multiple of 8.
 ATS_API int ats_gemm_skinny(const void* a, long long lda, const void* w, long long ldw, long long w_rows, const SkinnyArgs* args, int splits, void* stream) {
   SkinnyArgs p = *args;
+  if (splits == 0) return stream_product(a, lda, w, ldw, w_rows, p, static_cast<cudaStream_t>(stream));
   const int blocks = (p.K + SK_BK - 1) / SK_BK;
   if (p.T < 1 || p.T > 128 || p.N < 1 || p.K < 8 || splits < 1 || splits > blocks || (splits > SK_MAX_SPLIT && p.mode != kSkPart)) return 1003;
   const int nt = p.T <= 16 ? 16 : p.T <= 32 ? 32 : p.T <= 64 ? 64 : 128;

@@ -11,6 +11,7 @@
 // 2,560 x 2,048 5.2 / 3.7, pairs of 2,816 x 1,024 4.8 / 3.3; sixteen rows 5.0 / 3.8, 8.3 / 7.3, 5.6 / 4.6, 5.1 / 4.1.  Which products come here:
 // stream_fits() in ops/gemm.py.  Warps, ring and CTAs per SM are the fastest of nine forms (a ring of four steps for up to eight tokens, 16 warps:
 // 2,048 x 5,632 5.2, eight warps 7.3, rings of two steps 7.4).
+#include "skinny.cuh"
 #include "stream_step.cuh"
 
 namespace ats {
@@ -135,36 +136,35 @@ int launch_gemv(int ctas, const __nv_bfloat16* w, long long ldw, const __nv_bflo
                 long long ld_out, int M, int N, int K, int early, const StreamStep& st, cudaStream_t s) {
   constexpr int kRing = WARPS * DEPTH * bf16_stage_bytes(MODE == kStreamStore ? 1 : 2, NT);
   auto kernel = gemv_bf16_kernel<MODE, WARPS, NT, DEPTH, MINB>;
-  static bool attr_set = false;
-  if (!attr_set) {
-    if (cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing)) return int(ce);
-    attr_set = true;
-  }
+  if (cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kRing)) return int(ce);
   return int(launch_pdl(kernel, dim3(ctas), dim3(WARPS * 32), kRing, s, w, ldw, x, ldx, add, ld_add, out, ld_out, M, N, K, early, st));
 }
 
 }  // namespace
-}  // namespace ats
 
-using namespace ats;
-
-// out [M, N] (kStreamSwiGLU: [M, N / 2]) = x [M, K] @ w [N, K]^T (+ add), M <= 16, N a multiple of 16 (32 for pairs of tiles), K of 64, rows of x and w
-// 16-byte aligned; `w_ready`: no kernel that may still run writes w.  `step` may be null.
-ATS_API int ats_gemv_bf16(const void* w, long long ldw, const void* x, long long ldx, const void* add, long long ld_add, void* out, long long ld_out, int M, int N,
-                          int K, int mode, const StreamStep* step, int w_ready, void* stream) {
-  if (M < 1 || M > 16 || N < 16 || (N & 15) || K < 64 || (K & 63) || (ldx & 7) || (ldw & 7) || (reinterpret_cast<uintptr_t>(x) & 15) || (reinterpret_cast<uintptr_t>(w) & 15)) return 1003;
-  if (mode < kStreamStore || mode > kStreamRope || (mode != kStreamStore && (N & 31))) return 1003;
+// Takes kSkStore (+ add), kSkSwiglu and kSkRope of up to 16 tokens, N a multiple of 16 (of 32, and of the heads, for kSkRope), K of 64.
+int stream_product(const void* a, long long lda, const void* w, long long ldw, long long w_rows, const SkinnyArgs& p, cudaStream_t s) {
+  const int mode = p.mode == kSkStore ? kStreamStore : p.mode == kSkSwiglu ? kStreamSwiGLU : p.mode == kSkRope ? kStreamRope : -1;
+  const int M = p.T, K = p.K, N = mode == kStreamSwiGLU ? 2 * p.N : p.N;
+  if (mode < 0 || M < 1 || M > 16 || N < 16 || (p.N & 15) || K < 64 || (K & 63) || (lda & 7) || (ldw & 7) || w_rows < N || p.alpha != 1.f ||
+      (reinterpret_cast<uintptr_t>(a) & 15) || (reinterpret_cast<uintptr_t>(w) & 15) || (mode == kStreamSwiGLU && (p.up_offset != p.N || p.add)) ||
+      (mode == kStreamRope && (N & 31)))
+    return 1003;
   StreamStep st = {};
-  if (step) st = *step;
-  if (!stream_step_ok(st, mode, N, add != nullptr)) return 1003;
+  st.scale_parts = p.scale_parts; st.scale_n = p.scale_n; st.scale_inv = p.scale_inv; st.scale_eps = p.scale_eps;
+  st.next_w = p.next_w; st.next_out = p.next_out; st.next_parts = p.next_parts;
+  st.pos = p.pos; st.cos_t = p.w1; st.sin_t = p.w2; st.act_cols = p.act_cols; st.head_dim = p.head_dim;
+  if (!stream_step_ok(st, mode, N, p.add != nullptr)) return 1003;
   if (mode != kStreamRope) st.head_dim = 32;
-  const int early = w_ready && chained_launches(), tiles = N / 16, pairs = tiles / 2;
+  const int early = p.w_ready && chained_launches(), tiles = N / 16, pairs = tiles / 2;
   auto go = [&](auto launch, int ctas) {
-    return launch(ctas, static_cast<const __nv_bfloat16*>(w), ldw, static_cast<const __nv_bfloat16*>(x), ldx, static_cast<const __nv_bfloat16*>(add), ld_add,
-                  static_cast<__nv_bfloat16*>(out), ld_out, M, N, K, early, st, static_cast<cudaStream_t>(stream));
+    return launch(ctas, static_cast<const __nv_bfloat16*>(w), ldw, static_cast<const __nv_bfloat16*>(a), lda, p.add, p.ldadd, static_cast<__nv_bfloat16*>(p.out), p.ldo, M, N,
+                  K, early, st, s);
   };
   const bool two = M > 8;
   if (mode == kStreamSwiGLU) return two ? go(launch_gemv<kStreamSwiGLU, 8, 2, 2, 2>, pairs) : go(launch_gemv<kStreamSwiGLU, 8, 1, 2, 3>, pairs);
   if (mode == kStreamRope) return two ? go(launch_gemv<kStreamRope, 8, 2, 3, 2>, pairs) : go(launch_gemv<kStreamRope, 8, 1, 4, 2>, pairs);
   return two ? go(launch_gemv<kStreamStore, 16, 2, 2, 1>, tiles) : go(launch_gemv<kStreamStore, 16, 1, 4, 1>, tiles);
 }
+
+}  // namespace ats

@@ -1,6 +1,7 @@
 // Arguments of the decode-sized product (gemm_skinny.cu); mirrored by ops/gemm.py.
 #pragma once
 #include <cuda_bf16.h>
+#include <cuda_runtime.h>
 
 namespace ats {
 
@@ -39,5 +40,8 @@ struct SkinnyArgs {
   int* status;
   int w_ready;   // no kernel that may still run writes w (it is no result of the same step): in a chain of launches its first tiles are requested early
 };
+
+// The product as a stream through warps (gemv_bf16.cu): out, add, scale, next and the rotation as above, next_parts per 16 columns.
+int stream_product(const void* a, long long lda, const void* w, long long ldw, long long w_rows, const SkinnyArgs& p, cudaStream_t s);
 
 }  // namespace ats
