@@ -29,7 +29,7 @@ struct SkinnyArgs {
   const float *w1, *b1, *w2, *b2;
   const int* pos;
   // RMSNorm between two products.  The first one (kSkStore) also writes next_out [T, N] = bf16(out) * next_w and, per token and tile of 128
-  // columns, the sum of squares of its bf16 results (next_parts [T, tiles]); the second one reads next_out as its activations and multiplies
+  // columns (of 16 on the streaming kernel), the sum of squares of its bf16 results (next_parts [T, tiles]); the second one reads next_out as its activations and multiplies
   // its sums by rsqrt(sum of the scale_n parts of the token * scale_inv + scale_eps).
   const __nv_bfloat16* next_w;
   __nv_bfloat16* next_out;
