@@ -76,7 +76,7 @@ def _L():
 _P, _S, _CK = _lib.ptr, _lib.stream_ptr, _lib.check
 import os as _os
 
-_NORM_BLOCKS = int(_os.environ.get("ATS_NORM_BLOCKS", "1184"))  # CTAs of the row-walking backward kernels (8 per SM keeps enough rows in flight)
+_NORM_BLOCKS = int(_os.environ.get("ATS_NORM_BLOCKS", "1184"))  # most CTAs of the row-walking backward kernels (8 per SM; from 1,024 rows on the RMSNorm uses one per SM)
 
 
 # ----------------------------------------------------------------------------------------------------------

@@ -63,10 +63,11 @@ __device__ __forceinline__ void dq_word(uint32_t w, const Int4Consts& k, uint32_
   a[3] = dq_scale(and_or(shr_mulhi(w, k.m12), k.mask, k.magic), zB, sB);
 }
 
-// Asynchronous copies global -> shared (each lane copies into slots only it reads back, so no barrier is involved: a lane waits
-// for its own copy groups).  Loads into registers did not pipeline here: with five loads per step and stage the kernel waited
+// The ring of asynchronous copies (async_copy.cuh): each lane copies into slots only it reads back, so no barrier is involved: a lane waits
+// for its own copy groups.  Loads into registers did not pipeline here: with five loads per step and stage the kernel waited
 // a full round trip to memory in every step whatever the prefetch depth (1.9 TB/s, warps 68 % of the time on the long
 // scoreboard); copy groups are counted, not score-boarded.
+//
 // bytes one warp holds per stage: packed words and scale words of R tiles, 16 activations per lane and token tile
 __host__ __device__ constexpr int int4_stage_bytes(int R, int NT) { return 32 * (R * 16 + R * 8 + NT * 32); }
 __host__ __device__ constexpr int int4_ring_bytes(int WARPS, int R, int NT, int DEPTH) { return WARPS * DEPTH * int4_stage_bytes(R, NT); }
