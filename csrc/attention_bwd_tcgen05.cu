@@ -121,7 +121,8 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   uint64_t* ds_full = bars + 14;   // the same for dS (VIA_SMEM: P and dS written to shared memory)
   uint64_t* ds_free = bars + 15;   // without OVER: the products that read P and dS are done
   uint64_t* acc_done = bars + 16;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 17);
+  uint64_t* row_full = bars + 17;  // OVER: one arrival per softmax warp, its share of an iteration's statistics written and those before read
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -158,6 +159,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     mbar_init(ds_full, 4 * AB_SPLIT);
     mbar_init(ds_free, 1);
     mbar_init(acc_done, 1);
+    mbar_init(row_full, 4 * AB_SPLIT);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&map_q);
@@ -363,7 +365,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       if (MODE == 0 && ++to_diagonal == nq - fixed) to_diagonal = 0;
       const float* nl = sRow + (t & 1) * 256 + part * AB_COLS;   // of this thread's columns; 128 floats on those of delta
       if (OVER) {
-        asm volatile("bar.sync 1, %0;" ::"n"(128 * AB_SPLIT) : "memory");   // the values of this iteration are there, those of the one before are read
+        // The values of this iteration are there, those of the one before are read.  (No named barrier: a warp that has given up never comes to it.)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(row_full);
+        if (!mbar_wait_warp(row_full, t & 1, abort_flag, p.status, kTimeoutFull)) {
+          ok = false;
+          break;
+        }
         if (t + 1 < n_iter) sRow[((t + 1) & 1) * 256 + id] = ahead;
         next_tile();
         if (t + 2 < n_iter) ahead = row_stat(id & 127, id < 128);
@@ -372,7 +380,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         next_tile();
         if (t + 1 < n_iter) ahead = row_stat(r, true), ahead_d = row_stat(r, false);
       }
-      if (!mbar_wait_bounded(s_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) {
+      if (!mbar_wait_warp(s_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) {
         ok = false;
         break;
       }
@@ -389,7 +397,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       // dP^T or dP: without OVER it is on its way while the exponentials are taken
       uint32_t dv[AB_COLS];
       auto load_dp = [&] {
-        if (!mbar_wait_bounded(dp_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) return false;
+        if (!mbar_wait_warp(dp_full, t & 1, abort_flag, p.status, kTimeoutTmemFull)) return false;
         tc_fence_after();
 #pragma unroll
         for (int c = 0; c < AB_COLS / 32; ++c) tmem_ld_32x32(tmem_dP + col + c * 32, reinterpret_cast<uint32_t(&)[32]>(dv[c * 32]));
@@ -463,7 +471,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         }
       }
       // the products of the previous iteration must be done with P and dS before they are overwritten
-      if (!OVER && !mbar_wait_bounded(ds_free, (t & 1) ^ 1, abort_flag, p.status, kTimeoutTmemEmpty)) {
+      if (!OVER && !mbar_wait_warp(ds_free, (t & 1) ^ 1, abort_flag, p.status, kTimeoutTmemEmpty)) {
         ok = false;
         break;
       }
@@ -482,7 +490,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       __syncwarp();
       if (lane == 0) mbar_arrive(ds_full);
     }
-    if (ok && mbar_wait_bounded(acc_done, 0, abort_flag, p.status, kTimeoutTmemFull)) {
+    if (ok && mbar_wait_warp(acc_done, 0, abort_flag, p.status, kTimeoutTmemFull)) {
       tc_fence_after();
       const bool real = fixed * 128 + r < p.L;
       const long long tok = (long long)b * p.L + fixed * 128 + r;

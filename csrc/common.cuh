@@ -113,6 +113,10 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
   }
   return true;
 }
+// The same by a whole warp whose lanes go on together or give up together: one that left alone would leave the others at their next __syncwarp.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait_bounded(bar, parity, abort_flag, status, code));
+}
 
 // ----------------------------------------------------------------------------------------------
 // TMA (tiled, non-multicast). The innermost coordinate times the element size must be a multiple
