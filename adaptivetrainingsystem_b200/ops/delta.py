@@ -206,7 +206,7 @@ def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state:
         return out
     mma = scan_on_tensor_cores(mixed, s)
     groups = -(-L // (GROUP_MMA if mma else GROUP))
-    size = 832 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # layouts: csrc/delta_rule_mma.cu, csrc/delta_rule.cu
+    size = 836 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # layouts: csrc/delta_rule_mma.cu, csrc/delta_rule.cu
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
     o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
     args = _Scan(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0), B, L, H, KH, s.dim, s.vdim, groups, int(fresh))
@@ -269,7 +269,7 @@ def channel_delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor
         return out
     mma, DK = scan_on_tensor_cores(mixed, s), s.scan_rows
     groups = -(-L // (GROUP_MMA if mma else GROUP))
-    size = 73 * DK + 768 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # layouts: csrc/channel_delta_mma.cu, csrc/channel_delta.cu
+    size = 73 * DK + 784 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # layouts: csrc/channel_delta_mma.cu, csrc/channel_delta.cu
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
     o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
     args = _Channel(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(a), a.stride(0), _p(neg_rate), _p(dt_bias), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0),

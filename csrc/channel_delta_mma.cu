@@ -12,8 +12,8 @@
 // eight tokens with a later one factor at the eighth token, so that only the two 8 x 8 blocks on the diagonal are summed pair by pair.
 //
 // Bounded like delta_rule_mma.cu; 350 MMAs a group and warp.  Scan and pairs, us, fp32 FMA form (channel_delta.cu) / this one, 128 x 128 states: 8 sequences of
-// 2,048 tokens, 16 heads 1,213 / 808, 12 of 1,000 934 / 621, 3 of 1,501 537 / 326, one of 2,048 542 / 367, one of 512, 8 heads 121 / 99, one of 64 30 / 28.
-// State against 64 bits: 0.4e-6 (fast decays) to 1.6e-6 (slow ones, the errors of the decays' exponentials) on both.
+// 2,048 tokens, 16 heads 1,213 / 837, 12 of 1,000 934 / 635, 3 of 1,501 537 / 330, one of 2,048 542 / 371, one of 512, 8 heads 121 / 99, one of 64 30 / 29.
+// State against 64 bits: 0.84 to 0.995 of the FMA form's error on average (slow decays 1.2e-6 to 2.5e-6, the errors of the decays' exponentials; fast ones 0.5e-7).
 #include "delta_mma.cuh"
 
 namespace ats {
@@ -26,10 +26,10 @@ constexpr int CM_COLS = 64;              // value columns of a CTA
 constexpr int CM_STAGES = 2;
 constexpr int CM_ROWS = 3 * CM;          // P k, P q, k g_{j+1} .. g_C
 
-// Bytes per group and head: three pieces of the rows, T, R, P_C.
+// Bytes per group and head: three pieces of the rows, T without its diagonal, R, P_C, the diagonal (the step sizes).
 __host__ __device__ constexpr int cm_t_at(int DK) { return 3 * CM_ROWS * DK * 2; }
 __host__ __device__ constexpr int cm_p_at(int DK) { return cm_t_at(DK) + 2 * CM_B; }
-__host__ __device__ constexpr int cm_bytes(int DK) { return cm_p_at(DK) + DK * 4; }
+__host__ __device__ constexpr int cm_bytes(int DK) { return cm_p_at(DK) + DK * 4 + CM * 4; }
 // Byte of channel d (even) of a row: 16-byte pieces exchanged inside 128 bytes by the row's last three bits.
 __host__ __device__ constexpr int cm_at(int row, int d, int DK) { return row * DK * 2 + ((d >> 3 & ~7) | ((d >> 3 ^ row) & 7)) * 16 + (d & 7) * 2; }
 constexpr int CM_PITCH = 132;            // floats of a row that the off-diagonal block is computed from
@@ -101,7 +101,7 @@ __global__ void __launch_bounds__(128, 3) channel_pairs_mma_kernel(const Channel
       for (int i = 0; i < 8; ++i) {
         const float rk = i < n ? rl[(long long)i * 2 * p.KH + p.KH + kh] : 0.f, rq = i < n ? rl[(long long)i * 2 * p.KH + kh] : 0.f;
         const float2 fk = unpack_bf16x2(pk[i]), fq = unpack_bf16x2(pq[i]), fa = unpack_bf16x2(pa[i]);
-        kv[i][0] = fk.x * rk, kv[i][1] = fk.y * rk, qv[i][0] = fq.x * rq, qv[i][1] = fq.y * rq;
+        kv[i][0] = fk.x * rk, kv[i][1] = fk.y * rk; qv[i][0] = fq.x * rq, qv[i][1] = fq.y * rq;
         g[i][0] = i < n && d0 < p.dim ? decay_of<__nv_bfloat16>(fa.x + dt[0], rate) : 1.f;
         g[i][1] = i < n && d0 + 1 < p.dim ? decay_of<__nv_bfloat16>(fa.y + dt[1], rate) : 1.f;
       }
@@ -221,9 +221,11 @@ __global__ void __launch_bounds__(128, 3) channel_pairs_mma_kernel(const Channel
       }
     }
     __syncwarp();
-    if (lane < CM)
+    if (lane < CM) {
 #pragma unroll
-      for (int i = 0; i < CM; ++i) s_kk[i][lane] = y[i] * bc;   // T
+      for (int i = 0; i < CM; ++i) s_kk[i][lane] = i == lane ? 0.f : y[i] * bc;   // T
+      reinterpret_cast<float*>(co + cm_p_at(DK))[DK + lane] = bc;
+    }
     __syncwarp();
     store_split_b(s_kk, lane, reinterpret_cast<uint4*>(co + cm_t_at(DK)));
   }
@@ -335,7 +337,7 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
         mma_bf16(eq[x], a.hi, qb[2 * x], qb[2 * x + 1]);
       }
     }
-    float u[2][4];
+    float u[2][4], eu[2][4];
     Pieces a;
     {
       uint32_t vv[4];   // tokens 0..7 / 8..15 of column g, then of column g + 8
@@ -350,8 +352,14 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
       }
       split_tiles(sk[0], sk[1], a);
       split_product(a, mt, lane, u);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const float2 be = *reinterpret_cast<const float2*>(decay + DK + 8 * x + 2 * t);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) add_diagonal(e & 1 ? be.y : be.x, sk[x][e], u[x][e], eu[x][e]);
+      }
     }
-    split_tiles(u[0], u[1], a);
+    split_tiles(u[0], u[1], eu[0], eu[1], a);
 #pragma unroll
     for (int s = 0; s < KS; ++s) {   // the state first: the next group waits for it
       const uint32_t kat = at + cm_at(2 * CM + trow, 16 * s + 8 * tpiece, DK);
@@ -380,10 +388,10 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
       for (int x = 0; x < 2; ++x) {
         const float2 P = *reinterpret_cast<const float2*>(decay + 16 * s + 8 * x + 2 * t);
         float(&S_)[4] = S[2 * s + x];
-        S_[0] = fmaf(S_[0], P.x, d[x][0] + f[x][0]);
-        S_[1] = fmaf(S_[1], P.y, d[x][1] + f[x][1]);
-        S_[2] = fmaf(S_[2], P.x, d[x][2] + f[x][2]);
-        S_[3] = fmaf(S_[3], P.y, d[x][3] + f[x][3]);
+        S_[0] = fmaf(S_[0], P.x, f[x][0]) + d[x][0];
+        S_[1] = fmaf(S_[1], P.y, f[x][1]) + d[x][1];
+        S_[2] = fmaf(S_[2], P.x, f[x][2]) + d[x][2];
+        S_[3] = fmaf(S_[3], P.y, f[x][3]) + d[x][3];
       }
     }
     {
@@ -437,7 +445,7 @@ int launch_channel_mma(const ChannelArgs& p, int* status, cudaStream_t s) {
 using namespace ats;
 
 // bf16 rows whose values are whole 16-byte pieces (dim, vdim, ldm, ldo multiples of 8, mixed and o 16-byte aligned), dim up to DK (64 or 128), p->groups
-// groups of 16 tokens; coef: per (sequence, group, head) 292 DK + 3072 bytes (cm_bytes), 16-byte aligned.
+// groups of 16 tokens; coef: per (sequence, group, head) 292 DK + 3136 bytes (cm_bytes), 16-byte aligned.
 ATS_API int ats_channel_delta_mma(const ChannelArgs* p, int* status, void* stream) {
   if (p->B <= 0 || p->L <= 0) return 0;
   if (p->groups != (p->L + CM - 1) / CM || p->KH < 1 || p->H % p->KH || (p->DK != 64 && p->DK != 128) || p->dim < 1 || p->dim > p->DK ||

@@ -1,8 +1,11 @@
-// Warp-level tensor-core pieces of the delta-rule scans (delta_rule_mma.cu): fp32 operands as sums of bf16 values, fragments, asynchronous copies.
+// Warp-level tensor-core pieces of the delta-rule scans (delta_rule_mma.cu, channel_delta_mma.cu): fp32 operands as sums of bf16 values, fragments,
+// asynchronous copies.
 //
-// An fp32 value has 24 significant bits, three bf16 values have 8 each: cut off after every eight bits, the pieces add up to the value exactly,
-// and a product of a piece with a bf16 number is exact in fp32.  So a product of an fp32 matrix with a bf16 one is three
-// tensor-core products, one of two fp32 matrices six (the three pairs of pieces left out are below 2^-24 of the product).
+// An fp32 value has 24 significant bits, three bf16 values have 8 each: each rounded to nearest from what the ones before it leave, the pieces add up
+// to the value exactly, and a product of a piece with a bf16 number is exact in fp32.  So a product of an fp32 matrix with a bf16 one
+// is three tensor-core products, one of two fp32 matrices six: a middle piece is at most 2^-9 of its value, a lowest one 2^-18, so the three pairs left
+// out are within 2^-26 + 2^-36 of the product, of either sign.  (Pieces that are cut off and not rounded leave out up to 2^-21, always towards zero.)
+// The lowest piece has bits to spare: the rounding errors of a value that is on its way into a product go there.
 #pragma once
 #include "delta_common.cuh"
 
@@ -12,14 +15,12 @@ struct Pieces {   // of an A fragment (16 x 16): hi + mid + lo
   uint32_t hi[4], mid[4], lo[4];
 };
 
-// Two neighbouring values of a row as three words of two bf16 each.
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
-  const uint32_t ux = __float_as_uint(x), uy = __float_as_uint(y);
-  hi = __byte_perm(ux, uy, 0x7632);
-  const float rx = x - __uint_as_float(ux & 0xffff0000u), ry = y - __uint_as_float(uy & 0xffff0000u);
-  const uint32_t vx = __float_as_uint(rx), vy = __float_as_uint(ry);
-  mid = __byte_perm(vx, vy, 0x7632);
-  lo = __byte_perm(__float_as_uint(rx - __uint_as_float(vx & 0xffff0000u)), __float_as_uint(ry - __uint_as_float(vy & 0xffff0000u)), 0x7632);
+// Two neighbouring values of a row as three words of two bf16 each; ex, ey: what their own roundings cut off.
+__device__ __forceinline__ void split_pair(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo, float ex = 0.f, float ey = 0.f) {
+  hi = pack_bf16x2(x, y);
+  const float rx = x - __uint_as_float(hi << 16), ry = y - __uint_as_float(hi & 0xffff0000u);
+  mid = pack_bf16x2(rx, ry);
+  lo = pack_bf16x2(rx - __uint_as_float(mid << 16) + ex, ry - __uint_as_float(mid & 0xffff0000u) + ey);
 }
 
 // Accumulator tiles of columns 0..7 (a) and 8..15 (b) of a 16 x 16 block as the A operand of the next product.
@@ -30,12 +31,19 @@ __device__ __forceinline__ void split_tiles(const float (&a)[4], const float (&b
   split_pair(b[2], b[3], p.hi[3], p.mid[3], p.lo[3]);
 }
 
+__device__ __forceinline__ void split_tiles(const float (&a)[4], const float (&b)[4], const float (&ea)[4], const float (&eb)[4], Pieces& p) {
+  split_pair(a[0], a[1], p.hi[0], p.mid[0], p.lo[0], ea[0], ea[1]);
+  split_pair(a[2], a[3], p.hi[1], p.mid[1], p.lo[1], ea[2], ea[3]);
+  split_pair(b[0], b[1], p.hi[2], p.mid[2], p.lo[2], eb[0], eb[1]);
+  split_pair(b[2], b[3], p.hi[3], p.mid[3], p.lo[3], eb[2], eb[3]);
+}
+
 __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                : "+f"(c[0]), "+f"(c[1]), "+f"(c[2]), "+f"(c[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 // Tensor-core sums are cut off at the last place of the result: all in one direction, half a unit on average.  With c = a x b so computed, adds what was cut
-// off to `small`: the same product on top of -c.  (State of the scan after 300 tokens, relative error against 64 bits 1.28e-7 -> 0.92e-7.)
+// off to `small`: the same product on top of -c.  (Without it the state of a scan with fast decays is twice as far from 64 bits.)
 __device__ __forceinline__ void add_rest(const float (&c)[4], float (&small)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
   float rest[4] = {-c[0], -c[1], -c[2], -c[3]};
   mma_bf16(rest, a, b0, b1);
@@ -97,6 +105,14 @@ __device__ __forceinline__ void split_product(const Pieces& a, const uint4* b, i
   for (int n = 0; n < 2; ++n)
 #pragma unroll
     for (int e = 0; e < 4; ++e) c[n][e] += small[n][e];
+}
+
+// u + beta x rhs, with the rounding errors of both in `err`.  beta is the diagonal of a triangular factor, and mostly its largest term by far: a tensor-core
+// sum aligns its products with the largest one and loses the low bits of the others, so the product above takes the rest of the factor alone.
+__device__ __forceinline__ void add_diagonal(float beta, float rhs, float& u, float& err) {
+  const float p = __fmul_rn(beta, rhs), s = __fadd_rn(p, u), v = __fsub_rn(s, p);
+  err = __fmaf_rn(beta, rhs, -p) + (__fsub_rn(p, __fsub_rn(s, v)) + __fsub_rn(u, v));
+  u = s;
 }
 
 }  // namespace ats

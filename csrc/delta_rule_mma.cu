@@ -11,12 +11,13 @@
 // whole chain of its columns; no warp waits for another but for the rows that they share.  An accumulator tile of m16n8k16 has the
 // layout of half an A operand, so S^T multiplies K^T and Q^T (k, q rows by ldmatrix), the right-hand side T^T and U^T R^T and K without leaving the
 // registers.  k and q are bf16 as they come; S, the right-hand side, U, T and R are fp32 and enter as exact sums of three bf16 pieces (delta_mma.cuh),
-// products of the leading pieces and of the others summed apart; the state itself is updated by fp32 FMAs, since tensor-core sums are cut off, not rounded.
+// products of the leading pieces and of the others summed apart; the diagonal of T and the state's decay are fp32 FMAs, since tensor-core sums are cut off,
+// not rounded, and the rounding errors of U and of U D / |k| go into the state with them.
 //
 // What bounds it is the warp-level MMA pipe (some 13 cycles an instruction and SM quarter; 200 a group and warp) and, with one warp a quarter, the chain of
-// dependent products.  Scan and pairs, us, fp32 FMA form (delta_rule.cu) / this one, 128 x 128 states: 8 sequences of 2,048 tokens, 16 heads 1,129 / 420, 12 of
-// 1,000 878 / 330, 3 of 1,501 449 / 189, one of 2,048 435 / 247, one of 512, 8 heads 116 / 72, one of 64 24 / 22.  State against 64 bits (relative, 300 to 2,048
-// tokens): slow decays 2.5e-7 .. 2.9e-7 before, 1.6e-7 .. 2.4e-7 now; fast ones 0.7e-7 .. 1.2e-7, 0.9e-7; read-outs 1.66e-3 (their rounding to bf16) on both.
+// dependent products.  Scan and pairs, us, fp32 FMA form (delta_rule.cu) / this one, 128 x 128 states: 8 sequences of 2,048 tokens, 16 heads 1,129 / 447, 12 of
+// 1,000 878 / 352, 3 of 1,501 449 / 201, one of 2,048 435 / 263, one of 512, 8 heads 116 / 76, one of 64 24 / 21.  State against 64 bits: 0.65 to 0.86 of the FMA form's
+// error on average, from slow decays to those that forget a token at once; read-outs 1.66e-3 (their rounding to bf16) on both.
 #include "delta_mma.cuh"
 
 namespace ats {
@@ -25,8 +26,8 @@ namespace {
 
 constexpr int DM = 16;                          // tokens per group
 constexpr int DM_B = 3 * 32 * 16;               // bytes of a 16 x 16 matrix as split B operand
-constexpr int DM_VEC = 3 * DM + 16;             // floats: G_i / |k_i|, G_i c / |q_i|, D_Ci / |k_i|, then G_C
-constexpr int DM_COEF = 2 * DM_B + DM_VEC * 4;  // bytes per group and head: T, R, the vectors
+constexpr int DM_VEC = 4 * DM + 4;              // floats: G_i / |k_i|, G_i c / |q_i|, D_Ci / |k_i|, the diagonal of T (the step sizes), then G_C
+constexpr int DM_COEF = 2 * DM_B + DM_VEC * 4;  // bytes per group and head: T without its diagonal, R, the vectors
 constexpr int DM_COLS = 64;                     // value columns of a CTA
 constexpr int DM_STAGES = 3;
 
@@ -98,7 +99,7 @@ __global__ void __launch_bounds__(128) delta_pairs_mma_kernel(const ScanArgs p) 
         acc -= beta[i] * dec * s_kk[warp][i][j] * y[j];
       }
       y[i] = acc;
-      s_m[warp][r][0][i][c] = acc * bc;
+      s_m[warp][r][0][i][c] = i == c ? 0.f : acc * bc;
     }
     float dec = 1.f, G = 1.f, GC = 1.f;
 #pragma unroll
@@ -113,7 +114,8 @@ __global__ void __launch_bounds__(128) delta_pairs_mma_kernel(const ScanArgs p) 
       vec[c] = G * rk;
       vec[DM + c] = G * rq;
       vec[2 * DM + c] = dec * rk;   // dec has become g_{c+1} .. g_C
-      vec[3 * DM + c] = GC;
+      vec[3 * DM + c] = bc;
+      if (c == 0) vec[4 * DM] = GC;
     }
     __syncwarp();
     for (int x = 0; x < 2 && r0 + x < rep; ++x)
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
         mma_bf16(eq[x], a.mid, qb[2 * x], qb[2 * x + 1]);
       }
     }
-    float u[2][4];
+    float u[2][4], eu[2][4];
     Pieces a;
     {
       uint32_t vv[4];   // tokens 0..7 / 8..15 of column g, then of column g + 8
@@ -222,16 +224,27 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
       }
       split_tiles(sk[0], sk[1], a);
       split_product(a, mt, lane, u);
+#pragma unroll
+      for (int x = 0; x < 2; ++x) {
+        const float2 be = *reinterpret_cast<const float2*>(vec + 3 * DM + 8 * x + 2 * t);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) add_diagonal(e & 1 ? be.y : be.x, sk[x][e], u[x][e], eu[x][e]);
+      }
     }
     {   // the state first: the next group waits for it
-      float w[2][4];
+      float w[2][4], ew[2][4];
 #pragma unroll
       for (int x = 0; x < 2; ++x) {
         const float2 dk = *reinterpret_cast<const float2*>(vec + 2 * DM + 8 * x + 2 * t);
-        w[x][0] = u[x][0] * dk.x, w[x][1] = u[x][1] * dk.y, w[x][2] = u[x][2] * dk.x, w[x][3] = u[x][3] * dk.y;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          const float f = e & 1 ? dk.y : dk.x;
+          w[x][e] = u[x][e] * f;
+          ew[x][e] = fmaf(u[x][e], f, -w[x][e]) + eu[x][e] * f;
+        }
       }
-      split_tiles(w[0], w[1], a);
-      const float GC = vec[3 * DM];
+      split_tiles(w[0], w[1], ew[0], ew[1], a);
+      const float GC = vec[4 * DM];
 #pragma unroll
       for (int s = 0; s < KS; ++s) {
         uint32_t kt[4];
@@ -250,7 +263,7 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
 #pragma unroll
         for (int x = 0; x < 2; ++x)
 #pragma unroll
-          for (int e = 0; e < 4; ++e) S[2 * s + x][e] = fmaf(S[2 * s + x][e], GC, d[x][e] + f[x][e]);
+          for (int e = 0; e < 4; ++e) S[2 * s + x][e] = fmaf(S[2 * s + x][e], GC, f[x][e]) + d[x][e];
       }
     }
     {
@@ -291,7 +304,7 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
 using namespace ats;
 
 // bf16 rows whose parts are whole 16-byte pieces (dim, vdim, ldm, ldo multiples of 8, mixed and o 16-byte aligned), dim up to 128, p->groups groups of 16
-// tokens; coef: 832 floats per (sequence, group, head), 16-byte aligned.
+// tokens; coef: 836 floats per (sequence, group, head), 16-byte aligned.
 ATS_API int ats_delta_scan_mma(const ScanArgs* p, int fp32, void* stream) {
   if (p->B <= 0 || p->L <= 0) return 0;
   if (fp32 || p->groups != (p->L + DM - 1) / DM || p->KH < 1 || p->H % p->KH || p->dim < 1 || p->dim > 128 || ((p->dim | p->vdim | p->ldm | p->ldo) & 7) ||

@@ -5,9 +5,9 @@ import torch
 pytestmark = pytest.mark.gpu
 
 
-def _inputs(channel, B, L, H, KH, dim, vdim, slow):
+def _inputs(channel, B, L, H, KH, dim, vdim, shift, seed=None):
     from adaptivetrainingsystem_b200.ops import delta as D
-    g = torch.Generator(device="cuda").manual_seed(B + L + H + dim + vdim)
+    g = torch.Generator(device="cuda").manual_seed(B + L + H + dim + vdim if seed is None else seed)
 
     def r(*shape):
         return torch.randn(*shape, generator=g, device="cuda")
@@ -16,7 +16,7 @@ def _inputs(channel, B, L, H, KH, dim, vdim, slow):
     else:
         s = D.DeltaShape(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5)
     proj, conv, tail = r(B, L, s.proj_width).bfloat16(), r(s.taps, s.channels) * 0.5, r(B, 3, s.channels).bfloat16()
-    rate, shift = -torch.exp(r(H) * 0.5), -6.0 if slow else -2.0
+    rate = -torch.exp(r(H) * 0.5)
     start = r(2 * B, H, dim, vdim)[::2]      # sequences that do not lie side by side
     if channel:
         mixed, rlen, gb = D.delta_prep(proj, s, conv, None, None, tail)
@@ -32,6 +32,10 @@ def _inputs(channel, B, L, H, KH, dim, vdim, slow):
         def scan(state, fresh):
             return D.delta_scan(mixed, rlen, gb, state, s, L, fresh)
     return s, mixed, rlen, gb, decay, start, scan
+
+
+def _rel(a, b):
+    return float((a.double() - b).norm() / b.norm())
 
 
 def _exact(s, mixed, rlen, gb, decay, start, L, fresh):
@@ -56,7 +60,7 @@ def _exact(s, mixed, rlen, gb, decay, start, L, fresh):
 @pytest.mark.parametrize("fresh", [False, True])
 def test_against_recurrence_and_fma_scan(monkeypatch, channel, B, L, H, KH, dim, vdim, slow, fresh):
     from adaptivetrainingsystem_b200.ops import delta as D
-    s, mixed, rlen, gb, decay, start, scan = _inputs(channel, B, L, H, KH, dim, vdim, slow)
+    s, mixed, rlen, gb, decay, start, scan = _inputs(channel, B, L, H, KH, dim, vdim, -6.0 if slow else -2.0)
     assert D.scan_on_tensor_cores(mixed, s)
     state = start.clone()
     out = scan(state, fresh)
@@ -65,11 +69,30 @@ def test_against_recurrence_and_fma_scan(monkeypatch, channel, B, L, H, KH, dim,
     fma_state = start.clone()
     fma_out = scan(fma_state, fresh)
 
-    def rel(a, b):
-        return float((a.double() - b).norm() / b.norm())
     # Read-outs carry the rounding to bf16 (2^-9 an element at most).  States: 32-bit sums; with a decay per row the error of the fast exponential of
     # each token's decay (a few 1e-7) adds up over the tokens that a state remembers.  Neither is further off than the FMA scan by more than
-    # rounding errors differ from one order of sums to another.
-    assert rel(out, want) < 2.0 ** -8
-    assert rel(state, S) < (4e-6 if channel else 6e-7)
-    assert rel(state, S) < 1.5 * rel(fma_state, S) + 6e-8 and rel(out, want) < rel(fma_out, want) + 1e-5
+    # rounding errors of a single draw differ from one order of sums to another; the test below compares their averages.
+    assert _rel(out, want) < 2.0 ** -8
+    assert _rel(state, S) < (4e-6 if channel else 6e-7)
+    assert _rel(state, S) < 1.25 * _rel(fma_state, S) + 5e-9 and _rel(out, want) < _rel(fma_out, want) + 1e-5
+
+
+# From slow decays to those that forget a token at once, where a state is no further from 64 bits than a few of its own roundings: on average over draws
+# the scan is as close as the FMA scan (0.6 to 1.0 of its error; the mean of eight draws is good to 0.03).
+@pytest.mark.parametrize("shift", [-6.0, -2.0, 0.0, 2.0, 5.0])
+@pytest.mark.parametrize("L,dim", [(8, 64), (32, 64), (331, 128)])
+@pytest.mark.parametrize("channel", [False, True])
+def test_no_further_from_64_bits_than_the_fma_scan(monkeypatch, channel, L, dim, shift):
+    from adaptivetrainingsystem_b200.ops import delta as D
+    error = {True: 0.0, False: 0.0}
+    for seed in range(8):
+        s, mixed, rlen, gb, decay, start, scan = _inputs(channel, 4, L, 8, 4, dim, dim, shift, seed)
+        _, S = _exact(s, mixed, rlen, gb, decay, start, L, False)
+        for mma in error:
+            with monkeypatch.context() as m:
+                if not mma:
+                    m.setattr(D, "scan_on_tensor_cores", lambda *_: False)
+                state = start.clone()
+                scan(state, False)
+            error[mma] += _rel(state, S) / 8
+    assert error[True] < 1.03 * error[False], error
