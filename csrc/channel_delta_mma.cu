@@ -12,7 +12,7 @@
 // eight tokens with a later one factor at the eighth token, so that only the two 8 x 8 blocks on the diagonal are summed pair by pair.
 //
 // Bounded like delta_rule_mma.cu; 350 MMAs a group and warp.  Scan and pairs, us, fp32 FMA form (channel_delta.cu) / this one, 128 x 128 states: 8 sequences of
-// 2,048 tokens, 16 heads 1,213 / 837, 12 of 1,000 934 / 635, 3 of 1,501 537 / 330, one of 2,048 542 / 371, one of 512, 8 heads 121 / 99, one of 64 30 / 29.
+// 2,048 tokens, 16 heads 1,213 / 847, 12 of 1,000 934 / 640, 3 of 1,501 537 / 327, one of 2,048 542 / 367, one of 512, 8 heads 121 / 99, one of 64 30 / 29.
 // State against 64 bits: 0.84 to 0.995 of the FMA form's error on average (slow decays 1.2e-6 to 2.5e-6, the errors of the decays' exponentials; fast ones 0.5e-7).
 #include "delta_mma.cuh"
 
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(128, 3) channel_pairs_mma_kernel(const Channel
     __syncwarp();
     if (lane < CM) {
 #pragma unroll
-      for (int i = 0; i < CM; ++i) s_kk[i][lane] = i == lane ? 0.f : y[i] * bc;   // T
+      for (int i = 0; i < CM; ++i) s_kk[i][lane] = i <= lane ? 0.f : y[i] * bc;   // T
       reinterpret_cast<float*>(co + cm_p_at(DK))[DK + lane] = bc;
     }
     __syncwarp();
@@ -338,6 +338,8 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
       }
     }
     float u[2][4], eu[2][4];
+    int first[2];
+    bool spoilt;
     Pieces a;
     {
       uint32_t vv[4];   // tokens 0..7 / 8..15 of column g, then of column g + 8
@@ -350,14 +352,7 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
         sk[x][2] = hi.x - (sk[x][2] + ek[x][2]);
         sk[x][3] = hi.y - (sk[x][3] + ek[x][3]);
       }
-      split_tiles(sk[0], sk[1], a);
-      split_product(a, mt, lane, u);
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const float2 be = *reinterpret_cast<const float2*>(decay + DK + 8 * x + 2 * t);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) add_diagonal(e & 1 ? be.y : be.x, sk[x][e], u[x][e], eu[x][e]);
-      }
+      spoilt = solve_group(sk, mt, decay + DK, lane, u, eu, first);
     }
     split_tiles(u[0], u[1], eu[0], eu[1], a);
 #pragma unroll
@@ -401,6 +396,10 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
       for (int x = 0; x < 2; ++x)
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[x][e] += sq[x][e] + eq[x][e];
+      if (spoilt) {
+        spoil(o, t, first);
+        spoil_state(S, first);
+      }
       // [token][column] in shared memory: blocks (tokens 0..7, columns 0..7), (0..7, 8..15), (8..15, 0..7), (8..15, 8..15)
       stsm4_t(out_at + prow * OPITCH + ppiece * 16, pack_bf16x2(o[0][0], o[0][1]), pack_bf16x2(o[0][2], o[0][3]), pack_bf16x2(o[1][0], o[1][1]),
               pack_bf16x2(o[1][2], o[1][3]));

@@ -115,4 +115,78 @@ __device__ __forceinline__ void add_diagonal(float beta, float rhs, float& u, fl
   u = s;
 }
 
+// Values that are not finite.  A product with a triangular factor multiplies the later tokens of its group by zeros, and zero times NaN would reach the
+// earlier ones.  So once a column's U is not finite (which any value that is not finite in its right-hand side makes it), the product is taken again without
+// the values from the first such token on, and what those tokens leave is NaN.  Layout of all: lane (g, t), column g or g + 8, token 8 x + 2 t + (e & 1).
+__device__ __forceinline__ bool not_finite(const float (&v)[2][4]) {
+  float z = 0.f;
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int e = 0; e < 4; ++e) z = fmaf(v[x][e], 0.f, z);
+  return !(z == 0.f);
+}
+// Lowers `first` to the first token of each of the lane's columns that three pieces do not hold, and clears the values from there on.
+__device__ __forceinline__ void clear_spoilt(float (&v)[2][4], int t, int (&first)[2]) {
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (!(fabsf(v[x][e]) < 3.38e38f)) first[e >> 1] = min(first[e >> 1], 8 * x + 2 * t + (e & 1));
+#pragma unroll
+  for (int c = 0; c < 2; ++c) {
+    first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], 1));
+    first[c] = min(first[c], __shfl_xor_sync(0xffffffffu, first[c], 2));
+  }
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (8 * x + 2 * t + (e & 1) >= first[e >> 1]) v[x][e] = 0.f;
+}
+__device__ __forceinline__ void spoil(float (&v)[2][4], int t, const int (&first)[2]) {
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (8 * x + 2 * t + (e & 1) >= first[e >> 1]) v[x][e] = __int_as_float(0x7fffffff);
+}
+template <int NT>
+__device__ __forceinline__ void spoil_state(float (&S)[NT][4], const int (&first)[2]) {
+#pragma unroll
+  for (int j = 0; j < NT; ++j)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (first[e >> 1] < 16) S[j][e] = __int_as_float(0x7fffffff);
+}
+
+// U [column][token] = T x (right-hand side): `t_split` the factor below its diagonal, `beta` the diagonal; eu: what the roundings of U cut off.  Returns whether
+// some value of the warp is not finite; `first` then has the columns' first such tokens, from which on u is zero.
+__device__ __forceinline__ bool solve_group(float (&rhs)[2][4], const uint4* t_split, const float* beta, int lane, float (&u)[2][4], float (&eu)[2][4], int (&first)[2]) {
+  const int t = lane & 3;
+  auto solve = [&] {
+    Pieces a;
+    split_tiles(rhs[0], rhs[1], a);
+    split_product(a, t_split, lane, u);
+#pragma unroll
+    for (int x = 0; x < 2; ++x) {
+      const float2 be = *reinterpret_cast<const float2*>(beta + 8 * x + 2 * t);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) add_diagonal(e & 1 ? be.y : be.x, rhs[x][e], u[x][e], eu[x][e]);
+    }
+  };
+  solve();
+  if (!__any_sync(0xffffffffu, not_finite(u))) return false;
+  first[0] = first[1] = 16;
+  clear_spoilt(rhs, t, first);
+  solve();
+  clear_spoilt(u, t, first);
+#pragma unroll
+  for (int x = 0; x < 2; ++x)
+#pragma unroll
+    for (int e = 0; e < 4; ++e)
+      if (u[x][e] == 0.f || !(fabsf(eu[x][e]) < 3.38e38f)) eu[x][e] = 0.f;
+  return true;
+}
+
 }  // namespace ats

@@ -15,8 +15,8 @@
 // not rounded, and the rounding errors of U and of U D / |k| go into the state with them.
 //
 // What bounds it is the warp-level MMA pipe (some 13 cycles an instruction and SM quarter; 200 a group and warp) and, with one warp a quarter, the chain of
-// dependent products.  Scan and pairs, us, fp32 FMA form (delta_rule.cu) / this one, 128 x 128 states: 8 sequences of 2,048 tokens, 16 heads 1,129 / 447, 12 of
-// 1,000 878 / 352, 3 of 1,501 449 / 201, one of 2,048 435 / 263, one of 512, 8 heads 116 / 76, one of 64 24 / 21.  State against 64 bits: 0.65 to 0.86 of the FMA form's
+// dependent products.  Scan and pairs, us, fp32 FMA form (delta_rule.cu) / this one, 128 x 128 states: 8 sequences of 2,048 tokens, 16 heads 1,129 / 454, 12 of
+// 1,000 878 / 357, 3 of 1,501 449 / 204, one of 2,048 435 / 268, one of 512, 8 heads 116 / 77, one of 64 24 / 22.  State against 64 bits: 0.65 to 0.86 of the FMA form's
 // error on average, from slow decays to those that forget a token at once; read-outs 1.66e-3 (their rounding to bf16) on both.
 #include "delta_mma.cuh"
 
@@ -99,7 +99,7 @@ __global__ void __launch_bounds__(128) delta_pairs_mma_kernel(const ScanArgs p) 
         acc -= beta[i] * dec * s_kk[warp][i][j] * y[j];
       }
       y[i] = acc;
-      s_m[warp][r][0][i][c] = i == c ? 0.f : acc * bc;
+      s_m[warp][r][0][i][c] = i <= c ? 0.f : acc * bc;
     }
     float dec = 1.f, G = 1.f, GC = 1.f;
 #pragma unroll
@@ -210,6 +210,8 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
       }
     }
     float u[2][4], eu[2][4];
+    int first[2];
+    bool spoilt;
     Pieces a;
     {
       uint32_t vv[4];   // tokens 0..7 / 8..15 of column g, then of column g + 8
@@ -222,14 +224,7 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
         sk[x][2] = hi.x - gk.x * (sk[x][2] + ek[x][2]);
         sk[x][3] = hi.y - gk.y * (sk[x][3] + ek[x][3]);
       }
-      split_tiles(sk[0], sk[1], a);
-      split_product(a, mt, lane, u);
-#pragma unroll
-      for (int x = 0; x < 2; ++x) {
-        const float2 be = *reinterpret_cast<const float2*>(vec + 3 * DM + 8 * x + 2 * t);
-#pragma unroll
-        for (int e = 0; e < 4; ++e) add_diagonal(e & 1 ? be.y : be.x, sk[x][e], u[x][e], eu[x][e]);
-      }
+      spoilt = solve_group(sk, mt, vec + 3 * DM, lane, u, eu, first);
     }
     {   // the state first: the next group waits for it
       float w[2][4], ew[2][4];
@@ -277,6 +272,10 @@ __global__ void __launch_bounds__(128, 2) delta_scan_mma_kernel(const ScanArgs p
         o[x][1] += gq.y * (sq[x][1] + eq[x][1]);
         o[x][2] += gq.x * (sq[x][2] + eq[x][2]);
         o[x][3] += gq.y * (sq[x][3] + eq[x][3]);
+      }
+      if (spoilt) {
+        spoil(o, t, first);
+        spoil_state(S, first);
       }
       // [token][column] in shared memory: blocks (tokens 0..7, columns 0..7), (0..7, 8..15), (8..15, 0..7), (8..15, 8..15)
       stsm4_t(out_at + ((lane & 7) + (lane >> 4) * 8) * OPITCH + (lane >> 3 & 1) * 16, pack_bf16x2(o[0][0], o[0][1]), pack_bf16x2(o[0][2], o[0][3]),

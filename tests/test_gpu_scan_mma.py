@@ -96,3 +96,34 @@ def test_no_further_from_64_bits_than_the_fma_scan(monkeypatch, channel, L, dim,
                 scan(state, False)
             error[mma] += _rel(state, S) / 8
     assert error[True] < 1.03 * error[False], error
+
+
+# A value that is not finite reaches its own token and the later ones, as in the recurrence: in the first and the second eight tokens of a group, in a later
+# group, in the values, keys, queries, decays (the channel-wise rule makes its own) and step sizes, and in the state at the start.
+@pytest.mark.parametrize("channel,where", [(c, w) for c in (False, True) for w in ("v", "k", "q", "decay", "beta", "state") if not (c and w == "decay")])
+@pytest.mark.parametrize("token,bad", [(5, float("nan")), (13, float("inf")), (27, float("-inf"))])
+def test_values_that_are_not_finite_stay_behind_the_tokens_before_them(channel, where, token, bad):
+    B, L, H, KH, dim, vdim = 2, 40, 4, 2, 64, 80
+    if where in ("decay", "beta"):
+        bad = float("nan")
+    s, mixed, rlen, gb, decay, start, scan = _inputs(channel, B, L, H, KH, dim, vdim, -2.0)
+    clean = scan(start.clone(), False)
+    row = L + token                       # of the second sequence
+    if where == "v":
+        mixed[row, 2 * KH * dim + vdim + 3] = bad
+    elif where in "kq":
+        mixed[row, (KH * dim if where == "k" else 0) + dim + 7] = bad
+    elif where == "decay":
+        gb[row, 2] = bad
+        decay = gb.double()[:, :H].view(B, L, H, 1)
+    elif where == "beta":
+        gb[row, H + 2] = bad
+    else:
+        start = start.clone()
+        start[1, 2, 9, 4] = bad
+    state = start.clone()
+    out = scan(state, False)
+    want, S = _exact(s, mixed, rlen, gb, decay, start, L, False)
+    finite = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(out), finite) and torch.equal(torch.isfinite(state), torch.isfinite(S))
+    assert not bool(finite.all()) and torch.equal(out[finite], clean[finite])
