@@ -689,7 +689,7 @@ class _LinearCEFn(torch.autograd.Function):
         loss_row = torch.empty(T, dtype=torch.float32, device=dev)
         correct = torch.empty(T, dtype=torch.float32, device=dev)
         dh = torch.empty_like(h) if need_grad else None
-        whole = T <= chunk_rows
+        whole = 0 < T <= chunk_rows
         dw32 = torch.zeros(V, H, dtype=torch.float32, device=dev) if ctx.needs_input_grad[1] and not whole else None
         logits = None
         lib = _L()

@@ -1032,3 +1032,17 @@ def test_linear_cross_entropy_in_one_chunk(T, V):
     # the sums differ by T fp32 roundings, which can take the result to the neighbouring bf16 number (they are up to 2^-7 of the value apart)
     for a, b in ((one[2], many[2]), (one[3], many[3])):
         assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + T * 2.0 ** -23 * scale).all())
+
+
+@pytest.mark.parametrize("sink", [False, True])
+def test_linear_cross_entropy_of_no_rows_delivers_a_zero_weight_gradient(sink):
+    V, H = 64, 32
+    h, w = _rand(0, H).requires_grad_(), _rand(V, H).requires_grad_()
+    told = []
+    if sink:   # as an engine that reduces gradients has it
+        w._ats_grad, w._ats_grad_fresh, w._ats_grad_hook = torch.full((V, H), 3.0, device=DEV, dtype=torch.bfloat16), True, told.append
+    loss, raw, nvalid, acc = ops.linear_cross_entropy(h, w, torch.empty(0, dtype=torch.long, device=DEV))
+    loss.backward()
+    assert float(loss) == float(raw) == float(acc) == 0.0 and int(nvalid) == 0 and h.grad.shape == (0, H)
+    grad = w._ats_grad if sink else w.grad
+    assert bool((grad == 0).all()) and len(told) == int(sink)
