@@ -625,7 +625,9 @@ class DeepSeekTransformer(nn.Module):
                      attention_mask: Optional[torch.Tensor] = None, ignore_index: int = -100) -> Dict[str, torch.Tensor]:
         """Training objective with the output head fused into the loss."""
         x, aux_losses = self.hidden_states(input_ids, attention_mask)
-        loss, raw, nvalid, acc = ops.linear_cross_entropy(x, self.lm_head, labels, loss_weights, ignore_index, chunk_rows=ops.head_chunk_rows(self.lm_head.shape[0]))
+        w, rows = self.lm_head, labels.numel()
+        late = torch.is_grad_enabled() and w.requires_grad and rows <= ops.head_chunk_rows(w.shape[0])
+        loss, raw, nvalid, acc = ops.linear_cross_entropy(x, w, labels, loss_weights, ignore_index, **({"chunk_rows": rows, "late_weight_grad": True} if late else {}))
         total_aux = torch.stack(aux_losses).sum() if aux_losses else loss.new_zeros(())
         return {"loss": loss + total_aux.to(loss.dtype), "lm_loss": loss, "raw_loss": raw, "aux_loss": total_aux.detach(),
                 "valid_tokens": nvalid, "accuracy": acc}

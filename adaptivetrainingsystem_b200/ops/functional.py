@@ -671,12 +671,12 @@ def cross_entropy_reference(logits: torch.Tensor, labels: torch.Tensor, weights:
 
 class _LinearCEFn(torch.autograd.Function):
     """lm_head GEMM + cross-entropy, chunked over tokens; dlogits are produced in place right after each chunk's
-    logits.  With several chunks dh / dW are computed in the same pass, so the full [T, V] logits never exist, and dW is summed in an fp32 matrix.
-    With one chunk dlogits wait for the backward pass, where dW is one product straight into the gradient: no fp32 matrix to clear, to add
-    to and to round (32,000 x 4,096 of them: 86 + 81 + 129 us)."""
+    logits.  dh / dW are computed in the same pass, so the full [T, V] logits never exist, and dW is summed in an fp32 matrix.
+    With ``late_weight_grad`` and one chunk, h and dlogits wait for the backward pass, where dW is one product straight into the gradient: no fp32 matrix
+    to clear, to add to and to round (32,000 x 4,096 of them: 86 + 81 + 129 us)."""
 
     @staticmethod
-    def forward(ctx, h, w, labels, weights, ignore_index, chunk_rows):
+    def forward(ctx, h, w, labels, weights, ignore_index, chunk_rows, late_weight_grad):
         T, H = h.shape
         V = w.shape[0]
         dev = h.device
@@ -689,7 +689,7 @@ class _LinearCEFn(torch.autograd.Function):
         loss_row = torch.empty(T, dtype=torch.float32, device=dev)
         correct = torch.empty(T, dtype=torch.float32, device=dev)
         dh = torch.empty_like(h) if need_grad else None
-        whole = 0 < T <= chunk_rows
+        whole = late_weight_grad and 0 < T <= chunk_rows
         dw32 = torch.zeros(V, H, dtype=torch.float32, device=dev) if ctx.needs_input_grad[1] and not whole else None
         logits = None
         lib = _L()
@@ -733,30 +733,32 @@ class _LinearCEFn(torch.autograd.Function):
                     "cast")
                 return out
             dw = _deliver_grad(w, compute)
-        return dhs, dw, None, None, None, None
+        return dhs, dw, None, None, None, None, None
 
 
-HEAD_LOGITS_BYTES = 1 << 30   # logits of one chunk: 0.6 % of the memory, and at least 4,096 rows up to a vocabulary of 131,072
+HEAD_CHUNK_ROWS = 4096         # rows of a chunk of logits that is dropped again
+HEAD_LOGITS_BYTES = 1 << 30    # logits that a training step keeps from its loss to the backward pass: 0.6 % of the memory, and at least 4,096 rows up to a vocabulary of 131,072
 
 
 def head_chunk_rows(vocab: int) -> int:
-    """Rows of a chunk of :func:`linear_cross_entropy` for a training step, where one chunk is the fastest (16,384 rows of 32,000, 2,048 wide,
-    with their gradients: 5,620 to 6,230 us in four chunks, 5,460 to 5,510 in one)."""
-    return max(4096, HEAD_LOGITS_BYTES // (2 * vocab))
+    """Most rows of a training step that go through the output head as one chunk and whose logits' gradients are kept for the backward pass (16,384 rows of
+    32,000, 2,048 wide, with their gradients: 5,620 to 6,230 us in four chunks, 5,460 to 5,510 in one)."""
+    return max(HEAD_CHUNK_ROWS, HEAD_LOGITS_BYTES // (2 * vocab))
 
 
 def linear_cross_entropy(h: torch.Tensor, w: torch.Tensor, labels: torch.Tensor,
                          weights: Optional[torch.Tensor] = None, ignore_index: int = -100,
-                         chunk_rows: int = 4096):
+                         chunk_rows: int = 4096, late_weight_grad: bool = False):
     """Loss of ``softmax(h @ w.T)`` against ``labels`` -> (loss, raw_loss, valid_tokens, accuracy).
 
     The weight gradient is taken with unit upstream gradient (the loss is the root of the graph in training);
-    ``dh`` is scaled by the upstream gradient."""
+    ``dh`` is scaled by the upstream gradient.  ``late_weight_grad``: where one chunk holds all rows, the weight gradient is left to the backward
+    pass, for which ``h``, not to be modified before it, and the logits' gradients are kept."""
     h2 = h.reshape(-1, h.shape[-1])
     if _lib.use_cuda_kernels(h2):
         if not h2.is_contiguous():
             h2 = h2.contiguous()
-        return _LinearCEFn.apply(h2, w, labels, weights, ignore_index, chunk_rows)
+        return _LinearCEFn.apply(h2, w, labels, weights, ignore_index, chunk_rows, late_weight_grad)
     return cross_entropy_reference(F.linear(h2, w), labels, weights, ignore_index)
 
 

@@ -1017,13 +1017,13 @@ def test_linear_cross_entropy_in_one_chunk(T, V):
     labels = torch.randint(0, V, (T,), device=DEV)
     labels[:T // 10] = -100
     got = []
-    for rows in (T, max(1, T // 3)):
+    for rows, late in ((T, True), (max(1, T // 3), False)):
         h, w = h0.clone().requires_grad_(), w0.clone().requires_grad_()
-        loss = ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows)[0]
+        loss = ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows, late_weight_grad=late)[0]
         (loss * 0.37).backward()
         first, sink = w.grad.clone(), torch.full((V, H), 0.25, device=DEV, dtype=torch.bfloat16)
         w._ats_grad, w._ats_grad_fresh, w.grad = sink, False, None   # as an engine that sums micro-batches has it
-        ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows)[0].backward()
+        ops.linear_cross_entropy(h, w, labels, None, -100, chunk_rows=rows, late_weight_grad=late)[0].backward()
         assert w.grad is None
         got.append((loss.detach(), h.grad, first, sink))
     one, many = got
@@ -1034,15 +1034,31 @@ def test_linear_cross_entropy_in_one_chunk(T, V):
         assert bool(((a.float() - b.float()).abs() <= 2.0 ** -7 * b.float().abs() + T * 2.0 ** -23 * scale).all())
 
 
+@pytest.mark.parametrize("late", [False, True])
 @pytest.mark.parametrize("sink", [False, True])
-def test_linear_cross_entropy_of_no_rows_delivers_a_zero_weight_gradient(sink):
+def test_linear_cross_entropy_of_no_rows_delivers_a_zero_weight_gradient(late, sink):
     V, H = 64, 32
     h, w = _rand(0, H).requires_grad_(), _rand(V, H).requires_grad_()
     told = []
     if sink:   # as an engine that reduces gradients has it
         w._ats_grad, w._ats_grad_fresh, w._ats_grad_hook = torch.full((V, H), 3.0, device=DEV, dtype=torch.bfloat16), True, told.append
-    loss, raw, nvalid, acc = ops.linear_cross_entropy(h, w, torch.empty(0, dtype=torch.long, device=DEV))
+    loss, raw, nvalid, acc = ops.linear_cross_entropy(h, w, torch.empty(0, dtype=torch.long, device=DEV), late_weight_grad=late)
     loss.backward()
     assert float(loss) == float(raw) == float(acc) == 0.0 and int(nvalid) == 0 and h.grad.shape == (0, H)
     grad = w._ats_grad if sink else w.grad
     assert bool((grad == 0).all()) and len(told) == int(sink)
+
+
+def test_linear_cross_entropy_leaves_its_input_to_the_caller():
+    """Unless the weight gradient is left to the backward pass, the rows may be overwritten as soon as the loss is taken, and no logits are held."""
+    T, V, H = 512, 8192, 64
+    h, w, labels = _rand(T, H), _rand(V, H, scale=0.05).requires_grad_(), torch.randint(0, V, (T,), device=DEV)
+    ops.linear_cross_entropy(h, w, labels)[0].backward()
+    want, w.grad = w.grad.clone(), None
+    torch.cuda.synchronize()
+    before = torch.cuda.memory_allocated()
+    loss = ops.linear_cross_entropy(h, w, labels)[0]
+    assert torch.cuda.memory_allocated() - before < 4 * V * H + T * V   # the fp32 sums and change, where the logits are 2 T V
+    h.zero_()
+    loss.backward()
+    assert torch.equal(w.grad, want)
