@@ -738,7 +738,8 @@ class Config:
         optim = 12 * n / (w if self.zero_stage >= 1 else 1)
         tokens = self.micro_batch_size * self.seq_length
         act_per_layer = tokens * self.hidden_size * 2 * (2 if self.gradient_checkpointing else 18)
-        acts = act_per_layer * self.num_layers + tokens * self.vocab_size * 2 * 0.25
+        from .ops import head_bytes
+        acts = act_per_layer * self.num_layers + head_bytes(tokens, self.vocab_size, self.hidden_size)
         gb = 1024 ** 3
         out = {"parameters": params / gb, "gradients": grads / gb, "optimizer": optim / gb,
                "activations": acts / gb}

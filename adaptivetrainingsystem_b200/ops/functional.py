@@ -746,6 +746,11 @@ def head_chunk_rows(vocab: int) -> int:
     return max(HEAD_CHUNK_ROWS, HEAD_LOGITS_BYTES // (2 * vocab))
 
 
+def head_bytes(rows: int, vocab: int, width: int) -> int:
+    """What the output head of a training step of ``rows`` rows holds beside its input: the logits' gradients, or a chunk of them and the fp32 sums of its weight gradient."""
+    return 2 * rows * vocab if rows <= head_chunk_rows(vocab) else 2 * HEAD_CHUNK_ROWS * vocab + 4 * vocab * width
+
+
 def linear_cross_entropy(h: torch.Tensor, w: torch.Tensor, labels: torch.Tensor,
                          weights: Optional[torch.Tensor] = None, ignore_index: int = -100,
                          chunk_rows: int = 4096, late_weight_grad: bool = False):
