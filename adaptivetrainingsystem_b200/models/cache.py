@@ -23,16 +23,17 @@ class SequenceCache:
         self.device_lengths: Optional[torch.Tensor] = None
         self.device_positions: Optional[torch.Tensor] = None
         self.device_active: Optional[torch.Tensor] = None
+        self._device_counters: Optional[torch.Tensor] = None   # lengths and positions side by side: one launch moves both on
 
     def enable_device_lengths(self) -> None:
-        self._device_counters = torch.full((2, self.batch), self.length, dtype=torch.int32, device=self.device)   # (one launch moves both on)
+        self._device_counters = torch.full((2, self.batch), self.length, dtype=torch.int32, device=self.device)
         self.device_lengths, self.device_positions = self._device_counters
         self.device_active = torch.ones(self.batch, dtype=torch.int32, device=self.device)
 
     def device_advance(self) -> None:
         """One decoded token of every active row: called inside the captured step."""
         rows = (self.device_lengths, self.device_positions)
-        if [t.data_ptr() for t in rows] == [t.data_ptr() for t in self._device_counters]:
+        if self._device_counters is not None and [t.data_ptr() for t in rows] == [t.data_ptr() for t in self._device_counters]:
             self._device_counters += self.device_active
         else:   # (tensors of the caller's in their place)
             for t in rows:

@@ -253,3 +253,17 @@ def test_generation_without_kv_cache_matches_cached_generation():
     with pytest.raises(ValueError):
         GenerationEngine(model, kv_cache_dtype="fp8")
     GenerationEngine(model, kv_cache_dtype="fp32")
+
+
+@pytest.mark.parametrize("enabled", [False, True])
+def test_cache_counters_of_the_callers_advance(enabled):
+    from adaptivetrainingsystem_b200.models.cache import SequenceCache
+    cache = SequenceCache(3, 16, "cpu")
+    if enabled:
+        cache.enable_device_lengths()
+        cache.device_advance()
+        assert cache.device_lengths.tolist() == cache.device_positions.tolist() == [1, 1, 1]
+    cache.device_lengths, cache.device_positions = torch.tensor([4, 5, 6], dtype=torch.int32), torch.tensor([1, 2, 3], dtype=torch.int32)
+    cache.device_active = torch.tensor([1, 0, 1], dtype=torch.int32)
+    cache.device_advance()
+    assert cache.device_lengths.tolist() == [5, 5, 7] and cache.device_positions.tolist() == [2, 2, 4]
