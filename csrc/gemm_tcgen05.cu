@@ -1473,7 +1473,7 @@ ATS_API int ats_gemm_bf16_gathered(const void* A, long long lda, const void* B_l
   if (((long long)ready_rows * K * 2) % 4096) return 1003;
   if ((N & 7) || (K & 7) || (ldd & 7) || (b_rows % b_shards) || ((b_rows / b_shards) % ready_rows)) return 1003;
   if (ready_rows != 64 && ready_rows % 128) return 1003;  // chunks are halves or multiples of the 128-row boxes B is read in
-  if (epilogue == kF32 || (epilogue == kSwiGLU && (up_offset & 7))) return 1004;
+  if ((epilogue != kStore && epilogue != kAddC && epilogue != kSwiGLU) || (epilogue == kSwiGLU && (up_offset & 7))) return 1004;
   CUtensorMap ma, mb;
   int e;
   if ((e = make_tmap_2d(&ma, A, M, K, lda, 2, 64, 128))) return e;
