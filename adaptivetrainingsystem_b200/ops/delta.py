@@ -185,9 +185,17 @@ def delta_prep(proj: torch.Tensor, s: DeltaShape, conv: torch.Tensor, neg_rate: 
     return mixed, rlen, gb
 
 
+def _whole_pieces(t: torch.Tensor) -> torch.Tensor:
+    """``t`` [rows, columns] with rows that start at 16-byte pieces, as :func:`delta_prep` leaves them and the kernels read them; a copy of other rows."""
+    if t.data_ptr() % 16 == 0 and t.stride(0) * t.element_size() % 16 == 0 and t.stride(1) == 1:
+        return t
+    out = torch.empty(t.shape[0], pad8(t.shape[1]), dtype=t.dtype, device=t.device)[:, :t.shape[1]]
+    return out.copy_(t)
+
+
 def scan_on_tensor_cores(mixed: torch.Tensor, s: DeltaShape) -> bool:
-    """Whether portions run on ``csrc/delta_rule_mma.cu``: bf16 rows of 16-byte pieces, up to 128 state rows."""
-    return mixed.dtype == torch.bfloat16 and s.dim <= 128 and s.dim % 8 == 0 and s.vdim % 8 == 0 and mixed.stride(0) % 8 == 0 and mixed.data_ptr() % 16 == 0
+    """Whether portions (rows of whole pieces) run on ``csrc/delta_rule_mma.cu``: bf16, heads of 16-byte pieces, up to 128 state rows."""
+    return mixed.dtype == torch.bfloat16 and s.dim <= 128 and s.dim % 8 == 0 and s.vdim % 8 == 0
 
 
 def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, s: DeltaShape, L: int, fresh: bool) -> torch.Tensor:
@@ -204,9 +212,10 @@ def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state:
                 out[t] = o.reshape(-1).to(out.dtype)
             state[b] = S
         return out
+    mixed = _whole_pieces(mixed)
     mma = scan_on_tensor_cores(mixed, s)
     groups = -(-L // (GROUP_MMA if mma else GROUP))
-    size = 836 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # layouts: csrc/delta_rule_mma.cu, csrc/delta_rule.cu
+    size = 836 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # floats, laid out in csrc/delta_rule_mma.cu (3.3 KB per 16 tokens and head), csrc/delta_rule.cu (1.3 KB)
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
     o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
     args = _Scan(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0), B, L, H, KH, s.dim, s.vdim, groups, int(fresh))
@@ -267,9 +276,10 @@ def channel_delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor
                 out[t] = o.reshape(-1).to(out.dtype)
             state[b] = S
         return out
+    mixed, a = _whole_pieces(mixed), _whole_pieces(a)
     mma, DK = scan_on_tensor_cores(mixed, s), s.scan_rows
     groups = -(-L // (GROUP_MMA if mma else GROUP))
-    size = 73 * DK + 784 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # layouts: csrc/channel_delta_mma.cu, csrc/channel_delta.cu
+    size = 73 * DK + 784 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # csrc/channel_delta_mma.cu (40 KB, 128 rows), csrc/channel_delta.cu (27 KB)
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
     o = torch.empty(B * L, H * s.vdim, dtype=mixed.dtype, device=mixed.device)
     args = _Channel(_p(mixed), mixed.stride(0), _p(rlen), _p(gb), _p(a), a.stride(0), _p(neg_rate), _p(dt_bias), _p(coef), _p(state), state.stride(0), _p(o), o.stride(0),

@@ -37,7 +37,7 @@ constexpr int CM_PITCH = 132;            // floats of a row that the off-diagona
 constexpr int CM_PAIR_FLOATS = 24 * CM_PITCH + 2 * 128 + 2 * CM * 17;
 
 // Two warps per (group, head, sequence), one for each eight tokens, two channels per lane side by side.
-template <int DK, bool VEC>
+template <int DK>
 __global__ void __launch_bounds__(128, 3) channel_pairs_mma_kernel(const ChannelArgs p) {
   pdl_prologue();
   extern __shared__ __align__(16) float s_pair[];
@@ -75,18 +75,7 @@ __global__ void __launch_bounds__(128, 3) channel_pairs_mma_kernel(const Channel
     for (int i = 0; i < 64; ++i) sums[i] = 0.f;
 #pragma unroll 1
     for (int d0 = lane * 2; d0 < DK; d0 += 64) {
-      auto fetch = [&](const __nv_bfloat16* src, bool in) -> uint32_t {
-        uint32_t v = 0;
-        if (!in) return v;
-        if constexpr (VEC) {
-          if (d0 < p.dim) v = *reinterpret_cast<const uint32_t*>(src + d0);
-        } else {
-          const unsigned short* s = reinterpret_cast<const unsigned short*>(src);
-          if (d0 < p.dim) v = s[d0];
-          if (d0 + 1 < p.dim) v |= uint32_t(s[d0 + 1]) << 16;
-        }
-        return v;
-      };
+      auto fetch = [&](const __nv_bfloat16* src, bool in) -> uint32_t { return in && d0 < p.dim ? *reinterpret_cast<const uint32_t*>(src + d0) : 0; };
       uint32_t pk[8], pq[8], pa[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -428,8 +417,7 @@ __global__ void __launch_bounds__(128, 2) channel_scan_mma_kernel(const ChannelA
 template <int DK>
 int launch_channel_mma(const ChannelArgs& p, int* status, cudaStream_t s) {
   const int pair_smem = 2 * CM_PAIR_FLOATS * int(sizeof(float)), scan_smem = CM_STAGES * (cm_bytes(DK) + CM * (CM_COLS * 2 + 16));
-  const bool even = !((p.dim | p.ldm | p.lda) & 1);
-  auto pairs = even ? channel_pairs_mma_kernel<DK, true> : channel_pairs_mma_kernel<DK, false>;
+  auto pairs = channel_pairs_mma_kernel<DK>;
   if (cudaError_t e = cudaFuncSetAttribute(pairs, cudaFuncAttributeMaxDynamicSharedMemorySize, pair_smem)) return int(e);
   if (cudaError_t e = cudaFuncSetAttribute(channel_scan_mma_kernel<DK>, cudaFuncAttributeMaxDynamicSharedMemorySize, scan_smem)) return int(e);
   const long long groups = (long long)p.B * p.groups * p.H;
@@ -443,12 +431,12 @@ int launch_channel_mma(const ChannelArgs& p, int* status, cudaStream_t s) {
 
 using namespace ats;
 
-// bf16 rows whose values are whole 16-byte pieces (dim, vdim, ldm, ldo multiples of 8, mixed and o 16-byte aligned), dim up to DK (64 or 128), p->groups
+// bf16 rows whose values are whole 16-byte pieces (dim, vdim, ldm, ldo multiples of 8, mixed and o 16-byte aligned; decay inputs in pairs), dim up to DK (64 or 128), p->groups
 // groups of 16 tokens; coef: per (sequence, group, head) 292 DK + 3136 bytes (cm_bytes), 16-byte aligned.
 ATS_API int ats_channel_delta_mma(const ChannelArgs* p, int* status, void* stream) {
   if (p->B <= 0 || p->L <= 0) return 0;
   if (p->groups != (p->L + CM - 1) / CM || p->KH < 1 || p->H % p->KH || (p->DK != 64 && p->DK != 128) || p->dim < 1 || p->dim > p->DK ||
-      ((p->dim | p->vdim | p->ldm | p->ldo) & 7) || ((reinterpret_cast<uintptr_t>(p->mixed) | reinterpret_cast<uintptr_t>(p->o) | reinterpret_cast<uintptr_t>(p->coef)) & 15))
+      ((p->dim | p->vdim | p->ldm | p->ldo) & 7) || (p->lda & 1) || (reinterpret_cast<uintptr_t>(p->a) & 3) || ((reinterpret_cast<uintptr_t>(p->mixed) | reinterpret_cast<uintptr_t>(p->o) | reinterpret_cast<uintptr_t>(p->coef)) & 15))
     return 1006;
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   return p->DK == 64 ? launch_channel_mma<64>(*p, status, s) : launch_channel_mma<128>(*p, status, s);

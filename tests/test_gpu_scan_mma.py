@@ -127,3 +127,31 @@ def test_values_that_are_not_finite_stay_behind_the_tokens_before_them(channel, 
     finite = torch.isfinite(want)
     assert torch.equal(torch.isfinite(out), finite) and torch.equal(torch.isfinite(state), torch.isfinite(S))
     assert not bool(finite.all()) and torch.equal(out[finite], clean[finite])
+
+
+# Rows that do not start at 16-byte pieces (a slice of a wider matrix, an odd pitch) are copied to some that do: on both kinds of scan.
+@pytest.mark.parametrize("channel", [False, True])
+@pytest.mark.parametrize("dim,vdim", [(64, 48), (40, 20), (36, 20)])
+@pytest.mark.parametrize("offset,pad", [(1, 8), (2, 7), (0, 5), (4, 4)])
+def test_rows_at_any_address(channel, dim, vdim, offset, pad):
+    from adaptivetrainingsystem_b200.ops import delta as D
+    B, L, H, KH = 2, 21, 4, 2
+    s = (D.ChannelDeltaShape(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5, decay_rank=8, gate_rank=8) if channel
+         else D.DeltaShape(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5))
+    g = torch.Generator(device="cuda").manual_seed(dim + offset)
+    mixed = torch.randn(B * L, (s.channels + 7) // 8 * 8, generator=g, device="cuda").bfloat16()
+    a = torch.randn(B * L, H * dim, generator=g, device="cuda").bfloat16()
+    rlen, gb = 0.05 + 0.05 * torch.rand(B * L, 2 * KH, generator=g, device="cuda"), torch.rand(B * L, 2 * H, generator=g, device="cuda")
+    rate, bias = -torch.rand(H, generator=g, device="cuda"), torch.randn(H * dim, generator=g, device="cuda")
+
+    def elsewhere(t):
+        wide = torch.zeros(t.shape[0], offset + t.shape[1] + pad, dtype=t.dtype, device="cuda")
+        return wide[:, offset:offset + t.shape[1]].copy_(t)
+
+    def scan(m, x):
+        state = torch.ones(B, H, dim, vdim, device="cuda")
+        return (D.channel_delta_scan(m, rlen, gb, x, rate, bias, state, s, L, False) if channel else D.delta_scan(m, rlen, gb, state, s, L, False)), state
+    out, state = scan(mixed, a)
+    for m, x in ((elsewhere(mixed), a), (mixed, elsewhere(a)), (elsewhere(mixed), elsewhere(a))):
+        o, st = scan(m, x)
+        assert torch.equal(o, out) and torch.equal(st, state)
