@@ -150,42 +150,45 @@ rmsnorm_bwd_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __r
   }
 }
 
-// RMSNorm backward over many rows: one CTA of eight warps per SM, groups of WPR warps take a row each (up to 2,048 WPR columns with NV = 8 vectors of
-// eight per lane).  The kernel moves four matrices and does little with them, so what counts is what is in flight: every lane copies its vectors of
-// the group's next rows (x, dy and the gradient of the residual branch) asynchronously into slots that only it reads, two rows ahead, so that a row's
-// reduction never waits for its loads (98 KB in flight per SM at 2,048 columns; loading a row, reducing it and only then asking for the residual
-// branch kept a third of that).  16,384 x 2,048 with a residual branch 91.8 -> 47.6 us (41.6 at the copy rate),
-// 4,096 x 4,096 64.0 -> 29.5 (20.8) and 13.5 -> 3.5 for the fold of its partial sums, 16,384 x 5,120 446 -> 160, 3,000 x 1,024 9.3 -> 8.7.
+// RMSNorm backward over many rows: one CTA of eight warps per SM, groups of WPR warps take a row each, NV vectors of eight columns per lane, no more than
+// the width needs.  The kernel moves four matrices and does little with them, so what counts is what is in flight: every lane copies its vectors of
+// the group's next rows (x, dy and with RES the gradient of the residual branch) asynchronously into slots that only it reads, two rows ahead, so that a
+// row's reduction never waits for its loads.  Up to six vectors go to registers before the row is reduced and their slots are refilled at once; eight
+// would spill and are read twice.  Us, loading a row, reducing it and only then asking for the residual branch / this, with a residual branch: 16,384 x 2,048
+// 90.9 / 46.9 (41.6 at the copy rate), 4,096 x 2,048 19.4 / 13.9, 16,384 x 1,536 79.8 / 37.0, 12,000 x 1,024 22.3 / 15.7, 3,000 x 1,024 8.9 / 8.4, 8,000 x 768 12.7 / 10.5,
+// 12,000 x 512 15.0 / 10.5, 12,000 x 256 14.5 / 8.2, 1,024 x 64 5.9 / 5.0; 4,096 x 4,096 73.8 / 30.6, 16,384 x 4,096 244 / 93.  (Vectors beyond the width and
+// every value read twice made rows of up to 1,024 columns slower than the form before, 12,000 x 768 16.2 / 17.6.)
 // The weight-gradient sums of a lane's columns stay in registers and are folded over the groups at the end.
-template <int NV, int WPR>
+template <int NV, int WPR, bool RES>
 __global__ void __launch_bounds__(256, 1)
 rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16* __restrict__ w, const __nv_bfloat16* __restrict__ dy,
                         const float* __restrict__ rstd, const __nv_bfloat16* __restrict__ dres_in, __nv_bfloat16* __restrict__ dx,
                         float* __restrict__ dw_partial, int rows, int cols) {
-  constexpr int G = 8 / WPR, S = 2, SLOTS = 32 * WPR * NV;  // row groups, rows in flight, vectors of a row
+  constexpr int G = 8 / WPR, S = 2, SLOTS = 32 * WPR * NV, M = RES ? 3 : 2;  // row groups, rows in flight, vectors of a row, matrices
+  constexpr bool KEEP = NV < 8;
   extern __shared__ __align__(16) unsigned char rows_smem[];
   __shared__ float s_dot[2][8];
-  uint4* ring = reinterpret_cast<uint4*>(rows_smem);        // [G][S][3][SLOTS]
-  uint4* wsm = ring + G * S * 3 * SLOTS;                    // the weight, zero-padded
+  uint4* ring = reinterpret_cast<uint4*>(rows_smem);        // [G][S][M][SLOTS]
+  uint4* wsm = ring + G * S * M * SLOTS;                    // the weight, zero-padded
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, group = warp / WPR, at = (warp % WPR) * 32 + lane;
   const int nvec = cols >> 3;
   const float inv_cols = 1.f / float(cols);
   for (int v = threadIdx.x; v < SLOTS; v += 256) wsm[v] = v < nvec ? reinterpret_cast<const uint4*>(w)[v] : make_uint4(0, 0, 0, 0);
   __syncthreads();
-  uint4* mine = ring + group * S * 3 * SLOTS + at;
+  uint4* mine = ring + group * S * M * SLOTS + at;
   const long long first = (long long)blockIdx.x * G + group, stride = (long long)gridDim.x * G;
   float rq[S];
   auto issue = [&](int d, long long row) {
     if (row < rows) {
       rq[d] = rstd[row];
-      uint4* slot = mine + d * 3 * SLOTS;
+      uint4* slot = mine + d * M * SLOTS;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         const int v = at + 32 * WPR * i;
         if (v < nvec) {
           cp_async16(slot + 32 * WPR * i, reinterpret_cast<const uint4*>(x + row * cols) + v);
           cp_async16(slot + SLOTS + 32 * WPR * i, reinterpret_cast<const uint4*>(dy + row * cols) + v);
-          if (dres_in) cp_async16(slot + 2 * SLOTS + 32 * WPR * i, reinterpret_cast<const uint4*>(dres_in + row * cols) + v);
+          if (RES) cp_async16(slot + 2 * SLOTS + 32 * WPR * i, reinterpret_cast<const uint4*>(dres_in + row * cols) + v);
         }
       }
     }
@@ -205,13 +208,25 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
       const long long row = row0 + d * stride;
       if (row >= rows) break;  // the same for the whole group
       cp_async_wait<S - 1>();
-      const uint4* slot = mine + d * 3 * SLOTS;
+      const uint4* slot = mine + d * M * SLOTS;
       const float r = rq[d];
       auto vec = [&](int m, int i) { return at + 32 * WPR * i < nvec ? slot[m * SLOTS + 32 * WPR * i] : make_uint4(0, 0, 0, 0); };
+      uint4 kept[KEEP ? M : 1][KEEP ? NV : 1];
+      if constexpr (KEEP) {
+#pragma unroll
+        for (int i = 0; i < NV; ++i)
+#pragma unroll
+          for (int m = 0; m < M; ++m) kept[m][i] = vec(m, i);
+        issue(d, row + S * stride);  // (a lane refills the slots that it has just read itself)
+      }
+      auto value = [&](int m, int i) {
+        if constexpr (KEEP) return kept[m][i];
+        else return vec(m, i);
+      };
       float dot = 0.f;
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
-        const uint4 wq = wsm[at + 32 * WPR * i], a = vec(0, i), b = vec(1, i);
+        const uint4 wq = wsm[at + 32 * WPR * i], a = value(0, i), b = value(1, i);
         const uint32_t au[4] = {a.x, a.y, a.z, a.w}, bu[4] = {b.x, b.y, b.z, b.w};
         const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w};
 #pragma unroll
@@ -237,7 +252,9 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
 #pragma unroll
       for (int i = 0; i < NV; ++i) {
         const int v = at + 32 * WPR * i;
-        const uint4 wq = wsm[v], a = vec(0, i), b = vec(1, i), cq = dres_in ? vec(2, i) : make_uint4(0, 0, 0, 0);
+        const uint4 wq = wsm[v], a = value(0, i), b = value(1, i);
+        uint4 cq = make_uint4(0, 0, 0, 0);
+        if constexpr (RES) cq = value(2, i);
         const uint32_t au[4] = {a.x, a.y, a.z, a.w}, bu[4] = {b.x, b.y, b.z, b.w};
         const uint32_t wu[4] = {wq.x, wq.y, wq.z, wq.w}, cu[4] = {cq.x, cq.y, cq.z, cq.w};
         uint32_t o[4];
@@ -248,7 +265,7 @@ rmsnorm_bwd_rows_kernel(const __nv_bfloat16* __restrict__ x, const __nv_bfloat16
         }
         if (v < nvec) outr[v] = make_uint4(o[0], o[1], o[2], o[3]);
       }
-      issue(d, row + S * stride);  // (a lane refills the slots that it has just read itself)
+      if (!KEEP) issue(d, row + S * stride);
     }
   }
   cp_async_wait<0>();
@@ -513,6 +530,8 @@ ATS_API int ats_rmsnorm_fwd(const void* x, const void* res, const void* w, void*
   return int(cudaGetLastError());
 }
 
+template <int V> struct Const { static constexpr int value = V; };
+
 // dw_partial: fp32 scratch of nblocks*cols; dw written as bf16 (dw_bf16) and/or fp32 (dw_f32).
 static int rmsnorm_bwd_launch(const void* x, const void* w, const void* dy, const float* rstd, const void* dres_in, void* dx,
                               float* dw_partial, int nblocks, void* dw_bf16, float* dw_f32, int accumulate, long long rows,
@@ -526,18 +545,17 @@ static int rmsnorm_bwd_launch(const void* x, const void* w, const void* dy, cons
   auto DX = static_cast<__nv_bfloat16*>(dx);
   if (many_rows && rows >= 1024 && cols <= 16384 && nblocks >= 1) {
     const int nb = nblocks < 148 ? nblocks : 148;
-    auto go = [&](auto kernel, int nv, int wpr) -> int {
-      const int smem = (8 / wpr * 2 * 3 + 1) * 32 * wpr * nv * 16;
+    auto go = [&](auto nv_c, auto wpr_c) -> int {
+      constexpr int NV = decltype(nv_c)::value, WPR = decltype(wpr_c)::value;
+      auto kernel = DR ? rmsnorm_bwd_rows_kernel<NV, WPR, true> : rmsnorm_bwd_rows_kernel<NV, WPR, false>;
+      const int smem = (8 / WPR * 2 * (DR ? 3 : 2) + 1) * 32 * WPR * NV * 16;
       if (cudaError_t ce = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)) return int(ce);
       kernel<<<nb, 256, smem, s>>>(X, W, DY, rstd, DR, DX, dw_partial, (int)rows, cols);
       return int(cudaGetLastError());
     };
-    int e;
-    if (cols <= 1024) e = go(rmsnorm_bwd_rows_kernel<4, 1>, 4, 1);
-    else if (cols <= 2048) e = go(rmsnorm_bwd_rows_kernel<8, 1>, 8, 1);
-    else if (cols <= 4096) e = go(rmsnorm_bwd_rows_kernel<8, 2>, 8, 2);
-    else if (cols <= 8192) e = go(rmsnorm_bwd_rows_kernel<8, 4>, 8, 4);
-    else e = go(rmsnorm_bwd_rows_kernel<8, 8>, 8, 8);
+    const int e = cols <= 256 ? go(Const<1>(), Const<1>()) : cols <= 512 ? go(Const<2>(), Const<1>()) : cols <= 768 ? go(Const<3>(), Const<1>())
+                  : cols <= 1024 ? go(Const<4>(), Const<1>()) : cols <= 1536 ? go(Const<6>(), Const<1>()) : cols <= 2048 ? go(Const<4>(), Const<2>())
+                  : cols <= 4096 ? go(Const<8>(), Const<2>()) : cols <= 8192 ? go(Const<8>(), Const<4>()) : go(Const<8>(), Const<8>());
     if (e) return e;
     colsum_partial_kernel<<<(cols + 31) / 32, 256, 0, s>>>(dw_partial, nb, cols, static_cast<__nv_bfloat16*>(dw_bf16), dw_f32, accumulate);
     return int(cudaGetLastError());

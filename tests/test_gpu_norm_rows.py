@@ -10,7 +10,7 @@ DEV = "cuda"
 
 # rows: fewer than the groups of the grid, one more than a whole round of them, several rounds; columns around the widths of the groups
 @pytest.mark.parametrize("skip", [False, True])
-@pytest.mark.parametrize("rows,cols", [(1024, 8), (1185, 1000), (3000, 1024), (1184, 1032), (2500, 2048), (1030, 2056), (1777, 4096), (1024, 8192), (1100, 16384)])
+@pytest.mark.parametrize("rows,cols", [(1024, 8), (1190, 256), (1200, 264), (3111, 512), (1500, 520), (2369, 768), (1300, 776), (1185, 1000), (3000, 1024), (1184, 1032), (2000, 1536), (1500, 1544), (2500, 2048), (1030, 2056), (1777, 4096), (1024, 8192), (1100, 16384)])
 def test_backward_of_many_rows(rows, cols, skip):
     g = torch.Generator(device=DEV).manual_seed(rows + cols)
     x0, dy, ds = (torch.randn(rows, cols, generator=g, device=DEV).bfloat16() for _ in range(3))

@@ -1,4 +1,5 @@
-"""Scans of the delta rules (``csrc/delta_rule.cu``, ``csrc/channel_delta.cu``): four and eight value columns per lane are the same sums."""
+"""Scans of the delta rules: four and eight value columns per lane (``csrc/delta_rule.cu``, ``csrc/channel_delta.cu``) are the same sums; on the tensor-core
+scans, which have no such forms, a sequence is the same alone and among others."""
 import pytest
 import torch
 
@@ -6,15 +7,18 @@ pytestmark = pytest.mark.gpu
 
 
 # sequences on either side of the line (192 CTAs of 64 columns); vdim 96 and 100 leave the last CTA partly empty, dim 72 its state rows
-@pytest.mark.parametrize("dim,vdim,B,L", [(128, 128, 13, 41), (72, 96, 13, 8), (128, 100, 13, 9)])
+@pytest.mark.parametrize("dim,vdim,B,L,mma", [(128, 128, 13, 41, False), (72, 96, 13, 8, False), (128, 100, 13, 9, False), (128, 128, 13, 41, True), (72, 96, 13, 8, True)])
 @pytest.mark.parametrize("channel", [False, True])
 @pytest.mark.parametrize("fresh", [False, True])
-def test_batch_against_single_sequences(channel, dim, vdim, B, L, fresh):
+def test_batch_against_single_sequences(monkeypatch, channel, dim, vdim, B, L, mma, fresh):
     from adaptivetrainingsystem_b200.ops import delta as D
+    if not mma:
+        monkeypatch.setattr(D, "scan_on_tensor_cores", lambda *_: False)
     g = torch.Generator(device="cuda").manual_seed(dim + vdim + L)
     H, KH = 8, 4
     s = (D.ChannelDeltaShape if channel else D.DeltaShape)(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5)
     width = (s.channels + 7) // 8 * 8
+    assert not mma or D.scan_on_tensor_cores(torch.empty(1, width, dtype=torch.bfloat16), s)
     mixed = torch.randn(B * L, width, generator=g, device="cuda").bfloat16()
     rlen = 0.05 + 0.05 * torch.rand(B * L, 2 * KH, generator=g, device="cuda")
     gb = torch.rand(B * L, 2 * H, generator=g, device="cuda") * 0.5 + 0.5
