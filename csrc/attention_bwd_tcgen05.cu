@@ -16,10 +16,10 @@
 //   128 dimensions (OVER): those tiles would take the room of a second stage, and copies, products and exponentials would follow one another
 //           (568 us for one sequence of 4,096 tokens, 32 / 8 heads).  So the scores are computed transposed, S^T = K Q^T and dP^T = V dO^T, with keys
 //           as the lanes of tensor memory: P^T and dS^T are written over the scores they come from and are read from there.  The scores of pair t + 1
-//           run under dS of pair t, dP of t + 1 under the exponentials of t + 1: 309 us.  At 64 dimensions that form is the slower one (579 us
-//           against 543 for 8 x 2,048 tokens, 32 / 4 heads): products with an A operand in tensor memory and 64 columns take longer than from shared
-//           memory, and the statistics of a query are read per column.
-// In the other forms the scores of pair t + 1 run as soon as S of pair t is in registers, dP of t + 1 as soon as dP of t is (dQ pass 446 -> 435 us).
+//           run under dS of pair t, dP of t + 1 under the exponentials of t + 1: 263 us.  At 64 dimensions that form is the slower one (579 us
+//           for 8 x 2,048 tokens, 32 / 4 heads, where the other takes 397): products with an A operand in tensor memory and 64 columns take longer than
+//           from shared memory, and the statistics of a query are read per column.
+// In the other forms the scores of pair t + 1 run as soon as S of pair t is in registers, dP of t + 1 as soon as dP of t is.
 //
 //   warp 0: TMA producer   warp 1: TMEM owner + MMA issuer   warps 2..9: two threads per row of the scores (64 columns each)
 // Any sequence length: rows behind the end of a sequence read as zero (its length is a dimension of the tensor maps).  Queries there get a
@@ -51,16 +51,21 @@ struct AttnBwdArgs {
   long long* prof;  // optional [16]: cycle totals, written by one CTA (diagnostics; null in normal use)
 };
 
-template <int D, int MODE>
+enum : int { kNone, kAll, kDiagonal };
+template <int V> struct Masks { static constexpr int value = V; };
+
+// FORM 1: MODE 0 at 128 dimensions where each CTA has one pair of tiles (up to 128 tokens, no shared keys): there is nothing to run ahead of, and the form of 64
+// dimensions ends sooner (8 heads of 100 tokens 7.3 us, OVER 8.0); MODE 1 for more than eight tiles: see MASKS.
+template <int D, int MODE, int FORM>
 struct AttnBwdSmem {
   // streamed stages: a stage is held until the gradient products that read it have finished, and a refill takes a
   // TMA round trip, so the ring must be deep enough to have the next tiles in flight meanwhile
-  static constexpr int ST = (D == 64) ? 4 : 2;
+  static constexpr int ST = (D == 64) ? 4 : (MODE == 0 && FORM == 1) ? 1 : 2;
   static constexpr int TB = 128 * D * 2;
   static constexpr int R1 = 0, R2 = TB;
   static constexpr int T1 = 2 * TB;            // ST stages
   static constexpr int T2 = T1 + ST * TB;      // ST stages
-  static constexpr bool OVER = MODE == 0 && D == 128;
+  static constexpr bool OVER = MODE == 0 && D == 128 && FORM == 0;
   static constexpr int P_OFF = T2 + ST * TB;     // MODE 0 at 64 dimensions: P, dS
   static constexpr int DS_OFF = P_OFF + (MODE == 0 && !OVER ? 32768 : 0);
   static constexpr int ROW_OFF = DS_OFF + (MODE == 0 && !OVER ? 32768 : 0);   // OVER: [2][-lse, -delta][128 queries] of two iterations
@@ -94,11 +99,11 @@ __global__ void __launch_bounds__(256) attn_delta_kernel(const __nv_bfloat16* __
   }
 }
 
-template <int D, int MODE>
+template <int D, int MODE, int FORM>
 __global__ void __launch_bounds__(AB_THREADS, 1)
 attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                 const __grid_constant__ CUtensorMap map_v, const __grid_constant__ CUtensorMap map_do, const AttnBwdArgs p) {
-  using SM = AttnBwdSmem<D, MODE>;
+  using SM = AttnBwdSmem<D, MODE, FORM>;
   constexpr int ST = SM::ST;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -180,6 +185,9 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
   // in 64 columns of its own.
   constexpr bool OVER = SM::OVER, VIA_SMEM = MODE == 0 && !OVER;
   const uint32_t tmem_P = tmem_S, tmem_dS = OVER ? tmem_dP : tmem_base + 384;
+  // Masks of the pair on the diagonal: in every iteration where that is a large share of them (dQ of up to eight tiles: 8 x 384 tokens, 32 / 8 heads 32.3 us,
+  // two loops 33.5), else one loop with them and one without (one sequence of 4,096: 161 and 154).
+  constexpr int MASKS = MODE == 0 ? (FORM == 1 ? kAll : kNone) : (FORM == 0 ? kDiagonal : kNone);
   constexpr uint32_t HALF = OVER ? 64 : 32;   // columns from the first 64 reduction elements to the others
 
   // iteration t -> (query head, query tile, key tile)
@@ -338,12 +346,13 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     bool ok = true;
     // Query tile and head of the next statistics to fetch (MODE 1: of all of them), and of the iteration at hand whether it is on the diagonal.
     int tile = fixed, stat_head = MODE == 0 ? head * rep : head, to_diagonal = 0;
-    // log-sum-exp (times -log2 e) and delta (times -scale) of query `row` of that tile
+    // log-sum-exp or delta of query `row` of that tile, as they are: what is multiplied here would be waited for here
     auto row_stat = [&](int row, bool lse) {
       const long long idx = ((long long)b * p.Hq + stat_head) * p.L + tile * 128 + row;
       const bool real = tile * 128 + row < p.L;
-      return lse ? (real ? p.lse[idx] * -1.4426950408889634f : -INFINITY) : (real ? -p.delta[idx] * p.scale : 0.f);
+      return lse ? (real ? p.lse[idx] : INFINITY) : (real ? p.delta[idx] : 0.f);
     };
+    auto scaled = [&](float v, bool lse) { return lse ? v * -1.4426950408889634f : -v * p.scale; };
     auto next_tile = [&] {
       if (++tile == nq) tile = fixed, ++stat_head;
     };
@@ -352,7 +361,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
     const int id = int(threadIdx.x) - 64;
     float row_l = 0.f, row_d = 0.f, ahead = 0.f, ahead_d = 0.f;
     if (OVER) {
-      if (n_iter > 0) sRow[id] = row_stat(id & 127, id < 128);
+      if (n_iter > 0) sRow[id] = scaled(row_stat(id & 127, id < 128), id < 128);
       next_tile();
       if (n_iter > 1) ahead = row_stat(id & 127, id < 128);
     } else if (n_iter > 0) {
@@ -372,7 +381,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
           ok = false;
           break;
         }
-        if (t + 1 < n_iter) sRow[((t + 1) & 1) * 256 + id] = ahead;
+        if (t + 1 < n_iter) sRow[((t + 1) & 1) * 256 + id] = scaled(ahead, id < 128);
         next_tile();
         if (t + 2 < n_iter) ahead = row_stat(id & 127, id < 128);
       } else if (VIA_SMEM) {
@@ -407,26 +416,31 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
         ok = false;
         break;
       }
+      const float nl_row = scaled(row_l, true), nd_row = scaled(row_d, false);
       float2 pr[AB_COLS / 2];
+      auto exponentials = [&](auto masks) {
 #pragma unroll
-      for (int i = 0; i < AB_COLS / 2; i += 2) {
-        float4 n4 = make_float4(row_l, row_l, row_l, row_l);
-        if (OVER) n4 = *reinterpret_cast<const float4*>(nl + 2 * i);
+        for (int i = 0; i < AB_COLS / 2; i += 2) {
+          float4 n4 = make_float4(nl_row, nl_row, nl_row, nl_row);
+          if (OVER) n4 = *reinterpret_cast<const float4*>(nl + 2 * i);
 #pragma unroll
-        for (int x = 0; x < 2; ++x) {
-          const float2 xs = __ffma2_rn(make_float2(__uint_as_float(sv[2 * (i + x)]), __uint_as_float(sv[2 * (i + x) + 1])), sc2,
-                                       x ? make_float2(n4.z, n4.w) : make_float2(n4.x, n4.y));
-          pr[i + x] = make_float2(exp2f(xs.x), exp2f(xs.y));
+          for (int x = 0; x < 2; ++x) {
+            const float2 xs = __ffma2_rn(make_float2(__uint_as_float(sv[2 * (i + x)]), __uint_as_float(sv[2 * (i + x) + 1])), sc2,
+                                         x ? make_float2(n4.z, n4.w) : make_float2(n4.x, n4.y));
+            pr[i + x] = make_float2(exp2f(xs.x), exp2f(xs.y));
+            // keys behind the query: rows above the column (OVER) or columns behind the row
+            const int c = part * AB_COLS + 2 * (i + x);
+            if (masks.value == kAll || (masks.value == kDiagonal && diag)) {
+              if (OVER ? c < r : c > r) pr[i + x].x = 0.f;
+              if (OVER ? c + 1 < r : c + 1 > r) pr[i + x].y = 0.f;
+            }
+          }
         }
-      }
-      if (diag) {   // keys behind the query: rows above the column (OVER) or columns behind the row
-#pragma unroll
-        for (int i = 0; i < AB_COLS / 2; ++i) {
-          const int c = part * AB_COLS + 2 * i;
-          if (OVER ? c < r : c > r) pr[i].x = 0.f;
-          if (OVER ? c + 1 < r : c + 1 > r) pr[i].y = 0.f;
-        }
-      }
+      };
+      // (beside the exponentials, which take longer, the masks cost nothing; a pass of their own behind them made short sequences 4 to 11 % slower)
+      if constexpr (MASKS == kDiagonal) exponentials(Masks<kDiagonal>());
+      else if (MASKS == kAll || diag) exponentials(Masks<kAll>());
+      else exponentials(Masks<kNone>());
       if (!OVER) {
         tmem_ld_wait();
         tc_fence_before();
@@ -461,7 +475,7 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
       uint32_t dk[32];
 #pragma unroll
       for (int i = 0; i < 32; i += 2) {
-        float4 n4 = make_float4(row_d, row_d, row_d, row_d);
+        float4 n4 = make_float4(nd_row, nd_row, nd_row, nd_row);
         if (OVER) n4 = *reinterpret_cast<const float4*>(nl + 128 + 2 * i);
 #pragma unroll
         for (int x = 0; x < 2; ++x) {
@@ -532,14 +546,14 @@ attn_bwd_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant
 
 using namespace ats;
 
-template <int D, int MODE>
+template <int D, int MODE, int FORM>
 static int launch_attn_bwd(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mdo,
                            const AttnBwdArgs& p, cudaStream_t s) {
-  using SM = AttnBwdSmem<D, MODE>;
-  cudaError_t ce = cudaFuncSetAttribute(attn_bwd_kernel<D, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL);
+  using SM = AttnBwdSmem<D, MODE, FORM>;
+  cudaError_t ce = cudaFuncSetAttribute(attn_bwd_kernel<D, MODE, FORM>, cudaFuncAttributeMaxDynamicSharedMemorySize, SM::TOTAL);
   if (ce != cudaSuccess) return int(ce);
   dim3 grid(MODE == 0 ? p.Hkv : p.Hq, p.B, (p.L + 127) / 128);
-  attn_bwd_kernel<D, MODE><<<grid, AB_THREADS, SM::TOTAL, s>>>(mq, mk, mv, mdo, p);
+  attn_bwd_kernel<D, MODE, FORM><<<grid, AB_THREADS, SM::TOTAL, s>>>(mq, mk, mv, mdo, p);
   return int(cudaGetLastError());
 }
 
@@ -578,12 +592,12 @@ ATS_API int ats_attn_bwd(const void* q, long long ld_q, long long q_cols, int q_
   p.scale_log2 = 1.4426950408889634f * p.scale;
   p.status = status;
   p.prof = prof;
-  if (D == 128) {
-    if ((e = launch_attn_bwd<128, 0>(mq, mk, mv, mdo, p, s))) return e;
-    if (prof) p.prof = prof + 16;
-    return launch_attn_bwd<128, 1>(mq, mk, mv, mdo, p, s);
-  }
-  if ((e = launch_attn_bwd<64, 0>(mq, mk, mv, mdo, p, s))) return e;
+  const bool one_pair = L <= 128 && Hq == Hkv, many = L > 8 * 128;
+  if (D == 64) e = launch_attn_bwd<64, 0, 0>(mq, mk, mv, mdo, p, s);
+  else if (one_pair) e = launch_attn_bwd<128, 0, 1>(mq, mk, mv, mdo, p, s);
+  else e = launch_attn_bwd<128, 0, 0>(mq, mk, mv, mdo, p, s);
+  if (e) return e;
   if (prof) p.prof = prof + 16;
-  return launch_attn_bwd<64, 1>(mq, mk, mv, mdo, p, s);
+  if (D == 64) return many ? launch_attn_bwd<64, 1, 1>(mq, mk, mv, mdo, p, s) : launch_attn_bwd<64, 1, 0>(mq, mk, mv, mdo, p, s);
+  return many ? launch_attn_bwd<128, 1, 1>(mq, mk, mv, mdo, p, s) : launch_attn_bwd<128, 1, 0>(mq, mk, mv, mdo, p, s);
 }

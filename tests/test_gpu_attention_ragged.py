@@ -6,7 +6,8 @@ pytestmark = pytest.mark.gpu
 
 
 # lengths around the 128-row tiles and the pairs of them, single rows, both head sizes, with and without groups
-@pytest.mark.parametrize("B,L,hq,hkv,d", [(3, 1, 2, 2, 64), (2, 127, 4, 2, 128), (2, 129, 4, 1, 64), (3, 255, 4, 4, 64), (2, 257, 8, 2, 128), (3, 1000, 4, 2, 64), (1, 333, 4, 4, 128)])
+@pytest.mark.parametrize("B,L,hq,hkv,d", [(3, 1, 2, 2, 64), (2, 127, 4, 2, 128), (2, 129, 4, 1, 64), (3, 255, 4, 4, 64), (2, 257, 8, 2, 128), (3, 1000, 4, 2, 64), (1, 333, 4, 4, 128), (2, 128, 3, 3, 128), (2, 1, 2, 2, 128), (1, 128, 4, 2, 128), (1, 1024, 2, 1, 64), (1, 1025, 2, 2, 64),
+                                         (1, 1024, 2, 2, 128), (1, 1025, 2, 1, 128)])
 def test_ragged_lengths(B, L, hq, hkv, d):
     from adaptivetrainingsystem_b200 import ops
     from adaptivetrainingsystem_b200.ops import attention_native as N
