@@ -198,6 +198,22 @@ def scan_on_tensor_cores(mixed: torch.Tensor, s: DeltaShape) -> bool:
     return mixed.dtype == torch.bfloat16 and s.dim <= 128 and s.dim % 8 == 0 and s.vdim % 8 == 0
 
 
+def scan_pays(s: DeltaShape, L: int) -> bool:
+    """Whether portions of ``L`` tokens are faster on the tensor cores than in fp32 FMAs; the number of sequences plays no part, so that a sequence is the
+    same alone and among others.  A tensor-core group is 16 tokens whatever they hold, and the smallest launch takes longer (us, FMA / tensor cores, one
+    sequence of 16 heads unless said; 128 x 128 states):
+
+    * one decay a head: 8 tokens 9.3 / 12.4, 24 1.07 times the FMA form, 40 0.93 to 1.01, 48 0.87 to 0.94, 300 70.8 / 47.8; up to 64 state rows 8 tokens 8.8 / 10.1
+      (32 x 32), 12 0.74 to 0.95;
+    * one decay a row: 33 tokens 20.4 / 23.8, 64 1.02 to 1.05 times, 96 0.96 to 0.99, 300 74.2 / 63.1; fewer than 64 columns share the work of the pairs with too few:
+      12 sequences of 200, 128 x 32 1.08; up to 64 rows 24 tokens 1.02 to 1.06, 32 0.82 to 0.95, and from 12 on 0.89 to 1.01 with more than 32 rows and 64 columns."""
+    if not isinstance(s, ChannelDeltaShape):
+        return L > (40 if s.dim > 64 else 8)
+    if s.dim > 64:
+        return s.vdim >= 64 and L > 64
+    return L > 24 or (L > 8 and s.dim > 32 and s.vdim >= 64)
+
+
 def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state: torch.Tensor, s: DeltaShape, L: int, fresh: bool) -> torch.Tensor:
     """Advances ``state`` [B, H, dim, vdim] over portions of L tokens -> read-outs [B * L, H * vdim]; ``fresh``: the state starts at zero."""
     B = state.shape[0]
@@ -213,7 +229,7 @@ def delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor, state:
             state[b] = S
         return out
     mixed = _whole_pieces(mixed)
-    mma = scan_on_tensor_cores(mixed, s)
+    mma = scan_on_tensor_cores(mixed, s) and scan_pays(s, L)
     groups = -(-L // (GROUP_MMA if mma else GROUP))
     size = 836 if mma else 2 * GROUP * GROUP + 3 * GROUP + 8   # floats, laid out in csrc/delta_rule_mma.cu (3.3 KB per 16 tokens and head), csrc/delta_rule.cu (1.3 KB)
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)
@@ -277,7 +293,7 @@ def channel_delta_scan(mixed: torch.Tensor, rlen: torch.Tensor, gb: torch.Tensor
             state[b] = S
         return out
     mixed, a = _whole_pieces(mixed), _whole_pieces(a)
-    mma, DK = scan_on_tensor_cores(mixed, s), s.scan_rows
+    mma, DK = scan_on_tensor_cores(mixed, s) and scan_pays(s, L), s.scan_rows
     groups = -(-L // (GROUP_MMA if mma else GROUP))
     size = 73 * DK + 784 if mma else 2 * GROUP * GROUP + (3 * GROUP + 1) * DK   # csrc/channel_delta_mma.cu (40 KB, 128 rows), csrc/channel_delta.cu (27 KB)
     coef = torch.empty(B, groups, H, size, dtype=torch.float32, device=mixed.device)

@@ -12,8 +12,7 @@ pytestmark = pytest.mark.gpu
 @pytest.mark.parametrize("fresh", [False, True])
 def test_batch_against_single_sequences(monkeypatch, channel, dim, vdim, B, L, mma, fresh):
     from adaptivetrainingsystem_b200.ops import delta as D
-    if not mma:
-        monkeypatch.setattr(D, "scan_on_tensor_cores", lambda *_: False)
+    monkeypatch.setattr(D, "scan_pays", lambda *_: mma)
     g = torch.Generator(device="cuda").manual_seed(dim + vdim + L)
     H, KH = 8, 4
     s = (D.ChannelDeltaShape if channel else D.DeltaShape)(heads=H, kv_heads=KH, dim=dim, vdim=vdim, taps=4, eps=1e-5)
