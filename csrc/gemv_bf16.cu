@@ -128,7 +128,7 @@ gemv_bf16_kernel(const __nv_bfloat16* __restrict__ w, long long ldw, const __nv_
       s_red[warp][r][8 * n + 2 * t + 1][g + 8] = c[r][n][3];
     }
   __syncthreads();
-  stream_finish<MODE, WARPS, NT>(st, s_red, s_scale, tile, add, ld_add, out, ld_out, M, N);
+  stream_finish<MODE, WARPS, NT, true>(st, s_red, s_scale, tile, add, ld_add, out, ld_out, M, N);
 }
 
 template <int MODE, int WARPS, int NT, int DEPTH, int MINB>

@@ -77,7 +77,7 @@ __host__ __device__ constexpr int int4_ring_bytes(int WARPS, int R, int NT, int 
 // are spent streaming and not waiting for one round trip to memory per step.  One tile per CTA and MINB resident CTAs per SM keep
 // the grid fine-grained: with two tiles and 72 registers the 28,672-feature projection ran as 2.02 waves of CTAs, i.e. three.
 // NT: token tiles of eight rows (the code fragments of a step feed NT MMAs).
-template <int MODE, int WARPS, int NT, int DEPTH, int MINB>
+template <int MODE, int WARPS, int NT, int DEPTH, int MINB, bool STEP>
 __global__ void __launch_bounds__(WARPS * 32, MINB)
 gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta, const __nv_bfloat16* __restrict__ x, long long ldx,
                  const __nv_bfloat16* __restrict__ add, long long ld_add, __nv_bfloat16* __restrict__ out, long long ld_out,
@@ -86,7 +86,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
   if (!early) pdl_prologue();   // early: a chained launch, whose first packed words are requested under the kernel before it (common.cuh)
   else asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   __shared__ float s_red[WARPS][R][8 * NT][16];  // [warp][tile][token][feature of the tile]
-  __shared__ float s_scale[8 * NT];
+  __shared__ float s_scale[STEP ? 8 * NT : 1];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, g = lane >> 2, t = lane & 3;
   const int n_super = K >> 6, n_tiles = N >> 4;
   // constants the extraction wants in registers; built from a kernel argument so that they are not folded back into immediates
@@ -192,7 +192,7 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
     }
     cp_async_commit();
   }
-  stream_scales<WARPS, NT>(st, M, s_scale);  // (while the first copies travel)
+  if (STEP) stream_scales<WARPS, NT>(st, M, s_scale);  // (while the first copies travel)
   for (int S0 = warp; S0 < n_super; S0 += WARPS * DEPTH) {
 #pragma unroll
     for (int d = 0; d < DEPTH; ++d) {
@@ -218,8 +218,11 @@ gemv_int4_kernel(const uint4* __restrict__ wq, const uint32_t* __restrict__ meta
       s_red[warp][r][8 * n + 2 * t + 1][g + 8] = c[r][n][3];
     }
   __syncthreads();
-  stream_finish<MODE, WARPS, NT>(st, s_red, s_scale, tile, add, ld_add, out, ld_out, M, N);
+  stream_finish<MODE, WARPS, NT, STEP>(st, s_red, s_scale, tile, add, ld_add, out, ld_out, M, N);
 }
+
+struct StepYes { static constexpr bool value = true; };
+struct StepNo { static constexpr bool value = false; };
 
 // one thread per (tile, super-step, lane): 16 + 16 consecutive values of features g and g + 8
 __global__ void __launch_bounds__(256)
@@ -290,38 +293,44 @@ ATS_API int ats_gemv_int4(const void* wq, const void* meta, const void* x, long 
   cudaError_t err;
   constexpr int kSms = 148;
 #define ATS_GEMV4(MODE_, W_, NT_, D_, B_, GRID_)                                                                                      \
-  [&]() -> cudaError_t {                                                                                                             \
+  [&](auto with_step) -> cudaError_t {                                                                                               \
+    constexpr bool kStep = decltype(with_step)::value;                                                                               \
     constexpr int kRing = ats::int4_ring_bytes(W_, MODE_ == ats::kStreamStore ? 1 : 2, NT_, D_);                                         \
     static bool attr_set = false;                                                                                                    \
     if (!attr_set) {                                                                                                                 \
-      cudaError_t ce = cudaFuncSetAttribute(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
+      cudaError_t ce = cudaFuncSetAttribute(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_, kStep>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
                                             kRing);                                                                                  \
       if (ce != cudaSuccess) return ce;                                                                                              \
       attr_set = true;                                                                                                               \
     }                                                                                                                                \
-    return ats::launch_pdl(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_>, dim3(GRID_), dim3(W_ * 32), kRing, s, w4, mt, xp, ldx, ap, ld_add,     \
+    return ats::launch_pdl(ats::gemv_int4_kernel<MODE_, W_, NT_, D_, B_, kStep>, dim3(GRID_), dim3(W_ * 32), kRing, s, w4, mt, xp, ldx, ap, ld_add,     \
                            op, ld_out, M, N, K, gs, early, st);                                                                      \
-  }()
-  // Warps, ring and CTAs per SM, from a chain of launches (us a launch; one or four rows / sixteen rows):
-  // * one tile per CTA: with a CTA for each SM at most, sixteen warps have the whole of a short reduction in flight: 5,632 -> 2,048 8.2 -> 4.7 /
-  //   9.9 -> 5.9, 2,048 -> 2,048 3.0 -> 2.5 / 5.0 -> 3.1; with two, rings of three steps let both run at once: 14,336 -> 4,096 21.5 -> 14.9 / 23.2
-  //   (rings of four: 17.3); more tiles are more waves, and their CTAs stay small;
+  }
+  // Warps, ring and CTAs per SM (us a launch; up to eight / up to sixteen rows):
+  // * one tile per CTA: with fewer CTAs than SMs, sixteen warps have the whole of a short reduction in flight: in a chain of launches 5,632 -> 2,048 8.5 -> 4.6 /
+  //   9.5 -> 5.7, 2,048 -> 2,048 3.0 -> 2.4 / 4.6 -> 2.9, 1,024 -> 1,024 1.84 -> 1.78 / 2.9 -> 2.2 (launches that wait for the one before them have nothing in
+  //   flight to gain from 2,048 terms down: 1,024 -> 1,024 2.35 -> 2.5 / 2.7 -> 2.95; a product gives the same bits in a chain and outside, so the line is one of
+  //   shapes); with two per SM and up to eight rows, rings of three steps let both run at once: 14,336 -> 4,096 21.5 -> 14.9, 2,048 -> 4,736 4.3 -> 3.6.  A few CTAs
+  //   more than SMs are better off with eight warps (2,048 -> 2,384 3.1, sixteen 3.3), and so are up to two per SM with sixteen rows (2,048 -> 4,736 5.1 and 6.0);
   // * gate and up tiles: more than two CTAs per SM run at once with rings of two steps: 2,048 -> 11,264 7.6 -> 6.5 / 11.0 -> 10.1,
-  //   4,096 -> 28,672 26.7 -> 24.5 / 39.7 -> 36.0; two find the deep rings faster: 1,024 -> 5,632 3.0 (rings of two: 3.6), not with sixteen rows;
+  //   4,096 -> 28,672 26.7 -> 24.5 / 39.7 -> 36.0; fewer find the deep rings faster: 1,024 -> 5,632 3.0 (rings of two: 3.6), 2,048 -> 2,560 / 4.4 (5.6);
   // * heads of two tiles: deep rings (4,096 -> 6,144 8.5, rings of two 10.3), with sixteen rows while one CTA per SM is enough (2,048 -> 2,560 4.5,
   //   rings of two 5.8; 4,096 -> 6,144 13.7 and 11.8).
-  const bool two = M > 8;
+  const bool two = M > 8, alone = tiles < kSms, side_by_side = !two && tiles >= 160 && tiles <= 2 * kSms;
   const int pairs = tiles / 2;
-  if (mode == ats::kStreamSwiGLU)
-    err = two ? ATS_GEMV4(ats::kStreamSwiGLU, 8, 2, 2, 2, pairs) : pairs > 2 * kSms ? ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 2, 3, pairs) : ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 4, 2, pairs);
+  auto go = [&](auto launch) { return st.scale_parts || st.next_out ? launch(ats::StepYes()) : launch(ats::StepNo()); };
+  if (mode == ats::kStreamSwiGLU && pairs > 2 * kSms)
+    err = two ? go(ATS_GEMV4(ats::kStreamSwiGLU, 8, 2, 2, 2, pairs)) : go(ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 2, 3, pairs));
+  else if (mode == ats::kStreamSwiGLU)
+    err = two ? go(ATS_GEMV4(ats::kStreamSwiGLU, 8, 2, 3, 2, pairs)) : go(ATS_GEMV4(ats::kStreamSwiGLU, 8, 1, 4, 2, pairs));
   else if (mode == ats::kStreamRope)
-    err = !two ? ATS_GEMV4(ats::kStreamRope, 8, 1, 4, 2, pairs) : pairs > kSms ? ATS_GEMV4(ats::kStreamRope, 8, 2, 2, 2, pairs) : ATS_GEMV4(ats::kStreamRope, 8, 2, 4, 1, pairs);
-  else if (tiles > 2 * kSms)
-    err = two ? ATS_GEMV4(ats::kStreamStore, 8, 2, 4, 2, tiles) : ATS_GEMV4(ats::kStreamStore, 8, 1, 4, 3, tiles);
-  else if (two)
-    err = ATS_GEMV4(ats::kStreamStore, 16, 2, 2, 1, tiles);
+    err = !two ? go(ATS_GEMV4(ats::kStreamRope, 8, 1, 4, 2, pairs)) : pairs > kSms ? go(ATS_GEMV4(ats::kStreamRope, 8, 2, 2, 2, pairs)) : go(ATS_GEMV4(ats::kStreamRope, 8, 2, 4, 1, pairs));
+  else if (alone)
+    err = two ? go(ATS_GEMV4(ats::kStreamStore, 16, 2, 2, 1, tiles)) : go(ATS_GEMV4(ats::kStreamStore, 16, 1, 4, 1, tiles));
+  else if (side_by_side)
+    err = go(ATS_GEMV4(ats::kStreamStore, 16, 1, 3, 2, tiles));
   else
-    err = tiles > kSms ? ATS_GEMV4(ats::kStreamStore, 16, 1, 3, 2, tiles) : ATS_GEMV4(ats::kStreamStore, 16, 1, 4, 1, tiles);
+    err = two ? go(ATS_GEMV4(ats::kStreamStore, 8, 2, 4, 2, tiles)) : go(ATS_GEMV4(ats::kStreamStore, 8, 1, 4, 3, tiles));
 #undef ATS_GEMV4
   return int(err);
 }

@@ -288,7 +288,8 @@ def test_dequant_kernel_matches_reference_bit_for_bit(N, K, group):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("M,N,K,group", [(1, 64, 256, 128), (3, 2560, 2048, 128), (8, 2048, 5632, 128), (5, 32000, 2048, 128), (13, 512, 1024, 64),
-                                           (16, 28672, 1024, 256), (9, 2560, 2048, 128)])
+                                           (16, 28672, 1024, 256), (9, 2560, 2048, 128), (8, 2352, 512, 128), (16, 2352, 512, 128), (8, 2368, 512, 128), (9, 2368, 512, 128),
+                                           (1, 2544, 512, 128), (8, 2560, 512, 128), (2, 4736, 512, 128), (2, 4752, 512, 128)])
 def test_gemv_kernel_matches_fp32_product(M, N, K, group):
     """One tile per CTA (small N), two tiles per CTA (N / 32 >= 592), one and two token tiles, with and without the residual."""
     dev = torch.device("cuda")
