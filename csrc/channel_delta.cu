@@ -14,7 +14,7 @@
 // k_j g_{j+1} .. g_C, P_C in fp32; all decay products are running products of factors in (0, 1], so nothing overflows however fast a
 // channel decays.  channel_scan does three products with the state per token: sixteen lanes share eight columns, fp32 with packed
 // fma.f32x2, the next group's rows arriving in shared memory by asynchronous copies.  channel_delta_mma.cu is the faster form for bf16 rows of whole
-// 16-byte pieces and up to 128 state rows.
+// 16-byte pieces, up to 128 state rows and portions that are not short (ops/delta.py).
 #include "delta_common.cuh"
 
 namespace ats {
@@ -357,7 +357,8 @@ static int launch_channel(const ChannelArgs& p, cudaStream_t s) {
   if (even) launch_pdl(channel_pairs_kernel<T, 2, true>, grid, block, 0, s, p);
   else launch_pdl(channel_pairs_kernel<T, 2, false>, grid, block, 0, s, p);
   if (p.DK == 64) return launch_channel_scan<T, 4, 8>(p, s);
-  // (as in delta_rule.cu; us with eight / four columns: 16 CTAs 161 / 116, 96 516 / 471, 160 655 / 501, 192 499 / 405, 224 499 / 505, 256 1010 / 1034)
+  // (as in delta_rule.cu; us with eight / four columns, 500 tokens: bf16 32 CTAs 169 / 121, 96 184 / 178, 128 210 / 197, 160 299 / 248, 192 308 / 258, 224 311 / 312,
+  // 256 319 / 321; 32 bits 32 158 / 110, 96 174 / 174, 160 283 / 245, 192 293 / 255, 224 296 / 315)
   if (p.DK == 128 && (long long)((p.vdim + 63) / 64) * p.H * p.B <= SCAN_FEW) return launch_channel_scan<T, 8, 4>(p, s);
   if (p.DK == 128) return launch_channel_scan<T, 8, 8>(p, s);
   return launch_channel_scan<T, 16, 4>(p, s);

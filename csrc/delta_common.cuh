@@ -1,11 +1,12 @@
-// Pieces shared by the portion kernels of the delta rules (delta_rule.cu, channel_delta.cu).
+// Pieces shared by the portion kernels of the delta rules (delta_rule.cu, channel_delta.cu, delta_rule_mma.cu, channel_delta_mma.cu).
 #pragma once
 #include "typed.cuh"
 
 namespace ats {
 
 constexpr int DC = 8;  // tokens per group
-// Up to this many CTAs (of 64 columns) the scan kernels of 128 state rows take 32 columns a CTA instead.
+// Up to this many CTAs (of 64 columns) the fp32 FMA scans of 65 to 128 state rows take 32 columns a CTA instead: rows of 32 bits, bf16 heads that are no multiple of
+// eight wide, and portions too short for the tensor cores (ops/delta.py).
 constexpr int SCAN_FEW = 192;
 
 // exp(rate softplus(a)), rate < 0.  The bf16 form uses the fast functions and, where exp(a) is small, the series of log(1 + x), so that a

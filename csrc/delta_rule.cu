@@ -16,7 +16,7 @@
 // * delta_step: one decoded token per sequence: state read once and written once, output norm and gate in the same launch.
 //
 // delta_rule_mma.cu holds the portion kernels for bf16 rows of whole 16-byte pieces and up to 128 state rows (two to three times as fast); those below serve fp32,
-// larger states and odd widths.  channel_delta.cu holds the portion kernels of the form with one decay per state row; it shares delta_prep (without the decays),
+// larger states, odd widths and short portions.  channel_delta.cu holds the portion kernels of the form with one decay per state row; it shares delta_prep (without the decays),
 // delta_output and delta_step.
 //
 // A sequence at position 0 starts from a zero state and zero convolution inputs whatever its buffers hold.
@@ -855,8 +855,8 @@ static int launch_scan(const ScanArgs& p, cudaStream_t s) {
   if (p.dim <= 64) launch_pdl(delta_scan_kernel<T, 4, 8, 2>, grid(8), dim3(128), 0, s, p);
   else if (p.dim <= 128) {
     // Eight columns per lane read each k and q row for twice the products of four, but a CTA's groups follow one another, so while SMs are idle
-    // it is the time of one group that counts.  us with eight / four columns, by CTAs at eight: 16 187 / 117, 96 565 / 459, 128 388 / 312,
-    // 160 640 / 496, 192 532 / 416, 224 534 / 615, 256 1092 / 1270.
+    // it is the time of one group that counts.  us with eight / four columns, 500 tokens, by CTAs at eight: bf16 32 177 / 116, 96 185 / 159, 128 192 / 160,
+    // 160 268 / 220, 192 274 / 219, 224 274 / 303, 256 276 / 305; 32 bits, whose rows are twice as wide, 32 174 / 130, 96 174 / 198, 128 176 / 198, 192 288 / 321, 224 287 / 390.
     const dim3 g8 = grid(8);
     if ((long long)g8.x * g8.y * g8.z <= SCAN_FEW) launch_pdl(delta_scan_kernel<T, 8, 4, 2>, grid(4), dim3(128), 0, s, p);
     else launch_pdl(delta_scan_kernel<T, 8, 8, 2>, g8, dim3(128), 0, s, p);

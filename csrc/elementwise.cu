@@ -488,7 +488,7 @@ __global__ void cast_f32_bf16_kernel(const float* __restrict__ in, __nv_bfloat16
 }
 
 // out = bf16(in * bf16(*scale)): a gradient times the upstream one, which is on the device.  (The framework's product with a one-element tensor
-// does not vectorise: 84 us for 16,384 x 2,048, this 23.)  n is a multiple of 8.
+// does not vectorise: 78 us for 16,384 x 2,048, this 22.)  n is a multiple of 8.
 __global__ void __launch_bounds__(256) scale_bf16_kernel(const uint4* __restrict__ in, const float* __restrict__ scale, uint4* __restrict__ out, long long nvec) {
   const float s = __bfloat162float(__float2bfloat16(*scale));
   for (long long i = blockIdx.x * (long long)blockDim.x + threadIdx.x; i < nvec; i += (long long)gridDim.x * blockDim.x) {

@@ -4,13 +4,15 @@
 // barriers of a cluster are 3.2 us of every launch, where the weight of a 2,048-wide projection is streamed in 1.3.  Here a CTA owns 16 weight rows
 // (or two such tiles), its sixteen or eight warps split the reduction, and each keeps its share of the weight in flight in a ring of asynchronous
 // copies, as the 4-bit kernel does (int4.cu): a warp-level MMA takes the 16 rows as they are stored and up to eight tokens as its columns.  With a CTA
-// for every SM the whole weight of a projection is requested at once, in a captured step under the kernel before; there is no cluster and no
-// tensor memory to set up.  It is bound by one round trip to memory, the fold of the warps and the launch (1.4 us for 64 x 256).
+// for every SM the whole weight of a projection is requested at once, in a captured step under the kernel before where that leaves an SM free; there is no
+// cluster and no tensor memory to set up.  It is bound by one round trip to memory, the fold of the warps and the launch (1.4 us for 64 x 256).
 //
 // Us a launch in a chain, weights larger than L2 in turn, gemm_skinny.cu / here: one row 2,048 x 2,048 4.5 / 2.9, 2,048 x 5,632 8.0 / 5.9, rotated
 // 2,560 x 2,048 5.2 / 3.7, pairs of 2,816 x 1,024 4.8 / 3.3; sixteen rows 5.0 / 3.8, 8.3 / 7.3, 5.6 / 4.6, 5.1 / 4.1.  Which products come here:
-// stream_fits() in ops/gemm.py.  Warps, ring and CTAs per SM are the fastest of nine forms (a ring of four steps for up to eight tokens, 16 warps:
-// 2,048 x 5,632 5.2, eight warps 7.3, rings of two steps 7.4).
+// stream_fits() in ops/gemm.py.  Warps and ring are the fastest of nine forms (a ring of four steps for up to eight tokens, 16 warps:
+// 2,048 x 5,632 5.2, eight warps 7.3, rings of two steps 7.4).  Ring and sums are 200 KB for a plain tile (144 with more than eight tokens), 168 and 160 for heads, 88 and 112
+// for gate and up tiles: one CTA per SM, two of the last.  So where a launch has a CTA on every SM the next one asks for its weight as SMs become free, and with up to 2,048 terms,
+// two steps a warp, half of a plain ring is not used.  The last template number bounds the registers.
 #include "skinny.cuh"
 #include "stream_step.cuh"
 

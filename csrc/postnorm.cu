@@ -248,6 +248,7 @@ static int launch_postnorm(const PostNormArgs& p, cudaStream_t s) {
       default: return go(any);
     }
   };
+  // (a product of three slices, or of more than eight, walks them four at a time)
   if (q <= 1)
     by_splits(fold_postnorm_kernel<T, 1, 1>, fold_postnorm_kernel<T, 1, 2>, fold_postnorm_kernel<T, 1, 4>, fold_postnorm_kernel<T, 1, 8>, fold_postnorm_kernel<T, 1, 0>);
   else if (q <= 2)
